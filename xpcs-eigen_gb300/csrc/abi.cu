@@ -162,6 +162,7 @@ void free_series(Series *s) {
     s->n_part.release(st);
     s->side_pos.release(st);
     s->side_out.release(st);
+    s->side_cnt.release(st);
     DBuf<int32_t> *tti[] = {&s->tt_row_pix, &s->tt_row_grp, &s->tt_grp_ptr, &s->tt_order};
     for (auto *b : tti) b->release(st);
     DBuf<float> *ttf[] = {&s->tt_V, &s->tt_sg, &s->tt_sga, &s->tt_C, &s->tt_full, &s->tt_part};

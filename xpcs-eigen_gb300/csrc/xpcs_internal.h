@@ -294,6 +294,7 @@ struct Series {
   DBuf<int32_t> d_ppb;      // pixels per static bin
   DBuf<int64_t> side_pos;
   DBuf<float> side_out;
+  DBuf<uint32_t> side_cnt;  // integer sums of the side statistics
   DBuf<float> d_fscale;     // normalize_by_framesum: per-frame divisor frameSum/mean
   DBuf<int32_t> sc_frame;   // float-path scratch rows
   DBuf<float> sc_val;
