@@ -184,6 +184,7 @@ void run_twotime(Series &s, const TwoTimeReq &req, int mode, bool force_i64) {
                 Q = (int32_t)o.qbins.size();
   o.sg_rows = G;
   o.sg_cols = req.average ? 1 : F;
+  o.averaged = req.average != 0;
   auto up = [&](DBuf<int32_t> &b, const std::vector<int32_t> &v) {
     b.reserve(v.size() ? v.size() : 1, st);
     if (!v.empty())
@@ -250,7 +251,7 @@ void get_twotime(Series &s, int32_t *qbins, float *sg, float *c2t, float *g2full
   const size_t Q = o.qbins.size(), F = (size_t)o.frames;
   if (qbins) std::copy(o.qbins.begin(), o.qbins.end(), qbins);
   if (sg && o.sg_rows)
-    XG_CUDA(cudaMemcpyAsync(sg, o.sg_cols == 1 ? s.tt_sga.p : s.tt_sg.p,
+    XG_CUDA(cudaMemcpyAsync(sg, o.averaged ? s.tt_sga.p : s.tt_sg.p,
                             4 * (size_t)o.sg_rows * o.sg_cols, cudaMemcpyDeviceToHost, st));
   if (c2t && Q) XG_CUDA(cudaMemcpyAsync(c2t, s.tt_C.p, 4 * Q * F * F, cudaMemcpyDeviceToHost, st));
   if (g2full && Q) XG_CUDA(cudaMemcpyAsync(g2full, s.tt_full.p, 4 * F * Q, cudaMemcpyDeviceToHost, st));
