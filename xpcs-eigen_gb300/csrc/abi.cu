@@ -163,12 +163,15 @@ void free_series(Series *s) {
     s->side_pos.release(st);
     s->side_out.release(st);
     s->side_cnt.release(st);
-    DBuf<int32_t> *tti[] = {&s->tt_row_pix, &s->tt_row_grp, &s->tt_grp_ptr, &s->tt_order};
+    DBuf<int32_t> *tti[] = {&s->tt_row_pix, &s->tt_row_grp, &s->tt_grp_ptr, &s->tt_order,
+                            &s->tt_qptr, &s->tt_len};
     for (auto *b : tti) b->release(st);
     DBuf<float> *ttf[] = {&s->tt_V, &s->tt_sg, &s->tt_sga, &s->tt_C, &s->tt_full, &s->tt_part};
     for (auto *b : ttf) b->release(st);
     s->d_fscale.release(st);
     s->n_unsafe.release(st);
+    s->tt_cpos.release(st);
+    s->tt_cols.release(st);
     s->tt_err.release(st);
     s->tt_flags.release(st);
     s->tt_XT.release(st);

@@ -4,23 +4,26 @@
 // Replaces Corr::twotime (src/xpcs/corr.cpp:560-924) with SmoothingStaticMap /
 // SmoothingSymmetric (:433-547) and ComputeSG* (:1166-1305).  REFERENCE mode
 // reproduces the reference's float32 operations in its order:
-//   - the pixels of the processed q bins become rows of a dense matrix
-//     V [rows][F] in mapping order (q, static bin, pixel), zero where a pixel
-//     has no event;
+//   - the pixels of the processed q bins are rows in mapping order (q, static
+//     bin, pixel), as event lists (photon counting) or as a dense matrix
+//     V [rows][F], zero where a pixel has no event;
 //   - sg[g][f] = the float sum over the rows of smoothing group g (a static
 //     bin, or a q bin for the symmetric method) in mapping order, / pixels;
 //     with the average filter, the float mean over frames;
 //   - every event value is divided by its sg;
 //   - C_q[f0][f1] (f0 <= f1) = the float sum over the q bin's rows, in
 //     mapping order (ascending pixel index with frame threading), of
-//     v(f0) * v(f1) over pairs of events, then / pixels: a tiled CUDA-core
-//     Gram whose reduction runs over the rows in order, one separate multiply
-//     and add per pair (no fused multiply-add), products with a missing event
-//     skipped as the reference never forms them;
+//     v(f0) * v(f1) over pairs of events, then / pixels: one separate multiply
+//     and add per pair (no fused multiply-add), in row order, products with a
+//     missing event skipped as the reference never forms them.  Event lists:
+//     a warp per column f1 walks the column's events in row order
+//     (k_tt_gram_events); dense rows: a tiled CUDA-core Gram whose reduction
+//     runs over the rows in order (k_tt_gram);
 //   - g2full[ff] = the float mean of diagonal ff in order; g2partials[ff][w]
 //     the float sum of window w (`window` entries) of diagonal ff / window.
 #include <algorithm>
 #include <numeric>
+#include <utility>
 
 #include "xpcs_internal.h"
 
@@ -130,6 +133,207 @@ k_tt_gram(int32_t F, int32_t nrows, const int32_t *__restrict__ order,
     }
 }
 
+// ------------------------------------------------------------ event lists
+//
+// The Gram of sparse rows: of the F (F + 1) / 2 products of a row only those
+// of its events exist, and a column f1 of C needs, in row order, the rows
+// with an event at f1 and each one's earlier events.  The rows' events are
+// sorted by (q, frame), stably from row order, which gives every column's
+// rows in the order its sums take them.
+
+// Events of row order[j] (order null: row j) in build order.
+__global__ void k_tt_lens(int32_t R, const int32_t *__restrict__ order,
+                          const int32_t *__restrict__ row_pix,
+                          const int32_t *__restrict__ row_len, int32_t *__restrict__ len) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j < R) len[j] = row_len[row_pix[order ? order[j] : j]];
+}
+
+// One warp per row in build order: (key = q F + frame, a = row, b = the
+// event's position in its row).
+__global__ void k_tt_build(int32_t R, int32_t F, int32_t Q, const int32_t *__restrict__ order,
+                           const int32_t *__restrict__ q_ptr, const int32_t *__restrict__ row_pix,
+                           const int64_t *__restrict__ row_ptr,
+                           const int32_t *__restrict__ row_len,
+                           const int32_t *__restrict__ ev_frame, const int64_t *__restrict__ cpos,
+                           uint32_t *__restrict__ key, int32_t *__restrict__ a,
+                           float *__restrict__ b) {
+  const int64_t j = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (j >= R) return;
+  const int r = order ? order[j] : (int)j;
+  int q = 0, hi = Q - 1;  // the last q bin whose rows start at or before r
+  while (q < hi) {
+    const int mid = (q + hi + 1) >> 1;
+    if (q_ptr[mid] <= r) q = mid;
+    else hi = mid - 1;
+  }
+  const int p = row_pix[r], n = row_len[p];
+  const int64_t src = row_ptr[p], dst = cpos[j];
+  for (int i = threadIdx.x & 31; i < n; i += 32) {
+    key[dst + i] = (uint32_t)q * (uint32_t)F + (uint32_t)ev_frame[src + i];
+    a[dst + i] = r;
+    b[dst + i] = __int_as_float(i);
+  }
+}
+
+// col_ptr[c] = first event of column c = q F + frame
+__global__ void k_tt_cols(int64_t ncol, int64_t n, const uint32_t *__restrict__ key,
+                          int64_t *__restrict__ col_ptr) {
+  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (c > ncol) return;
+  int64_t first = 0, len = n;
+  while (len > 0) {
+    const int64_t h = len >> 1;
+    if (key[first + h] < (uint64_t)c) {
+      first += h + 1;
+      len -= h + 1;
+    } else {
+      len = h;
+    }
+  }
+  col_ptr[c] = first;
+}
+
+// sg[g][f] as k_tt_sg forms it (a row without an event at f adds 0): one warp
+// per (group, frame) over the column's events of the group's rows, in row
+// order (the lists sorted from mapping order).
+__global__ void k_tt_sg_events(int32_t F, const int32_t *__restrict__ grp_ptr,
+                               const int32_t *__restrict__ grp_q,
+                               const int64_t *__restrict__ col_ptr, const int32_t *__restrict__ a,
+                               const float *__restrict__ b, const int32_t *__restrict__ row_pix,
+                               const int64_t *__restrict__ row_ptr,
+                               const float *__restrict__ ev_val, float *__restrict__ sg) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int f = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5), g = blockIdx.y;
+  if (f >= F) return;
+  const int r0 = grp_ptr[g], r1 = grp_ptr[g + 1];
+  const int64_t c = (int64_t)grp_q[g] * F + f, end = col_ptr[c + 1];
+  int64_t lo = col_ptr[c], len = end - lo;
+  while (len > 0) {  // the group's first row in the column
+    const int64_t h = len >> 1;
+    if (a[lo + h] < r0) {
+      lo += h + 1;
+      len -= h + 1;
+    } else {
+      len = h;
+    }
+  }
+  float acc = 0.f;
+  for (int64_t e0 = lo;; e0 += 32) {
+    const int64_t e = e0 + lane;
+    const int r = e < end ? a[e] : r1;
+    const bool in = r < r1;
+    const float v = in ? ev_val[row_ptr[row_pix[r]] + __float_as_int(b[e])] : 0.f;
+    const int n = __popc(__ballot_sync(FULL, in));
+    for (int k = 0; k < n; k++) acc = __fadd_rn(acc, __shfl_sync(FULL, v, k));
+    if (n < 32) break;
+  }
+  if (lane == 0) sg[(size_t)g * F + f] = __fdiv_rn(acc, (float)(r1 - r0));
+}
+
+// Smoothed values of the rows' events, beside their frames (one warp per row).
+__global__ void k_tt_smooth_events(int32_t R, int32_t F, int32_t average,
+                                   const int32_t *__restrict__ row_pix,
+                                   const int32_t *__restrict__ row_grp,
+                                   const int64_t *__restrict__ row_ptr,
+                                   const int32_t *__restrict__ row_len,
+                                   const int32_t *__restrict__ ev_frame,
+                                   const float *__restrict__ ev_val, const float *__restrict__ sg,
+                                   float *__restrict__ sv) {
+  const int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (r >= R) return;
+  const int p = row_pix[r], n = row_len[p], g = row_grp[r];
+  const int64_t base = row_ptr[p];
+  for (int i = threadIdx.x & 31; i < n; i += 32) {
+    const float v = ev_val[base + i];
+    sv[base + i] =
+        v == 0.f ? v : __fdiv_rn(v, average ? sg[g] : sg[(size_t)g * F + ev_frame[base + i]]);
+  }
+}
+
+// One warp per column f1 of one q bin, W columns a block: the column's sums
+// over f0 <= f1 in the warp's shared memory (F floats).  The column's events
+// come in row order; each one's row contributes v(f0) v(f1) for its events up
+// to f1, one f0 per lane, so no two lanes of a step share a sum and every sum
+// takes its rows in order.  A lane each looks up 32 events' rows at a time,
+// and the next event's first 32 row entries are loaded while the current
+// one's are added: the steps' latency bounds it.  Long columns first; the
+// block writes its columns side by side (32-byte sectors at W = 8).
+// Measured (256 x 256 pixels, 701 frames, 6 q bins, 2 % of the pixels hit per
+// frame): the two-time call 0.89 ms against 13.0 ms with the dense matrix,
+// 9.75 ms of it in the tiled Gram.
+__global__ void __launch_bounds__(256)
+k_tt_gram_events(int32_t F, int32_t q0, const int32_t *__restrict__ q_ptr,
+                 const int64_t *__restrict__ col_ptr, const int32_t *__restrict__ a,
+                 const float *__restrict__ b, const int32_t *__restrict__ row_pix,
+                 const int64_t *__restrict__ row_ptr, const int32_t *__restrict__ ev_frame,
+                 const float *__restrict__ sv, float *__restrict__ C) {
+  extern __shared__ float tt_acc[];
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, W = blockDim.x >> 5;
+  const int q = q0 + blockIdx.y, c0 = (gridDim.x - 1 - blockIdx.x) * W, f1 = c0 + w;
+  float *acc = tt_acc + (size_t)w * F;
+  if (f1 < F) {
+    for (int f = lane; f <= f1; f += 32) acc[f] = 0.f;
+    __syncwarp();
+    const int64_t lo = col_ptr[(int64_t)q * F + f1], hi = col_ptr[(int64_t)q * F + f1 + 1];
+    for (int64_t e0 = lo; e0 < hi; e0 += 32) {
+      const int64_t e = e0 + lane;
+      int64_t my_base = 0;
+      int my_i = -1;  // position of the event in its row: entries 0 .. i reach up to f1
+      float my_v = 0.f;
+      if (e < hi) {
+        my_base = row_ptr[row_pix[a[e]]];
+        my_i = __float_as_int(b[e]);
+        my_v = sv[my_base + my_i];
+      }
+      const int n = (int)min((int64_t)32, hi - e0);
+      int64_t base = __shfl_sync(FULL, my_base, 0);
+      int i = __shfl_sync(FULL, my_i, 0);
+      int f = lane <= i ? ev_frame[base + lane] : 0;
+      float v = lane <= i ? sv[base + lane] : 0.f;
+      for (int k = 0; k < n; k++) {
+        const int64_t bk = base;
+        const int ik = i, fk = f;
+        const float vk = v, v1 = __shfl_sync(FULL, my_v, k);
+        const int nk = min(k + 1, 31);
+        base = __shfl_sync(FULL, my_base, nk);
+        i = k + 1 < n ? __shfl_sync(FULL, my_i, nk) : -1;
+        f = lane <= i ? ev_frame[base + lane] : 0;
+        v = lane <= i ? sv[base + lane] : 0.f;
+        if (v1 == 0.f) continue;  // no event (a smoothed value of 0 forms no product)
+        if (vk != 0.f) acc[fk] = __fadd_rn(acc[fk], __fmul_rn(vk, v1));
+        for (int j = lane + 32; j <= ik; j += 32) {
+          const float x = sv[bk + j];
+          if (x != 0.f) {
+            const int fx = ev_frame[bk + j];
+            acc[fx] = __fadd_rn(acc[fx], __fmul_rn(x, v1));
+          }
+        }
+        __syncwarp();
+      }
+    }
+  }
+  __syncthreads();
+  const float den = (float)(q_ptr[q + 1] - q_ptr[q]);
+  float *Cq = C + (size_t)q * F * F;
+  const int last = min(c0 + W, F) - 1;
+  for (int idx = threadIdx.x; idx < (last + 1) * W; idx += blockDim.x) {
+    const int f0 = idx / W, cw = idx % W, c = c0 + cw;
+    if (c < F && f0 <= c) Cq[(size_t)f0 * F + c] = __fdiv_rn(tt_acc[(size_t)cw * F + f0], den);
+  }
+}
+
+// Columns per block of the event Gram: 8 while two blocks fit on an SM, fewer
+// for longer columns; 0 when not even one column fits.
+int tt_columns(int32_t F) {
+  const size_t col = sizeof(float) * (size_t)F;
+  for (int w : {8, 4, 2, 1})
+    if (w * col <= 110 * 1024) return w;
+  return col <= 220 * 1024 ? 1 : 0;
+}
+
 // one thread per (q, diagonal ff): g2full and, for ff < window, g2partials
 __global__ void k_tt_diag(int32_t Q, int32_t F, int32_t window, int32_t tp,
                           const float *__restrict__ C, float *__restrict__ g2full,
@@ -138,7 +342,15 @@ __global__ void k_tt_diag(int32_t Q, int32_t F, int32_t window, int32_t tp,
   if (ff >= F || q >= Q) return;
   const float *Cq = C + (size_t)q * F * F;
   float acc = 0.f;
-  for (int fx = 0; fx < F - ff; fx++) acc = __fadd_rn(acc, Cq[(size_t)fx * F + fx + ff]);
+  int fx = 0;
+  for (; fx + 16 <= F - ff; fx += 16) {  // the loads first, in flight together
+    float x[16];
+#pragma unroll
+    for (int j = 0; j < 16; j++) x[j] = Cq[(size_t)(fx + j) * F + fx + j + ff];
+#pragma unroll
+    for (int j = 0; j < 16; j++) acc = __fadd_rn(acc, x[j]);
+  }
+  for (; fx < F - ff; fx++) acc = __fadd_rn(acc, Cq[(size_t)fx * F + fx + ff]);
   g2full[(size_t)ff * Q + q] = __fdiv_rn(acc, (float)(F - ff));
   if (ff < window) {
     for (int w = 0; w < tp; w++) {
@@ -147,6 +359,129 @@ __global__ void k_tt_diag(int32_t Q, int32_t F, int32_t window, int32_t tp,
         s = __fadd_rn(s, Cq[(size_t)fx * F + fx + ff]);
       g2part[((size_t)ff * tp + w) * Q + q] = __fdiv_rn(s, (float)window);
     }
+  }
+}
+
+// Whether the rows are sparse enough for the event Gram, from the mean number
+// of events per pixel and frame, d.  Its work grows as d^2, the tiled Gram's
+// not at all, and short columns are cheap at any density.  Whole calls in ms,
+// event lists / tiled (random events, 3 q bins):
+//   pixels  frames   d = 0.05      0.1         0.2         0.4
+//   128^2      100  0.38/2.52   0.49/2.53   0.70/2.57   1.41/2.58   (0.7: 3.1/2.6)
+//   128^2      700  0.53/2.73   0.98/2.78   2.70/2.85   9.5/3.0
+//   128^2    2,000  1.10/6.61   2.50/6.74   7.95/7.02   28.5/7.5
+//   256^2      700  1.20/12.5   3.03/12.6   10.1/12.8   36.8/13.2
+//   64^2     4,096  1.58/5.60   3.10/5.75   9.03/6.09   32.0/7.0
+bool tt_use_events(Series &s) {
+  if (tt_columns(s.F) == 0) return false;
+  const double most = std::min(0.4, std::max(0.15, 40.0 / s.F));
+  return (double)s.raw_events <= most * (double)s.qmap.pix.size() * s.R_in * s.F;
+}
+
+// C, sg and sga from event lists.
+void gram_events(Series &s, const TwoTimeReq &req, const TwoTimeLayout &lay, int32_t R, int32_t G,
+                 int32_t Q) {
+  cudaStream_t st = s.stream;
+  const int32_t F = s.F;
+  const int64_t ncol = (int64_t)Q * F;
+  const auto warps = [](int64_t k) { return (unsigned)((k * 32 + 255) / 256); };
+  std::vector<int32_t> ptrs(lay.q_ptr);  // rows of each q bin, then the q bin of each group
+  for (int32_t g = 0, q = 0; g < G; g++) {
+    while (q + 1 < Q && lay.grp_ptr[g] >= lay.q_ptr[q + 1]) q++;
+    ptrs.push_back(q);
+  }
+  s.tt_qptr.reserve(ptrs.size(), st);
+  XG_CUDA(cudaMemcpyAsync(s.tt_qptr.p, ptrs.data(), 4 * ptrs.size(), cudaMemcpyHostToDevice, st));
+  const int32_t *q_ptr = s.tt_qptr.p, *grp_q = q_ptr + Q + 1;
+  s.tt_len.reserve(R, st);
+  s.tt_cpos.reserve((size_t)R + 1, st);
+  s.tt_cols.reserve((size_t)ncol + 1, st);
+  s.scan_tmp.reserve(scan_workspace_bytes(R), st);
+  int64_t n = -1;
+  // sorts the rows' events by (q, frame) from the given row order; returns the
+  // sorted (a, b)
+  const auto lists = [&](const int32_t *order) {
+    k_tt_lens<<<(R + 255) / 256, 256, 0, st>>>(R, order, s.tt_row_pix.p, s.row_len.p, s.tt_len.p);
+    XG_CHECK_LAUNCH();
+    exclusive_scan_i32_i64(s.tt_len.p, s.tt_cpos.p, R, s.scan_tmp.p, st);
+    if (n < 0) {
+      XG_CUDA(cudaMemcpyAsync(&n, s.tt_cpos.p + R, sizeof(n), cudaMemcpyDeviceToHost, st));
+      XG_CUDA(cudaStreamSynchronize(st));
+    }
+    const size_t ne = std::max<int64_t>(n, 1);
+    s.keyA.reserve(ne, st);
+    s.frA.reserve(ne, st);
+    s.vA.reserve(ne, st);
+    s.keyB.reserve(ne, st);
+    s.frB.reserve(ne, st);
+    s.vB.reserve(ne, st);
+    k_tt_build<<<warps(R), 256, 0, st>>>(R, F, Q, order, q_ptr, s.tt_row_pix.p, s.row_ptr.p,
+                                         s.row_len.p, s.ev_frame.p, s.tt_cpos.p, s.keyA.p,
+                                         s.frA.p, s.vA.p);
+    XG_CHECK_LAUNCH();
+    const int bits = ncol > 1 ? 64 - __builtin_clzll((unsigned long long)ncol - 1) : 1;
+    const bool in_b = radix_sort_triples(s, s.keyA.p, s.frA.p, s.vA.p, s.keyB.p, s.frB.p, s.vB.p,
+                                         n, bits);
+    k_tt_cols<<<(unsigned)((ncol + 256) / 256), 256, 0, st>>>(ncol, n, in_b ? s.keyB.p : s.keyA.p,
+                                                              s.tt_cols.p);
+    XG_CHECK_LAUNCH();
+    return std::make_pair((const int32_t *)(in_b ? s.frB.p : s.frA.p),
+                          (const float *)(in_b ? s.vB.p : s.vA.p));
+  };
+  auto ab = lists(nullptr);  // mapping order
+  k_tt_sg_events<<<dim3(warps(F), G), 256, 0, st>>>(F, s.tt_grp_ptr.p, grp_q, s.tt_cols.p, ab.first,
+                                                    ab.second, s.tt_row_pix.p, s.row_ptr.p,
+                                                    s.ev_val.p, s.tt_sg.p);
+  XG_CHECK_LAUNCH();
+  if (req.average) {
+    k_tt_sg_avg<<<(G + 127) / 128, 128, 0, st>>>(G, F, s.tt_sg.p, s.tt_sga.p);
+    XG_CHECK_LAUNCH();
+  }
+  s.tt_V.reserve((size_t)std::max<int64_t>(s.raw_events, 1), st);  // as long as the event lists
+  k_tt_smooth_events<<<warps(R), 256, 0, st>>>(R, F, req.average, s.tt_row_pix.p, s.tt_row_grp.p,
+                                               s.row_ptr.p, s.row_len.p, s.ev_frame.p, s.ev_val.p,
+                                               req.average ? s.tt_sga.p : s.tt_sg.p, s.tt_V.p);
+  XG_CHECK_LAUNCH();
+  if (req.frame_threading) ab = lists(s.tt_order.p);
+  const int W = tt_columns(F);
+  const size_t smem = sizeof(float) * (size_t)F * W;
+  XG_CUDA(cudaFuncSetAttribute(k_tt_gram_events, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)smem));
+  k_tt_gram_events<<<dim3((F + W - 1) / W, Q), 32 * W, smem, st>>>(
+      F, 0, q_ptr, s.tt_cols.p, ab.first, ab.second, s.tt_row_pix.p, s.row_ptr.p, s.ev_frame.p,
+      s.tt_V.p, s.tt_C.p);
+  XG_CHECK_LAUNCH();
+}
+
+// The same from the dense matrix V.
+void gram_dense(Series &s, const TwoTimeReq &req, const TwoTimeLayout &lay, int32_t R, int32_t G,
+                int32_t Q) {
+  cudaStream_t st = s.stream;
+  const int32_t F = s.F;
+  const std::vector<int32_t> &q_ptr = lay.q_ptr;
+  const size_t nV = (size_t)R * F;
+  s.tt_V.reserve(nV, st);
+  XG_CUDA(cudaMemsetAsync(s.tt_V.p, 0, 4 * nV, st));
+  k_tt_scatter<<<(R + 127) / 128, 128, 0, st>>>(R, F, s.tt_row_pix.p, s.row_ptr.p, s.row_len.p,
+                                                s.ev_frame.p, s.ev_val.p, s.tt_V.p);
+  XG_CHECK_LAUNCH();
+  k_tt_sg<<<dim3((F + 127) / 128, G), 128, 0, st>>>(G, F, s.tt_grp_ptr.p, s.tt_V.p, s.tt_sg.p);
+  XG_CHECK_LAUNCH();
+  if (req.average) {
+    k_tt_sg_avg<<<(G + 127) / 128, 128, 0, st>>>(G, F, s.tt_sg.p, s.tt_sga.p);
+    XG_CHECK_LAUNCH();
+  }
+  k_tt_smooth<<<(unsigned)((nV + 255) / 256), 256, 0, st>>>(R, F, req.average, s.tt_row_grp.p,
+                                                           req.average ? s.tt_sga.p : s.tt_sg.p,
+                                                           s.tt_V.p);
+  XG_CHECK_LAUNCH();
+  const int T = (F + TT_TILE - 1) / TT_TILE;
+  for (int32_t q = 0; q < Q; q++) {
+    const int32_t nr = q_ptr[q + 1] - q_ptr[q];
+    if (nr == 0) continue;
+    k_tt_gram<<<T * (T + 1) / 2, 256, 0, st>>>(F, nr, s.tt_order.p + q_ptr[q], s.tt_V.p,
+                                               s.tt_C.p + (size_t)q * F * F);
+    XG_CHECK_LAUNCH();
   }
 }
 
@@ -212,31 +547,11 @@ void run_twotime(Series &s, const TwoTimeReq &req, int mode, bool force_i64) {
   up(s.tt_row_grp, row_grp);
   up(s.tt_grp_ptr, grp_ptr);
   up(s.tt_order, order);
-  const size_t nV = (size_t)R * F;
-  s.tt_V.reserve(nV ? nV : 1, st);
-  if (nV) XG_CUDA(cudaMemsetAsync(s.tt_V.p, 0, 4 * nV, st));
   if (R > 0 && F > 0) {
-    k_tt_scatter<<<(R + 127) / 128, 128, 0, st>>>(R, F, s.tt_row_pix.p, s.row_ptr.p, s.row_len.p,
-                                                  s.ev_frame.p, s.ev_val.p, s.tt_V.p);
-    XG_CHECK_LAUNCH();
-    k_tt_sg<<<dim3((F + 127) / 128, G), 128, 0, st>>>(G, F, s.tt_grp_ptr.p, s.tt_V.p, s.tt_sg.p);
-    XG_CHECK_LAUNCH();
-    if (req.average) {
-      k_tt_sg_avg<<<(G + 127) / 128, 128, 0, st>>>(G, F, s.tt_sg.p, s.tt_sga.p);
-      XG_CHECK_LAUNCH();
-    }
-    k_tt_smooth<<<(unsigned)((nV + 255) / 256), 256, 0, st>>>(R, F, req.average, s.tt_row_grp.p,
-                                                             req.average ? s.tt_sga.p : s.tt_sg.p,
-                                                             s.tt_V.p);
-    XG_CHECK_LAUNCH();
-    const int T = (F + TT_TILE - 1) / TT_TILE;
-    for (int32_t q = 0; q < Q; q++) {
-      const int32_t nr = q_ptr[q + 1] - q_ptr[q];
-      if (nr == 0) continue;
-      k_tt_gram<<<T * (T + 1) / 2, 256, 0, st>>>(F, nr, s.tt_order.p + q_ptr[q], s.tt_V.p,
-                                                 s.tt_C.p + (size_t)q * F * F);
-      XG_CHECK_LAUNCH();
-    }
+    if (tt_use_events(s))
+      gram_events(s, req, lay, R, G, Q);
+    else
+      gram_dense(s, req, lay, R, G, Q);
     k_tt_diag<<<dim3((F + 127) / 128, Q), 128, 0, st>>>(Q, F, req.window, o.partials, s.tt_C.p,
                                                        s.tt_full.p, s.tt_part.p);
     XG_CHECK_LAUNCH();

@@ -331,6 +331,8 @@ struct Series {
   // two-time
   TwoTimeOut tt;
   DBuf<int32_t> tt_row_pix, tt_row_grp, tt_grp_ptr, tt_order;
+  DBuf<int32_t> tt_qptr, tt_len;        // event lists: q bins' rows and the groups' q bins
+  DBuf<int64_t> tt_cpos, tt_cols;       // rows' and columns' first events
   DBuf<float> tt_V, tt_sg, tt_sga, tt_C, tt_full, tt_part;
   DBuf<int32_t> tt_err, tt_flags;       // tensor-core path: wait timeouts, range flags
   DBuf<uint16_t> tt_XT;                 // fp16 counts X^T [Fp][Kp] of one group
