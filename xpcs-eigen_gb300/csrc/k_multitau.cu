@@ -161,20 +161,14 @@ __device__ __forceinline__ void bins_pairs(const uint32_t *row, int m, int lf, i
     if (k < count) acc[k * 32] = a[k];
 }
 
-// One warp's 32 consecutive pixels p0 .. p0+31 of a series: the body of the
-// thread-per-pixel kernel, shared by its per-series launch and by the batch's
-// work-queue launch.  wbase: the warp's (CAP + scratch words) x 32 words of
-// shared memory.
+// The 32 consecutive pixels of a warp (this lane's is p, possibly past P),
+// each lane's row of n0 events packed in its column of wbase, the warp's (CAP
+// + scratch words) x 32 words of shared memory: the body of the
+// thread-per-pixel kernels after the rows are loaded.
 template <int CAP>
-__device__ __forceinline__ void mt_thread_warp(const uint8_t *__restrict__ plan_g,
-                                               const int64_t *__restrict__ row_ptr,
-                                               const int32_t *__restrict__ row_len,
-                                               const uint8_t *__restrict__ pclass,
-                                               const int32_t *__restrict__ ev_frame,
-                                               const float *__restrict__ ev_val,
+__device__ __forceinline__ void mt_thread_rows(const uint8_t *__restrict__ plan_g, int p, int n0,
                                                float *__restrict__ G2, float *__restrict__ IP,
-                                               float *__restrict__ IF, int p0,
-                                               uint32_t *wbase) {
+                                               float *__restrict__ IF, uint32_t *wbase) {
   // the plan is read from global memory: every lane of a warp reads the same
   // words (one L1-cached broadcast), and shared memory is left to the rows
   const McPlan *pl = (const McPlan *)plan_g;
@@ -185,53 +179,6 @@ __device__ __forceinline__ void mt_thread_warp(const uint8_t *__restrict__ plan_
   const int lane = threadIdx.x & 31;
   uint32_t *row = wbase + lane;
   int32_t *acc = (int32_t *)(row + CAP * 32);  // scratch, also S(t_end) per level
-
-  if (p0 >= P) return;
-  const int p = p0 + lane;
-  const bool mine = p < P && pclass[p] == PCLASS_THREAD;
-  const int n0 = mine ? row_len[p] : 0;
-
-  // cooperative, coalesced load of the warp's rows (consecutive pixels have
-  // consecutive rows), scattered to the owning lane's slots; four chunks of
-  // 32 events in flight per lane.  Positions are relative to the warp's first
-  // event: when a lane owns a packed row every frame is below 65536, so the
-  // 32 rows span fewer than 2^21 events.
-  if (__any_sync(0xffffffffu, n0 > 0)) {
-    const unsigned FULL = 0xffffffffu;
-    const int plast = min(p0 + 32, P);
-    const int64_t e0 = row_ptr[p0];
-    const int nw = (int)(row_ptr[plast] - e0);
-    const int my_b = p < P ? (int)(row_ptr[p] - e0) : nw;
-    const int lo = __reduce_min_sync(FULL, n0 > 0 ? my_b : INT_MAX);
-    const int hi = __reduce_max_sync(FULL, n0 > 0 ? my_b + n0 : 0);
-    for (int base = lo; base < hi; base += 128) {
-      int dst[4], fr[4];
-      float vl[4];
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        const int e = base + u * 32 + lane;
-        int owner = 0;  // last lane whose row starts at or before e
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          const int cand = owner + o;
-          const int cb = __shfl_sync(FULL, my_b, cand & 31);
-          if (cand < 32 && cb <= e) owner = cand;
-        }
-        const int slot = e - __shfl_sync(FULL, my_b, owner);
-        const int olen = __shfl_sync(FULL, n0, owner);
-        dst[u] = (e < hi && slot < olen) ? slot * 32 + owner : -1;
-        if (dst[u] >= 0) {
-          fr[u] = ev_frame[e0 + e];
-          vl[u] = ev_val[e0 + e];
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 4; u++)
-        if (dst[u] >= 0) wbase[dst[u]] = pk(fr[u], __float2int_rn(vl[u]));
-    }
-  }
-  __syncwarp();
-
   // total and S(t_end) per level (sweep from the end; t_end non-increasing)
   int total = 0;
   for (int i = 0; i < n0; i++) total += pk_v(row[i * 32]);
@@ -422,6 +369,68 @@ __device__ __forceinline__ void mt_thread_warp(const uint8_t *__restrict__ plan_
   }
 }
 
+// One warp's 32 consecutive pixels p0 .. p0+31 of a series: the rows loaded
+// and run, shared by the per-series launch and by the batch's work-queue
+// launch.
+template <int CAP>
+__device__ __forceinline__ void mt_thread_warp(const uint8_t *__restrict__ plan_g,
+                                               const int64_t *__restrict__ row_ptr,
+                                               const int32_t *__restrict__ row_len,
+                                               const uint8_t *__restrict__ pclass,
+                                               const int32_t *__restrict__ ev_frame,
+                                               const float *__restrict__ ev_val,
+                                               float *__restrict__ G2, float *__restrict__ IP,
+                                               float *__restrict__ IF, int p0,
+                                               uint32_t *wbase) {
+  const int P = ((const McPlan *)plan_g)->P, lane = threadIdx.x & 31;
+  if (p0 >= P) return;
+  const int p = p0 + lane;
+  const bool mine = p < P && pclass[p] == PCLASS_THREAD;
+  const int n0 = mine ? row_len[p] : 0;
+
+  // cooperative, coalesced load of the warp's rows (consecutive pixels have
+  // consecutive rows), scattered to the owning lane's slots; four chunks of
+  // 32 events in flight per lane.  Positions are relative to the warp's first
+  // event: when a lane owns a packed row every frame is below 65536, so the
+  // 32 rows span fewer than 2^21 events.
+  if (__any_sync(0xffffffffu, n0 > 0)) {
+    const unsigned FULL = 0xffffffffu;
+    const int plast = min(p0 + 32, P);
+    const int64_t e0 = row_ptr[p0];
+    const int nw = (int)(row_ptr[plast] - e0);
+    const int my_b = p < P ? (int)(row_ptr[p] - e0) : nw;
+    const int lo = __reduce_min_sync(FULL, n0 > 0 ? my_b : INT_MAX);
+    const int hi = __reduce_max_sync(FULL, n0 > 0 ? my_b + n0 : 0);
+    for (int base = lo; base < hi; base += 128) {
+      int dst[4], fr[4];
+      float vl[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const int e = base + u * 32 + lane;
+        int owner = 0;  // last lane whose row starts at or before e
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          const int cand = owner + o;
+          const int cb = __shfl_sync(FULL, my_b, cand & 31);
+          if (cand < 32 && cb <= e) owner = cand;
+        }
+        const int slot = e - __shfl_sync(FULL, my_b, owner);
+        const int olen = __shfl_sync(FULL, n0, owner);
+        dst[u] = (e < hi && slot < olen) ? slot * 32 + owner : -1;
+        if (dst[u] >= 0) {
+          fr[u] = ev_frame[e0 + e];
+          vl[u] = ev_val[e0 + e];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (dst[u] >= 0) wbase[dst[u]] = pk(fr[u], __float2int_rn(vl[u]));
+    }
+  }
+  __syncwarp();
+  mt_thread_rows<CAP>(plan_g, p, n0, G2, IP, IF, wbase);
+}
+
 template <int CAP>
 __global__ void __launch_bounds__(MT_WARPS * 32, 8)
 k_mt_thread(const uint8_t *__restrict__ plan_g, const int64_t *__restrict__ row_ptr,
@@ -501,14 +510,13 @@ __device__ int compact_row(uint32_t *row, int m, int lastframe, int lane) {
 //     reads the 64 bins after it, finds its first partner's index by a
 //     population count over the bins below tau_lo and visits only the
 //     occupied bins of the delay window.
-// One pixel p of a series with a row of n0 events (min_n < n0 <= cap): the
-// body of the warp-per-pixel kernel, shared by its per-series launches and by
+// One pixel p of a series with a row of n0 events from event b on (min_n < n0
+// <= cap): the body of the warp-per-pixel kernel, shared by its per-series launches and by
 // the batch's work-queue launches.  pl / ar: the plan (shared or global
 // memory); row, S: the warp's 2 x cap words; acc: this lane's accumulators
 // (acc[k * 32]).
 __device__ __forceinline__ void mt_warp_pixel(const McPlan *pl, const McArrays &ar, int p,
-                                              const int64_t *__restrict__ row_ptr,
-                                              const int32_t *__restrict__ row_len,
+                                              int64_t b, int n0,
                                               const int32_t *__restrict__ ev_frame,
                                               const float *__restrict__ ev_val,
                                               float *__restrict__ G2, float *__restrict__ IP,
@@ -517,8 +525,6 @@ __device__ __forceinline__ void mt_warp_pixel(const McPlan *pl, const McArrays &
   const int P = pl->P, mode = pl->mode, D = pl->D;
   const int lane = threadIdx.x & 31;
   const unsigned FULL = 0xffffffffu;
-  const int n0 = row_len[p];
-  const int64_t b = row_ptr[p];
   int carry = 0;
   for (int c0 = 0; c0 < n0; c0 += 32) {
     const int i = c0 + lane;
@@ -674,7 +680,7 @@ k_mt_warp(const uint8_t *__restrict__ plan_g, const int32_t *__restrict__ list,
     const int p = list[q];
     const int n0 = row_len[p];
     if (n0 <= min_n || n0 > cap) continue;  // another launch's share of the list
-    mt_warp_pixel(pl, ar, p, row_ptr, row_len, ev_frame, ev_val, G2, IP, IF, cap, row, S, acc);
+    mt_warp_pixel(pl, ar, p, row_ptr[p], n0, ev_frame, ev_val, G2, IP, IF, cap, row, S, acc);
   }
 }
 
@@ -753,8 +759,8 @@ k_mt_warp_queue(const MtQueueMember *__restrict__ tab, int32_t n, int32_t use_lo
     if (n0 <= min_n || n0 > cap) continue;
     const McPlan *pl = (const McPlan *)m.plan;
     const McArrays ar = mc_arrays(m.plan, pl->D);
-    mt_warp_pixel(pl, ar, p, m.row_ptr, m.row_len, m.ev_frame, m.ev_val, m.G2, m.IP, m.IF, cap,
-                  row, S, acc);
+    mt_warp_pixel(pl, ar, p, m.row_ptr[p], n0, m.ev_frame, m.ev_val, m.G2, m.IP, m.IF, cap, row,
+                  S, acc);
   }
 }
 
@@ -877,20 +883,18 @@ __device__ __forceinline__ bool fw_findable(uint64_t fmask, int j) {
   return (fmask >> (j & 63)) & 1u;
 }
 
-__global__ void __launch_bounds__(FW_WARPS * 32, 7)
-k_mt_fwarp(const uint8_t *__restrict__ plan_g, const int32_t *__restrict__ flist,
-           DevStats *__restrict__ stats, const int64_t *__restrict__ row_ptr,
-           const int32_t *__restrict__ row_len, const int32_t *__restrict__ ev_frame,
-           const float *__restrict__ ev_val, const float *__restrict__ fscale,
-           int32_t *__restrict__ sc_frame, float *__restrict__ sc_val, float *__restrict__ G2,
-           float *__restrict__ IP, float *__restrict__ IF) {
-  extern __shared__ __align__(16) uint8_t fw_smem[];
-  const McPlan *pl = (const McPlan *)plan_g;
-  const int D = pl->D, P = pl->P, nlev = pl->nlev, acc_max = pl->acc;
+// One pixel p with a row of n0 events from event b on: the scratch row idx /
+// val, the warp's shared memory wb (fw_warp_bytes).
+__device__ __forceinline__ void fw_pixel(const McPlan *pl, const McArrays &ar, int p, int64_t b,
+                                         int n0, const int32_t *__restrict__ ev_frame,
+                                         const float *__restrict__ ev_val,
+                                         const float *__restrict__ fscale, int32_t *idx,
+                                         float *val, float *__restrict__ G2,
+                                         float *__restrict__ IP, float *__restrict__ IF,
+                                         uint8_t *wb) {
+  const int P = pl->P, nlev = pl->nlev, acc_max = pl->acc;
   const bool ref = pl->mode == XPCS_MODE_REFERENCE;
-  const McArrays ar = mc_arrays(plan_g, D);
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  uint8_t *wb = fw_smem + (size_t)w * fw_warp_bytes(acc_max);
+  const int lane = threadIdx.x & 31;
   int32_t *ridx = (int32_t *)wb;
   float *rval = (float *)(wb + 256);
   // bin b of the window: the value of the entry at b0 + b when it is
@@ -900,6 +904,241 @@ k_mt_fwarp(const uint8_t *__restrict__ plan_g, const int32_t *__restrict__ flist
   float *bval = (float *)(wb + 512);
   float *terms = (float *)(wb + 512 + FW_WIN * 4);
   float *vrow = terms + (size_t)3 * acc_max * FW_TSTRIDE;
+  for (int i0 = 0; i0 < n0; i0 += 4 * 32) {
+    int32_t f[4];
+    float x[4];
+#pragma unroll
+    for (int h = 0; h < 4; h++) {  // the loads first, in flight together
+      const int i = i0 + h * 32 + lane;
+      if (i < n0) {
+        f[h] = ev_frame[b + i];
+        x[h] = ev_val[b + i];
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 4; h++) {
+      const int i = i0 + h * 32 + lane;
+      if (i < n0) {
+        idx[i] = f[h];
+        // normalize_by_framesum: v / (frameSum[f] / mean) (main.cpp:330-333)
+        val[i] = fscale ? __fdiv_rn(x[h], fscale[f[h]]) : x[h];
+      }
+    }
+  }
+  __syncwarp();
+  int L = n0;
+  bool tail_sorted = true, dead = false;
+  for (int gi = 0; gi < nlev; gi++) {
+    const McLevel lv = pl->lv[gi];
+    const int lastframe = lv.lastframe, cnt = lv.count, t0 = lv.tau_lo;
+    if (lv.compact && !dead) {
+      const int prevL = L;
+      // the junction between the previous prefix and the older tail
+      bool junction_ok = true;
+      if (prevL < n0) junction_ok = idx[prevL - 1] <= idx[prevL];
+      if ((idx[0] >> 1) >= lastframe) {
+        dead = true;  // nothing is kept: lastIndex becomes 1 on a stale entry
+      } else {
+        int out = 0, carry_h = -1;
+        // chunks of 32 entries, each loaded two chunks ahead: a chunk's
+        // pass writes only below its own end, so the entries in flight
+        // are never overwritten before they are used
+        int32_t ia = lane < prevL ? idx[lane] : INT_MAX;
+        float va = lane < prevL ? val[lane] : 0.f;
+        int32_t ia1 = 32 + lane < prevL ? idx[32 + lane] : INT_MAX;
+        float va1 = 32 + lane < prevL ? val[32 + lane] : 0.f;
+        for (int base = 0; base < prevL; base += 32) {
+          const int a2 = base + 64 + lane;
+          const int32_t ia2 = a2 < prevL ? idx[a2] : INT_MAX;
+          const float va2 = a2 < prevL ? val[a2] : 0.f;
+          const int a = base + lane;
+          const bool in = a < prevL;
+          const bool has_b = a + 1 < prevL;
+          // the next entry: the lane above's, or the next chunk's first
+          int32_t ib = __shfl_down_sync(0xffffffffu, ia, 1);
+          float vb = __shfl_down_sync(0xffffffffu, va, 1);
+          const int32_t ib1 = __shfl_sync(0xffffffffu, ia1, 0);
+          const float vb1 = __shfl_sync(0xffffffffu, va1, 0);
+          if (lane == 31) {
+            ib = ib1;
+            vb = vb1;
+          }
+          const int h = ia >> 1, hb = ib >> 1;
+          int hp = __shfl_up_sync(0xffffffffu, h, 1);
+          if (lane == 0) hp = carry_h;
+          const bool keep = in && (a == 0 || h != hp) && h < lastframe;
+          const bool merge = keep && has_b && hb == h;
+          float sv = va;
+          if (merge) sv = __fadd_rn(va, vb);
+          sv = __fmul_rn(sv, 0.5f);  // == sv / 2 (exact scaling)
+          const unsigned bal = __ballot_sync(0xffffffffu, keep);
+          const bool stop = __any_sync(0xffffffffu, in && h >= lastframe);
+          carry_h = __shfl_sync(0xffffffffu, h, 31);
+          __syncwarp();
+          if (keep) {
+            const int o = out + __popc(bal & ((1u << lane) - 1u));
+            idx[o] = h;
+            val[o] = sv;
+          }
+          out += __popc(bal);
+          __syncwarp();
+          if (stop) break;
+          ia = ia1;
+          va = va1;
+          ia1 = ia2;
+          va1 = va2;
+        }
+        L = out;
+        tail_sorted = tail_sorted && (L >= prevL || junction_ok);
+      }
+    }
+    if (dead) {
+      for (int c = lane; c < cnt; c += 32) {
+        const size_t o = (size_t)(lv.first + c) * P + p;
+        G2[o] = 0.f;
+        IP[o] = 0.f;
+        IF[o] = 0.f;
+      }
+      continue;
+    }
+    // every prefix entry is findable unless the reference searches a buffer
+    // that is out of order
+    const bool all_find = !ref || (tail_sorted && (L >= n0 || idx[L - 1] <= idx[L]));
+    const int kmax = t0 + cnt - 1;
+    const int nchain = 3 * cnt;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    // ring slots past the row end are never read (partners stop at L)
+    uint64_t fmask = 0;
+    fw_put(0, lane, L, fw_fetch(0, lane, L, n0, all_find, idx, val), ridx, rval, fmask);
+    fw_put(32, lane, L, fw_fetch(32, lane, L, n0, all_find, idx, val), ridx, rval, fmask);
+    for (int base = 0; base < L; base += 32) {
+      // the tile after next, in flight while this one is processed
+      const FwEntry nx = fw_fetch(base + 64, lane, L, n0, all_find, idx, val);
+      __syncwarp();
+      const int r = base + lane;
+      const bool valid = r < L;
+      const int nt = min(32, L - base);  // entries in this tile
+      const int32_t src = valid ? ridx[r & 63] : 0;
+      const float v = valid ? rval[r & 63] : 0.f;
+      // partners: when the tile and its partners span fewer than FW_WIN
+      // bins, through a per-warp bin array (one lookup per delay), else by
+      // scanning the following entries
+      const int32_t b0 = ridx[base & 63];
+      const bool use_bins = ridx[(base + nt - 1) & 63] + kmax - b0 < FW_WIN;
+      if (use_bins) {
+        ((float4 *)bval)[lane] = make_float4(0.f, 0.f, 0.f, 0.f);  // FW_WIN = 128 bins
+        __syncwarp();
+        if (valid) bval[src - b0] = fw_findable(fmask, r) ? v : 0.f;
+        const int q2 = base + 32 + lane;
+        if (lane < kmax && q2 < L) {
+          const int tb = ridx[q2 & 63] - b0;
+          if (tb < FW_WIN) bval[tb] = fw_findable(fmask, q2) ? rval[q2 & 63] : 0.f;
+        }
+        __syncwarp();
+      }
+      // inside [kmax, lastframe - kmax) every IP and IF term of the tile is v:
+      // the IP/IF chains then read one shared row
+      const bool bulk = b0 >= kmax && ridx[(base + nt - 1) & 63] < lastframe - kmax;
+      if (valid) {
+        if (bulk) {
+          vrow[lane] = v;
+        } else {
+          float *tp = terms + (size_t)cnt * FW_TSTRIDE + lane;
+          float *tf = tp + (size_t)cnt * FW_TSTRIDE;
+#pragma unroll
+          for (int c = 0; c < FW_MAXC; c++) {
+            if (c >= cnt) break;
+            const int tau = t0 + c;
+            tp[c * FW_TSTRIDE] = src < lastframe - tau ? v : 0.f;
+            tf[c * FW_TSTRIDE] = (src >= tau && src < lastframe) ? v : 0.f;
+          }
+        }
+        // a partner is a prefix entry, so it lies below lastframe and the
+        // reference's src < lastframe - tau test holds for every pair found
+        if (use_bins) {
+          const float *bw = bval + (src + t0 - b0);  // + c <= src - b0 + kmax < FW_WIN
+          float *tg = terms + lane;
+          if ((cnt & 3) == 0) {  // e.g. every level of 8 delays: one test per 4 delays
+#pragma unroll
+            for (int c = 0; c < FW_MAXC; c += 4) {
+              if (c >= cnt) break;
+#pragma unroll
+              for (int u = 0; u < 4; u++) tg[(c + u) * FW_TSTRIDE] = __fmul_rn(v, bw[c + u]);
+            }
+          } else {
+#pragma unroll
+            for (int c = 0; c < FW_MAXC; c++) {
+              if (c >= cnt) break;
+              tg[c * FW_TSTRIDE] = __fmul_rn(v, bw[c]);
+            }
+          }
+        } else {
+          for (int c = 0; c < cnt; c++) terms[(size_t)c * FW_TSTRIDE + lane] = 0.f;
+          for (int k = t0 > 0 ? 1 : 0; k <= kmax; k++) {
+            const int qk = r + k;
+            if (qk >= L) break;
+            const int d = ridx[qk & 63] - src;
+            if (d > kmax) break;
+            if (d >= t0 && fw_findable(fmask, qk))
+              terms[(size_t)(d - t0) * FW_TSTRIDE + lane] = __fmul_rn(v, rval[qk & 63]);
+          }
+        }
+      }
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const int ch = lane + 32 * j;
+        if (ch < nchain) {
+          const float *tr = (bulk && ch >= cnt) ? vrow : terms + (size_t)ch * FW_TSTRIDE;
+          float a = acc[j];
+          if (nt == 32) {
+            const float4 *t4 = (const float4 *)tr;
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+              const float4 y = t4[i];
+              a = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(a, y.x), y.y), y.z), y.w);
+            }
+          } else {
+#pragma unroll
+            for (int i = 0; i < 32; i++) {
+              if (i >= nt) break;
+              a = __fadd_rn(a, tr[i]);
+            }
+          }
+          acc[j] = a;
+        }
+      }
+      __syncwarp();
+      // the tile after next replaces this one in the ring
+      fw_put(base + 64, lane, L, nx, ridx, rval, fmask);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int ch = lane + 32 * j;
+      if (ch < nchain) {
+        const int type = ch / cnt, c = ch - type * cnt;
+        const int d = lv.first + c;
+        const float den = ar.denom[d];
+        const float x = den > 0.f ? __fdiv_rn(acc[j], den) : acc[j];
+        float *dst = type == 0 ? G2 : (type == 1 ? IP : IF);
+        dst[(size_t)d * P + p] = x;
+      }
+    }
+  }
+}
+
+__global__ void __launch_bounds__(FW_WARPS * 32, 7)
+k_mt_fwarp(const uint8_t *__restrict__ plan_g, const int32_t *__restrict__ flist,
+           DevStats *__restrict__ stats, const int64_t *__restrict__ row_ptr,
+           const int32_t *__restrict__ row_len, const int32_t *__restrict__ ev_frame,
+           const float *__restrict__ ev_val, const float *__restrict__ fscale,
+           int32_t *__restrict__ sc_frame, float *__restrict__ sc_val, float *__restrict__ G2,
+           float *__restrict__ IP, float *__restrict__ IF) {
+  extern __shared__ __align__(16) uint8_t fw_smem[];
+  const McPlan *pl = (const McPlan *)plan_g;
+  const McArrays ar = mc_arrays(plan_g, pl->D);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  uint8_t *wb = fw_smem + (size_t)w * fw_warp_bytes(pl->acc);
   const int nf = stats->nfloat;
   // pixels are handed out one per warp from a counter: rows differ in length
   for (;;) {
@@ -909,232 +1148,181 @@ k_mt_fwarp(const uint8_t *__restrict__ plan_g, const int32_t *__restrict__ flist
     if (q >= nf) break;
     const int p = flist[q];
     const int64_t b = row_ptr[p];
-    const int n0 = row_len[p];
-    int32_t *idx = sc_frame + b;
-    float *val = sc_val + b;
-    for (int i0 = 0; i0 < n0; i0 += 4 * 32) {
-      int32_t f[4];
-      float x[4];
-#pragma unroll
-      for (int h = 0; h < 4; h++) {  // the loads first, in flight together
-        const int i = i0 + h * 32 + lane;
-        if (i < n0) {
-          f[h] = ev_frame[b + i];
-          x[h] = ev_val[b + i];
-        }
-      }
-#pragma unroll
-      for (int h = 0; h < 4; h++) {
-        const int i = i0 + h * 32 + lane;
-        if (i < n0) {
-          idx[i] = f[h];
-          // normalize_by_framesum: v / (frameSum[f] / mean) (main.cpp:330-333)
-          val[i] = fscale ? __fdiv_rn(x[h], fscale[f[h]]) : x[h];
-        }
-      }
-    }
-    __syncwarp();
-    int L = n0;
-    bool tail_sorted = true, dead = false;
-    for (int gi = 0; gi < nlev; gi++) {
-      const McLevel lv = pl->lv[gi];
-      const int lastframe = lv.lastframe, cnt = lv.count, t0 = lv.tau_lo;
-      if (lv.compact && !dead) {
-        const int prevL = L;
-        // the junction between the previous prefix and the older tail
-        bool junction_ok = true;
-        if (prevL < n0) junction_ok = idx[prevL - 1] <= idx[prevL];
-        if ((idx[0] >> 1) >= lastframe) {
-          dead = true;  // nothing is kept: lastIndex becomes 1 on a stale entry
-        } else {
-          int out = 0, carry_h = -1;
-          // chunks of 32 entries, each loaded two chunks ahead: a chunk's
-          // pass writes only below its own end, so the entries in flight
-          // are never overwritten before they are used
-          int32_t ia = lane < prevL ? idx[lane] : INT_MAX;
-          float va = lane < prevL ? val[lane] : 0.f;
-          int32_t ia1 = 32 + lane < prevL ? idx[32 + lane] : INT_MAX;
-          float va1 = 32 + lane < prevL ? val[32 + lane] : 0.f;
-          for (int base = 0; base < prevL; base += 32) {
-            const int a2 = base + 64 + lane;
-            const int32_t ia2 = a2 < prevL ? idx[a2] : INT_MAX;
-            const float va2 = a2 < prevL ? val[a2] : 0.f;
-            const int a = base + lane;
-            const bool in = a < prevL;
-            const bool has_b = a + 1 < prevL;
-            // the next entry: the lane above's, or the next chunk's first
-            int32_t ib = __shfl_down_sync(0xffffffffu, ia, 1);
-            float vb = __shfl_down_sync(0xffffffffu, va, 1);
-            const int32_t ib1 = __shfl_sync(0xffffffffu, ia1, 0);
-            const float vb1 = __shfl_sync(0xffffffffu, va1, 0);
-            if (lane == 31) {
-              ib = ib1;
-              vb = vb1;
-            }
-            const int h = ia >> 1, hb = ib >> 1;
-            int hp = __shfl_up_sync(0xffffffffu, h, 1);
-            if (lane == 0) hp = carry_h;
-            const bool keep = in && (a == 0 || h != hp) && h < lastframe;
-            const bool merge = keep && has_b && hb == h;
-            float sv = va;
-            if (merge) sv = __fadd_rn(va, vb);
-            sv = __fmul_rn(sv, 0.5f);  // == sv / 2 (exact scaling)
-            const unsigned bal = __ballot_sync(0xffffffffu, keep);
-            const bool stop = __any_sync(0xffffffffu, in && h >= lastframe);
-            carry_h = __shfl_sync(0xffffffffu, h, 31);
-            __syncwarp();
-            if (keep) {
-              const int o = out + __popc(bal & ((1u << lane) - 1u));
-              idx[o] = h;
-              val[o] = sv;
-            }
-            out += __popc(bal);
-            __syncwarp();
-            if (stop) break;
-            ia = ia1;
-            va = va1;
-            ia1 = ia2;
-            va1 = va2;
-          }
-          L = out;
-          tail_sorted = tail_sorted && (L >= prevL || junction_ok);
-        }
-      }
-      if (dead) {
-        for (int c = lane; c < cnt; c += 32) {
-          const size_t o = (size_t)(lv.first + c) * P + p;
-          G2[o] = 0.f;
-          IP[o] = 0.f;
-          IF[o] = 0.f;
-        }
-        continue;
-      }
-      // every prefix entry is findable unless the reference searches a buffer
-      // that is out of order
-      const bool all_find = !ref || (tail_sorted && (L >= n0 || idx[L - 1] <= idx[L]));
-      const int kmax = t0 + cnt - 1;
-      const int nchain = 3 * cnt;
-      float acc[4] = {0.f, 0.f, 0.f, 0.f};
-      // ring slots past the row end are never read (partners stop at L)
-      uint64_t fmask = 0;
-      fw_put(0, lane, L, fw_fetch(0, lane, L, n0, all_find, idx, val), ridx, rval, fmask);
-      fw_put(32, lane, L, fw_fetch(32, lane, L, n0, all_find, idx, val), ridx, rval, fmask);
-      for (int base = 0; base < L; base += 32) {
-        // the tile after next, in flight while this one is processed
-        const FwEntry nx = fw_fetch(base + 64, lane, L, n0, all_find, idx, val);
-        __syncwarp();
-        const int r = base + lane;
-        const bool valid = r < L;
-        const int nt = min(32, L - base);  // entries in this tile
-        const int32_t src = valid ? ridx[r & 63] : 0;
-        const float v = valid ? rval[r & 63] : 0.f;
-        // partners: when the tile and its partners span fewer than FW_WIN
-        // bins, through a per-warp bin array (one lookup per delay), else by
-        // scanning the following entries
-        const int32_t b0 = ridx[base & 63];
-        const bool use_bins = ridx[(base + nt - 1) & 63] + kmax - b0 < FW_WIN;
-        if (use_bins) {
-          ((float4 *)bval)[lane] = make_float4(0.f, 0.f, 0.f, 0.f);  // FW_WIN = 128 bins
-          __syncwarp();
-          if (valid) bval[src - b0] = fw_findable(fmask, r) ? v : 0.f;
-          const int q2 = base + 32 + lane;
-          if (lane < kmax && q2 < L) {
-            const int tb = ridx[q2 & 63] - b0;
-            if (tb < FW_WIN) bval[tb] = fw_findable(fmask, q2) ? rval[q2 & 63] : 0.f;
-          }
-          __syncwarp();
-        }
-        // inside [kmax, lastframe - kmax) every IP and IF term of the tile is v:
-        // the IP/IF chains then read one shared row
-        const bool bulk = b0 >= kmax && ridx[(base + nt - 1) & 63] < lastframe - kmax;
-        if (valid) {
-          if (bulk) {
-            vrow[lane] = v;
-          } else {
-            float *tp = terms + (size_t)cnt * FW_TSTRIDE + lane;
-            float *tf = tp + (size_t)cnt * FW_TSTRIDE;
-#pragma unroll
-            for (int c = 0; c < FW_MAXC; c++) {
-              if (c >= cnt) break;
-              const int tau = t0 + c;
-              tp[c * FW_TSTRIDE] = src < lastframe - tau ? v : 0.f;
-              tf[c * FW_TSTRIDE] = (src >= tau && src < lastframe) ? v : 0.f;
-            }
-          }
-          // a partner is a prefix entry, so it lies below lastframe and the
-          // reference's src < lastframe - tau test holds for every pair found
-          if (use_bins) {
-            const float *bw = bval + (src + t0 - b0);  // + c <= src - b0 + kmax < FW_WIN
-            float *tg = terms + lane;
-            if ((cnt & 3) == 0) {  // e.g. every level of 8 delays: one test per 4 delays
-#pragma unroll
-              for (int c = 0; c < FW_MAXC; c += 4) {
-                if (c >= cnt) break;
-#pragma unroll
-                for (int u = 0; u < 4; u++) tg[(c + u) * FW_TSTRIDE] = __fmul_rn(v, bw[c + u]);
-              }
-            } else {
-#pragma unroll
-              for (int c = 0; c < FW_MAXC; c++) {
-                if (c >= cnt) break;
-                tg[c * FW_TSTRIDE] = __fmul_rn(v, bw[c]);
-              }
-            }
-          } else {
-            for (int c = 0; c < cnt; c++) terms[(size_t)c * FW_TSTRIDE + lane] = 0.f;
-            for (int k = t0 > 0 ? 1 : 0; k <= kmax; k++) {
-              const int qk = r + k;
-              if (qk >= L) break;
-              const int d = ridx[qk & 63] - src;
-              if (d > kmax) break;
-              if (d >= t0 && fw_findable(fmask, qk))
-                terms[(size_t)(d - t0) * FW_TSTRIDE + lane] = __fmul_rn(v, rval[qk & 63]);
-            }
-          }
-        }
-        __syncwarp();
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-          const int ch = lane + 32 * j;
-          if (ch < nchain) {
-            const float *tr = (bulk && ch >= cnt) ? vrow : terms + (size_t)ch * FW_TSTRIDE;
-            float a = acc[j];
-            if (nt == 32) {
-              const float4 *t4 = (const float4 *)tr;
-#pragma unroll
-              for (int i = 0; i < 8; i++) {
-                const float4 y = t4[i];
-                a = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(a, y.x), y.y), y.z), y.w);
-              }
-            } else {
-#pragma unroll
-              for (int i = 0; i < 32; i++) {
-                if (i >= nt) break;
-                a = __fadd_rn(a, tr[i]);
-              }
-            }
-            acc[j] = a;
-          }
-        }
-        __syncwarp();
-        // the tile after next replaces this one in the ring
-        fw_put(base + 64, lane, L, nx, ridx, rval, fmask);
-      }
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const int ch = lane + 32 * j;
-        if (ch < nchain) {
-          const int type = ch / cnt, c = ch - type * cnt;
-          const int d = lv.first + c;
-          const float den = ar.denom[d];
-          const float x = den > 0.f ? __fdiv_rn(acc[j], den) : acc[j];
-          float *dst = type == 0 ? G2 : (type == 1 ? IP : IF);
-          dst[(size_t)d * P + p] = x;
-        }
-      }
-    }
+    fw_pixel(pl, ar, p, b, row_len[p], ev_frame, ev_val, fscale, sc_frame + b, sc_val + b, G2, IP,
+             IF, wb);
     __syncwarp();
   }
+}
+
+// ------------------------------------------- caller rows, nothing allocated
+//
+// The row kernels for rows that come without classes, lengths or work lists
+// (noalloc.cu): every kernel finds its own rows among the caller's row
+// pointers and reads a row's class from its events, so no per-pixel array is
+// needed.  A row is regular when its frames ascend strictly within [0, F) and
+// its values are below 2^126 (the float-row kernel multiplies by 0 where the
+// reference forms no product, and halving sums must not overflow); regular
+// rows take the kernels of a series, the others the replay (noalloc.cu).
+// status[1] collects the kinds of rows seen, so that a kernel without rows
+// returns at once; status[2 ..] are the kernels' pixel counters.
+// Measured (256 x 250 pixels, 3,000 frames, 2.8 M events): the call 4,700 us
+// with one thread replaying each row from global memory, 574 us now.
+constexpr int NA_GRAB = 4;  // pixels a warp takes at a time
+
+// Row p: its first event and length; false (and the status bit) when it lies
+// outside the events.
+__device__ __forceinline__ bool na_row(const NaRows &v, int p, int64_t &b, int &n) {
+  b = v.row_ptr[p];
+  const int64_t e = v.row_ptr[p + 1];
+  const bool ok = b >= 0 && e >= b && e <= v.events;
+  n = ok ? (int)(e - b) : 0;
+  return ok;
+}
+
+// Class of row [b, b + n), the same in every lane: NA_INT (n <= MT_LONG_CAP),
+// NA_FLOAT or NA_IRREGULAR.
+__device__ __forceinline__ int na_class(const NaRows &v, int64_t b, int n) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  bool reg = true, integ = v.F <= 65536 && n <= MT_LONG_CAP;
+  int total = 0;  // a lane's share: at most 128 values of at most 4,096 while integ
+  int last = -1;
+  for (int i0 = 0; i0 < n; i0 += 32) {
+    const int i = i0 + lane;
+    const int f = i < n ? v.frame[b + i] : INT_MAX;
+    const float x = i < n ? v.value[b + i] : 0.f;
+    int prev = __shfl_up_sync(FULL, f, 1);
+    if (lane == 0) prev = last;
+    last = __shfl_sync(FULL, f, 31);
+    if (i < n) {
+      reg = reg && f > prev && f < v.F && fabsf(x) < 0x1p126f;
+      integ = integ && x == truncf(x) && fabsf(x) < 16777216.f;
+      total += integ ? (int)fminf(fabsf(x), 4096.f) : 0;
+    }
+  }
+  reg = __all_sync(FULL, reg);
+  integ = __all_sync(FULL, integ);
+  if (!reg) return NA_IRREGULAR;
+  return integ && __reduce_add_sync(FULL, total) < 4096 ? NA_INT : NA_FLOAT;
+}
+
+// One thread per pixel: rows of up to CAP events, each lane loading and
+// classifying its own; every other pixel gets zeros here, overwritten by the
+// kernels below.
+template <int CAP>
+__global__ void __launch_bounds__(MT_WARPS * 32, 8) k_na_thread(NaRows v) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  const int scr = ((const McPlan *)v.plan)->scr;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t *wbase = (uint32_t *)smem + (size_t)warp * (CAP + scr) * 32;
+  uint32_t *row = wbase + lane;
+  const int64_t p0 = ((int64_t)blockIdx.x * MT_WARPS + warp) * 32;
+  if (p0 >= v.P) return;
+  const int p = (int)p0 + lane;
+  int64_t b = 0;
+  int n = 0, n0 = 0, kinds = 0;
+  if (lane < v.P - p0 && !na_row(v, p, b, n)) atomicOr(v.status, 1);
+  if (n > CAP) {
+    kinds = n <= MT_WARP_CAP ? 1 : (n <= MT_MID_CAP ? 2 : (n <= MT_LONG_CAP ? 4 : NA_FLOAT));
+  } else if (n > 0) {
+    bool reg = true, integ = v.F <= 65536;
+    int total = 0, prev = -1;
+    for (int i0 = 0; i0 < n; i0 += 4) {
+      int f[4];
+      float x[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) {  // the loads first, in flight together
+        f[u] = i0 + u < n ? v.frame[b + i0 + u] : 0;
+        x[u] = i0 + u < n ? v.value[b + i0 + u] : 0.f;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        if (i0 + u >= n) break;
+        reg = reg && f[u] > prev && f[u] < v.F && fabsf(x[u]) < 0x1p126f;
+        integ = integ && x[u] == truncf(x[u]) && fabsf(x[u]) < 16777216.f;
+        total += integ ? (int)fminf(fabsf(x[u]), 4096.f) : 0;
+        row[(i0 + u) * 32] = pk(f[u], __float2int_rn(x[u]));
+        prev = f[u];
+      }
+    }
+    if (reg && integ && total < 4096)
+      n0 = n;
+    else
+      kinds = reg ? NA_FLOAT : NA_IRREGULAR;
+  }
+  kinds = __reduce_or_sync(0xffffffffu, (unsigned)kinds);
+  if (lane == 0 && kinds) atomicOr(v.status + 1, kinds);
+  __syncwarp();
+  mt_thread_rows<CAP>(v.plan, p, n0, v.G2, v.IP, v.IF, wbase);
+}
+
+// The pixels of a warp, NA_GRAB at a time from the counter `next`: calls
+// row(p, b, n) for those whose row has min_n < n <= max_n events.
+template <class Row>
+__device__ __forceinline__ void na_pixels(const NaRows &v, int32_t *next, int min_n, int max_n,
+                                          Row row) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int groups = v.P / NA_GRAB + (v.P % NA_GRAB != 0);
+  for (;;) {
+    int g = 0;
+    if (lane == 0) g = atomicAdd(next, 1);
+    g = __shfl_sync(FULL, g, 0);
+    if (g >= groups) break;
+    const int p0 = g * NA_GRAB;
+    int64_t b = 0;
+    int n = 0;
+    if (lane < min(NA_GRAB, v.P - p0)) na_row(v, p0 + lane, b, n);
+    unsigned m = __ballot_sync(FULL, n > min_n && n <= max_n);
+    while (m) {
+      const int l = __ffs(m) - 1;
+      m &= m - 1u;
+      row(p0 + l, __shfl_sync(FULL, b, l), __shfl_sync(FULL, n, l));
+      __syncwarp();
+    }
+  }
+}
+
+// One warp per pixel: integer rows of min_n < n <= cap events (kind bit
+// `kind`); rows that are not get their kind recorded for the kernels after.
+__global__ void __launch_bounds__(256)
+k_na_warp(NaRows v, int32_t kind, int32_t min_n, int32_t cap, int32_t *next) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  if (!(v.status[1] & kind)) return;
+  const McPlan *pl = (const McPlan *)v.plan;
+  const McArrays ar = mc_arrays(v.plan, pl->D);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int ACC = max(pl->acc, pl->nlev);
+  uint32_t *row = (uint32_t *)smem + (size_t)warp * (2 * cap + 32 * ACC);
+  int32_t *S = (int32_t *)(row + cap);
+  int32_t *acc = S + cap + lane;
+  na_pixels(v, next, min_n, cap, [&](int p, int64_t b, int n) {
+    const int c = na_class(v, b, n);
+    if (c != NA_INT) {
+      if (lane == 0) atomicOr(v.status + 1, c);
+      return;
+    }
+    mt_warp_pixel(pl, ar, p, b, n, v.frame, v.value, v.G2, v.IP, v.IF, cap, row, S, acc);
+  });
+}
+
+// One warp per pixel: float rows of any length.  It works on scratch copies
+// of its rows; a descending row pointer (reported by the thread kernel) can
+// make rows share scratch words, so the replay takes the float rows then.
+__global__ void __launch_bounds__(FW_WARPS * 32, 7) k_na_fwarp(NaRows v, int32_t *next) {
+  extern __shared__ __align__(16) uint8_t fw_smem[];
+  if (v.status[0] || !(v.status[1] & NA_FLOAT)) return;
+  const McPlan *pl = (const McPlan *)v.plan;
+  const McArrays ar = mc_arrays(v.plan, pl->D);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  uint8_t *wb = fw_smem + (size_t)w * fw_warp_bytes(pl->acc);
+  na_pixels(v, next, 0, INT_MAX, [&](int p, int64_t b, int n) {
+    const int c = na_class(v, b, n);
+    if (c == NA_IRREGULAR && lane == 0) atomicOr(v.status + 1, c);
+    if (c != NA_FLOAT) return;
+    fw_pixel(pl, ar, p, b, n, v.frame, v.value, nullptr, v.sc_frame + b, v.sc_val + b, v.G2, v.IP,
+             v.IF, wb);
+  });
 }
 
 // Host-side plan: level groups of the delay schedule with the lastframe each
@@ -1235,9 +1423,7 @@ void launch_float_rows(Series &s, const McPlan &hp, cudaStream_t st, int sms) {
     prepare_framesum_scale(s);
     fscale = s.d_fscale.p;
   }
-  int kmax = 0;
-  for (int g = 0; g < hp.nlev; g++) kmax = std::max(kmax, hp.lv[g].tau_lo + hp.lv[g].count - 1);
-  if (kmax <= FW_MAXC && hp.acc <= FW_MAXC) {
+  if (mt_float_rows_warp(hp)) {
     const size_t smf = FW_WARPS * fw_warp_bytes(hp.acc);
     XG_CUDA(cudaFuncSetAttribute(k_mt_fwarp, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smf));
@@ -1420,6 +1606,75 @@ void mt_queue_run(const std::vector<Series *> &ss, MtQueue &q, cudaStream_t st) 
     const McPlan hp = *(const McPlan *)make_plan(s, s.plan_mode).data();
     launch_float_rows(s, hp, st, sms);
   }
+}
+
+// Loads the kernels of mt_noalloc_rows on the current device and lifts their
+// shared-memory limit, so that later calls find them in place.
+cudaError_t mt_noalloc_setup() {
+  const void *k[] = {(const void *)k_na_thread<32>, (const void *)k_na_thread<80>,
+                     (const void *)k_na_warp, (const void *)k_na_fwarp};
+  for (const void *f : k) {
+    cudaFuncAttributes a;
+    cudaError_t e = cudaFuncGetAttributes(&a, f);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               227 * 1024 - (int)a.sharedSizeBytes);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
+// Whether the row kernels take the schedule: shared memory, at most 32 delays
+// a level (the warp kernels' lanes), consecutive delays and monotone
+// thresholds, as make_plan requires.
+bool mt_noalloc_supported(const McPlan &hp, const McArrays &ar) {
+  const int scr = std::max(hp.acc, hp.nlev);
+  if (hp.D <= 0 || hp.P > (1 << 30) || hp.acc > 32 || thread_smem(hp.scr, 80) > 227 * 1024 ||
+      warp_smem(0, scr, MT_WARP_CAP, WP_WARPS) > 227 * 1024 ||
+      warp_smem(0, scr, MT_MID_CAP, MID_WARPS) > 227 * 1024 ||
+      warp_smem(0, scr, MT_LONG_CAP, LONG_WARPS) > 227 * 1024)
+    return false;
+  for (int k = 1; k < hp.D; k++)
+    if (ar.t_ip[k] >= ar.t_ip[k - 1] || ar.tau_abs[k] <= ar.tau_abs[k - 1]) return false;
+  for (int g = 0; g < hp.nlev; g++) {
+    const McLevel &L = hp.lv[g];
+    if (g > 0 && L.t_end > hp.lv[g - 1].t_end) return false;
+    for (int k = 0; k < L.count; k++)
+      if (ar.tau_lvl[L.first + k] != L.tau_lo + k) return false;
+  }
+  return true;
+}
+
+// Whether float rows go to the warp-per-row kernel (else the replay).
+bool mt_float_rows_warp(const McPlan &hp) {
+  int kmax = 0;
+  for (int g = 0; g < hp.nlev; g++) kmax = std::max(kmax, hp.lv[g].tau_lo + hp.lv[g].count - 1);
+  return kmax <= FW_MAXC && hp.acc <= FW_MAXC;
+}
+
+// Enqueues the row kernels over the caller's rows: outputs of every regular
+// row (and zeros for the others); status[1] then holds the kinds of rows left.
+cudaError_t mt_noalloc_rows(const McPlan &hp, const NaRows &v, int sms, cudaStream_t st) {
+  const int scr = std::max(hp.acc, hp.nlev);
+  const unsigned blocks = (unsigned)(((int64_t)v.P + MT_WARPS * 32 - 1) / (MT_WARPS * 32));
+  // rows of about 1.5 times the mean fit the thread kernel (default_knobs has
+  // more steps; two keep the kernels loaded at set-up few)
+  const int cap = 1.5 * (double)v.events <= 32.0 * (double)v.P ? 32 : 80;
+  if (cap == 32)
+    k_na_thread<32><<<blocks, MT_WARPS * 32, thread_smem(hp.scr, 32), st>>>(v);
+  else
+    k_na_thread<80><<<blocks, MT_WARPS * 32, thread_smem(hp.scr, 80), st>>>(v);
+  const int tiers[3][3] = {{cap, MT_WARP_CAP, WP_WARPS},
+                           {MT_WARP_CAP, MT_MID_CAP, MID_WARPS},
+                           {MT_MID_CAP, MT_LONG_CAP, LONG_WARPS}};
+  for (int t = 0; t < 3; t++) {
+    const size_t sm = warp_smem(0, scr, tiers[t][1], tiers[t][2]);
+    k_na_warp<<<sms * std::max(1, (int)((227 * 1024) / sm)), tiers[t][2] * 32, sm, st>>>(
+        v, 1 << t, tiers[t][0], tiers[t][1], v.status + 2 + t);
+  }
+  if (mt_float_rows_warp(hp))
+    k_na_fwarp<<<sms * 7, FW_WARPS * 32, FW_WARPS * fw_warp_bytes(hp.acc), st>>>(v, v.status + 5);
+  return cudaGetLastError();
 }
 
 }  // namespace xg

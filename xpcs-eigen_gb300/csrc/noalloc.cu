@@ -10,9 +10,11 @@
 // working copy of the rows that the in-place level compaction destroys, and a
 // status word) is one file-scope __device__ array of fixed size.
 //
-// Every pixel is replayed with the reference's own float operations in its
-// order (the order-preserving path of k_multitau.cu), so the result is
-// bit-identical to xpcs_multitau2 for any input rows.
+// Rows whose frames ascend strictly and whose values are finite take the row
+// kernels of a series, which find and classify their rows themselves
+// (k_multitau.cu); any other row is replayed with the reference's own float
+// operations in its order.  The result is bit-identical to that replay, and
+// to xpcs_multitau2, for any input rows.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -56,35 +58,53 @@ __host__ __device__ inline NaView na_view(unsigned char *base) {
                           (size_t)NA_MAX_EVENTS * sizeof(int32_t))};
 }
 
-__global__ void __launch_bounds__(128)
-k_mt_float_noalloc(unsigned char *scratch, const int64_t *__restrict__ row_ptr,
-                   const int32_t *__restrict__ frame, const float *__restrict__ value,
-                   int32_t P, int64_t events, float *__restrict__ G2, float *__restrict__ IP,
-                   float *__restrict__ IF) {
-  const NaView v = na_view(scratch);
+// The rows the row kernels left, one thread per pixel.  mode 0: irregular
+// rows; 1: every row outside the integer class (schedules the float-row kernel
+// does not take, or row pointers that descend); 2: every row (schedules the
+// row kernels do not take).
+__global__ void __launch_bounds__(128) k_mt_float_noalloc(NaRows v, int32_t mode) {
+  if (mode == 0 && v.status[0]) mode = 1;  // the float-row kernel left its rows
+  if (mode < 2 && !(v.status[1] & (mode == 0 ? NA_IRREGULAR : NA_IRREGULAR | NA_FLOAT))) return;
   const McPlan *pl = (const McPlan *)v.plan;
-  const int D = pl->D;
+  const int D = pl->D, P = v.P;
   const McArrays ar = mc_arrays(v.plan, D);
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < P; p += gridDim.x * blockDim.x) {
-    const int64_t b = row_ptr[p];
-    const int64_t n64 = row_ptr[p + 1] - b;
-    if (b < 0 || n64 < 0 || b + n64 > events) {
+  for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < P;
+       q += (int64_t)gridDim.x * blockDim.x) {
+    const int p = (int)q;
+    const int64_t b = v.row_ptr[p], e = v.row_ptr[p + 1];
+    if (b < 0 || e < b || e > v.events) {
+      if (mode < 2) continue;  // reported and zeroed by the row kernels
       atomicOr(v.status, 1);
       for (int d = 0; d < D; d++) {
-        G2[(size_t)d * P + p] = 0.f;
-        IP[(size_t)d * P + p] = 0.f;
-        IF[(size_t)d * P + p] = 0.f;
+        v.G2[(size_t)d * P + p] = 0.f;
+        v.IP[(size_t)d * P + p] = 0.f;
+        v.IF[(size_t)d * P + p] = 0.f;
       }
       continue;
     }
-    const int n0 = (int)n64;
-    int32_t *idx = v.frame + b;
-    float *val = v.value + b;
-    for (int i = 0; i < n0; i++) {
-      idx[i] = frame[b + i];
-      val[i] = value[b + i];
+    const int n0 = (int)(e - b);
+    if (mode < 2) {  // the class the row kernels gave it
+      if (n0 == 0) continue;
+      bool reg = true, integ = v.F <= 65536 && n0 <= MT_LONG_CAP;
+      int64_t total = 0;
+      int32_t prev = -1;
+      for (int i = 0; i < n0 && reg; i++) {
+        const int32_t f = v.frame[b + i];
+        const float x = v.value[b + i];
+        reg = f > prev && f < v.F && fabsf(x) < 0x1p126f;
+        integ = integ && x == truncf(x) && fabsf(x) < 16777216.f;
+        if (integ) total += (int64_t)fabsf(x);
+        prev = f;
+      }
+      if (reg && (mode == 0 || (integ && total < 4096))) continue;
     }
-    replay_pixel(pl, ar, P, p, idx, val, n0, G2, IP, IF);
+    int32_t *idx = v.sc_frame + b;
+    float *val = v.sc_val + b;
+    for (int i = 0; i < n0; i++) {
+      idx[i] = v.frame[b + i];
+      val[i] = v.value[b + i];
+    }
+    replay_pixel(pl, ar, P, p, idx, val, n0, v.G2, v.IP, v.IF);
   }
 }
 
@@ -118,6 +138,7 @@ int na_build_plan(int32_t P, int32_t F, int32_t dpl, int32_t mode, uint8_t *buf,
   int32_t *tau_lvl = base;
   float *denom = (float *)(base + D);
   int32_t *tau_abs = base + 2 * D, *t_ip = base + 3 * D, *gi = base + 4 * D;
+  float *rcp = (float *)(base + 5 * D);
   pl->P = P;
   pl->D = D;
   pl->F = F;
@@ -141,6 +162,7 @@ int na_build_plan(int32_t P, int32_t F, int32_t dpl, int32_t mode, uint8_t *buf,
       tau_lvl[k] = tau;
       tau_abs[k] = tau_frames;
       denom[k] = (lastframe - tau) > 0 ? (float)(lastframe - tau) : 0.f;
+      rcp[k] = denom[k] > 0.f && lastframe - tau <= (1 << 24) ? recip_rn(lastframe - tau) : 0.f;
       t_ip[k] = (int32_t)std::max<int64_t>(0, (int64_t)(lastframe - tau) << level);
       if (level != prev_level) {
         if (nlev >= MAX_LEVELS) return -1;
@@ -162,7 +184,8 @@ int na_build_plan(int32_t P, int32_t F, int32_t dpl, int32_t mode, uint8_t *buf,
   }
   pl->nlev = nlev;
   pl->acc = 1;
-  pl->scr = nlev > 1 ? nlev : 1;
+  for (int g = 0; g < nlev; g++) pl->acc = std::max(pl->acc, pl->lv[g].count);
+  pl->scr = std::max(pl->acc, nlev) + (F >= 16384 ? 8 : 0);  // as default_knobs
   return D;
 }
 
@@ -207,6 +230,11 @@ extern "C" int xpcs_multitau2_noalloc(const int64_t *row_ptr, const int32_t *fra
                     "device (its first call loads the library's device code and reserves the "
                     "array; make that call at initialisation, with device memory to spare)");
       }
+      e = mt_noalloc_setup();
+      if (e != cudaSuccess) {
+        cudaGetLastError();
+        return fail(XPCS_ERR_CUDA, "xpcs_multitau2_noalloc: its kernels could not be loaded");
+      }
       g_na_ptr[dev] = (unsigned char *)ptr;
     }
     scratch = g_na_ptr[dev];
@@ -219,15 +247,26 @@ extern "C" int xpcs_multitau2_noalloc(const int64_t *row_ptr, const int32_t *fra
                 "(XPCS_NOALLOC_MAX_DELAYS)");
   cudaStream_t st = (cudaStream_t)stream;
   const NaView v = na_view(scratch);
-  if (cudaMemsetAsync(v.status, 0, sizeof(int32_t), st) != cudaSuccess ||
-      cudaMemcpyAsync((void *)v.plan, plan, sizeof(plan), cudaMemcpyHostToDevice, st) != cudaSuccess)
+  if (cudaMemsetAsync(v.status, 0, 8 * sizeof(int32_t), st) != cudaSuccess ||
+      cudaMemcpyAsync((void *)v.plan, plan, mc_plan_bytes(D), cudaMemcpyHostToDevice, st) !=
+          cudaSuccess)
     return fail(XPCS_ERR_CUDA, "xpcs_multitau2_noalloc: copy to the scratch failed");
   if (D > 0) {
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int grid = std::max(1, std::min((pixels + 127) / 128, std::max(sms, 1) * 8));
-    k_mt_float_noalloc<<<grid, 128, 0, st>>>(scratch, row_ptr, frame, value, pixels, events, G2,
-                                             IP, IF);
+    sms = std::max(sms, 1);
+    const McPlan &hp = *(const McPlan *)plan;
+    const NaRows rows{v.plan, row_ptr, frame, value, pixels, frames, events, v.status, v.frame,
+                      v.value, G2, IP, IF};
+    int mode = 2;
+    if (mt_noalloc_supported(hp, mc_arrays(plan, D))) {
+      mode = mt_float_rows_warp(hp) ? 0 : 1;
+      if (mt_noalloc_rows(hp, rows, sms, st) != cudaSuccess)
+        return fail(XPCS_ERR_CUDA, "xpcs_multitau2_noalloc: kernel launch failed");
+    }
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)pixels + 127) / 128,
+                                                                 sms * 8));
+    k_mt_float_noalloc<<<grid, 128, 0, st>>>(rows, mode);
     if (cudaGetLastError() != cudaSuccess)
       return fail(XPCS_ERR_CUDA, "xpcs_multitau2_noalloc: kernel launch failed");
   }

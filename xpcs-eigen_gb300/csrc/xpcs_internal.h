@@ -442,6 +442,25 @@ void reset_blocks(Series &s);
 void run_multitau(Series &s, int mode);                      // k_multitau.cu
 void run_normalize(Series &s, bool want64, bool want32);     // k_normalize.cu
 void build_norm_chunks(Series &s);                           // k_normalize.cu
+bool mt_float_rows_warp(const McPlan &hp);                    // k_multitau.cu
+// The rows of xpcs_multitau2_noalloc (k_multitau.cu): the caller's arrays and
+// the fixed scratch.  No allocation, no exception.
+enum : int32_t { NA_INT = 0, NA_FLOAT = 8, NA_IRREGULAR = 16 };  // kinds of rows in status[1]
+struct NaRows {
+  const uint8_t *plan;
+  const int64_t *row_ptr;
+  const int32_t *frame;
+  const float *value;
+  int32_t P, F;
+  int64_t events;
+  int32_t *status;  // [0] input error, [1] kinds of rows seen, [2 ..] pixel counters
+  int32_t *sc_frame;
+  float *sc_val;
+  float *G2, *IP, *IF;
+};
+cudaError_t mt_noalloc_setup();
+bool mt_noalloc_supported(const McPlan &hp, const McArrays &ar);
+cudaError_t mt_noalloc_rows(const McPlan &hp, const NaRows &v, int sms, cudaStream_t st);
 // The float nearest to 1/b (ties to even) for an integer b in [1, 2^24].
 float recip_rn(int32_t b);                                   // k_multitau.cu
 
