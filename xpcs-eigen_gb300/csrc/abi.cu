@@ -157,6 +157,9 @@ void free_series(Series *s) {
     s->d_mask.release(st);
     s->pclass.release(st);
     s->scan_tmp.release(st);
+    s->ft_slots.release(st);
+    s->ft_list.release(st);
+    s->ft_out.release(st);
     s->plan.release(st);
     s->d_flat.release(st);
     s->n_part.release(st);
@@ -340,7 +343,7 @@ int xpcs_series_get_info(xpcs_series *h, xpcs_series_info *info) {
       XG_CUDA(cudaMemcpy(&st, s.stats.p, sizeof(st), cudaMemcpyDeviceToHost));
       info->events = (int64_t)st.events;
       info->valid_pixels = st.nvalid;
-      info->float_path_pixels = st.nfloat;
+      info->float_path_pixels = st.nfloat + st.nfthread;
     }
   });
 }

@@ -26,6 +26,7 @@ __device__ __forceinline__ void record_class_warp(bool has, int32_t p, uint8_t c
   const unsigned mw = __ballot_sync(FULL, live && c == PCLASS_WARP);
   const unsigned ml = __ballot_sync(FULL, live && c == PCLASS_LONG);
   const unsigned mf = __ballot_sync(FULL, live && c == PCLASS_FLOAT);
+  const unsigned mt = __ballot_sync(FULL, live && c == PCLASS_FTHREAD);
   const unsigned ev = __reduce_add_sync(FULL, live ? (unsigned)n : 0u);
   int bw = 0, bl = 0, bf = 0;
   if (lane == 0) {
@@ -33,6 +34,7 @@ __device__ __forceinline__ void record_class_warp(bool has, int32_t p, uint8_t c
       atomicAdd(&stats->nvalid, __popc(mv));
       atomicAdd(&stats->events, (unsigned long long)ev);
     }
+    if (mt) atomicAdd(&stats->nfthread, __popc(mt));
     if (mw) bw = atomicAdd(&stats->nwarp, __popc(mw));
     if (ml) bl = atomicAdd(&stats->nlong, __popc(ml));
     if (mf) bf = atomicAdd(&stats->nfloat, __popc(mf));

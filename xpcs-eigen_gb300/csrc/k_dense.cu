@@ -507,7 +507,7 @@ __global__ void k_px_totals(int32_t P, int32_t nblk, const int32_t *__restrict__
 constexpr int KB_VT = 128;  // raw values from a pixel's threshold up in its value table
 
 struct PxGather {
-  int32_t P, F, tcap, force_float, nblk, has_dark;
+  int32_t P, F, tcap, fcap, force_float, nblk, has_dark;
   const int64_t *blk_base;
   const int32_t *blk_r0, *blk_off, *blk_len;
   const uint32_t *pk;
@@ -608,6 +608,7 @@ k_dense_gather_px(PxGather g) {
     uint8_t c = has && g.mask[p] ? pixel_class(n, s_nonint[lane] == 0, s_tot[lane], g.F, g.tcap)
                                  : (uint8_t)PCLASS_EMPTY;
     if (g.force_float && c != PCLASS_EMPTY) c = PCLASS_FLOAT;  // values rescaled later
+    c = float_class(c, n, g.fcap);
     record_class_warp(has, p, c, n, g.pclass, g.cl, g.stats);
   }
 }
@@ -786,7 +787,7 @@ void dense_px_gather(Series &s) {
     XG_CUDA(cudaMemsetAsync(s.blk_tot.p, 0, sizeof(int32_t) * (size_t)P, st));
   }
   exclusive_scan_i32_i64(s.blk_tot.p, s.row_ptr.p, P, s.scan_tmp.p, st);
-  PxGather g{P, s.F, s.thread_cap, s.desc.normalize_by_framesum, nblk, s.has_dark ? 1 : 0,
+  PxGather g{P, s.F, s.thread_cap, s.float_cap, s.desc.normalize_by_framesum, nblk, s.has_dark ? 1 : 0,
              s.d_blk_base.p, s.d_blk_r0.p, s.blk_off.p, s.blk_len.p, s.blk_pk.p, s.row_ptr.p,
              s.d_mask.p, s.rmin.p, s.dark_avg.p, s.has_flat ? s.d_flat.p : nullptr,
              (const DensePrep *)s.dn_prep.p, s.ev_frame.p, s.ev_val.p, s.row_len.p, s.pclass.p,

@@ -161,12 +161,13 @@ __device__ __forceinline__ void bins_pairs(const uint32_t *row, int m, int lf, i
     if (k < count) acc[k * 32] = a[k];
 }
 
-// The 32 consecutive pixels of a warp (this lane's is p, possibly past P),
-// each lane's row of n0 events packed in its column of wbase, the warp's (CAP
+// The 32 consecutive pixels of a warp (this lane's is p; mine: its outputs are
+// written here, zeros for a row of 0 events), each lane's row of n0 events packed in its column of wbase, the warp's (CAP
 // + scratch words) x 32 words of shared memory: the body of the
 // thread-per-pixel kernels after the rows are loaded.
 template <int CAP>
 __device__ __forceinline__ void mt_thread_rows(const uint8_t *__restrict__ plan_g, int p, int n0,
+                                               bool mine,
                                                float *__restrict__ G2, float *__restrict__ IP,
                                                float *__restrict__ IF, uint32_t *wbase) {
   // the plan is read from global memory: every lane of a warp reads the same
@@ -247,7 +248,7 @@ __device__ __forceinline__ void mt_thread_rows(const uint8_t *__restrict__ plan_
             }
           }
           // lanes without a row of this kernel have n0 = 0: both numerators are 0
-          if (p < P) {
+          if (mine) {
             const size_t o = (size_t)(d0 + k) * P + p;
             IP[o] = scaled_quotient_nb(total - rsum, lvl, den, rc);
             IF[o] = scaled_quotient_nb(s_end - ssum, lvl, den, rc);
@@ -361,7 +362,7 @@ __device__ __forceinline__ void mt_thread_rows(const uint8_t *__restrict__ plan_
       }
       for (int k = 0; k < nd; k++) {
         const float den = __shfl_sync(0xffffffffu, den_l, k), rc = __shfl_sync(0xffffffffu, rc_l, k);
-        if (p < P)
+        if (mine)
           G2[(size_t)(d0 + k) * P + p] =
               scaled_quotient_nb(acc[(d0 - L.first + k) * 32], 2 * L.level, den, rc);
       }
@@ -385,8 +386,19 @@ __device__ __forceinline__ void mt_thread_warp(const uint8_t *__restrict__ plan_
   const int P = ((const McPlan *)plan_g)->P, lane = threadIdx.x & 31;
   if (p0 >= P) return;
   const int p = p0 + lane;
-  const bool mine = p < P && pclass[p] == PCLASS_THREAD;
-  const int n0 = mine ? row_len[p] : 0;
+  const int c = p < P ? pclass[p] : PCLASS_FTHREAD;
+  const bool mine = c != PCLASS_FTHREAD;  // those are written by k_mt_fthread
+  if (!__any_sync(0xffffffffu, mine)) return;
+  const int n0 = c == PCLASS_THREAD ? row_len[p] : 0;
+  if (!__any_sync(0xffffffffu, n0 > 0)) {  // zeros only
+    if (!mine) return;
+    const int D = ((const McPlan *)plan_g)->D;
+    for (int d = 0; d < D; d++) {
+      const size_t o = (size_t)d * P + p;
+      G2[o] = IP[o] = IF[o] = 0.f;
+    }
+    return;
+  }
 
   // cooperative, coalesced load of the warp's rows (consecutive pixels have
   // consecutive rows), scattered to the owning lane's slots; four chunks of
@@ -428,7 +440,7 @@ __device__ __forceinline__ void mt_thread_warp(const uint8_t *__restrict__ plan_
     }
   }
   __syncwarp();
-  mt_thread_rows<CAP>(plan_g, p, n0, G2, IP, IF, wbase);
+  mt_thread_rows<CAP>(plan_g, p, n0, mine, G2, IP, IF, wbase);
 }
 
 template <int CAP>
@@ -1253,7 +1265,7 @@ __global__ void __launch_bounds__(MT_WARPS * 32, 8) k_na_thread(NaRows v) {
   kinds = __reduce_or_sync(0xffffffffu, (unsigned)kinds);
   if (lane == 0 && kinds) atomicOr(v.status + 1, kinds);
   __syncwarp();
-  mt_thread_rows<CAP>(v.plan, p, n0, v.G2, v.IP, v.IF, wbase);
+  mt_thread_rows<CAP>(v.plan, p, n0, lane < v.P - p0, v.G2, v.IP, v.IF, wbase);
 }
 
 // The pixels of a warp, NA_GRAB at a time from the counter `next`: calls
@@ -1323,6 +1335,380 @@ __global__ void __launch_bounds__(FW_WARPS * 32, 7) k_na_fwarp(NaRows v, int32_t
     fw_pixel(pl, ar, p, b, n, v.frame, v.value, nullptr, v.sc_frame + b, v.sc_val + b, v.G2, v.IP,
              v.IF, wb);
   });
+}
+
+// ---------------------------------------------- float rows, thread per pixel
+//
+// The same float sums with one pixel per thread, for rows of up to
+// Series::float_cap events.  A warp takes 32 rows of about the same length
+// (k_ft_sort) and keeps them in a scratch slot of its own in device memory
+// (L2 for the usual rows), entry-interleaved: entry j of every lane is one
+// coalesced 256-byte line of (bin, value) pairs, and the warp walks j in
+// lockstep, the loads two entries ahead.  One pass per
+// level forms the level's sums and, in the same step, writes the next level's
+// compacted row in place, exactly as the reference leaves it (stale tail
+// included).  A 32-bit mask of the bins before the current one (bit d - 1: an
+// entry d bins back) tells which delays have a partner that ends in it, and a
+// ring of the last 16 values in shared memory holds those partners, so that
+// every delay's sum takes its products in the order of the reference (by the
+// earlier entry, which is also the order of the later one).  The IF sums
+// start at their first entry; the IP sums are one running sum, read off where
+// it passes each delay's threshold.
+// Bound by instruction issue (about 94 k warp instructions for 32 rows of 154
+// events, 60 % issue) and, where the slots outgrow the L2, by their traffic.
+// Measured against the warp-per-row kernel, which spends about 430 warp
+// instructions on 32 entries of one row (float rows as a whole, ms):
+//   dense  960^2 x 2,000 frames, 154 events a row   11.15 -> 4.53
+//   dense  640^2 x 4,000, 294                        8.28 -> 4.58
+//   flat   509 x 387 x 1,500, 58                     1.72 -> 0.72
+//   flat   1024^2 x 1,000, 9                         5.45 -> 1.64
+constexpr int FT_WARPS = 4;
+constexpr int FT_AHEAD = 2;  // entries loaded ahead
+constexpr int FT_PREF = 4;   // entries fetched into L1 ahead
+constexpr double FT_MEAN_MAX = 2000.0;                   // longest mean row it is used for
+constexpr double FT_PIX_FACTOR = 1.4e-5;                 // rows of up to this x pixels means
+constexpr size_t FT_SLOT_BYTES = (size_t)3 << 30;        // most device memory of the slots
+constexpr int FT_WIN_PIX = 4096;  // pixels sorted by row length together
+constexpr int FT_TILE = 33;  // row of the 32 x 32 staging tile, padded
+constexpr int FT_MAXC = 16;  // delays per level, and the ring's entries
+constexpr int FT_MAXD = 16;  // largest delay in bins: the partners are among the last 16 entries
+
+// Shared memory of a warp: the staging tiles while the rows are loaded, then
+// the ring (each value at slots j & 15 and 16 + (j & 15), so that a partner's
+// predecessors lie below it) and the IP sums of a level.
+constexpr int FT_WORDS = 2 * 32 * FT_TILE;
+static_assert(FT_WORDS >= 3 * FT_MAXC * 32, "the ring and the IP sums reuse the staging tiles");
+
+struct FtState {
+  uint2 *S;          // this lane's column of the slot: entry j at S[j * 32]
+  float *ring, *ip;  // this lane's columns in shared memory
+  int n0, m;         // events of the row, entries of the level's prefix
+  bool tail_sorted;  // the buffer from m on ascends
+  bool sorted;       // the whole buffer ascends
+  int tail0;         // first bin of the tail
+
+  __device__ __forceinline__ int lower_bound(int x) const {  // libstdc++'s halving
+    int first = 0, len = n0;
+    while (len > 0) {
+      const int half = len >> 1;
+      if ((int)S[(first + half) * 32].x < x) {
+        first += half + 1;
+        len -= half + 1;
+      } else {
+        len = half;
+      }
+    }
+    return first;
+  }
+  // After the prefix of prev entries (last bin t_last) became `out` entries
+  // (last bin o_last) in place.
+  __device__ __forceinline__ void compacted(int prev, int t_last, int out, int o_last) {
+    const bool junction_ok = prev >= n0 || t_last <= (int)S[prev * 32].x;
+    m = out;
+    tail_sorted = tail_sorted && (m >= prev || junction_ok);
+    tail0 = m < n0 ? (int)S[m * 32].x : INT_MAX;
+    sorted = m == 0 || (tail_sorted && o_last <= tail0);
+  }
+};
+
+// One pass over the level's entries.  SUMS: the sums of cnt <= KM delays from
+// tlo on (lf: the level's lastframe); CHECK: an entry counts as a partner only
+// where the search over the whole buffer finds it; NEXT: the entries compacted
+// for the next level (lfn: its lastframe).
+template <int KM, bool SUMS, bool CHECK, bool NEXT>
+__device__ __forceinline__ void ft_pass(FtState &f, int lf, int tlo, int cnt, int lfn,
+                                        float (&g2)[KM], float (&iff)[KM]) {
+  const unsigned FULL = 0xffffffffu;
+  const int m = f.m, mmax = __reduce_max_sync(FULL, m);
+  const int thi = tlo + cnt - 1;
+  const uint32_t cmask = (1u << cnt) - 1u, gap = (1u << (tlo - 1)) - 1u;
+  float run = 0.f;
+  int kip = cnt - 1;       // IP sums of the delays above kip are read off
+  uint32_t before = 0u;    // bins before the previous entry's
+  int tp = 0;
+  int out = 0, ph = -1;    // next level: entries written, pending bin and value
+  float pv = 0.f;
+  uint2 pf[FT_AHEAD];
+#pragma unroll
+  for (int u = 0; u < FT_AHEAD; u++) pf[u] = u < m ? f.S[u * 32] : make_uint2(0u, 0u);
+  for (int j0 = 0; j0 < mmax; j0 += FT_AHEAD) {
+#pragma unroll
+    for (int u = 0; u < FT_AHEAD; u++) {
+      const int j = j0 + u;
+      const bool act = j < m;
+      const int t = act ? (int)pf[u].x : tp + 1;  // idle lanes: no partner, +0 to the sums
+      const float v = act ? __uint_as_float(pf[u].y) : 0.f;
+      if (FT_PREF && j + FT_PREF < m)
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(f.S + (j + FT_PREF) * 32));
+      if (j + FT_AHEAD < m) pf[u] = f.S[(j + FT_AHEAD) * 32];
+      if (SUMS) {
+        const int step = t - tp;
+        before = j == 0 || step > 32 ? 0u : ((before << 1 | 1u) << (step - 1));
+        uint32_t w = act ? (before >> (tlo - 1)) & cmask : 0u;
+        if (CHECK && w && !f.sorted && !(f.tail_sorted && t <= f.tail0) && f.lower_bound(t) != j)
+          w = 0u;
+        const float *pr = f.ring + (16 + ((j - 1 - __popc(before & gap)) & 15)) * 32;
+#pragma unroll
+        for (int k = 0; k < KM; k++) {
+          if (w & (1u << k)) {
+            g2[k] = __fadd_rn(g2[k], __fmul_rn(*pr, v));
+            pr -= 32;
+          }
+        }
+        f.ring[(j & 15) * 32] = v;
+        f.ring[(16 + (j & 15)) * 32] = v;
+        if (__all_sync(FULL, t >= thi)) {
+#pragma unroll
+          for (int k = 0; k < KM; k++) iff[k] = __fadd_rn(iff[k], v);
+        } else {
+#pragma unroll
+          for (int k = 0; k < KM; k++)
+            if (t >= tlo + k) iff[k] = __fadd_rn(iff[k], v);
+        }
+        while (act && kip >= 0 && t >= lf - tlo - kip) {
+          f.ip[kip * 32] = run;
+          kip--;
+        }
+        run = __fadd_rn(run, v);
+      }
+      if (NEXT && act) {
+        const int h = t >> 1;
+        if (h == ph) {
+          pv = __fadd_rn(pv, v);  // distinct frames: pairs at most
+        } else {
+          if (ph >= 0 && ph < lfn) {
+            f.S[out * 32] = make_uint2((uint32_t)ph, __float_as_uint(__fmul_rn(pv, 0.5f)));
+            out++;
+          }
+          ph = h;
+          pv = v;
+        }
+      }
+      tp = act ? t : tp;
+    }
+  }
+  if (SUMS)
+    for (; kip >= 0; kip--) f.ip[kip * 32] = run;
+  if (NEXT && m > 0) {
+    int o_last = -1;
+    if (ph < lfn) {
+      f.S[out * 32] = make_uint2((uint32_t)ph, __float_as_uint(__fmul_rn(pv, 0.5f)));
+      out++;
+      o_last = ph;
+    } else if (out > 0) {
+      o_last = (int)f.S[(out - 1) * 32].x;
+    }
+    f.compacted(m, tp, out, o_last);
+  }
+}
+
+template <int KM>
+__device__ __forceinline__ void ft_run_level(FtState &f, const McPlan *pl, const McArrays &ar,
+                                             int gi, bool ref, bool mine, float *out,
+                                             int32_t Dp) {
+  const McLevel L = pl->lv[gi];
+  const int lfn = gi + 1 < pl->nlev ? pl->lv[gi + 1].lastframe : 0;  // 0: nothing is kept
+  float g2[KM], iff[KM];
+#pragma unroll
+  for (int k = 0; k < KM; k++) g2[k] = iff[k] = 0.f;
+  if (gi > 0 && ref && __any_sync(0xffffffffu, !f.sorted)) {
+    // the search needs the buffer as it is: the sums first, then the compaction
+    ft_pass<KM, true, true, false>(f, L.lastframe, L.tau_lo, L.count, 0, g2, iff);
+    float none[1];
+    ft_pass<1, false, false, true>(f, 0, 1, 1, lfn, none, none);
+  } else {
+    ft_pass<KM, true, false, true>(f, L.lastframe, L.tau_lo, L.count, lfn, g2, iff);
+  }
+  if (!mine) return;
+  float ip[KM];
+#pragma unroll
+  for (int k = 0; k < KM; k++) {
+    const float den = k < L.count ? ar.denom[L.first + k] : 0.f;
+    ip[k] = k < L.count ? f.ip[k * 32] : 0.f;
+    if (den > 0.f) {
+      g2[k] = __fdiv_rn(g2[k], den);
+      ip[k] = __fdiv_rn(ip[k], den);
+      iff[k] = __fdiv_rn(iff[k], den);
+    }
+  }
+  float *o = out + L.first;
+  if (L.count == KM && KM % 4 == 0 && (L.first & 3) == 0) {  // the usual level: whole sectors
+#pragma unroll
+    for (int k = 0; k < KM; k += 4) {
+      *(float4 *)(o + k) = make_float4(g2[k], g2[k + 1], g2[k + 2], g2[k + 3]);
+      *(float4 *)(o + Dp + k) = make_float4(ip[k], ip[k + 1], ip[k + 2], ip[k + 3]);
+      *(float4 *)(o + 2 * Dp + k) = make_float4(iff[k], iff[k + 1], iff[k + 2], iff[k + 3]);
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < KM; k++) {
+      if (k >= L.count) break;
+      o[k] = g2[k];
+      o[Dp + k] = ip[k];
+      o[2 * Dp + k] = iff[k];
+    }
+  }
+}
+
+// The float rows of every window of FT_WIN_PIX pixels, longest first, into the
+// window's part of `list` (-1 past the last): a counting sort by length / 4.
+// A warp lasts as long as its longest row, and neighbouring pixels' rows can
+// differ tenfold (dense frames: each pixel's gain decides how much of the
+// noise passes its threshold).  The window is small enough for the partly
+// written output lines of the windows at work to stay in L2.
+__global__ void __launch_bounds__(256)
+k_ft_sort(int32_t P, const int32_t *__restrict__ row_len, const uint8_t *__restrict__ pclass,
+          int32_t *__restrict__ list) {
+  constexpr int NB = 1024, PER = FT_WIN_PIX / 256;
+  __shared__ int32_t cnt[NB];
+  __shared__ int32_t wsum[8];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t base = (int64_t)blockIdx.x * FT_WIN_PIX;
+  for (int k = threadIdx.x; k < NB; k += 256) cnt[k] = 0;
+  __syncthreads();
+  int bin[PER];
+#pragma unroll
+  for (int i = 0; i < PER; i++) {
+    const int64_t p = base + i * 256 + threadIdx.x;
+    bin[i] = -1;
+    if (p < P && pclass[p] == PCLASS_FTHREAD) {
+      bin[i] = max(0, NB - 1 - (row_len[p] >> 2));  // longest first
+      atomicAdd(&cnt[bin[i]], 1);
+    }
+  }
+  __syncthreads();
+  // exclusive scan of the NB counters, 4 per thread
+  int c[4], s = 0;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    c[k] = s;
+    s += cnt[threadIdx.x * 4 + k];
+  }
+  int x = s;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) wsum[w] = x;
+  __syncthreads();
+  int off = x - s, total = 0;
+  for (int k = 0; k < 8; k++) {
+    if (k < w) off += wsum[k];
+    total += wsum[k];
+  }
+#pragma unroll
+  for (int k = 0; k < 4; k++) cnt[threadIdx.x * 4 + k] = off + c[k];
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < PER; i++)
+    if (bin[i] >= 0) list[base + atomicAdd(&cnt[bin[i]], 1)] = (int32_t)(base + i * 256 + threadIdx.x);
+  for (int k = total + threadIdx.x; k < FT_WIN_PIX; k += 256) list[base + k] = -1;
+}
+
+// 32 entries of the sorted lists at a time, handed out per warp from a
+// counter; slots: `cap` lines of 32 entries for every warp of the grid.  KA /
+// KB: the most delays of level 0 and of the others.
+template <int KA, int KB>
+__global__ void __launch_bounds__(FT_WARPS * 32, 5)
+k_mt_fthread(const uint8_t *__restrict__ plan_g, int32_t cap, uint2 *__restrict__ slots,
+             const int32_t *__restrict__ list, const int64_t *__restrict__ row_ptr,
+             const int32_t *__restrict__ row_len, const int32_t *__restrict__ ev_frame,
+             const float *__restrict__ ev_val, const float *__restrict__ fscale,
+             DevStats *__restrict__ stats, int32_t Dp, float *__restrict__ stage) {
+  __shared__ float ft_sm[FT_WARPS][FT_WORDS];
+  const unsigned FULL = 0xffffffffu;
+  const McPlan *pl = (const McPlan *)plan_g;
+  const McArrays ar = mc_arrays(plan_g, pl->D);
+  const int P = pl->P, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const bool ref = pl->mode == XPCS_MODE_REFERENCE;
+  const int groups = (P + FT_WIN_PIX - 1) / FT_WIN_PIX * (FT_WIN_PIX / 32);
+  float *tf = ft_sm[w], *tv = tf + 32 * FT_TILE;
+  FtState f;
+  f.S = slots + ((size_t)blockIdx.x * FT_WARPS + w) * cap * 32 + lane;
+  f.ring = ft_sm[w] + lane;
+  f.ip = ft_sm[w] + 2 * FT_MAXC * 32 + lane;
+  for (;;) {
+    int g = 0;
+    if (lane == 0) g = atomicAdd(&stats->ftnext, 1);
+    g = __shfl_sync(FULL, g, 0);
+    if (g >= groups) break;
+    const int p = list[(size_t)g * 32 + lane];
+    const bool mine = p >= 0;
+    if (!__any_sync(FULL, mine)) continue;
+    f.n0 = f.m = mine ? row_len[p] : 0;
+    const int64_t b0 = mine ? row_ptr[p] : 0;
+    // 32 entries of every row at a time: read coalesced row by row into the
+    // padded tiles, then taken by the owning lanes
+    const int nmax = __reduce_max_sync(FULL, f.n0);
+    for (int e0 = 0; e0 < nmax; e0 += 32) {
+      __syncwarp();
+#pragma unroll 8
+      for (int q = 0; q < 32; q++) {
+        const int64_t bq = __shfl_sync(FULL, b0, q);
+        const bool in = e0 + lane < __shfl_sync(FULL, f.n0, q);
+        tf[q * FT_TILE + lane] = in ? __int_as_float(ev_frame[bq + e0 + lane]) : 0.f;
+        tv[q * FT_TILE + lane] = in ? ev_val[bq + e0 + lane] : 0.f;
+      }
+      __syncwarp();
+#pragma unroll 4
+      for (int s = 0; s < 32; s++) {
+        const uint32_t fr = __float_as_uint(tf[lane * FT_TILE + s]);
+        float v = tv[lane * FT_TILE + s];
+        if (e0 + s < f.n0) {
+          // normalize_by_framesum: v / (frameSum[f] / mean) (main.cpp:330-333)
+          if (fscale) v = __fdiv_rn(v, fscale[fr]);
+          f.S[(e0 + s) * 32] = make_uint2(fr, __float_as_uint(v));
+        }
+      }
+    }
+    __syncwarp();
+    f.tail_sorted = f.sorted = true;
+    f.tail0 = INT_MAX;
+    float *out = stage + (mine ? (size_t)p * 3 * Dp : 0);
+    ft_run_level<KA>(f, pl, ar, 0, ref, mine, out, Dp);
+    for (int gi = 1; gi < pl->nlev; gi++) ft_run_level<KB>(f, pl, ar, gi, ref, mine, out, Dp);
+    __syncwarp();
+  }
+}
+
+// The kernel's results [pixel][G2, IP, IF][Dp] into G2 / IP / IF [D][P]: 32 x
+// 32 tiles through shared memory.  A warp's lanes hold pixels from all over
+// their window, and storing each delay's 32 values where they belong took 1.8
+// of 5.6 ms (960 x 960 pixels, 70 delays); with whole sectors per pixel and
+// this pass over them (0.41 ms) all of it takes 4.5 ms.
+__global__ void __launch_bounds__(256)
+k_ft_out(int32_t P, int32_t D, int32_t Dp, const uint8_t *__restrict__ pclass,
+         const float *__restrict__ stage, float *__restrict__ G2, float *__restrict__ IP,
+         float *__restrict__ IF) {
+  __shared__ float tile[8][32][33];  // a warp each: no barrier, all loads in flight
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int p0 = blockIdx.x * 32;
+  const bool mine = p0 + lane < P && pclass[p0 + lane] == PCLASS_FTHREAD;
+  const unsigned rows = __ballot_sync(FULL, mine);
+  if (!rows) return;
+  const float *src = stage + (size_t)p0 * 3 * Dp + lane;
+  for (int c0 = w * 32; c0 < 3 * Dp; c0 += 8 * 32) {
+    const bool in = c0 + lane < 3 * Dp;
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 32; q++)
+      tile[w][q][lane] = in && (rows >> q & 1u) ? src[(size_t)q * 3 * Dp + c0] : 0.f;
+    __syncwarp();
+    int which = c0 / Dp, d = c0 - which * Dp;
+#pragma unroll 8
+    for (int r = 0; r < 32; r++) {
+      if (mine && which < 3 && d < D) {
+        float *o = which == 0 ? G2 : (which == 1 ? IP : IF);
+        o[(size_t)d * P + p0 + lane] = tile[w][lane][r];
+      }
+      if (++d == Dp) {
+        d = 0;
+        which++;
+      }
+    }
+  }
 }
 
 // Host-side plan: level groups of the delay schedule with the lastframe each
@@ -1423,6 +1809,30 @@ void launch_float_rows(Series &s, const McPlan &hp, cudaStream_t st, int sms) {
     prepare_framesum_scale(s);
     fscale = s.d_fscale.p;
   }
+  XG_CUDA(cudaMemsetAsync(&s.stats.p->fnext, 0, 2 * sizeof(int32_t), st));  // and ftnext
+  if (s.float_cap) {
+    const auto kernel = s.desc.delays_per_level <= 4 ? k_mt_fthread<8, 4> : k_mt_fthread<16, 8>;
+    int per_sm = 0;
+    XG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, FT_WARPS * 32, 0));
+    // the slots of the grid within FT_SLOT_BYTES
+    const size_t block_bytes = (size_t)FT_WARPS * 32 * s.float_cap * sizeof(uint2);
+    per_sm = std::min(per_sm, (int)(FT_SLOT_BYTES / (block_bytes * (size_t)sms)));
+    const int windows = (P + FT_WIN_PIX - 1) / FT_WIN_PIX;
+    const int blocks = std::min(sms * std::max(1, per_sm), windows * (FT_WIN_PIX / 32 / FT_WARPS));
+    s.ft_slots.reserve(blocks * block_bytes, st);
+    s.ft_list.reserve((size_t)windows * FT_WIN_PIX, st);
+    const int Dp = (s.D + 3) & ~3;
+    s.ft_out.reserve((size_t)P * 3 * Dp, st);
+    k_ft_sort<<<windows, 256, 0, st>>>(P, s.row_len.p, s.pclass.p, s.ft_list.p);
+    XG_CHECK_LAUNCH();
+    kernel<<<blocks, FT_WARPS * 32, 0, st>>>(
+        s.plan.p, s.float_cap, (uint2 *)s.ft_slots.p, s.ft_list.p, s.row_ptr.p, s.row_len.p,
+        s.ev_frame.p, s.ev_val.p, fscale, s.stats.p, Dp, s.ft_out.p);
+    XG_CHECK_LAUNCH();
+    k_ft_out<<<(P + 31) / 32, 256, 0, st>>>(P, s.D, Dp, s.pclass.p, s.ft_out.p, s.G2.p, s.IP.p,
+                                            s.IF.p);
+    XG_CHECK_LAUNCH();
+  }
   if (mt_float_rows_warp(hp)) {
     const size_t smf = FW_WARPS * fw_warp_bytes(hp.acc);
     XG_CUDA(cudaFuncSetAttribute(k_mt_fwarp, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1430,7 +1840,6 @@ void launch_float_rows(Series &s, const McPlan &hp, cudaStream_t st, int sms) {
     int per_sm = 0;
     XG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mt_fwarp, FW_WARPS * 32,
                                                           smf));
-    XG_CUDA(cudaMemsetAsync(&s.stats.p->fnext, 0, sizeof(int32_t), st));
     k_mt_fwarp<<<sms * std::max(1, per_sm), FW_WARPS * 32, smf, st>>>(
         s.plan.p, s.flist.p, s.stats.p, s.row_ptr.p, s.row_len.p, s.ev_frame.p, s.ev_val.p,
         fscale, s.sc_frame.p, s.sc_val.p, s.G2.p, s.IP.p, s.IF.p);
@@ -1462,6 +1871,31 @@ float recip_rn(int32_t b) {
     }
   }
   return best;
+}
+
+// Row capacity of the thread-per-pixel float kernel.  It serves series whose
+// values are floats as a rule (flatfield, averaging, dense frames,
+// normalize_by_framesum) with at most 16 delays a level.  Longer rows go to
+// the warp-per-row kernel: one of them would keep a warp busy longer than the
+// rest of the series takes.  Dense frames' rows differ most (the threshold
+// passes much of some pixels' noise): at 960 x 960 x 2,000 frames the float
+// rows take 6.2 / 5.6 / 5.1 / 4.5 / 4.5 ms with 2 / 3 / 4 / 6 / 9 times the
+// mean; photon counting series do not depend on it (0.72 ms at 509 x 387 x
+// 1,500 frames from 2 to 9 times the mean).  The kernel's time is at least the
+// longest row's (about 1.1 us an event) and the other kernel's grows with all
+// events (0.08 ns each), so the longest row is limited to a multiple of the
+// mean that falls with the pixel count, and below 90,000 pixels the kernel is
+// not used: at 320 x 320 dense pixels, rows of 736 events, 6 times the mean
+// takes 6.0 ms, this rule 4.5 and the warp-per-row kernel alone 4.7.  Rows of
+// 4,000 events on average gain nothing any more (320^2 x 60,000 frames).
+int32_t mt_float_cap(const Series &s, double mean) {
+  if (!(s.has_flat || s.desc.avg_frames > 1 || s.desc.dense || s.desc.normalize_by_framesum))
+    return 0;
+  const int dpl = s.desc.delays_per_level;
+  if (s.D == 0 || dpl < 1 || 2 * dpl > FT_MAXC || mean > FT_MEAN_MAX) return 0;
+  static_assert(FT_MAXC == FT_MAXD, "a level's largest delay is at most 2 dpl bins");
+  const double factor = std::min(s.desc.dense ? 6.0 : 3.0, FT_PIX_FACTOR * s.P);
+  return factor < 1.25 ? 0 : (int32_t)std::min<double>(s.F, factor * mean + 64.0);
 }
 
 void run_multitau(Series &s, int mode) {

@@ -413,7 +413,8 @@ __device__ void merge_row(int32_t p, int32_t n, int64_t b, float favg, int32_t *
 // otherwise each lane merges its own row / sums it in frame order.  Pixels
 // outside the mask get empty rows.
 __global__ void __launch_bounds__(256, 6)
-k_merge_classify(int32_t P, int32_t F, int32_t avg, int32_t tcap, int32_t force_float,
+k_merge_classify(int32_t P, int32_t F, int32_t avg, int32_t tcap, int32_t fcap,
+                 int32_t force_float,
                  const int64_t *__restrict__ row_ptr, const uint8_t *__restrict__ mask,
                  int32_t *__restrict__ fr, float *__restrict__ val, int32_t *__restrict__ row_len,
                  uint8_t *__restrict__ pclass, ClassLists cl, float *__restrict__ pixels_sum,
@@ -516,6 +517,7 @@ k_merge_classify(int32_t P, int32_t F, int32_t avg, int32_t tcap, int32_t force_
   }
   uint8_t c = keep ? pixel_class(out, integral, total, F, tcap) : (uint8_t)PCLASS_EMPTY;
   if (force_float && c != PCLASS_EMPTY) c = PCLASS_FLOAT;  // values rescaled after the filter
+  c = float_class(c, out, fcap);
   record_class_warp(has, p, c, out, pclass, cl, stats);
 }
 
@@ -724,7 +726,7 @@ void reserve_lists(Series &s) {
 void merge_classify(Series &s, int32_t avg) {
   const int pix_per_block = 256;
   k_merge_classify<<<(s.P + pix_per_block - 1) / pix_per_block, 256, 0, s.stream>>>(
-      s.P, s.F, avg, s.thread_cap, s.desc.normalize_by_framesum, s.row_ptr.p, s.d_mask.p,
+      s.P, s.F, avg, s.thread_cap, s.float_cap, s.desc.normalize_by_framesum, s.row_ptr.p, s.d_mask.p,
       s.ev_frame.p, s.ev_val.p, s.row_len.p, s.pclass.p,
       ClassLists{s.wlist.p, s.llist.p, s.flist.p}, s.pixels_sum.p, s.stats.p);
   XG_CHECK_LAUNCH();
@@ -894,13 +896,16 @@ void reset_blocks(Series &s) {
 // rows of 25, 52 and 100 events (1 Mi pixels, 5,000-20,000 frames), and the
 // extra scratch words it picks from 16,384 frames on.
 void default_knobs(Series &s) {
-  if (s.knobs_set) return;
   if (s.valid_pixels < 0) {
     s.valid_pixels = 0;
     for (uint8_t v : s.qmap.valid) s.valid_pixels += v;
   }
   const double mean =
       (double)s.raw_events / ((double)std::max<int64_t>(s.valid_pixels, 1) * s.R_in);
+  // raw events of a row that the filter uses: the stride's skipped sub-frames
+  // are among a sparse series' events
+  s.float_cap = mt_float_cap(s, mean * s.R_in / (s.desc.dense ? 1 : s.desc.stride_frames));
+  if (s.knobs_set) return;
   int32_t cap = MT_THREAD_CAPS[MT_THREAD_NCAPS - 1];
   for (int c : MT_THREAD_CAPS)
     if (c >= 1.5 * mean) {

@@ -170,7 +170,7 @@ constexpr int MT_THREAD_CAP_DEFAULT = 80;
 constexpr int MT_WARP_CAP = 256;
 constexpr int MT_LONG_CAP = 4096;  // an integer row with sum |v| < 4096 has fewer non-zero events
 enum : uint8_t { PCLASS_EMPTY = 0, PCLASS_THREAD = 1, PCLASS_WARP = 2, PCLASS_FLOAT = 3,
-                 PCLASS_LONG = 4 };
+                 PCLASS_LONG = 4, PCLASS_FTHREAD = 5 };
 
 __host__ __device__ inline uint8_t pixel_class(int n, bool integral, long long total, int F,
                                                int thread_cap) {
@@ -182,6 +182,10 @@ __host__ __device__ inline uint8_t pixel_class(int n, bool integral, long long t
   if (n <= MT_LONG_CAP) return PCLASS_LONG;
   return PCLASS_FLOAT;
 }
+// A float row by length: the thread-per-pixel float kernel's share.
+__host__ __device__ inline uint8_t float_class(uint8_t c, int n, int float_cap) {
+  return c == PCLASS_FLOAT && n <= float_cap ? (uint8_t)PCLASS_FTHREAD : c;
+}
 
 // Counters written by device passes.
 struct DevStats {
@@ -190,7 +194,8 @@ struct DevStats {
   int32_t nvalid;
   int32_t nwarp;
   int32_t nlong;
-  int32_t fnext;  // next float-path pixel to hand out (k_mt_fwarp)
+  int32_t nfthread;  // float rows of the thread-per-pixel float kernel
+  int32_t fnext, ftnext;  // ftnext: next 32 pixels of k_mt_fthread; fnext: next float-path pixel to hand out (k_mt_fwarp)
   unsigned long long events;
   unsigned long long dropped;  // K-a items sorted last (unused frames, bad pixel indices)
 };
@@ -299,6 +304,9 @@ struct Series {
   DBuf<float> d_fscale;     // normalize_by_framesum: per-frame divisor frameSum/mean
   DBuf<int32_t> sc_frame;   // float-path scratch rows
   DBuf<float> sc_val;
+  DBuf<uint8_t> ft_slots;   // thread-per-pixel float kernel: its warps' row slots
+  DBuf<int32_t> ft_list;    // its pixels, sorted by row length in windows
+  DBuf<float> ft_out;       // its results, pixel by pixel
   DBuf<uint8_t> scan_tmp;
   DBuf<DevStats> stats;
 
@@ -306,6 +314,7 @@ struct Series {
   DBuf<uint8_t> plan;       // McPlan + tau_lvl[D] + denom[D]
   int32_t plan_mode = -1;   // mode of the plan in `plan` (-1: none uploaded)
   int32_t thread_cap = MT_THREAD_CAP_DEFAULT;  // rows up to this length: thread per pixel
+  int32_t float_cap = 0;    // float rows up to this length: thread per pixel (default_knobs)
   int32_t scr_extra = 0;    // scratch words beyond max(delays of a level, levels)
   int32_t radix_ipt = 0;    // transpose items per lane (event tile / 256); 0: by series size
   int32_t plan_scr = -1;    // scratch words of the uploaded plan
@@ -443,6 +452,9 @@ void run_multitau(Series &s, int mode);                      // k_multitau.cu
 void run_normalize(Series &s, bool want64, bool want32);     // k_normalize.cu
 void build_norm_chunks(Series &s);                           // k_normalize.cu
 bool mt_float_rows_warp(const McPlan &hp);                    // k_multitau.cu
+// Longest row of the thread-per-pixel float kernel for a series whose rows
+// hold `mean` events on average, 0 for no row at all.
+int32_t mt_float_cap(const Series &s, double mean);           // k_multitau.cu
 // The rows of xpcs_multitau2_noalloc (k_multitau.cu): the caller's arrays and
 // the fixed scratch.  No allocation, no exception.
 enum : int32_t { NA_INT = 0, NA_FLOAT = 8, NA_IRREGULAR = 16 };  // kinds of rows in status[1]
