@@ -6,27 +6,31 @@
 // range is cut into chunks of at most NCH pixels.
 //
 // float64 result (the reported one):
-//   k_norm_chunk   one block per (chunk, tau) reads G2/IP/IF of the chunk's
-//                  pixels once and produces, for the chunk: sum G2, sum IP,
-//                  sum IF, sum x and sum (x - mean_chunk)^2 with
-//                  x = G2 / (IP IF), NaN -> 0 and still counted (quirk Q8).
+//   k_norm_part    one warp per (chunk, NT delays) reads G2/IP/IF of the
+//                  chunk's pixels once and produces, per delay: sum G2, sum
+//                  IP, sum IF, sum (x - s) and sum (x - s)^2 with x = G2 / (IP
+//                  IF), NaN -> 0 and still counted (quirk Q8), and s the mean
+//                  of the chunk's first 32 ratios, so that the variance loses
+//                  nothing to cancellation and one pass suffices.
 //                  Per-element arithmetic is double-word ("float-float") on
 //                  the FP32 pipes -- TwoSum, FMA-based TwoProd, the quotient
 //                  of a float by a double-word, and Sum2 compensated sums of
-//                  Ogita, Rump & Oishi (2005) for the per-thread totals --
+//                  Ogita, Rump & Oishi (2005) for the per-lane totals --
 //                  because GB300's FP64 rate is a small fraction of its FP32
-//                  rate; the block reductions use the double-word addition of
-//                  Joldes, Muller & Popescu (ACM TOMS 2017), and the block
-//                  totals and everything after are FP64.
-//   k_norm_finish  one thread per (q, tau): entry ratio (G2/n)/((IP/n)(IF/n))
-//                  (:966-1013), g2 = mean of the non-NaN ratios (:1018-1040),
-//                  and the chunks' (n, mean, M2) merged in order with Chan's
-//                  pairwise update; stderr = sqrt(1/n) sqrt(M2/n) (:1043-1087).
+//                  rate; the sums over a warp use the double-word addition of
+//                  Joldes, Muller & Popescu (ACM TOMS 2017), and everything
+//                  after is FP64.
+//   k_norm_finish  one warp per (q, tau): entry ratio (G2/n)/((IP/n)(IF/n))
+//                  (:966-1013), g2 = mean of the non-NaN ratios (:1018-1040);
+//                  the ring's mean from the chunks' sums and its M2 as the sum
+//                  of every chunk's own and of n (chunk mean - mean)^2;
+//                  stderr = sqrt(1/n) sqrt(M2/n) (:1043-1087).
 // float32 result (optional, bit-identical to the reference's float output):
 //   k_f32_transpose / k_entry_f32 / k_q_f32 replay the reference's sequential
 //   float operations in its order, including the running-mean/M2 update of
 //   every pixel.
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "xpcs_internal.h"
@@ -34,9 +38,10 @@
 namespace xg {
 namespace {
 
-constexpr int NB = 256;          // threads per chunk block
-constexpr int NIPT = 16;         // pixels per thread
-constexpr int NCH = NB * NIPT;   // pixels per chunk
+constexpr int NT = 4;            // delays a warp takes together
+constexpr int NW = 4;            // warps per block
+constexpr int NPART = 6;         // doubles per (chunk, delay)
+constexpr int NCH_MIN = 128, NCH_MAX = 1024;  // pixels per chunk
 
 // ------------------------------------------------ double-word arithmetic
 
@@ -94,142 +99,244 @@ __device__ __forceinline__ void s2_add(sum2 &a, dw x) {
   a.c = __fadd_rn(a.c, x.l);
 }
 __device__ __forceinline__ dw s2_value(const sum2 &a) { return two_sum(a.s, a.c); }
-__device__ __forceinline__ dw dw_from_double(double x) {
-  float h = __double2float_rn(x);
-  return {h, __double2float_rn(x - (double)h)};
-}
 __device__ __forceinline__ double to_double(dw x) { return (double)x.h + (double)x.l; }
 
-// Block sum of N double-word values: warp reduction in double-word arithmetic
-// on the FP32 pipes, FP64 only for the per-warp partials, which thread 0 adds
-// up: out is valid in thread 0 only (FP64 runs at a small fraction of the FP32
-// rate here, so the other threads do not repeat those additions).
-template <int N>
-__device__ __forceinline__ void block_sum_dw(dw (&x)[N], double (&out)[N], double *sh) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-  for (int k = 0; k < N; k++)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      dw y{__shfl_down_sync(0xffffffffu, x[k].h, o), __shfl_down_sync(0xffffffffu, x[k].l, o)};
-      x[k] = dw_add(x[k], y);
-    }
-  if (lane == 0)
-#pragma unroll
-    for (int k = 0; k < N; k++) sh[k * (NB / 32) + w] = to_double(x[k]);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int k = 0; k < N; k++) {
-      double r = 0.0;
-#pragma unroll
-      for (int ww = 0; ww < NB / 32; ww++) r += sh[k * (NB / 32) + ww];
-      out[k] = r;
-    }
-  }
-  __syncthreads();
+__device__ __forceinline__ float rcp_approx(float b) {  // within 1 ulp
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
+  return r;
 }
 
-// part layout: [chunk][tau][5] = sum G2, sum IP, sum IF, sum x, M2 about the chunk mean
-__global__ void __launch_bounds__(NB)
-k_norm_chunk(int D, int P, const int32_t *__restrict__ ch_k0, const int32_t *__restrict__ ch_k1,
-             const int32_t *__restrict__ pix, const float *__restrict__ G2,
-             const float *__restrict__ IP, const float *__restrict__ IF, double *__restrict__ part) {
-  __shared__ double sh[4 * (NB / 32) + 1];
-  __shared__ float s_mean[2];
-  __shared__ float xh[NCH], xl[NCH];
-  const int c = blockIdx.x, t = blockIdx.y;
+// x = g / (a b) as a double-word, NaN -> 0.  The quotient of the approximate
+// reciprocal is corrected by two FMA residuals (relative error a few 2^-48);
+// quotients whose residuals could underflow, and non-finite ones, take the
+// general form.
+__device__ __forceinline__ dw ratio_dw(float g, float a, float b) {
+  const dw p = two_prod(a, b);
+  const float rb = rcp_approx(p.h);
+  const float q = __fmul_rn(g, rb);
+  const float r = __fmaf_rn(-q, p.l, __fmaf_rn(-q, p.h, g));
+  float ql = __fmul_rn(r, rb);
+  ql = __fmaf_rn(__fmaf_rn(-ql, p.h, r), rb, ql);
+  dw x = {q, ql};
+  const float aq = fabsf(q), ag = fabsf(g), ap = fabsf(p.h);
+  if (!(aq > 0x1p-60f && aq < 0x1p60f && ag > 0x1p-60f && ap > 0x1p-60f && ap < 0x1p60f)) {
+    x = g == 0.f ? dw{0.f, 0.f} : f_div_dw(g, p);
+    if (isnan(x.h) || isnan(x.l)) x = {0.f, 0.f};
+  }
+  return x;
+}
+
+// part layout: [chunk][tau][NPART] = sum G2, sum IP, sum IF, sum (x - s),
+// sum (x - s)^2, s.
+// Bound by instruction issue, about 120 instructions per element at 85-90 %
+// issue.  Against a block per (chunk of 4,096 pixels, delay) with the ratios
+// kept in shared memory for a second pass (168 instructions per element, a
+// quarter of them in the block's reductions): 1,024 x 1,024 pixels, 88 delays
+// 359 us instead of 602; 512 x 512, 34 delays 50 instead of 73.  Four delays
+// together share the pixel list and let one transposing reduction over the
+// warp sum all 20 values (21 double-word additions instead of 100).  The
+// largest relative error of stderr against FP64 over seven series was 1.9e-14
+// (3.5e-14 before), its rms 0.6 to 0.8 of what it was.
+__global__ void __launch_bounds__(NW * 32)
+k_norm_part(int D, int P, int NC, const int32_t *__restrict__ ch_k0,
+            const int32_t *__restrict__ ch_k1, const int32_t *__restrict__ pix,
+            const float *__restrict__ G2, const float *__restrict__ IP,
+            const float *__restrict__ IF, double *__restrict__ part) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int c = blockIdx.x * NW + (threadIdx.x >> 5), t0 = blockIdx.y * NT;
+  if (c >= NC) return;
   const int k0 = ch_k0[c], k1 = ch_k1[c];
-  const size_t o = (size_t)t * P;
-  sum2 sg{0.f, 0.f}, si{0.f, 0.f}, sf{0.f, 0.f}, sx{0.f, 0.f};
+  // the block's rows of the arrays: delays past the last one repeat it, unused
+  const float *rg[NT], *ra[NT], *rb[NT];
 #pragma unroll
-  for (int j = 0; j < NIPT; j++) {
-    const int k = k0 + j * NB + threadIdx.x;
-    if (k < k1) {
-      const int p = pix[k];
-      const float g = G2[o + p], a = IP[o + p], b = IF[o + p];
-      s2_add(sg, g);
-      s2_add(si, a);
-      s2_add(sf, b);
-      dw x = f_div_dw(g, two_prod(a, b));
-      if (isnan(x.h) || isnan(x.l)) x = {0.f, 0.f};
-      s2_add(sx, x);
-      xh[j * NB + threadIdx.x] = x.h;
-      xl[j * NB + threadIdx.x] = x.l;
+  for (int j = 0; j < NT; j++) {
+    const size_t o = (size_t)min(t0 + j, D - 1) * P;
+    rg[j] = G2 + o;
+    ra[j] = IP + o;
+    rb[j] = IF + o;
+  }
+  sum2 sg[NT], si[NT], sf[NT], sd[NT], sq[NT];
+  float s[NT];
+#pragma unroll
+  for (int j = 0; j < NT; j++) sg[j] = si[j] = sf[j] = sd[j] = sq[j] = {0.f, 0.f};
+  // the next 32 pixels' values are in flight while these are summed, their
+  // pixel indices one step earlier
+  float gn[NT], an[NT], bn[NT];
+  const auto load = [&](int p) {
+#pragma unroll
+    for (int j = 0; j < NT; j++) {
+      gn[j] = p >= 0 ? rg[j][(uint32_t)p] : 0.f;
+      an[j] = p >= 0 ? ra[j][(uint32_t)p] : 0.f;
+      bn[j] = p >= 0 ? rb[j][(uint32_t)p] : 0.f;
+    }
+  };
+  load(k0 + lane < k1 ? pix[k0 + lane] : -1);
+  int pn = k0 + 32 + lane < k1 ? pix[k0 + 32 + lane] : -1;
+  for (int k = k0; k < k1; k += 32) {
+    const bool in = k + lane < k1;
+    float g[NT], a[NT], b[NT];
+#pragma unroll
+    for (int j = 0; j < NT; j++) {
+      g[j] = gn[j];
+      a[j] = an[j];
+      b[j] = bn[j];
+    }
+    load(pn);
+    pn = k + 64 + lane < k1 ? pix[k + 64 + lane] : -1;
+    dw x[NT];
+#pragma unroll
+    for (int j = 0; j < NT; j++) x[j] = ratio_dw(g[j], a[j], b[j]);
+    if (k == k0) {  // the shift: the mean of the first ratios
+      const float n = (float)min(32, k1 - k0);
+#pragma unroll
+      for (int j = 0; j < NT; j++) {
+        float m = x[j].h;
+#pragma unroll
+        for (int w = 16; w > 0; w >>= 1) m = __fadd_rn(m, __shfl_xor_sync(FULL, m, w));
+        s[j] = __fdiv_rn(m, n);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < NT; j++) {
+      s2_add(sg[j], g[j]);
+      s2_add(si[j], a[j]);
+      s2_add(sf[j], b[j]);
+      if (in) {
+        const dw d0 = two_sum(x[j].h, -s[j]);
+        const float dl = __fadd_rn(d0.l, x[j].l);
+        s2_add(sd[j], dw{d0.h, dl});
+        const dw q = two_prod(d0.h, d0.h);
+        s2_add(sq[j], dw{q.h, __fmaf_rn(__fmul_rn(2.f, d0.h), dl, __fmaf_rn(dl, dl, q.l))});
+      }
     }
   }
-  const double n = (double)(k1 - k0);
-  dw parts[4] = {s2_value(sg), s2_value(si), s2_value(sf), s2_value(sx)};
-  double sums[4];
-  block_sum_dw<4>(parts, sums, sh);  // thread 0 holds the sums
-  if (threadIdx.x == 0) {
-    const dw mu = dw_from_double(sums[3] / n);
-    s_mean[0] = mu.h;
-    s_mean[1] = mu.l;
-  }
-  __syncthreads();
-  const float mh = -s_mean[0], ml = -s_mean[1];
-  sum2 m2{0.f, 0.f};
+  // sums over the warp: at each step a lane keeps one half of its values and
+  // hands the other to its partner, so that a lane ends with one value
+  constexpr int NV = 5 * NT;
+  static_assert(NV == 20, "the steps below halve 20 values");
+  dw v[NV + 1];
 #pragma unroll
-  for (int j = 0; j < NIPT; j++) {
-    const int k = k0 + j * NB + threadIdx.x;
-    if (k < k1) {
-      // d = x - mean as an exact high difference and a low remainder; d^2
-      // as the exact square of the high part and the rest by FMA
-      const dw d0 = two_sum(xh[j * NB + threadIdx.x], mh);
-      const float dl = __fadd_rn(__fadd_rn(d0.l, xl[j * NB + threadIdx.x]), ml);
-      const dw q = two_prod(d0.h, d0.h);
-      s2_add(m2, dw{q.h, __fmaf_rn(__fmul_rn(2.f, d0.h), dl, __fmaf_rn(dl, dl, q.l))});
+  for (int j = 0; j < NT; j++) {
+    v[5 * j] = s2_value(sg[j]);
+    v[5 * j + 1] = s2_value(si[j]);
+    v[5 * j + 2] = s2_value(sf[j]);
+    v[5 * j + 3] = s2_value(sd[j]);
+    v[5 * j + 4] = s2_value(sq[j]);
+  }
+  const auto halve = [&](auto cnt, int w) {
+    constexpr int n = decltype(cnt)::value, h = (n + 1) / 2;
+    const bool up = lane & w;
+    if (n & 1) v[n] = {0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < h; i++) {
+      const dw keep = up ? v[i + h] : v[i], send = up ? v[i] : v[i + h];
+      v[i] = dw_add(keep, dw{__shfl_xor_sync(FULL, send.h, w), __shfl_xor_sync(FULL, send.l, w)});
     }
-  }
-  dw mparts[1] = {s2_value(m2)};
-  double msum[1];
-  block_sum_dw<1>(mparts, msum, sh);
-  if (threadIdx.x == 0) {
-    double *q = part + ((size_t)c * D + t) * 5;
-    q[0] = sums[0];
-    q[1] = sums[1];
-    q[2] = sums[2];
-    q[3] = sums[3];
-    q[4] = msum[0];
-  }
+  };
+  halve(std::integral_constant<int, 20>{}, 16);
+  halve(std::integral_constant<int, 10>{}, 8);
+  halve(std::integral_constant<int, 5>{}, 4);
+  halve(std::integral_constant<int, 3>{}, 2);
+  halve(std::integral_constant<int, 2>{}, 1);
+  // the value this lane ended with: 20 -> 10 + 10 -> 5 + 5 -> 3 + 2 -> 2 + 1
+  // (2 + 0) -> 1 + 1
+  const int c4 = lane & 4 ? 2 : 3, c2 = lane & 2 ? c4 - 2 : 2;
+  const int id = (lane & 16 ? 10 : 0) + (lane & 8 ? 5 : 0) + (lane & 4 ? 3 : 0) +
+                 (lane & 2 ? 2 : 0) + (lane & 1);
+  const int t = t0 + id / 5;
+  if ((lane & 1) < c2 && t < D)
+    part[((size_t)c * D + t) * NPART + id % 5] = to_double(v[0]);
+#pragma unroll
+  for (int j = 0; j < NT; j++)
+    if (lane == j && t0 + j < D) part[((size_t)c * D + t0 + j) * NPART + 5] = (double)s[j];
 }
 
+__device__ __forceinline__ double warp_sum(double x) {
+#pragma unroll
+  for (int w = 16; w > 0; w >>= 1) x += __shfl_xor_sync(0xffffffffu, x, w);
+  return x;
+}
+
+// Five sums over the warp, the same in every lane: 8 FP64 additions by
+// halving the values as above (5 -> 3 + 2 -> 2 + 1 -> 1 + 1) instead of 25.
+__device__ __forceinline__ void warp_sum5(double (&v)[5]) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  double a[3], b[2];
+  const bool u16 = lane & 16, u8 = lane & 8, u4 = lane & 4;
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    const double hi = i < 2 ? v[i + 3] : 0.0;
+    a[i] = (u16 ? hi : v[i]) + __shfl_xor_sync(FULL, u16 ? v[i] : hi, 16);
+  }
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    const double hi = i < 1 ? a[2] : 0.0;
+    b[i] = (u8 ? hi : a[i]) + __shfl_xor_sync(FULL, u8 ? a[i] : hi, 8);
+  }
+  double c = (u4 ? b[1] : b[0]) + __shfl_xor_sync(FULL, u4 ? b[0] : b[1], 4);
+  c += __shfl_xor_sync(FULL, c, 2);
+  c += __shfl_xor_sync(FULL, c, 1);
+  v[0] = __shfl_sync(FULL, c, 0);
+  v[1] = __shfl_sync(FULL, c, 4);
+  v[2] = __shfl_sync(FULL, c, 8);
+  v[3] = __shfl_sync(FULL, c, 16);
+  v[4] = __shfl_sync(FULL, c, 20);
+}
+
+// One warp per (q, tau), lanes over the ring's chunks.  Bound by FP64 issue
+// (a division is some 25 instructions at 1/64 of the FP32 rate), so the
+// formulas keep the divisions to one per entry and three per ring.  One
+// thread merging the chunks in turn took 62 us at 18 rings x 88 delays and 40
+// at 9 x 34; 19 and 14 now.
 __global__ void k_norm_finish(int NQ, int D, const int32_t *__restrict__ qep,
                               const int32_t *__restrict__ qrow,
                               const int32_t *__restrict__ e_chunk_ptr,
                               const int32_t *__restrict__ ch_k0, const int32_t *__restrict__ ch_k1,
                               const double *__restrict__ part, double *__restrict__ g2,
                               double *__restrict__ se) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const int idx = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   if (idx >= NQ * D) return;
   const int qi = idx / D, t = idx - qi * D;
-  double gacc = 0.0, gcnt = 0.0;
-  double n = 0.0, mean = 0.0, M2 = 0.0;
+  double gacc = 0.0, n = 0.0, sx = 0.0;
+  int gcnt = 0;
   for (int e = qep[qi]; e < qep[qi + 1]; e++) {
-    double sg = 0.0, si = 0.0, sf = 0.0, ne = 0.0;
-    for (int c = e_chunk_ptr[e]; c < e_chunk_ptr[e + 1]; c++) {
-      const double *q = part + ((size_t)c * D + t) * 5;
+    double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // sum G2, IP, IF, x; pixels
+    for (int c = e_chunk_ptr[e] + lane; c < e_chunk_ptr[e + 1]; c += 32) {
+      const double *q = part + ((size_t)c * D + t) * NPART;
       const double nc = (double)(ch_k1[c] - ch_k0[c]);
-      sg += q[0];
-      si += q[1];
-      sf += q[2];
-      ne += nc;
-      // Chan et al.: merge (n, mean, M2) of the chunk into the running one
-      const double mc = q[3] / nc;
-      const double nn = n + nc;
-      const double delta = mc - mean;
-      mean = n == 0.0 ? mc : mean + delta * (nc / nn);
-      M2 = n == 0.0 ? q[4] : M2 + q[4] + delta * delta * (n * nc / nn);
-      n = nn;
+      v[0] += q[0];
+      v[1] += q[1];
+      v[2] += q[2];
+      v[3] += fma(nc, q[5], q[3]);
+      v[4] += nc;
     }
-    const double r = (sg / ne) / ((si / ne) * (sf / ne));
-    gacc += isnan(r) ? 0.0 : r;
-    gcnt += isnan(r) ? 0.0 : 1.0;
+    warp_sum5(v);
+    n += v[4];
+    sx += v[3];
+    const double r = v[0] * v[4] / (v[1] * v[2]);  // (G2/n) / ((IP/n) (IF/n))
+    if (!isnan(r)) {
+      gacc += r;
+      gcnt++;
+    }
   }
-  const int row = qrow[qi];
-  g2[(size_t)t * NQ + row] = gacc / gcnt;
-  se[(size_t)t * NQ + row] = sqrt(1.0 / n) * sqrt(M2 / n);
+  // sum (x - mean)^2 = sum (x - s)^2 + 2 (s - mean) sum (x - s) + n (s - mean)^2
+  const double mean = sx / n;
+  double M2 = 0.0;
+  for (int c = e_chunk_ptr[qep[qi]] + lane; c < e_chunk_ptr[qep[qi + 1]]; c += 32) {
+    const double *q = part + ((size_t)c * D + t) * NPART;
+    const double nc = (double)(ch_k1[c] - ch_k0[c]), d = q[5] - mean;
+    M2 += fma(d, fma(nc, d, 2.0 * q[3]), q[4]);
+  }
+  M2 = warp_sum(M2);
+  if (lane == 0) {
+    const int row = qrow[qi];
+    g2[(size_t)t * NQ + row] = gacc / (double)gcnt;
+    se[(size_t)t * NQ + row] = sqrt(M2) / n;  // sqrt(1/n) sqrt(M2/n)
+  }
 }
 
 // ------------------------------------------------ float32, reference order
@@ -520,13 +627,18 @@ __global__ void k_q_f32(int NQ, int D, int Dp, int FR_CH, const int32_t *__restr
 
 }  // namespace
 
+// Chunks of up to 1,024 pixels, smaller ones where those would leave fewer
+// than 16 warps per SM (152 SMs) for the series' pixels and delays.
 void build_norm_chunks(Series &s) {
   const QMap &q = s.qmap;
+  const double units = (double)q.pix.size() * ((s.D + NT - 1) / NT);
+  int nch = NCH_MAX;
+  while (nch > NCH_MIN && units / nch < 152.0 * 16) nch /= 2;
   std::vector<int32_t> k0, k1, eptr(1, 0);
   for (int e = 0; e < q.nentries(); e++) {
-    for (int a = q.entry_pix_ptr[e]; a < q.entry_pix_ptr[e + 1]; a += NCH) {
+    for (int a = q.entry_pix_ptr[e]; a < q.entry_pix_ptr[e + 1]; a += nch) {
       k0.push_back(a);
-      k1.push_back(std::min(a + NCH, q.entry_pix_ptr[e + 1]));
+      k1.push_back(std::min(a + nch, q.entry_pix_ptr[e + 1]));
     }
     eptr.push_back((int32_t)k0.size());
   }
@@ -550,14 +662,14 @@ void run_normalize(Series &s, bool want64, bool want32) {
     s.n_g2.reserve((size_t)NQ * D, st);
     s.n_se.reserve((size_t)NQ * D, st);
     const int NC = s.n_chunks;
-    s.n_part.reserve((size_t)(NC > 0 ? NC : 1) * D * 5, st);
+    s.n_part.reserve((size_t)(NC > 0 ? NC : 1) * D * NPART, st);
     if (NC > 0) {
-      k_norm_chunk<<<dim3(NC, D), NB, 0, st>>>(D, P, s.n_ch_k0.p, s.n_ch_k1.p, s.n_pix.p, s.G2.p,
-                                              s.IP.p, s.IF.p, s.n_part.p);
+      k_norm_part<<<dim3((NC + NW - 1) / NW, (D + NT - 1) / NT), NW * 32, 0, st>>>(
+          D, P, NC, s.n_ch_k0.p, s.n_ch_k1.p, s.n_pix.p, s.G2.p, s.IP.p, s.IF.p, s.n_part.p);
       XG_CHECK_LAUNCH();
     }
     const int bs = 128;
-    k_norm_finish<<<(NQ * D + bs - 1) / bs, bs, 0, st>>>(NQ, D, s.n_q_entry_ptr.p, s.n_q_row.p,
+    k_norm_finish<<<(unsigned)(((int64_t)NQ * D * 32 + bs - 1) / bs), bs, 0, st>>>(NQ, D, s.n_q_entry_ptr.p, s.n_q_row.p,
                                                         s.n_e_chunk_ptr.p, s.n_ch_k0.p,
                                                         s.n_ch_k1.p, s.n_part.p, s.n_g2.p,
                                                         s.n_se.p);
