@@ -374,151 +374,325 @@ __global__ void k_row_ptr(const uint32_t *__restrict__ keys, int64_t n,
   row_ptr[p] = first;
 }
 
-// Per-lane merge of one pixel's row: events of the same filter frame summed in
-// stream order as pixels_value_[pix] += v, then / avg (sparse_filter.cpp:
-// 146-172); pixelSum accumulated in frame order.
-__device__ void merge_row(int32_t p, int32_t n, int64_t b, float favg, int32_t *fr, float *val,
-                          int32_t &out, bool &integral, long long &total, float &psum) {
-  int32_t i = 0;
+// The events of one row (b, n) merged in place by a warp: events of the same
+// filter frame summed in stream order as pixels_value_[pix] += v, then / avg
+// (sparse_filter.cpp:146-172); psum: the merged values summed in frame order.
+// A group that reaches the end of a 32-event chunk stays open (its frame and
+// sum so far) until the next chunk.  The same results in every lane, except
+// total, which each lane holds its share of (saturating at 2^24).
+__device__ __forceinline__ void merge_row(int64_t b, int32_t n, float favg,
+                                          int32_t *__restrict__ fr, float *__restrict__ val,
+                                          int32_t &out, bool &integral, uint32_t &total,
+                                          float &psum) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
   out = 0;
   integral = true;
   total = 0;
   psum = 0.f;
-  while (i < n) {
-    int32_t f = fr[b + i];
-    float acc = 0.f;
-    do {
-      acc = __fadd_rn(acc, val[b + i]);
-      i++;
-    } while (i < n && fr[b + i] == f);
-    float x = __fdiv_rn(acc, favg);
-    fr[b + out] = f;
-    val[b + out] = x;
-    out++;
-    psum = __fadd_rn(psum, x);
-    if (integral) {
-      if (x == truncf(x) && fabsf(x) < 16777216.f)
-        total += llabs((long long)x);
-      else
-        integral = false;
+  int32_t cf = -1;  // the open group
+  float ca = 0.f;
+  const auto count = [&](float x, bool mine) {
+    if (!mine) return;
+    if (x == truncf(x) && fabsf(x) < 16777216.f)
+      total = min(total + (uint32_t)fabsf(x), 1u << 24);
+    else
+      integral = false;
+  };
+  int32_t f_nx = lane < n ? fr[b + lane] : -1;
+  float x_nx = lane < n ? val[b + lane] : 0.f;
+  for (int32_t i0 = 0; i0 < n; i0 += 32) {
+    const int32_t f = f_nx;
+    float x = x_nx;
+    const bool in = i0 + lane < n;
+    f_nx = i0 + 32 + lane < n ? fr[b + i0 + 32 + lane] : -1;
+    x_nx = i0 + 32 + lane < n ? val[b + i0 + 32 + lane] : 0.f;
+    const int cnt = min(32, n - i0);
+    // the open group's events at the chunk's start
+    const unsigned other = __ballot_sync(FULL, !in || f != cf);
+    const int lead = other ? __ffs(other) - 1 : 32;
+    for (int k = 0; k < lead; k++) ca = __fadd_rn(ca, __shfl_sync(FULL, x, k));
+    if (lead == cnt) continue;  // only possible with events left in the group or row
+    if (cf >= 0) {
+      const float v = __fdiv_rn(ca, favg);
+      if (lane == 0) {
+        fr[b + out] = cf;
+        val[b + out] = v;
+      }
+      count(v, lane == 0);
+      psum = __fadd_rn(psum, v);
+      out++;
     }
+    // groups that start in this chunk
+    const int32_t fp = __shfl_up_sync(FULL, f, 1);
+    const bool head = in && lane >= lead && (lane == lead || f != fp);
+    const unsigned heads = __ballot_sync(FULL, head);
+    const unsigned after = lane == 31 ? 0u : heads >> (lane + 1);
+    const int run = head ? (after ? __ffs(after) : cnt - lane) : 0;
+    const int longest = __reduce_max_sync(FULL, run);
+    float acc = __fadd_rn(0.f, x);
+    for (int k = 1; k < longest; k++) {
+      const float y = __shfl_down_sync(FULL, x, k);
+      if (k < run) acc = __fadd_rn(acc, y);
+    }
+    const int last = 31 - __clz(heads);  // stays open
+    cf = __shfl_sync(FULL, f, last);
+    ca = __shfl_sync(FULL, acc, last);
+    const unsigned done = heads & ~(1u << last);
+    const float v = __fdiv_rn(acc, favg);
+    const bool emit = done >> lane & 1u;
+    __syncwarp();
+    if (emit) {
+      const int32_t o = out + __popc(done & ((1u << lane) - 1u));
+      fr[b + o] = f;
+      val[b + o] = v;
+    }
+    count(v, emit);
+    for (unsigned m = done; m; m &= m - 1u)
+      psum = __fadd_rn(psum, __shfl_sync(FULL, v, __ffs(m) - 1));
+    out += __popc(done);
   }
+  if (cf >= 0) {
+    const float v = __fdiv_rn(ca, favg);
+    if (lane == 0) {
+      fr[b + out] = cf;
+      val[b + out] = v;
+    }
+    count(v, lane == 0);
+    psum = __fadd_rn(psum, v);
+    out++;
+  }
+  integral = __all_sync(FULL, integral);
 }
 
-// One warp per 32 consecutive pixels (their rows are contiguous): events are
-// read coalesced to detect duplicate frames and to collect, per pixel, whether
-// every value is an integer, sum |v| and sum v.  Without duplicates and with
-// avg == 1 the rows are final as sorted, and for integer rows with sum |v| <
-// 2^24 every float partial sum of pixelSum is exact, so pixelSum = (float)sum v;
-// otherwise each lane merges its own row / sums it in frame order.  Pixels
-// outside the mask get empty rows.
-__global__ void __launch_bounds__(256, 6)
-k_merge_classify(int32_t P, int32_t F, int32_t avg, int32_t tcap, int32_t fcap,
+constexpr int MC_WARPS = 4;             // warps per block of 32 pixels
+constexpr int MC_ROWS = 32 / MC_WARPS;  // rows per warp
+
+// Long rows, and rows to merge.  One block per 32 consecutive pixels, 8 rows
+// per warp, a warp's lanes over a row's events: repeated frames, whether every
+// value is an integer, sum |v| and sum v are found in one pass (the next
+// chunk, of this row or the next, in flight), reduced once per row.  Without
+// duplicates and with avg == 1 the row is final as sorted, and for integer
+// rows with sum |v| < 2^24 every float partial sum of pixelSum is exact, so
+// pixelSum = (float)sum v; otherwise the row is merged / summed in frame
+// order.  Pixels outside the mask get empty rows.  The block's first warp
+// classifies the 32 pixels.
+__global__ void __launch_bounds__(MC_WARPS * 32)
+k_merge_rows(int32_t P, int32_t F, int32_t avg, int32_t tcap, int32_t fcap,
                  int32_t force_float,
                  const int64_t *__restrict__ row_ptr, const uint8_t *__restrict__ mask,
                  int32_t *__restrict__ fr, float *__restrict__ val, int32_t *__restrict__ row_len,
                  uint8_t *__restrict__ pclass, ClassLists cl, float *__restrict__ pixels_sum,
                  DevStats *__restrict__ stats) {
-  __shared__ long long s_total[8][32];
-  __shared__ long long s_sum[8][32];
-  __shared__ int32_t s_nonint[8][32];
+  __shared__ int32_t s_len[32];
+  __shared__ uint8_t s_cls[32];
+  const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int p0 = (blockIdx.x * 8 + w) * 32;
+  const int pb = blockIdx.x * 32, p0 = pb + w * MC_ROWS;
+  int64_t my_b = 0;
+  int32_t my_n = 0;
+  if (lane < MC_ROWS && p0 + lane < P && mask[p0 + lane]) {
+    my_b = row_ptr[p0 + lane];
+    my_n = (int32_t)(row_ptr[p0 + lane + 1] - my_b);
+  }
+  if (lane < MC_ROWS) {  // rows without events
+    s_len[w * MC_ROWS + lane] = 0;
+    s_cls[w * MC_ROWS + lane] = PCLASS_EMPTY;
+    if (p0 + lane < P && my_n == 0) pixels_sum[p0 + lane] = 0.f;
+  }
+  __syncwarp();
+  unsigned rows = __ballot_sync(FULL, my_n > 0);
+  int q = rows ? __ffs(rows) - 1 : 0;
+  int64_t b = __shfl_sync(FULL, my_b, q);
+  int32_t n = __shfl_sync(FULL, my_n, q), i0 = 0;
+  int32_t f = lane < n ? fr[b + lane] : -1;
+  float x = lane < n ? val[b + lane] : 0.f;
+  int32_t last_f = -1;  // the previous chunk's last frame
+  bool dup = false, nonint = false;
+  uint32_t total = 0;  // this lane's share, saturating at 2^24
+  int32_t sum = 0;     // exact while the total is below 2^24
+  while (rows) {
+    const bool in = i0 + lane < n;
+    const int32_t fc = f;
+    const float xc = x;
+    const int32_t nc = n;
+    const int64_t bc = b;
+    const int qc = q;
+    const bool end = i0 + 32 >= n;  // the row's last chunk
+    i0 += 32;
+    if (end) {
+      rows &= rows - 1u;
+      q = rows ? __ffs(rows) - 1 : 0;
+      b = __shfl_sync(FULL, my_b, q);
+      n = rows ? __shfl_sync(FULL, my_n, q) : 0;
+      i0 = 0;
+    }
+    f = i0 + lane < n ? fr[b + i0 + lane] : -1;
+    x = i0 + lane < n ? val[b + i0 + lane] : 0.f;
+    int32_t fp = __shfl_up_sync(FULL, fc, 1);
+    if (lane == 0) fp = last_f;
+    if (in) {
+      dup = dup || fc == fp;
+      const bool ni = !(xc == truncf(xc) && fabsf(xc) < 16777216.f);
+      nonint = nonint || ni;
+      if (!ni) {
+        total = min(total + (uint32_t)fabsf(xc), 1u << 24);
+        sum += (int32_t)xc;
+      }
+    }
+    if (!end) {
+      last_f = __shfl_sync(FULL, fc, 31);
+      continue;
+    }
+    int32_t out = nc;
+    bool integral = !__any_sync(FULL, nonint);
+    float psum = 0.f;
+    if (__any_sync(FULL, dup) || avg != 1) {
+      merge_row(bc, nc, (float)avg, fr, val, out, integral, total, psum);
+      total = __reduce_add_sync(FULL, total);
+    } else {
+      total = __reduce_add_sync(FULL, total);
+      if (integral && total < 16777216u) {
+        psum = (float)__reduce_add_sync(FULL, sum);
+      } else {
+        for (int32_t j0 = 0; j0 < nc; j0 += 32) {
+          const float y = j0 + lane < nc ? val[bc + j0 + lane] : 0.f;
+          const int m = min(32, nc - j0);
+          if (m == 32) {
+#pragma unroll
+            for (int k = 0; k < 32; k++) psum = __fadd_rn(psum, __shfl_sync(FULL, y, k));
+          } else {
+            for (int k = 0; k < m; k++) psum = __fadd_rn(psum, __shfl_sync(FULL, y, k));
+          }
+        }
+      }
+    }
+    if (lane == 0) {
+      uint8_t c = pixel_class(out, integral, total, F, tcap);
+      if (force_float && c != PCLASS_EMPTY) c = PCLASS_FLOAT;  // values rescaled after the filter
+      s_len[w * MC_ROWS + qc] = out;
+      s_cls[w * MC_ROWS + qc] = float_class(c, out, fcap);
+      pixels_sum[p0 + qc] = psum;
+    }
+    last_f = -1;
+    dup = nonint = false;
+    total = 0;
+    sum = 0;
+  }
+  __syncthreads();
+  if (w == 0) {
+    const int p = pb + lane;
+    const bool has = p < P;
+    if (has) row_len[p] = s_len[lane];
+    record_class_warp(has, p, s_cls[lane], s_len[lane], pclass, cl, stats);
+  }
+}
+
+// Short rows.  One warp per 32 consecutive pixels, whose rows are contiguous:
+// tiles of 1,024 events are read coalesced, repeated frames are found between
+// neighbouring events (a bit per row start tells which neighbours share a
+// row), and the values go to shared memory, where each lane adds up its own
+// row in order: the running sum is pixelSum as the reference forms it, and
+// sum |v|, exact below 2^24, classifies the row.  A warp that finds a repeated
+// frame merges its rows one by one.  Pixels outside the mask get empty rows.
+// Bound by instruction issue, about 6 per event and row of a lane; a warp's
+// former walk of the events in chunks that straddle rows searched every
+// event's row and reduced three sums per run, 155 instructions a chunk (times
+// at merge_classify).
+constexpr int MS_TILE = 1024;
+constexpr int MS_WARPS = 8;
+constexpr double MS_MEAN_MAX = 256.0;  // see merge_classify
+__global__ void __launch_bounds__(MS_WARPS * 32)
+k_merge_short(int32_t P, int32_t F, int32_t tcap, int32_t fcap, int32_t force_float,
+              const int64_t *__restrict__ row_ptr, const uint8_t *__restrict__ mask,
+              int32_t *__restrict__ fr, float *__restrict__ val, int32_t *__restrict__ row_len,
+              uint8_t *__restrict__ pclass, ClassLists cl, float *__restrict__ pixels_sum,
+              DevStats *__restrict__ stats) {
+  __shared__ float s_val[MS_WARPS][MS_TILE];
+  __shared__ uint32_t s_start[MS_WARPS][MS_TILE / 32];
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int p0 = (blockIdx.x * MS_WARPS + w) * 32;
   if (p0 >= P) return;
   const int p = p0 + lane;
-  const bool has = p < P;
-  const int plast = min(p0 + 32, P);
-  const int64_t e0 = row_ptr[p0], e1 = row_ptr[plast];
+  const bool has = p < P, keep = has && mask[p] != 0;
+  const int64_t e0 = row_ptr[p0], e1 = row_ptr[min(p0 + 32, P)];
   const int64_t my_b = has ? row_ptr[p] : e1;
-  const int32_t my_n = has ? (int32_t)(row_ptr[p + 1] - my_b) : 0;
-  const bool keep = has && mask[p] != 0;
-  s_total[w][lane] = 0;
-  s_sum[w][lane] = 0;
-  s_nonint[w][lane] = 0;
-  __syncwarp();
-  bool dup = false;
-  // The chunks of the warp's rows, in positions relative to e0 of type T:
-  // 32-bit when the rows span less than 2^30 events (one shuffle and one
-  // compare per step of the owner search), else 64-bit.  Each 32-event chunk
-  // is loaded one chunk ahead; the previous chunk's last frame carries over
-  // to lane 0.
-  auto chunks = [&](auto zero) {
-    using T = decltype(zero);
-    const int32_t *frw = fr + e0;
-    const float *valw = val + e0;
-    const T n_all = (T)(e1 - e0), my_bt = (T)(my_b - e0);
-    int32_t f_nx = lane < n_all ? frw[lane] : 0;
-    float x_nx = lane < n_all ? valw[lane] : 0.f;
-    int32_t carry_f = 0;
-    for (T base = 0; base < n_all; base += 32) {
-      const T e = base + lane;
-      const int32_t f = f_nx;
-      const float x = x_nx;
-      const bool in_nx = base + 32 + lane < n_all;
-      f_nx = in_nx ? frw[base + 32 + lane] : 0;
-      x_nx = in_nx ? valw[base + 32 + lane] : 0.f;
-      int owner = 0;  // last lane whose row starts at or before e
+  const int64_t my_e = has ? row_ptr[p + 1] : e1;
+  float *tile = s_val[w];
+  uint32_t *start = s_start[w];
+  float total = 0.f, psum = 0.f;
+  bool dup = false, nonint = false;
+  int32_t last_f = -1;
+  for (int64_t t0 = e0; t0 < e1; t0 += MS_TILE) {
+    const int n = (int)min((int64_t)MS_TILE, e1 - t0);
+    __syncwarp();
+    start[lane] = 0u;
+    __syncwarp();
+    if (my_b >= t0 && my_b < t0 + n)
+      atomicOr(&start[(int)(my_b - t0) >> 5], 1u << ((int)(my_b - t0) & 31));
+    __syncwarp();
+    for (int c0 = 0; c0 * 32 < n; c0 += 4) {
+      int32_t f[4];
+      float x[4];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const int cand = owner + o;  // at most 31
-        const T cb = __shfl_sync(0xffffffffu, my_bt, cand);
-        if (cb <= e) owner = cand;
+      for (int u = 0; u < 4; u++) {  // the loads first, in flight together
+        const int i = (c0 + u) * 32 + lane;
+        f[u] = i < n ? fr[t0 + i] : -1;
+        x[u] = i < n ? val[t0 + i] : 0.f;
       }
-      const T ob = __shfl_sync(0xffffffffu, my_bt, owner);
-      const bool in = e < n_all;
-      int32_t fprev = __shfl_up_sync(0xffffffffu, f, 1);
-      if (lane == 0) fprev = carry_f;  // e > 0: the previous chunk's last frame
-      carry_f = __shfl_sync(0xffffffffu, f, 31);
-      if (in && e > ob && f == fprev) dup = true;
-      const bool nonint = in && !(x == truncf(x) && fabsf(x) < 16777216.f);
-      // a row's lanes are one run (owners do not decrease across the lanes)
-      const int ow = in ? owner : 32;
-      const int oprev = __shfl_up_sync(0xffffffffu, ow, 1);
-      const unsigned starts = __ballot_sync(0xffffffffu, lane == 0 || ow != oprev);
-      const unsigned upto = lane == 31 ? 0xffffffffu : ((2u << lane) - 1u);
-      const int rs = 31 - __clz(starts & upto);
-      const unsigned after = starts & ~upto;
-      const unsigned peers =
-          (after ? ((1u << (__ffs(after) - 1)) - 1u) : 0xffffffffu) & ~((1u << rs) - 1u);
-      const unsigned a = in ? (unsigned)fminf(fabsf(x), 16777216.f) : 0u;
-      const int xi = (in && !nonint) ? (int)x : 0;
-      const unsigned sum = __reduce_add_sync(peers, a);
-      const int ssum = __reduce_add_sync(peers, xi);
-      const unsigned anynon = __reduce_or_sync(peers, nonint ? 1u : 0u);
-      if (in && lane == __ffs(peers) - 1) {
-        s_total[w][owner] += sum;
-        s_sum[w][owner] += ssum;
-        s_nonint[w][owner] |= (int)anynon;
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const int i = (c0 + u) * 32 + lane;
+        int32_t fp = __shfl_up_sync(FULL, f[u], 1);
+        if (lane == 0) fp = last_f;
+        last_f = __shfl_sync(FULL, f[u], 31);
+        if (i < n) {
+          dup = dup || (f[u] == fp && !(start[c0 + u] >> lane & 1u));
+          tile[i] = x[u];
+        }
       }
-      __syncwarp();
     }
-  };
-  if (e1 - e0 < ((int64_t)1 << 30))
-    chunks(int32_t{0});
-  else
-    chunks(int64_t{0});
-  dup = __any_sync(0xffffffffu, dup);
-  int32_t out = keep ? my_n : 0;
-  bool integral = s_nonint[w][lane] == 0;
-  long long total = s_total[w][lane];
-  float psum = 0.f;
-  if (keep) {
-    if (dup || avg != 1) {
-      merge_row(p, my_n, my_b, (float)avg, fr, val, out, integral, total, psum);
-    } else if (integral && total < 16777216) {
-      psum = (float)s_sum[w][lane];
-    } else {
-      for (int32_t i = 0; i < my_n; i++) psum = __fadd_rn(psum, val[my_b + i]);
+    __syncwarp();
+    const int i0 = (int)(max(my_b, t0) - t0), i1 = (int)(min(my_e, t0 + n) - t0);
+    for (int i = i0; i < i1; i++) {
+      const float x = tile[i];
+      total = __fadd_rn(total, fabsf(x));
+      psum = __fadd_rn(psum, x);
+      nonint = nonint || x != truncf(x);
+    }
+  }
+  int32_t out = keep ? (int32_t)(my_e - my_b) : 0;
+  bool integral = !nonint;
+  // sum |v| as an integer: exact below 2^24, and only compared with less above
+  long long tot = total < 16777216.f ? (long long)total : 1ll << 24;
+  if (__any_sync(FULL, dup)) {
+    unsigned rows = __ballot_sync(FULL, out > 0);
+    while (rows) {
+      const int q = __ffs(rows) - 1;
+      rows &= rows - 1u;
+      int32_t o;
+      bool in;
+      uint32_t share;
+      float ps;
+      merge_row(__shfl_sync(FULL, my_b, q), __shfl_sync(FULL, out, q), 1.f, fr, val, o, in, share,
+                ps);
+      share = __reduce_add_sync(FULL, share);
+      if (lane == q) {
+        out = o;
+        integral = in;
+        tot = share;
+        psum = ps;
+      }
     }
   }
   if (has) {
     row_len[p] = out;
-    pixels_sum[p] = psum;
+    pixels_sum[p] = keep ? psum : 0.f;
   }
-  uint8_t c = keep ? pixel_class(out, integral, total, F, tcap) : (uint8_t)PCLASS_EMPTY;
+  uint8_t c = keep ? pixel_class(out, integral, tot, F, tcap) : (uint8_t)PCLASS_EMPTY;
   if (force_float && c != PCLASS_EMPTY) c = PCLASS_FLOAT;  // values rescaled after the filter
-  c = float_class(c, out, fcap);
-  record_class_warp(has, p, c, out, pclass, cl, stats);
+  record_class_warp(has, p, float_class(c, out, fcap), out, pclass, cl, stats);
 }
 
 template <int IPT, bool FIRST, bool LAST, bool PK>
@@ -723,12 +897,28 @@ void reserve_lists(Series &s) {
   s.stats.reserve(1, st);
 }
 
+// The lane-per-row form while rows are short (mean raw events per mapped
+// pixel); to merge (avg != 1) or for long rows, which leave its lanes idle and
+// its warps few, the warp-per-row form.  The whole filter stage in ms, short
+// form / long form / before both (MS_MEAN_MAX lies between the two):
+//   512^2 x 1,000 frames,     9 events a row  0.168 / 0.189 / 0.189
+//   1024^2 x 10,000,         47               1.510 / 1.633 / 1.630
+//   256^2 x 16,000,         151               0.395 / 0.399 / 0.443
+//   512^2 x 4,000,          181               1.432 / 1.468 / 1.527
+//   263^2 x 16,000,         676               1.626 / 1.451 / 1.629
+//   509^2 x 1,500, average 2, 55 (to merge)       - / 0.825 / 1.114
 void merge_classify(Series &s, int32_t avg) {
-  const int pix_per_block = 256;
-  k_merge_classify<<<(s.P + pix_per_block - 1) / pix_per_block, 256, 0, s.stream>>>(
-      s.P, s.F, avg, s.thread_cap, s.float_cap, s.desc.normalize_by_framesum, s.row_ptr.p, s.d_mask.p,
-      s.ev_frame.p, s.ev_val.p, s.row_len.p, s.pclass.p,
-      ClassLists{s.wlist.p, s.llist.p, s.flist.p}, s.pixels_sum.p, s.stats.p);
+  const ClassLists cl{s.wlist.p, s.llist.p, s.flist.p};
+  const double mean = (double)s.raw_events / (double)std::max<int64_t>(s.valid_pixels, 1);
+  if (avg == 1 && mean < MS_MEAN_MAX)
+    k_merge_short<<<(s.P + MS_WARPS * 32 - 1) / (MS_WARPS * 32), MS_WARPS * 32, 0, s.stream>>>(
+        s.P, s.F, s.thread_cap, s.float_cap, s.desc.normalize_by_framesum, s.row_ptr.p, s.d_mask.p,
+        s.ev_frame.p, s.ev_val.p, s.row_len.p, s.pclass.p, cl, s.pixels_sum.p, s.stats.p);
+  else
+    k_merge_rows<<<(s.P + 31) / 32, MC_WARPS * 32, 0, s.stream>>>(
+        s.P, s.F, avg, s.thread_cap, s.float_cap, s.desc.normalize_by_framesum, s.row_ptr.p,
+        s.d_mask.p, s.ev_frame.p, s.ev_val.p, s.row_len.p, s.pclass.p, cl, s.pixels_sum.p,
+        s.stats.p);
   XG_CHECK_LAUNCH();
 }
 
