@@ -190,7 +190,6 @@ void free_series(Series *s) {
     s->keyA.release(st);
     s->keyB.release(st);
     s->hist.release(st);
-    s->hist_scan.release(st);
     s->d_blk_base.release(st);
     s->blk_fr.release(st);
     s->blk_val.release(st);

@@ -12,7 +12,7 @@
 //            unused stride sub-frames and frames past the end (key = P, sorts
 //            last), and forms v = (float)(value * flatfield) as the reference
 //            does (sparse_filter.cpp:149-153).
-//   pass k   8-bit digit k of the pixel index: tile histograms -> digit-major
+//   pass k   7- or 8-bit digit k of the pixel index: tile histograms -> digit-major
 //            exclusive scan -> stable scatter.  Ranking inside a tile uses
 //            per-bit warp ballots + per-warp digit counters, so equal digits
 //            keep stream order (tile, warp, round, lane).
@@ -36,8 +36,13 @@ constexpr int RS_WARPS = RS_THREADS / 32;
 // Items per lane: 8 (tiles of 2048) keeps more blocks resident; above
 // RS_BIG_N events 16 (tiles of 4096) halves the tile histograms.
 constexpr int64_t RS_BIG_N = (int64_t)1 << 27;
-constexpr int RS_DIGITS = 256;
-static_assert(RS_THREADS == RS_DIGITS, "one digit per thread in the downsweep scan");
+// Digits of 7 or 8 bits (DB): 7 wherever they need no pass more (keys of 9-14,
+// 17-21 or 25-28 bits).  Half the digits halve the tile histograms and their
+// scan, take a ballot less per item to rank and double a tile's runs of
+// consecutive addresses.  A downsweep of 52 M items takes 312 / 269 / 254 us in
+// the three passes (353 / 305 / 281 with 8 bits).
+constexpr int RS_DIGITS_MAX = 256;
+static_assert(RS_DIGITS_MAX <= RS_THREADS, "a thread per digit in the downsweep scan");
 
 // The raw frames [r0, r0 + nframes) of a series: idx/val/valf start at their
 // first event e0, frame_off/frame_map at r0, and frame_off holds absolute
@@ -67,8 +72,16 @@ struct PassCfg {
   float *v_out;
   int64_t n;
   int shift;
-  int ntiles;
+  int ntiles;       // tiles, and the row length of the digit-major histogram
+  int hstride;      // (a multiple of 4)
   uint32_t sentinel;
+};
+
+// Per-pass workspace after the histogram: the digits' totals, then their
+// first positions, then the count of scanned digits.
+struct DigitSums {
+  uint32_t total[RS_DIGITS_MAX], base[RS_DIGITS_MAX];
+  uint32_t done;
 };
 
 // Raw frame of the first item of every chunk of 32 * IPT items (one warp's
@@ -144,11 +157,13 @@ __device__ __forceinline__ int64_t item_index(int tile, int w, int k, int lane) 
   return (int64_t)tile * (RS_THREADS * IPT) + (int64_t)w * 32 * IPT + k * 32 + lane;
 }
 
-template <int IPT, bool FIRST>
+template <int IPT, int DB, bool FIRST>
 __global__ void __launch_bounds__(RS_THREADS)
-k_upsweep(RawCfg rc, PassCfg pc, uint32_t *__restrict__ hist) {
+k_upsweep(RawCfg rc, PassCfg pc, uint32_t *__restrict__ hist, DigitSums *__restrict__ ds) {
+  constexpr int RS_DIGITS = 1 << DB;
   __shared__ uint32_t h[RS_DIGITS];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, tile = blockIdx.x;
+  if (tile == 0 && threadIdx.x == 0) ds->done = 0;  // for the pass's digit scan
   for (int d = threadIdx.x; d < RS_DIGITS; d += RS_THREADS) h[d] = 0;
   __syncthreads();
   uint32_t key[IPT];
@@ -198,31 +213,114 @@ k_upsweep(RawCfg rc, PassCfg pc, uint32_t *__restrict__ hist) {
   }
   __syncthreads();
   for (int d = threadIdx.x; d < RS_DIGITS; d += RS_THREADS)
-    hist[(int64_t)d * pc.ntiles + tile] = h[d];
+    hist[(int64_t)d * pc.hstride + tile] = h[d];
+}
+
+// One block per digit: the exclusive scan of its tile counts, in place, and
+// its total; the last block to finish turns the totals into the digits' first
+// positions.  One launch per pass instead of the three of a device-wide scan:
+// 12 us at 25,469 tiles (42 before, with twice the digits), 5 us at 1,204 (12).
+constexpr int DSC_THREADS = 1024;
+constexpr int DSC_IPT = 8;
+__global__ void __launch_bounds__(DSC_THREADS)
+k_digit_scan(int digits, int ntiles, int hstride, uint32_t *__restrict__ hist,
+             DigitSums *__restrict__ ds) {
+  __shared__ uint32_t wsum[DSC_THREADS / 32];
+  __shared__ bool last;
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  uint32_t *row = hist + (int64_t)blockIdx.x * hstride;
+  uint32_t carry = 0;
+  for (int base = 0; base < ntiles; base += DSC_THREADS * DSC_IPT) {
+    const int i = base + threadIdx.x * DSC_IPT;
+    uint32_t v[DSC_IPT];
+#pragma unroll
+    for (int k = 0; k < DSC_IPT; k += 4) {  // rows are 16-byte aligned, hstride a multiple of 4
+      const uint4 x = i + k < hstride ? *(const uint4 *)(row + i + k) : make_uint4(0u, 0u, 0u, 0u);
+      v[k] = x.x;
+      v[k + 1] = x.y;
+      v[k + 2] = x.z;
+      v[k + 3] = x.w;
+    }
+    uint32_t s = 0;
+#pragma unroll
+    for (int k = 0; k < DSC_IPT; k++) {
+      if (i + k >= ntiles) v[k] = 0;  // the row's padding is not written by the upsweep
+      const uint32_t c = v[k];
+      v[k] = s;
+      s += c;
+    }
+    uint32_t x = s;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(FULL, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) wsum[w] = x;
+    __syncthreads();
+    uint32_t y = wsum[lane];  // DSC_THREADS / 32 == 32 warps
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t z = __shfl_up_sync(FULL, y, o);
+      if (lane >= o) y += z;
+    }
+    const uint32_t before = w ? __shfl_sync(FULL, y, w - 1) : 0u;
+    const uint32_t all = __shfl_sync(FULL, y, 31);
+    const uint32_t off = carry + before + x - s;
+#pragma unroll
+    for (int k = 0; k < DSC_IPT; k += 4)
+      if (i + k < hstride)
+        *(uint4 *)(row + i + k) =
+            make_uint4(off + v[k], off + v[k + 1], off + v[k + 2], off + v[k + 3]);
+    carry += all;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    ds->total[blockIdx.x] = carry;
+    __threadfence();
+    last = atomicAdd(&ds->done, 1u) == (uint32_t)digits - 1u;
+  }
+  __syncthreads();
+  if (!last || w != 0) return;
+  __threadfence();
+  uint32_t run = 0;
+  for (int d0 = 0; d0 < digits; d0 += 32) {
+    const uint32_t c = ((volatile uint32_t *)ds->total)[d0 + lane];
+    uint32_t x = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(FULL, x, o);
+      if (lane >= o) x += y;
+    }
+    ds->base[d0 + lane] = run + x - c;
+    run += __shfl_sync(FULL, x, 31);
+  }
 }
 
 // Shared memory of the downsweep: per-warp digit counters, the tile's global
 // and local digit offsets, and the tile staged in digit order.
-template <int IPT, bool PK>
+template <int IPT, int DB, bool PK>
 struct DsSmem {
-  uint32_t wcnt[RS_WARPS][RS_DIGITS];
-  uint32_t toff[RS_DIGITS];
-  uint32_t tstart[RS_DIGITS];
+  uint32_t wcnt[RS_WARPS][1 << DB];
+  uint32_t toff[1 << DB];
+  uint32_t tstart[1 << DB];
   uint32_t wtot[RS_THREADS / 32];
   uint32_t key[RS_THREADS * IPT];
   int32_t fr[RS_THREADS * IPT];      // frame, or the packed item
   float v[PK ? 1 : RS_THREADS * IPT];
 };
 
-template <int IPT, bool FIRST, bool LAST, bool PK>
+template <int IPT, int DB, bool FIRST, bool LAST, bool PK>
 __global__ void __launch_bounds__(RS_THREADS)
-k_downsweep(RawCfg rc, PassCfg pc, const uint32_t *__restrict__ offsets) {
+k_downsweep(RawCfg rc, PassCfg pc, const uint32_t *__restrict__ offsets,
+            const DigitSums *__restrict__ dsum) {
+  constexpr int RS_DIGITS = 1 << DB;
   extern __shared__ __align__(16) uint8_t ds_raw[];
-  DsSmem<IPT, PK> &sm = *reinterpret_cast<DsSmem<IPT, PK> *>(ds_raw);
+  DsSmem<IPT, DB, PK> &sm = *reinterpret_cast<DsSmem<IPT, DB, PK> *>(ds_raw);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, tile = blockIdx.x;
   for (int d = lane; d < RS_DIGITS; d += 32) sm.wcnt[w][d] = 0;
   for (int d = threadIdx.x; d < RS_DIGITS; d += RS_THREADS)
-    sm.toff[d] = offsets[(int64_t)d * pc.ntiles + tile];
+    sm.toff[d] = offsets[(int64_t)d * pc.hstride + tile] + dsum->base[d];
   __syncwarp();
 
   uint32_t key[IPT];
@@ -277,11 +375,11 @@ k_downsweep(RawCfg rc, PassCfg pc, const uint32_t *__restrict__ offsets) {
   for (int k = 0; k < IPT; k++) {
     const bool ok = key[k] != 0xffffffffu;
     uint32_t d = ok ? ((key[k] >> pc.shift) & (RS_DIGITS - 1)) : RS_DIGITS;
-    // lanes with the same digit (9 bits with the invalid marker), one ballot
-    // per bit: cheaper here than match_any
+    // lanes with the same digit (and the invalid marker's bit), one ballot per
+    // bit: cheaper here than match_any
     unsigned peers = 0xffffffffu;
 #pragma unroll
-    for (int b = 0; b < 9; b++) {
+    for (int b = 0; b <= DB; b++) {
       const bool bit = (d >> b) & 1u;
       const unsigned bal = __ballot_sync(0xffffffffu, bit);
       peers &= bit ? bal : ~bal;
@@ -298,25 +396,27 @@ k_downsweep(RawCfg rc, PassCfg pc, const uint32_t *__restrict__ offsets) {
   __syncthreads();
   // per digit: exclusive over warps; tile total -> tile-local digit starts
   {
-    const int d = threadIdx.x;  // RS_THREADS == RS_DIGITS
-    uint32_t run = 0;
+    const int d = threadIdx.x;  // whole warps of digits
+    uint32_t run = 0, x = 0;
+    if (d < RS_DIGITS) {
 #pragma unroll
-    for (int ww = 0; ww < RS_WARPS; ww++) {
-      uint32_t c = sm.wcnt[ww][d];
-      sm.wcnt[ww][d] = run;
-      run += c;
-    }
-    uint32_t x = run;
+      for (int ww = 0; ww < RS_WARPS; ww++) {
+        uint32_t c = sm.wcnt[ww][d];
+        sm.wcnt[ww][d] = run;
+        run += c;
+      }
+      x = run;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
+      for (int o = 1; o < 32; o <<= 1) {
+        uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
     }
-    if (lane == 31) sm.wtot[w] = x;
+    if (lane == 31) sm.wtot[w] = x;  // 0 past the digits
     __syncthreads();
     uint32_t before = 0;
     for (int ww = 0; ww < w; ww++) before += sm.wtot[ww];
-    sm.tstart[d] = before + x - run;
+    if (d < RS_DIGITS) sm.tstart[d] = before + x - run;
   }
   __syncthreads();
   // stage the tile in digit order
@@ -352,26 +452,68 @@ k_downsweep(RawCfg rc, PassCfg pc, const uint32_t *__restrict__ offsets) {
   }
 }
 
-// Row pointers from the sorted keys: row_ptr[p] = first position whose key
+// Row pointers from the sorted keys: row_ptr[p] = the first position whose key
 // is >= p (std::lower_bound over the kept items), row_ptr[P] = the kept total.
-// One thread per pixel; neighbouring pixels share the upper search steps.
-__global__ void k_row_ptr(const uint32_t *__restrict__ keys, int64_t n,
-                          const DevStats *__restrict__ stats, int32_t P,
-                          int64_t *__restrict__ row_ptr) {
-  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p > P) return;
+// One pass over the keys, 512 per warp in four 16-byte loads a lane: where the
+// key changes, the rows up to it start there; a warp fills longer gaps (rows
+// without events) together.  Bound by HBM: 4 B per event read.  One binary
+// search per pixel took 64 us at 49.6 M events in 1 Mi pixels and 12 at 2.5 M
+// in 512^2, this pass 64 and 9.
+constexpr int RP_U = 4;
+__global__ void __launch_bounds__(256)
+k_row_ptr(const uint32_t *__restrict__ keys, int64_t n, const DevStats *__restrict__ stats,
+          int32_t P, int64_t *__restrict__ row_ptr) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
   const int64_t nv = n - (int64_t)stats->dropped;
-  int64_t first = 0, len = nv;
-  while (len > 0) {
-    const int64_t half = len >> 1;
-    if ((int64_t)keys[first + half] < p) {
-      first += half + 1;
-      len -= half + 1;
+  // the warp's first key; position nv is the end of the last rows
+  const int64_t w0 =
+      (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (RP_U * 128);
+  if (w0 > nv) return;
+  int32_t key[RP_U][5];  // keys i0 - 1 .. i0 + 3 of a group: -1 before the first, P past the end
+#pragma unroll
+  for (int u = 0; u < RP_U; u++) {
+    const int64_t i0 = w0 + u * 128 + lane * 4;
+    if (i0 + 3 < nv) {
+      const uint4 x = *(const uint4 *)(keys + i0);
+      key[u][1] = (int32_t)x.x;
+      key[u][2] = (int32_t)x.y;
+      key[u][3] = (int32_t)x.z;
+      key[u][4] = (int32_t)x.w;
     } else {
-      len = half;
+#pragma unroll
+      for (int k = 1; k < 5; k++) key[u][k] = i0 - 1 + k < nv ? (int32_t)keys[i0 - 1 + k] : P;
     }
   }
-  row_ptr[p] = first;
+  int32_t before = w0 > 0 ? (int32_t)keys[w0 - 1] : -1;
+#pragma unroll
+  for (int u = 0; u < RP_U; u++) {
+    const int64_t i0 = w0 + u * 128 + lane * 4;
+    key[u][0] = __shfl_up_sync(FULL, key[u][4], 1);
+    if (lane == 0) key[u][0] = before;
+    before = __shfl_sync(FULL, key[u][4], 31);
+    // rows (key[k - 1], key[k]] start at position i0 - 1 + k; most lanes see no
+    // change
+    if (key[u][4] != key[u][0]) {
+#pragma unroll
+      for (int k = 1; k < 5; k++)
+        if (key[u][k] - key[u][k - 1] <= 8)
+          for (int32_t p = key[u][k - 1] + 1; p <= key[u][k]; p++) row_ptr[p] = i0 - 1 + k;
+    }
+    if (!__any_sync(FULL, key[u][4] - key[u][0] > 8)) continue;
+#pragma unroll
+    for (int k = 1; k < 5; k++) {
+      unsigned big = __ballot_sync(FULL, key[u][k] - key[u][k - 1] > 8);
+      while (big) {
+        const int l = __ffs(big) - 1;
+        big &= big - 1u;
+        const int32_t a = __shfl_sync(FULL, key[u][k - 1], l);
+        const int32_t e = __shfl_sync(FULL, key[u][k], l);
+        const int64_t pos = __shfl_sync(FULL, i0 - 1 + k, l);
+        for (int32_t p = a + 1 + lane; p <= e; p += 32) row_ptr[p] = pos;
+      }
+    }
+  }
 }
 
 // The events of one row (b, n) merged in place by a warp: events of the same
@@ -695,46 +837,73 @@ k_merge_short(int32_t P, int32_t F, int32_t tcap, int32_t fcap, int32_t force_fl
   record_class_warp(has, p, float_class(c, out, fcap), out, pclass, cl, stats);
 }
 
-template <int IPT, bool FIRST, bool LAST, bool PK>
-void launch_downsweep(int ntiles, cudaStream_t st, const RawCfg &rc, const PassCfg &pc,
-                      const uint32_t *offsets) {
-  const size_t smem = sizeof(DsSmem<IPT, PK>);
-  XG_CUDA(cudaFuncSetAttribute(k_downsweep<IPT, FIRST, LAST, PK>,
+template <int IPT, int DB, bool FIRST, bool LAST, bool PK>
+void launch_downsweep(Series &s, int ntiles, const RawCfg &rc, const PassCfg &pc,
+                      const DigitSums *ds) {
+  const size_t smem = sizeof(DsSmem<IPT, DB, PK>);
+  XG_CUDA(cudaFuncSetAttribute(k_downsweep<IPT, DB, FIRST, LAST, PK>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k_downsweep<IPT, FIRST, LAST, PK><<<ntiles, RS_THREADS, smem, st>>>(rc, pc, offsets);
+  k_downsweep<IPT, DB, FIRST, LAST, PK><<<ntiles, RS_THREADS, smem, s.stream>>>(rc, pc, s.hist.p,
+                                                                               ds);
 }
 
 // One radix pass: tile histograms, digit-major scan, stable scatter.
-template <int IPT>
-void radix_pass(Series &s, bool first, bool last, bool packed, int ntiles, const RawCfg &rc,
-                const PassCfg &pc) {
+template <int IPT, int DB, bool PK>
+void radix_pass(Series &s, bool first, bool last, const RawCfg &rc, PassCfg pc) {
   cudaStream_t st = s.stream;
+  const int ntiles = pc.ntiles;
+  pc.hstride = (ntiles + 3) & ~3;
+  DigitSums *ds = (DigitSums *)(s.hist.p + ((size_t)pc.hstride << DB));
   if (first)
-    k_upsweep<IPT, true><<<ntiles, RS_THREADS, 0, st>>>(rc, pc, s.hist.p);
+    k_upsweep<IPT, DB, true><<<ntiles, RS_THREADS, 0, st>>>(rc, pc, s.hist.p, ds);
   else
-    k_upsweep<IPT, false><<<ntiles, RS_THREADS, 0, st>>>(rc, pc, s.hist.p);
+    k_upsweep<IPT, DB, false><<<ntiles, RS_THREADS, 0, st>>>(rc, pc, s.hist.p, ds);
   XG_CHECK_LAUNCH();
-  exclusive_scan_u32(s.hist.p, s.hist_scan.p, (int64_t)RS_DIGITS * ntiles, s.scan_tmp.p, st);
+  k_digit_scan<<<1 << DB, DSC_THREADS, 0, st>>>(1 << DB, ntiles, pc.hstride, s.hist.p, ds);
+  XG_CHECK_LAUNCH();
+  if (first && last)
+    launch_downsweep<IPT, DB, true, true, PK>(s, ntiles, rc, pc, ds);
+  else if (first)
+    launch_downsweep<IPT, DB, true, false, PK>(s, ntiles, rc, pc, ds);
+  else if (last)
+    launch_downsweep<IPT, DB, false, true, PK>(s, ntiles, rc, pc, ds);
+  else
+    launch_downsweep<IPT, DB, false, false, PK>(s, ntiles, rc, pc, ds);
+  XG_CHECK_LAUNCH();
+}
+
+// Passes and digit bits for keys of nbits bits.
+struct Digits {
+  int passes, bits;
+};
+Digits digits_for(int nbits) {
+  const int passes = (nbits + 7) / 8;
+  return {passes, nbits <= 7 * passes ? 7 : 8};
+}
+
+void radix_pass(Series &s, int ipt, int bits, bool packed, bool first, bool last, const RawCfg &rc,
+                const PassCfg &pc) {
   if (packed) {
-    if (first && last)
-      launch_downsweep<IPT, true, true, true>(ntiles, st, rc, pc, s.hist_scan.p);
-    else if (first)
-      launch_downsweep<IPT, true, false, true>(ntiles, st, rc, pc, s.hist_scan.p);
-    else if (last)
-      launch_downsweep<IPT, false, true, true>(ntiles, st, rc, pc, s.hist_scan.p);
+    if (ipt == 16)
+      bits == 7 ? radix_pass<16, 7, true>(s, first, last, rc, pc)
+                : radix_pass<16, 8, true>(s, first, last, rc, pc);
     else
-      launch_downsweep<IPT, false, false, true>(ntiles, st, rc, pc, s.hist_scan.p);
+      bits == 7 ? radix_pass<8, 7, true>(s, first, last, rc, pc)
+                : radix_pass<8, 8, true>(s, first, last, rc, pc);
   } else {
-    if (first && last)
-      launch_downsweep<IPT, true, true, false>(ntiles, st, rc, pc, s.hist_scan.p);
-    else if (first)
-      launch_downsweep<IPT, true, false, false>(ntiles, st, rc, pc, s.hist_scan.p);
-    else if (last)
-      launch_downsweep<IPT, false, true, false>(ntiles, st, rc, pc, s.hist_scan.p);
+    if (ipt == 16)
+      bits == 7 ? radix_pass<16, 7, false>(s, first, last, rc, pc)
+                : radix_pass<16, 8, false>(s, first, last, rc, pc);
     else
-      launch_downsweep<IPT, false, false, false>(ntiles, st, rc, pc, s.hist_scan.p);
+      bits == 7 ? radix_pass<8, 7, false>(s, first, last, rc, pc)
+                : radix_pass<8, 8, false>(s, first, last, rc, pc);
   }
-  XG_CHECK_LAUNCH();
+}
+
+// The histogram of a pass, its rows padded to 16 bytes, and the digits' sums.
+void reserve_hist(Series &s, int ntiles, int bits) {
+  const size_t hstride = ((size_t)ntiles + 3) & ~(size_t)3;
+  s.hist.reserve((hstride << bits) + sizeof(DigitSums) / sizeof(uint32_t), s.stream);
 }
 
 int items_per_lane(int64_t n) { return n >= RS_BIG_N ? 16 : 8; }
@@ -746,14 +915,12 @@ int items_per_lane(int64_t n) { return n >= RS_BIG_N ? 16 : 8; }
 // Returns true when the sorted triples ended in the scratch arrays.
 bool radix_sort_triples(Series &s, uint32_t *key, int32_t *a, float *b, uint32_t *key2,
                         int32_t *a2, float *b2, int64_t n, int key_bits) {
-  cudaStream_t st = s.stream;
   if (n <= 0 || key_bits <= 0) return false;
-  const int passes = (key_bits + 7) / 8;
+  const Digits dg = digits_for(key_bits);
+  const int passes = dg.passes;
   const int ipt = items_per_lane(n);
   const int ntiles = (int)((n + RS_THREADS * ipt - 1) / (RS_THREADS * ipt));
-  s.hist.reserve((size_t)RS_DIGITS * ntiles, st);
-  s.hist_scan.reserve((size_t)RS_DIGITS * ntiles, st);
-  s.scan_tmp.reserve(scan_workspace_bytes((int64_t)RS_DIGITS * ntiles), st);
+  reserve_hist(s, ntiles, dg.bits);
   RawCfg rc{};
   uint32_t *kb[2] = {key, key2};
   int32_t *ab[2] = {a, a2};
@@ -761,7 +928,7 @@ bool radix_sort_triples(Series &s, uint32_t *key, int32_t *a, float *b, uint32_t
   for (int pass = 0; pass < passes; pass++) {
     PassCfg pc{};
     pc.n = n;
-    pc.shift = 8 * pass;
+    pc.shift = dg.bits * pass;
     pc.ntiles = ntiles;
     pc.sentinel = 0xfffffffeu;
     pc.key_in = kb[pass & 1];
@@ -770,10 +937,7 @@ bool radix_sort_triples(Series &s, uint32_t *key, int32_t *a, float *b, uint32_t
     pc.key_out = kb[(pass + 1) & 1];
     pc.fr_out = ab[(pass + 1) & 1];
     pc.v_out = bb[(pass + 1) & 1];
-    if (ipt == 16)
-      radix_pass<16>(s, false, false, false, ntiles, rc, pc);
-    else
-      radix_pass<8>(s, false, false, false, ntiles, rc, pc);
+    radix_pass(s, ipt, dg.bits, false, false, false, rc, pc);
   }
   return (passes & 1) != 0;
 }
@@ -816,13 +980,11 @@ void transpose_range(Series &s, int32_t r0, int32_t r1, int32_t *ev_fr, float *e
   // the count of items sorted last, read by the row pointers, is per range
   XG_CUDA(cudaMemsetAsync(&s.stats.p->dropped, 0, sizeof(unsigned long long), st));
   const int nbits = 32 - __builtin_clz((unsigned)P);  // bits to hold P (the drop key)
-  const int passes = (nbits + 7) / 8;
+  const Digits dg = digits_for(nbits);
+  const int passes = dg.passes;
   const int ipt = s.radix_ipt == 8 || s.radix_ipt == 16 ? s.radix_ipt : items_per_lane(n);
   const int ntiles = (int)((n + RS_THREADS * ipt - 1) / (RS_THREADS * ipt));
-  s.hist.reserve((size_t)RS_DIGITS * ntiles, st);
-  s.hist_scan.reserve((size_t)RS_DIGITS * ntiles, st);
-  const size_t ws = scan_workspace_bytes((int64_t)RS_DIGITS * ntiles);
-  s.scan_tmp.reserve(std::max(ws, scan_workspace_bytes(P)), st);
+  reserve_hist(s, ntiles, dg.bits);
   // sparse series below 65,536 filter frames carry one packed word per item
   // (frame, raw value) through the passes instead of a frame and a value
   const bool dense = s.desc.dense != 0;
@@ -856,7 +1018,7 @@ void transpose_range(Series &s, int32_t r0, int32_t r1, int32_t *ev_fr, float *e
     bool first = pass == 0, last = pass == passes - 1;
     PassCfg pc{};
     pc.n = n;
-    pc.shift = 8 * pass;
+    pc.shift = dg.bits * pass;
     pc.ntiles = ntiles;
     pc.sentinel = (uint32_t)P;
     if (!first) {
@@ -873,14 +1035,10 @@ void transpose_range(Series &s, int32_t r0, int32_t r1, int32_t *ev_fr, float *e
       pc.fr_out = fbuf[pass & 1];
       pc.v_out = vbuf[pass & 1];
     }
-    if (ipt == 16)
-      radix_pass<16>(s, first, last, packed, ntiles, rc, pc);
-    else
-      radix_pass<8>(s, first, last, packed, ntiles, rc, pc);
+    radix_pass(s, ipt, dg.bits, packed, first, last, rc, pc);
   }
   const uint32_t *keys = (passes % 2 == 0) ? s.keyB.p : s.keyA.p;  // written by the last pass
-  k_row_ptr<<<(unsigned)(((int64_t)P + 1 + 255) / 256), 256, 0, st>>>(keys, n, s.stats.p, P,
-                                                                      row_ptr);
+  k_row_ptr<<<(unsigned)((n + 1 + RP_U * 1024 - 1) / (RP_U * 1024)), 256, 0, st>>>(keys, n, s.stats.p, P, row_ptr);
   XG_CHECK_LAUNCH();
 }
 

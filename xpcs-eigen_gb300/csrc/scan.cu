@@ -1,6 +1,5 @@
 // Device-wide exclusive prefix sums (reduce-then-scan, recursive over block
-// totals).  Used for radix-sort digit offsets and for the pixel-major row
-// offsets of the event lists.
+// totals).  Used for the pixel-major row offsets of the event lists.
 #include "xpcs_internal.h"
 
 namespace xg {
@@ -111,10 +110,6 @@ void scan_rec(const TI *in, int64_t n_in, int64_t n_out, TO *out, uint8_t *ws, c
 }  // namespace
 
 size_t scan_workspace_bytes(int64_t n) { return ws_bytes<int64_t>(n + 1); }
-
-void exclusive_scan_u32(const uint32_t *in, uint32_t *out, int64_t n, void *ws, cudaStream_t st) {
-  scan_rec<uint32_t, uint32_t>(in, n, n, out, (uint8_t *)ws, st);
-}
 
 // out has n+1 entries; out[n] is the total.
 void exclusive_scan_i32_i64(const int32_t *in, int64_t *out, int64_t n, void *ws,

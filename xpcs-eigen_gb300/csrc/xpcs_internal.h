@@ -275,7 +275,7 @@ struct Series {
   DBuf<uint32_t> keyA, keyB;
   DBuf<int32_t> frA, frB;
   DBuf<float> vA, vB;
-  DBuf<uint32_t> hist, hist_scan;
+  DBuf<uint32_t> hist;
   // incremental transposes (block_frames > 0): block-local pixel-major rows
   int32_t block_frames = 0;   // filter frames per block; 0: one transpose at xpcs_multitau
   int32_t blk_raw_done = 0;   // raw frames already transposed into blocks
@@ -437,7 +437,6 @@ void xpcs_set_last_error(const char *msg);
 
 // Scans (scan.cu)
 size_t scan_workspace_bytes(int64_t n);
-void exclusive_scan_u32(const uint32_t *in, uint32_t *out, int64_t n, void *ws, cudaStream_t st);
 void exclusive_scan_i32_i64(const int32_t *in, int64_t *out, int64_t n, void *ws,
                             cudaStream_t st);
 
