@@ -372,8 +372,9 @@ int xpcs_get_twotime(xpcs_series *s, int32_t *qbins, float *sg, float *c2t, floa
  * process.  A batch holds several series handles of one device (uneven frame
  * counts, detector sizes and occupancies) and runs the whole path for all of
  * them -- filter/transpose, multi-tau and normalisation -- as one CUDA graph,
- * captured on the first run and replayed until a member's frames, the mode or
- * the flags change (then it is captured again).  Members are dealt, largest
+ * captured by the second run on the same frames and replayed until a member's
+ * frames, the mode or the flags change; a first run enqueues the same schedule
+ * directly.  Members are dealt, largest
  * first, onto a number of concurrent chains.  Two forms:
  *  - work queue (the default): the chains run every member's transpose, then
  *    the multi-tau of all members runs as persistent launches over a device

@@ -234,3 +234,29 @@ def test_both_batch_forms_equal_each_series_alone(queue):
     finally:
         for s in series:
             s.close()
+
+
+def test_first_run_replay_and_a_change_of_form_give_the_same_bits():
+    """The first run on new frames enqueues the members' work directly, the
+    next ones replay a captured graph; a form chosen in between, and calls on
+    a member alone, leave the results as they are."""
+    series = [open_member(*synth_member(i, *m)) for i, m in enumerate(MIX[:4])]
+    golden = [golden_member(n)[1] for n in ("sparse_flat", "dense_dark")]
+    members = series + golden
+    try:
+        solo = [alone(s, xg.MODE_REFERENCE) for s in members]
+        with xg.Batch(members) as b:
+            for queue in (True, True, False, False, True):
+                b.set_form(queue)
+                for _ in range(3):
+                    b.run(xg.MODE_REFERENCE, f64=True, f32=True)
+                    for s, r in zip(members, solo):
+                        assert_same(results(s), r)
+                    members[1].side_stats(max(members[1].frames // 10, 1))
+            b.run(xg.MODE_EXACT, f64=True)
+            b.run(xg.MODE_REFERENCE, f64=True, f32=True)
+            for s, r in zip(members, solo):
+                assert_same(results(s), r)
+    finally:
+        for s in members:
+            s.close()

@@ -1898,9 +1898,8 @@ int32_t mt_float_cap(const Series &s, double mean) {
   return factor < 1.25 ? 0 : (int32_t)std::min<double>(s.F, factor * mean + 64.0);
 }
 
-void run_multitau(Series &s, int mode) {
+std::vector<uint8_t> prepare_multitau(Series &s, int mode) {
   cudaStream_t st = s.stream;
-  const int D = s.D, P = s.P;
   // the plan depends on the series' shape and the mode only; it is uploaded
   // once per mode (a captured batch graph must not copy from host memory)
   std::vector<uint8_t> plan = make_plan(s, mode);
@@ -1912,10 +1911,18 @@ void run_multitau(Series &s, int mode) {
     s.plan_mode = mode;
     s.plan_scr = hp->scr;
   }
-  const size_t nD = (size_t)D * P;
+  const size_t nD = (size_t)s.D * s.P;
   s.G2.reserve(nD ? nD : 1, st);
   s.IP.reserve(nD ? nD : 1, st);
   s.IF.reserve(nD ? nD : 1, st);
+  return plan;
+}
+
+void run_multitau(Series &s, int mode) {
+  cudaStream_t st = s.stream;
+  const int D = s.D, P = s.P;
+  const std::vector<uint8_t> plan = prepare_multitau(s, mode);
+  const McPlan *hp = (const McPlan *)plan.data();
   if (D == 0 || P == 0) return;
   const int scr = std::max(hp->acc, hp->nlev);
   const ThreadKernel ktt = thread_kernel(s.thread_cap);

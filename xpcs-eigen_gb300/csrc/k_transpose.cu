@@ -901,9 +901,12 @@ void radix_pass(Series &s, int ipt, int bits, bool packed, bool first, bool last
 }
 
 // The histogram of a pass, its rows padded to 16 bytes, and the digits' sums.
-void reserve_hist(Series &s, int ntiles, int bits) {
+// Sized for 8-bit digits whichever the keys take, so that sorts of one
+// series' events by different keys never move the buffer under a captured
+// batch.
+void reserve_hist(Series &s, int ntiles) {
   const size_t hstride = ((size_t)ntiles + 3) & ~(size_t)3;
-  s.hist.reserve((hstride << bits) + sizeof(DigitSums) / sizeof(uint32_t), s.stream);
+  s.hist.reserve(hstride * RS_DIGITS_MAX + sizeof(DigitSums) / sizeof(uint32_t), s.stream);
 }
 
 int items_per_lane(int64_t n) { return n >= RS_BIG_N ? 16 : 8; }
@@ -920,7 +923,7 @@ bool radix_sort_triples(Series &s, uint32_t *key, int32_t *a, float *b, uint32_t
   const int passes = dg.passes;
   const int ipt = items_per_lane(n);
   const int ntiles = (int)((n + RS_THREADS * ipt - 1) / (RS_THREADS * ipt));
-  reserve_hist(s, ntiles, dg.bits);
+  reserve_hist(s, ntiles);
   RawCfg rc{};
   uint32_t *kb[2] = {key, key2};
   int32_t *ab[2] = {a, a2};
@@ -984,7 +987,7 @@ void transpose_range(Series &s, int32_t r0, int32_t r1, int32_t *ev_fr, float *e
   const int passes = dg.passes;
   const int ipt = s.radix_ipt == 8 || s.radix_ipt == 16 ? s.radix_ipt : items_per_lane(n);
   const int ntiles = (int)((n + RS_THREADS * ipt - 1) / (RS_THREADS * ipt));
-  reserve_hist(s, ntiles, dg.bits);
+  reserve_hist(s, ntiles);
   // sparse series below 65,536 filter frames carry one packed word per item
   // (frame, raw value) through the passes instead of a frame and a value
   const bool dense = s.desc.dense != 0;

@@ -385,8 +385,8 @@ struct MtQueue {
   std::vector<int32_t> cap_first, cap_count, cap_groups;  // per MT_THREAD_CAPS entry
   int32_t scr_max = 0, acc_max = 0;
 };
-// Builds the table (after an eager pass has sized every buffer and uploaded
-// every plan); enqueues the multi-tau of every member as work-queue launches
+// Builds the table (once every member's transpose is enqueued and its
+// multi-tau prepared: every buffer has its place then); enqueues the multi-tau of every member as work-queue launches
 // (k_multitau.cu).
 void mt_queue_build(const std::vector<Series *> &ss, MtQueue &q, cudaStream_t st);
 void mt_queue_run(const std::vector<Series *> &ss, MtQueue &q, cudaStream_t st);
@@ -448,6 +448,8 @@ void default_knobs(Series &s);
 void transpose_ready_blocks(Series &s);
 void reset_blocks(Series &s);
 void run_multitau(Series &s, int mode);                      // k_multitau.cu
+// Its plan (uploaded) and output buffers, without running it.
+std::vector<uint8_t> prepare_multitau(Series &s, int mode);  // k_multitau.cu
 void run_normalize(Series &s, bool want64, bool want32);     // k_normalize.cu
 void build_norm_chunks(Series &s);                           // k_normalize.cu
 bool mt_float_rows_warp(const McPlan &hp);                    // k_multitau.cu
