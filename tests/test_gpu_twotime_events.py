@@ -41,3 +41,36 @@ def test_twotime_event_lists_and_dense_rows_vs_oracle(W, H, F, density, static_m
         assert same_bits_nan(r["c2t"][q], o["c2t"][q])
     for k in ("sg", "g2full", "g2partials"):
         assert same_bits_nan(r[k], o[k]), k
+
+
+@pytest.mark.parametrize("W,H,F,density,most", [
+    (9, 7, 1, 0.04, 3), (12, 11, 8, 0.05, 9), (40, 30, 33, 0.03, 9), (13, 12, 65, 0.04, 2048),
+    (30, 30, 900, 0.045, 4), (16, 16, 300, 0.02, 30000), (5, 5, 3600, 0.02, 9),
+    (6, 5, 9500, 0.01, 9), (20, 20, 130, 0.3, 9),
+])
+@pytest.mark.parametrize("static_map,average", [(True, False), (False, True), (True, True),
+                                                (False, False)])
+def test_exact_twotime_from_event_lists_equals_the_int64_gram(W, H, F, density, most, static_map,
+                                                              average):
+    """EXACT mode from the event lists (one and several smoothing groups per q
+    bin, columns of one and of many blocks, counts past what int32 or fp16 sums
+    hold) equals the int64 CUDA-core Gram in every output."""
+    rng = np.random.default_rng(W * F + most)
+    P = W * H
+    sq = (rng.integers(0, 6, P) + 1).astype(np.int32)
+    sq[:12] = np.repeat(np.arange(1, 7), 2)
+    dq = (sq + 1) // 2
+    hit = rng.random((F, P)) < density
+    nnz, idx = hit.sum(1).astype(np.uint32), np.nonzero(hit)[1].astype(np.int32)
+    val = rng.integers(1, most + 1, idx.size).astype(np.int16)
+    out = []
+    for mode in (xg.MODE_EXACT, xg.TWOTIME_EXACT_CUDA_CORES):
+        with xg.Series(W, H, F, 4, dq.reshape(H, W), sq.reshape(H, W)) as s:
+            s.ingest_sparse(nnz, idx, val)
+            out.append(s.twotime([1, 3], static_map=static_map, average=average, window=3,
+                                 mode=mode))
+    e, i = out
+    for q in (1, 3):
+        assert same_bits_nan(e["c2t"][q], i["c2t"][q])
+    for k in ("sg", "g2full", "g2partials"):
+        assert same_bits_nan(e[k], i[k]), k

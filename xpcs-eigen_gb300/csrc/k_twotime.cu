@@ -135,6 +135,20 @@ k_tt_gram(int32_t F, int32_t nrows, const int32_t *__restrict__ order,
 
 // ------------------------------------------------------------ event lists
 //
+// Smoothing group of every row.
+__global__ void k_tt_groups(int32_t R, int32_t G, const int32_t *__restrict__ grp_ptr,
+                            int32_t *__restrict__ row_grp) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= R) return;
+  int lo = 0, hi = G - 1;  // the last group that starts at or before r
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (grp_ptr[mid] <= r) lo = mid;
+    else hi = mid - 1;
+  }
+  row_grp[r] = lo;
+}
+
 // The Gram of sparse rows: of the F (F + 1) / 2 products of a row only those
 // of its events exist, and a column f1 of C needs, in row order, the rows
 // with an event at f1 and each one's earlier events.  The rows' events are
@@ -252,68 +266,87 @@ __global__ void k_tt_smooth_events(int32_t R, int32_t F, int32_t average,
   }
 }
 
+__device__ __forceinline__ void tt_add(float &acc, float x, float y) {
+  acc = __fadd_rn(acc, __fmul_rn(x, y));
+}
+__device__ __forceinline__ void tt_add(int32_t &acc, int32_t x, int32_t y) { acc += x * y; }
+__device__ __forceinline__ void tt_value(float v, float &x) { x = v; }
+__device__ __forceinline__ void tt_value(float v, int32_t &x) { x = __float2int_rn(v); }
+
+// The events [lo, hi) of column f1, in row order, by one warp: each one's row
+// contributes v(f0) v(f1) to acc[f0] for its events up to f1, one f0 per lane,
+// so no two lanes of a step share a sum and every sum takes its rows in order.
+// A lane each looks up 32 events' rows at a time, and the next event's first
+// 32 row entries are loaded while the current one's are added: the steps'
+// latency bounds it.
+template <class T>
+__device__ __forceinline__ void tt_column(int64_t lo, int64_t hi, const int32_t *__restrict__ a,
+                                          const float *__restrict__ b,
+                                          const int32_t *__restrict__ row_pix,
+                                          const int64_t *__restrict__ row_ptr,
+                                          const int32_t *__restrict__ ev_frame,
+                                          const float *__restrict__ val, T *acc) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  for (int64_t e0 = lo; e0 < hi; e0 += 32) {
+    const int64_t e = e0 + lane;
+    int64_t my_base = 0;
+    int my_i = -1;  // position of the event in its row: entries 0 .. i reach up to f1
+    T my_v = 0;
+    if (e < hi) {
+      my_base = row_ptr[row_pix[a[e]]];
+      my_i = __float_as_int(b[e]);
+      tt_value(val[my_base + my_i], my_v);
+    }
+    const int n = (int)min((int64_t)32, hi - e0);
+    int64_t base = __shfl_sync(FULL, my_base, 0);
+    int i = __shfl_sync(FULL, my_i, 0);
+    int f = lane <= i ? ev_frame[base + lane] : 0;
+    float v = lane <= i ? val[base + lane] : 0.f;
+    for (int k = 0; k < n; k++) {
+      const int64_t bk = base;
+      const int ik = i, fk = f;
+      T vk;
+      tt_value(v, vk);
+      const T v1 = __shfl_sync(FULL, my_v, k);
+      const int nk = min(k + 1, 31);
+      base = __shfl_sync(FULL, my_base, nk);
+      i = k + 1 < n ? __shfl_sync(FULL, my_i, nk) : -1;
+      f = lane <= i ? ev_frame[base + lane] : 0;
+      v = lane <= i ? val[base + lane] : 0.f;
+      if (v1 == 0) continue;  // no event (a smoothed value of 0 forms no product)
+      if (vk != 0) tt_add(acc[fk], vk, v1);
+      for (int j = lane + 32; j <= ik; j += 32) {
+        T x;
+        tt_value(val[bk + j], x);
+        if (x != 0) tt_add(acc[ev_frame[bk + j]], x, v1);
+      }
+      __syncwarp();
+    }
+  }
+}
+
 // One warp per column f1 of one q bin, W columns a block: the column's sums
-// over f0 <= f1 in the warp's shared memory (F floats).  The column's events
-// come in row order; each one's row contributes v(f0) v(f1) for its events up
-// to f1, one f0 per lane, so no two lanes of a step share a sum and every sum
-// takes its rows in order.  A lane each looks up 32 events' rows at a time,
-// and the next event's first 32 row entries are loaded while the current
-// one's are added: the steps' latency bounds it.  Long columns first; the
-// block writes its columns side by side (32-byte sectors at W = 8).
+// over f0 <= f1 in the warp's shared memory (F floats).  Long columns first;
+// the block writes its columns side by side (32-byte sectors at W = 8).
 // Measured (256 x 256 pixels, 701 frames, 6 q bins, 2 % of the pixels hit per
-// frame): the two-time call 0.89 ms against 13.0 ms with the dense matrix,
+// frame): the two-time call 0.84 ms against 11.3 ms with the dense matrix,
 // 9.75 ms of it in the tiled Gram.
 __global__ void __launch_bounds__(256)
-k_tt_gram_events(int32_t F, int32_t q0, const int32_t *__restrict__ q_ptr,
+k_tt_gram_events(int32_t F, const int32_t *__restrict__ q_ptr,
                  const int64_t *__restrict__ col_ptr, const int32_t *__restrict__ a,
                  const float *__restrict__ b, const int32_t *__restrict__ row_pix,
                  const int64_t *__restrict__ row_ptr, const int32_t *__restrict__ ev_frame,
                  const float *__restrict__ sv, float *__restrict__ C) {
   extern __shared__ float tt_acc[];
-  const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, W = blockDim.x >> 5;
-  const int q = q0 + blockIdx.y, c0 = (gridDim.x - 1 - blockIdx.x) * W, f1 = c0 + w;
+  const int q = blockIdx.y, c0 = (gridDim.x - 1 - blockIdx.x) * W, f1 = c0 + w;
   float *acc = tt_acc + (size_t)w * F;
   if (f1 < F) {
     for (int f = lane; f <= f1; f += 32) acc[f] = 0.f;
     __syncwarp();
-    const int64_t lo = col_ptr[(int64_t)q * F + f1], hi = col_ptr[(int64_t)q * F + f1 + 1];
-    for (int64_t e0 = lo; e0 < hi; e0 += 32) {
-      const int64_t e = e0 + lane;
-      int64_t my_base = 0;
-      int my_i = -1;  // position of the event in its row: entries 0 .. i reach up to f1
-      float my_v = 0.f;
-      if (e < hi) {
-        my_base = row_ptr[row_pix[a[e]]];
-        my_i = __float_as_int(b[e]);
-        my_v = sv[my_base + my_i];
-      }
-      const int n = (int)min((int64_t)32, hi - e0);
-      int64_t base = __shfl_sync(FULL, my_base, 0);
-      int i = __shfl_sync(FULL, my_i, 0);
-      int f = lane <= i ? ev_frame[base + lane] : 0;
-      float v = lane <= i ? sv[base + lane] : 0.f;
-      for (int k = 0; k < n; k++) {
-        const int64_t bk = base;
-        const int ik = i, fk = f;
-        const float vk = v, v1 = __shfl_sync(FULL, my_v, k);
-        const int nk = min(k + 1, 31);
-        base = __shfl_sync(FULL, my_base, nk);
-        i = k + 1 < n ? __shfl_sync(FULL, my_i, nk) : -1;
-        f = lane <= i ? ev_frame[base + lane] : 0;
-        v = lane <= i ? sv[base + lane] : 0.f;
-        if (v1 == 0.f) continue;  // no event (a smoothed value of 0 forms no product)
-        if (vk != 0.f) acc[fk] = __fadd_rn(acc[fk], __fmul_rn(vk, v1));
-        for (int j = lane + 32; j <= ik; j += 32) {
-          const float x = sv[bk + j];
-          if (x != 0.f) {
-            const int fx = ev_frame[bk + j];
-            acc[fx] = __fadd_rn(acc[fx], __fmul_rn(x, v1));
-          }
-        }
-        __syncwarp();
-      }
-    }
+    const int64_t *cp = col_ptr + (int64_t)q * F + f1;
+    tt_column<float>(cp[0], cp[1], a, b, row_pix, row_ptr, ev_frame, sv, acc);
   }
   __syncthreads();
   const float den = (float)(q_ptr[q + 1] - q_ptr[q]);
@@ -325,10 +358,167 @@ k_tt_gram_events(int32_t F, int32_t q0, const int32_t *__restrict__ q_ptr,
   }
 }
 
-// Columns per block of the event Gram: 8 while two blocks fit on an SM, fewer
-// for longer columns; 0 when not even one column fits.
-int tt_columns(int32_t F) {
-  const size_t col = sizeof(float) * (size_t)F;
+// ----------------------------------------- EXACT mode from the event lists
+//
+// The counts' Gram products are integers, so the lists give EXACT mode's
+// matrices as well, and for sparse counts with less work than the dense Gram
+// on the tensor cores, which multiplies (and first stores) mostly zeros:
+// int32 sums in shared memory, exact while sum over a group's rows of (max
+// count)^2 < 2^31, then the same double operations on them as after the
+// tensor-core Gram (k_twotime_tc.cu).
+
+// Per group: sum over its rows of (max |count|)^2; flag 1: a value that is not
+// an integer count.  One warp per row.
+__global__ void k_tt_check(int32_t R, const int32_t *__restrict__ row_pix,
+                           const int32_t *__restrict__ row_grp,
+                           const int64_t *__restrict__ row_ptr,
+                           const int32_t *__restrict__ row_len, const float *__restrict__ ev_val,
+                           unsigned long long *__restrict__ bound, int32_t *__restrict__ flags) {
+  const int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (r >= R) return;
+  const int lane = threadIdx.x & 31, p = row_pix[r], n = row_len[p];
+  const int64_t base = row_ptr[p];
+  unsigned mx = 0;
+  bool bad = false;
+  for (int i = lane; i < n; i += 32) {
+    const float v = ev_val[base + i];
+    const bool ok = v == truncf(v) && fabsf(v) <= 65536.f;
+    bad = bad || !ok;
+    mx = max(mx, ok ? (unsigned)fabsf(v) : 0u);
+  }
+  bad = __any_sync(0xffffffffu, bad);
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if (lane == 0) {
+    if (bad) atomicOr(flags, 1);
+    if (mx) atomicAdd(&bound[row_grp[r]], (unsigned long long)mx * mx);
+  }
+}
+
+// The part of column c's events whose rows lie in [r0, r1) (ascending rows).
+__device__ __forceinline__ int64_t tt_first_row(const int32_t *__restrict__ a, int64_t lo,
+                                                int64_t hi, int32_t r) {
+  int64_t len = hi - lo;
+  while (len > 0) {
+    const int64_t h = len >> 1;
+    if (a[lo + h] < r) {
+      lo += h + 1;
+      len -= h + 1;
+    } else {
+      len = h;
+    }
+  }
+  return lo;
+}
+
+// sg[g][f] = (sum of the group's counts at f) / pixels in double, and its
+// reciprocal; sg as float.  One warp per (group, frame).
+__global__ void k_tt_sg_counts(int32_t F, const int32_t *__restrict__ grp_ptr,
+                               const int32_t *__restrict__ grp_q,
+                               const int64_t *__restrict__ col_ptr, const int32_t *__restrict__ a,
+                               const float *__restrict__ b, const int32_t *__restrict__ row_pix,
+                               const int64_t *__restrict__ row_ptr,
+                               const float *__restrict__ ev_val, double *__restrict__ sgd,
+                               double *__restrict__ isg, float *__restrict__ sg) {
+  const int lane = threadIdx.x & 31;
+  const int f = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5), g = blockIdx.y;
+  if (f >= F) return;
+  const int r0 = grp_ptr[g], r1 = grp_ptr[g + 1];
+  const int64_t c = (int64_t)grp_q[g] * F + f;
+  const int64_t lo = tt_first_row(a, col_ptr[c], col_ptr[c + 1], r0);
+  const int64_t hi = tt_first_row(a, lo, col_ptr[c + 1], r1);
+  long long s = 0;
+  for (int64_t e = lo + lane; e < hi; e += 32)
+    s += (long long)ev_val[row_ptr[row_pix[a[e]]] + __float_as_int(b[e])];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0) {
+    const double v = (double)s / (r1 - r0);
+    sgd[(size_t)g * F + f] = v;
+    isg[(size_t)g * F + f] = 1.0 / v;
+    sg[(size_t)g * F + f] = (float)v;
+  }
+}
+
+// The averaged form: the mean over the frames, in order; one thread per group.
+__global__ void k_tt_sg_counts_avg(int32_t G, int32_t F, const double *__restrict__ sgd,
+                                   double *__restrict__ isg, float *__restrict__ sga) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= G) return;
+  double mean = 0.0;
+  for (int f = 0; f < F; f++) mean += sgd[(size_t)g * F + f];
+  mean /= F;
+  isg[(size_t)g * F] = 1.0 / mean;
+  sga[g] = (float)mean;
+}
+
+// One warp per column as k_tt_gram_events, on the counts: the int32 sums of
+// every smoothing group of the q bin in turn, folded into double sums where
+// there are several (multi), C and its double form Cq as k_tc_single /
+// k_tc_accum and k_tc_final give them.
+// Measured (512 x 512 pixels, 1,536 frames, 9 q bins, 1 % of the pixels hit per
+// frame, one group per q bin): the call 1.05 ms against 3.58 with the
+// tensor-core Gram (1.45 in the Gram, the rest in building, clearing and
+// scaling its matrices and in a synchronisation per group).
+__global__ void __launch_bounds__(256)
+k_tt_gram_counts(int32_t F, int32_t q0, int32_t multi, int32_t average,
+                 const int32_t *__restrict__ q_ptr, const int32_t *__restrict__ q_grp,
+                 const int32_t *__restrict__ grp_ptr, const int64_t *__restrict__ col_ptr,
+                 const int32_t *__restrict__ a, const float *__restrict__ b,
+                 const int32_t *__restrict__ row_pix, const int64_t *__restrict__ row_ptr,
+                 const int32_t *__restrict__ ev_frame, const float *__restrict__ ev_val,
+                 const double *__restrict__ isg, double *__restrict__ Cd, float *__restrict__ C) {
+  extern __shared__ __align__(16) uint8_t tt_raw[];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, W = blockDim.x >> 5;
+  const int q = q0 + blockIdx.y, c0 = (gridDim.x - 1 - blockIdx.x) * W, f1 = c0 + w;
+  double *dsum = (double *)tt_raw;  // [W][F] when multi
+  int32_t *isum = (int32_t *)(dsum + (multi ? (size_t)W * F : 0));
+  int32_t *acc = isum + (size_t)w * F;
+  double *dac = dsum + (size_t)w * F;
+  const int g0 = q_grp[q], g1 = q_grp[q + 1];
+  if (f1 < F) {
+    const int64_t lo = col_ptr[(int64_t)q * F + f1], hi = col_ptr[(int64_t)q * F + f1 + 1];
+    if (multi)
+      for (int f = lane; f <= f1; f += 32) dac[f] = 0.0;
+    for (int g = g0; g < g1; g++) {
+      for (int f = lane; f <= f1; f += 32) acc[f] = 0;
+      __syncwarp();
+      const int64_t l = multi ? tt_first_row(a, lo, hi, grp_ptr[g]) : lo;
+      const int64_t h = multi ? tt_first_row(a, l, hi, grp_ptr[g + 1]) : hi;
+      tt_column<int32_t>(l, h, a, b, row_pix, row_ptr, ev_frame, ev_val, acc);
+      if (!multi) break;
+      const double *ig = isg + (size_t)g * F;
+      const double y = average ? ig[0] : ig[f1];
+      for (int f = lane; f <= f1; f += 32)
+        if (acc[f]) dac[f] += (double)acc[f] * (average ? ig[0] : ig[f]) * y;
+      __syncwarp();
+    }
+  }
+  __syncthreads();
+  const int32_t npix = q_ptr[q + 1] - q_ptr[q];
+  const double inv = npix ? 1.0 / npix : 0.0;
+  const double *ig = isg + (size_t)g0 * F;
+  double *Cdq = Cd + (size_t)blockIdx.y * F * F;
+  float *Cq = C + (size_t)q * F * F;
+  const int last = min(c0 + W, F) - 1;
+  for (int idx = threadIdx.x; idx < (last + 1) * W; idx += blockDim.x) {
+    const int f0 = idx / W, cw = idx % W, c = c0 + cw;
+    if (c >= F || f0 > c) continue;
+    double v;
+    if (multi) {
+      v = dsum[(size_t)cw * F + f0] * inv;
+    } else {
+      const int32_t n = isum[(size_t)cw * F + f0];
+      v = n ? (double)n * (average ? ig[0] : ig[f0]) * (average ? ig[0] : ig[c]) * inv : 0.0;
+    }
+    Cdq[(size_t)f0 * F + c] = v;
+    Cq[(size_t)f0 * F + c] = (float)v;
+  }
+}
+
+// Columns per block of the event Grams, of `bytes` per frame: 8 while two
+// blocks fit on an SM, fewer for longer columns; 0 when not even one fits.
+int tt_columns(int32_t F, size_t bytes) {
+  const size_t col = bytes * (size_t)F;
   for (int w : {8, 4, 2, 1})
     if (w * col <= 110 * 1024) return w;
   return col <= 220 * 1024 ? 1 : 0;
@@ -373,9 +563,71 @@ __global__ void k_tt_diag(int32_t Q, int32_t F, int32_t window, int32_t tp,
 //   256^2      700  1.20/12.5   3.03/12.6   10.1/12.8   36.8/13.2
 //   64^2     4,096  1.58/5.60   3.10/5.75   9.03/6.09   32.0/7.0
 bool tt_use_events(Series &s) {
-  if (tt_columns(s.F) == 0) return false;
+  if (tt_columns(s.F, sizeof(float)) == 0) return false;
   const double most = std::min(0.4, std::max(0.15, 40.0 / s.F));
   return (double)s.raw_events <= most * (double)s.qmap.pix.size() * s.R_in * s.F;
+}
+
+// Warps of 256-thread blocks for k units of one warp.
+unsigned tt_warps(int64_t k) { return (unsigned)((k * 32 + 255) / 256); }
+
+struct EventLists {
+  const int32_t *q_ptr, *grp_q, *q_grp;  // rows of each q bin; q bin of each group; groups of each
+  int64_t n;                             // events of the rows
+};
+
+// Row counts for the lists, and the tables of q bins and groups; enqueues the
+// copy of the event count to *n (valid after a synchronisation).
+EventLists lists_prepare(Series &s, const TwoTimeLayout &lay, int32_t R, int32_t G, int32_t Q,
+                         const int32_t *order, int64_t *n) {
+  cudaStream_t st = s.stream;
+  std::vector<int32_t> tab(lay.q_ptr);
+  for (int32_t g = 0, q = 0; g < G; g++) {
+    while (q + 1 < Q && lay.grp_ptr[g] >= lay.q_ptr[q + 1]) q++;
+    tab.push_back(q);
+  }
+  tab.push_back(0);
+  tab.insert(tab.end(), lay.q_grp_end.begin(), lay.q_grp_end.end());
+  s.tt_qptr.reserve(tab.size(), st);
+  XG_CUDA(cudaMemcpyAsync(s.tt_qptr.p, tab.data(), 4 * tab.size(), cudaMemcpyHostToDevice, st));
+  s.tt_len.reserve(R, st);
+  s.tt_cpos.reserve((size_t)R + 1, st);
+  s.tt_cols.reserve((size_t)Q * s.F + 1, st);
+  s.scan_tmp.reserve(scan_workspace_bytes(R), st);
+  k_tt_lens<<<(R + 255) / 256, 256, 0, st>>>(R, order, s.tt_row_pix.p, s.row_len.p, s.tt_len.p);
+  XG_CHECK_LAUNCH();
+  exclusive_scan_i32_i64(s.tt_len.p, s.tt_cpos.p, R, s.scan_tmp.p, st);
+  if (n) XG_CUDA(cudaMemcpyAsync(n, s.tt_cpos.p + R, sizeof(*n), cudaMemcpyDeviceToHost, st));
+  const int32_t *q_ptr = s.tt_qptr.p;
+  return {q_ptr, q_ptr + Q + 1, q_ptr + Q + 1 + G, 0};
+}
+
+// Sorts the rows' events by (q, frame) from the given row order (null: mapping
+// order); the sorted (row, position) pairs, and the columns' first events in
+// tt_cols.
+std::pair<const int32_t *, const float *> lists_build(Series &s, const EventLists &l, int32_t R,
+                                                      int32_t Q, const int32_t *order) {
+  cudaStream_t st = s.stream;
+  const int32_t F = s.F;
+  const int64_t ncol = (int64_t)Q * F;
+  const size_t ne = std::max<int64_t>(l.n, 1);
+  s.keyA.reserve(ne, st);
+  s.frA.reserve(ne, st);
+  s.vA.reserve(ne, st);
+  s.keyB.reserve(ne, st);
+  s.frB.reserve(ne, st);
+  s.vB.reserve(ne, st);
+  k_tt_build<<<tt_warps(R), 256, 0, st>>>(R, F, Q, order, l.q_ptr, s.tt_row_pix.p, s.row_ptr.p,
+                                          s.row_len.p, s.ev_frame.p, s.tt_cpos.p, s.keyA.p,
+                                          s.frA.p, s.vA.p);
+  XG_CHECK_LAUNCH();
+  const int bits = ncol > 1 ? 64 - __builtin_clzll((unsigned long long)ncol - 1) : 1;
+  const bool in_b =
+      radix_sort_triples(s, s.keyA.p, s.frA.p, s.vA.p, s.keyB.p, s.frB.p, s.vB.p, l.n, bits);
+  k_tt_cols<<<(unsigned)((ncol + 256) / 256), 256, 0, st>>>(ncol, l.n, in_b ? s.keyB.p : s.keyA.p,
+                                                            s.tt_cols.p);
+  XG_CHECK_LAUNCH();
+  return {in_b ? s.frB.p : s.frA.p, in_b ? s.vB.p : s.vA.p};
 }
 
 // C, sg and sga from event lists.
@@ -383,74 +635,109 @@ void gram_events(Series &s, const TwoTimeReq &req, const TwoTimeLayout &lay, int
                  int32_t Q) {
   cudaStream_t st = s.stream;
   const int32_t F = s.F;
-  const int64_t ncol = (int64_t)Q * F;
-  const auto warps = [](int64_t k) { return (unsigned)((k * 32 + 255) / 256); };
-  std::vector<int32_t> ptrs(lay.q_ptr);  // rows of each q bin, then the q bin of each group
-  for (int32_t g = 0, q = 0; g < G; g++) {
-    while (q + 1 < Q && lay.grp_ptr[g] >= lay.q_ptr[q + 1]) q++;
-    ptrs.push_back(q);
-  }
-  s.tt_qptr.reserve(ptrs.size(), st);
-  XG_CUDA(cudaMemcpyAsync(s.tt_qptr.p, ptrs.data(), 4 * ptrs.size(), cudaMemcpyHostToDevice, st));
-  const int32_t *q_ptr = s.tt_qptr.p, *grp_q = q_ptr + Q + 1;
-  s.tt_len.reserve(R, st);
-  s.tt_cpos.reserve((size_t)R + 1, st);
-  s.tt_cols.reserve((size_t)ncol + 1, st);
-  s.scan_tmp.reserve(scan_workspace_bytes(R), st);
-  int64_t n = -1;
-  // sorts the rows' events by (q, frame) from the given row order; returns the
-  // sorted (a, b)
-  const auto lists = [&](const int32_t *order) {
-    k_tt_lens<<<(R + 255) / 256, 256, 0, st>>>(R, order, s.tt_row_pix.p, s.row_len.p, s.tt_len.p);
-    XG_CHECK_LAUNCH();
-    exclusive_scan_i32_i64(s.tt_len.p, s.tt_cpos.p, R, s.scan_tmp.p, st);
-    if (n < 0) {
-      XG_CUDA(cudaMemcpyAsync(&n, s.tt_cpos.p + R, sizeof(n), cudaMemcpyDeviceToHost, st));
-      XG_CUDA(cudaStreamSynchronize(st));
-    }
-    const size_t ne = std::max<int64_t>(n, 1);
-    s.keyA.reserve(ne, st);
-    s.frA.reserve(ne, st);
-    s.vA.reserve(ne, st);
-    s.keyB.reserve(ne, st);
-    s.frB.reserve(ne, st);
-    s.vB.reserve(ne, st);
-    k_tt_build<<<warps(R), 256, 0, st>>>(R, F, Q, order, q_ptr, s.tt_row_pix.p, s.row_ptr.p,
-                                         s.row_len.p, s.ev_frame.p, s.tt_cpos.p, s.keyA.p,
-                                         s.frA.p, s.vA.p);
-    XG_CHECK_LAUNCH();
-    const int bits = ncol > 1 ? 64 - __builtin_clzll((unsigned long long)ncol - 1) : 1;
-    const bool in_b = radix_sort_triples(s, s.keyA.p, s.frA.p, s.vA.p, s.keyB.p, s.frB.p, s.vB.p,
-                                         n, bits);
-    k_tt_cols<<<(unsigned)((ncol + 256) / 256), 256, 0, st>>>(ncol, n, in_b ? s.keyB.p : s.keyA.p,
-                                                              s.tt_cols.p);
-    XG_CHECK_LAUNCH();
-    return std::make_pair((const int32_t *)(in_b ? s.frB.p : s.frA.p),
-                          (const float *)(in_b ? s.vB.p : s.vA.p));
-  };
-  auto ab = lists(nullptr);  // mapping order
-  k_tt_sg_events<<<dim3(warps(F), G), 256, 0, st>>>(F, s.tt_grp_ptr.p, grp_q, s.tt_cols.p, ab.first,
-                                                    ab.second, s.tt_row_pix.p, s.row_ptr.p,
-                                                    s.ev_val.p, s.tt_sg.p);
+  int64_t n = 0;
+  EventLists l = lists_prepare(s, lay, R, G, Q, nullptr, &n);
+  XG_CUDA(cudaStreamSynchronize(st));
+  l.n = n;
+  auto ab = lists_build(s, l, R, Q, nullptr);  // mapping order
+  k_tt_sg_events<<<dim3(tt_warps(F), G), 256, 0, st>>>(F, s.tt_grp_ptr.p, l.grp_q, s.tt_cols.p,
+                                                       ab.first, ab.second, s.tt_row_pix.p,
+                                                       s.row_ptr.p, s.ev_val.p, s.tt_sg.p);
   XG_CHECK_LAUNCH();
   if (req.average) {
     k_tt_sg_avg<<<(G + 127) / 128, 128, 0, st>>>(G, F, s.tt_sg.p, s.tt_sga.p);
     XG_CHECK_LAUNCH();
   }
   s.tt_V.reserve((size_t)std::max<int64_t>(s.raw_events, 1), st);  // as long as the event lists
-  k_tt_smooth_events<<<warps(R), 256, 0, st>>>(R, F, req.average, s.tt_row_pix.p, s.tt_row_grp.p,
-                                               s.row_ptr.p, s.row_len.p, s.ev_frame.p, s.ev_val.p,
-                                               req.average ? s.tt_sga.p : s.tt_sg.p, s.tt_V.p);
+  k_tt_smooth_events<<<tt_warps(R), 256, 0, st>>>(R, F, req.average, s.tt_row_pix.p,
+                                                  s.tt_row_grp.p, s.row_ptr.p, s.row_len.p,
+                                                  s.ev_frame.p, s.ev_val.p,
+                                                  req.average ? s.tt_sga.p : s.tt_sg.p, s.tt_V.p);
   XG_CHECK_LAUNCH();
-  if (req.frame_threading) ab = lists(s.tt_order.p);
-  const int W = tt_columns(F);
+  if (req.frame_threading) {
+    lists_prepare(s, lay, R, G, Q, s.tt_order.p, nullptr);
+    ab = lists_build(s, l, R, Q, s.tt_order.p);
+  }
+  const int W = tt_columns(F, sizeof(float));
   const size_t smem = sizeof(float) * (size_t)F * W;
   XG_CUDA(cudaFuncSetAttribute(k_tt_gram_events, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)smem));
   k_tt_gram_events<<<dim3((F + W - 1) / W, Q), 32 * W, smem, st>>>(
-      F, 0, q_ptr, s.tt_cols.p, ab.first, ab.second, s.tt_row_pix.p, s.row_ptr.p, s.ev_frame.p,
+      F, l.q_ptr, s.tt_cols.p, ab.first, ab.second, s.tt_row_pix.p, s.row_ptr.p, s.ev_frame.p,
       s.tt_V.p, s.tt_C.p);
   XG_CHECK_LAUNCH();
+}
+
+// EXACT mode from the counts' event lists; false when the series takes the
+// other forms: rows too dense for the lists, or counts too large for int32
+// sums.  The lists' work grows with the square of the events per pixel and
+// frame, d, and the tensor-core Gram's hardly at all; longer columns leave the
+// lists fewer warps per SM.  Whole calls in ms, lists / tensor cores:
+//   pixels  frames  q bins   d = 0.01       0.02        0.03        0.05
+//   256^2      300       3  0.38/0.85   0.50/0.89   0.58/0.88   0.77/0.94  (0.1: 1.35/1.13)
+//   512^2    1,536       9  1.05/3.58   1.54/3.74   2.37/4.04   4.50/4.62
+//     (two groups a q bin)  1.55/4.54   2.39/4.83   3.61/5.22   7.02/6.04
+//   1024^2     700       9  2.13/9.83   3.14/10.3   4.10/11.4   7.87/13.3
+//   512^2    4,096       9  4.02/6.50   8.57/7.08   15.7/8.02   38.1/9.72
+bool gram_counts(Series &s, const TwoTimeReq &req, const TwoTimeLayout &lay, int32_t R, int32_t G,
+                 int32_t Q) {
+  cudaStream_t st = s.stream;
+  const int32_t F = s.F;
+  const double most = std::min(0.06, 65.0 / F);
+  if (F > 65535 || (double)s.raw_events > most * (double)s.qmap.pix.size() * s.R_in * F)
+    return false;
+  const bool multi = G > Q;
+  const size_t col = sizeof(int32_t) + (multi ? sizeof(double) : 0);
+  const int W = tt_columns(F, col);
+  if (W == 0) return false;
+  int64_t n = 0;
+  int32_t flags = 0;
+  std::vector<unsigned long long> bound(G);
+  s.tt_bound.reserve(std::max(G, 2), st);
+  s.tt_flags.reserve(1, st);
+  XG_CUDA(cudaMemsetAsync(s.tt_bound.p, 0, sizeof(unsigned long long) * G, st));
+  XG_CUDA(cudaMemsetAsync(s.tt_flags.p, 0, sizeof(int32_t), st));
+  k_tt_check<<<tt_warps(R), 256, 0, st>>>(R, s.tt_row_pix.p, s.tt_row_grp.p, s.row_ptr.p,
+                                          s.row_len.p, s.ev_val.p, s.tt_bound.p, s.tt_flags.p);
+  XG_CHECK_LAUNCH();
+  EventLists l = lists_prepare(s, lay, R, G, Q, nullptr, &n);
+  XG_CUDA(cudaMemcpyAsync(bound.data(), s.tt_bound.p, sizeof(unsigned long long) * G,
+                          cudaMemcpyDeviceToHost, st));
+  XG_CUDA(cudaMemcpyAsync(&flags, s.tt_flags.p, sizeof(flags), cudaMemcpyDeviceToHost, st));
+  XG_CUDA(cudaStreamSynchronize(st));
+  l.n = n;
+  if (flags & 1) tt_not_counts();
+  for (unsigned long long b : bound)
+    if (b >= (1ull << 31)) return false;
+  const auto ab = lists_build(s, l, R, Q, nullptr);
+  s.tt_sgd.reserve(2 * (size_t)G * F, st);
+  double *sgd = s.tt_sgd.p, *isg = sgd + (size_t)G * F;
+  k_tt_sg_counts<<<dim3(tt_warps(F), G), 256, 0, st>>>(F, s.tt_grp_ptr.p, l.grp_q, s.tt_cols.p,
+                                                       ab.first, ab.second, s.tt_row_pix.p,
+                                                       s.row_ptr.p, s.ev_val.p, sgd, isg,
+                                                       s.tt_sg.p);
+  XG_CHECK_LAUNCH();
+  if (req.average) {
+    k_tt_sg_counts_avg<<<(G + 31) / 32, 32, 0, st>>>(G, F, sgd, isg, s.tt_sga.p);
+    XG_CHECK_LAUNCH();
+  }
+  const size_t smem = col * (size_t)F * W;
+  XG_CUDA(cudaFuncSetAttribute(k_tt_gram_counts, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)smem));
+  // q bins at a time: their double matrices within 2 GB
+  const size_t F2 = (size_t)F * F;
+  const int32_t step = (int32_t)std::max<size_t>(1, std::min<size_t>(Q, (2ull << 30) / (8 * F2)));
+  s.tt_Cq.reserve(F2 * step, st);
+  for (int32_t q = 0; q < Q; q += step) {
+    const int32_t nq = std::min(step, Q - q);
+    k_tt_gram_counts<<<dim3((F + W - 1) / W, nq), 32 * W, smem, st>>>(
+        F, q, multi, req.average, l.q_ptr, l.q_grp, s.tt_grp_ptr.p, s.tt_cols.p, ab.first,
+        ab.second, s.tt_row_pix.p, s.row_ptr.p, s.ev_frame.p, s.ev_val.p, isg, s.tt_Cq.p,
+        s.tt_C.p);
+    XG_CHECK_LAUNCH();
+    twotime_exact_diag(s, req.window, Q, q, nq);
+  }
+  return true;
 }
 
 // The same from the dense matrix V.
@@ -496,27 +783,32 @@ void run_twotime(Series &s, const TwoTimeReq &req, int mode, bool force_i64) {
   o.frames = F;
   o.window = req.window;
   o.partials = req.window > 0 ? std::max(0, (F - req.window) / req.window) : 0;
-  // rows of the processed q bins in mapping order; smoothing groups; q row ranges
+  // rows of the processed q bins in mapping order (ranges of the mapping's
+  // pixel list, which is on the device already); smoothing groups; q row ranges
   TwoTimeLayout lay;
+  int32_t R = 0;
+  std::vector<std::pair<int32_t, int32_t>> runs;  // [first, end) of the pixel list
   for (int32_t i = 0; i < qm.nq(); i++) {
     const int32_t q = qm.q_ids[i];
     if (std::find(req.qbins.begin(), req.qbins.end(), q) == req.qbins.end()) continue;
-    for (int32_t e = qm.q_entry_ptr[i]; e < qm.q_entry_ptr[i + 1]; e++) {
-      for (int32_t k = qm.entry_pix_ptr[e]; k < qm.entry_pix_ptr[e + 1]; k++) {
-        lay.row_pix.push_back(qm.pix[k]);
-        lay.row_grp.push_back((int32_t)lay.grp_ptr.size() - 1);
-      }
-      if (req.static_map) lay.grp_ptr.push_back((int32_t)lay.row_pix.size());
-    }
-    if (!req.static_map) lay.grp_ptr.push_back((int32_t)lay.row_pix.size());
-    lay.q_ptr.push_back((int32_t)lay.row_pix.size());
+    const int32_t k0 = qm.entry_pix_ptr[qm.q_entry_ptr[i]];
+    const int32_t k1 = qm.entry_pix_ptr[qm.q_entry_ptr[i + 1]];
+    if (req.static_map)
+      for (int32_t e = qm.q_entry_ptr[i]; e < qm.q_entry_ptr[i + 1]; e++)
+        lay.grp_ptr.push_back(R + qm.entry_pix_ptr[e + 1] - k0);
+    else
+      lay.grp_ptr.push_back(R + k1 - k0);
+    R += k1 - k0;
+    if (!runs.empty() && runs.back().second == k0)
+      runs.back().second = k1;
+    else
+      runs.push_back({k0, k1});
+    lay.q_ptr.push_back(R);
     lay.q_grp_end.push_back((int32_t)lay.grp_ptr.size() - 1);
     o.qbins.push_back(q);
   }
-  const std::vector<int32_t> &row_pix = lay.row_pix, &row_grp = lay.row_grp,
-                             &grp_ptr = lay.grp_ptr, &q_ptr = lay.q_ptr;
-  const int32_t R = (int32_t)row_pix.size(), G = (int32_t)grp_ptr.size() - 1,
-                Q = (int32_t)o.qbins.size();
+  const std::vector<int32_t> &grp_ptr = lay.grp_ptr, &q_ptr = lay.q_ptr;
+  const int32_t G = (int32_t)grp_ptr.size() - 1, Q = (int32_t)o.qbins.size();
   o.sg_rows = G;
   o.sg_cols = req.average ? 1 : F;
   o.averaged = req.average != 0;
@@ -525,7 +817,20 @@ void run_twotime(Series &s, const TwoTimeReq &req, int mode, bool force_i64) {
     if (!v.empty())
       XG_CUDA(cudaMemcpyAsync(b.p, v.data(), 4 * v.size(), cudaMemcpyHostToDevice, st));
   };
-  up(s.tt_row_pix, row_pix);
+  s.tt_row_pix.reserve(R ? R : 1, st);
+  int32_t at = 0;
+  for (const auto &r : runs) {
+    if (r.second > r.first)
+      XG_CUDA(cudaMemcpyAsync(s.tt_row_pix.p + at, s.n_pix.p + r.first,
+                              4 * (size_t)(r.second - r.first), cudaMemcpyDeviceToDevice, st));
+    at += r.second - r.first;
+  }
+  up(s.tt_grp_ptr, grp_ptr);
+  s.tt_row_grp.reserve(R ? R : 1, st);
+  if (R > 0) {
+    k_tt_groups<<<(R + 255) / 256, 256, 0, st>>>(R, G, s.tt_grp_ptr.p, s.tt_row_grp.p);
+    XG_CHECK_LAUNCH();
+  }
   s.tt_sg.reserve((size_t)(G ? G : 1) * (F ? F : 1), st);
   s.tt_sga.reserve(G ? G : 1, st);
   s.tt_C.reserve((size_t)(Q ? Q : 1) * F * F + 1, st);
@@ -533,22 +838,26 @@ void run_twotime(Series &s, const TwoTimeReq &req, int mode, bool force_i64) {
   s.tt_part.reserve((size_t)req.window * o.partials * (Q ? Q : 1) + 1, st);
   XG_CUDA(cudaMemsetAsync(s.tt_C.p, 0, 4 * ((size_t)Q * F * F + 1), st));
   if (mode == XPCS_MODE_EXACT) {
-    if (R > 0 && F > 0) run_twotime_exact(s, req, lay, force_i64);
+    if (R > 0 && F > 0 && (force_i64 || !gram_counts(s, req, lay, R, G, Q)))
+      run_twotime_exact(s, req, lay, force_i64);
     o.ready = true;
     return;
   }
   // Gram order of every q bin's rows
   std::vector<int32_t> order(R);
   std::iota(order.begin(), order.end(), 0);
-  if (req.frame_threading)
+  if (req.frame_threading) {
+    std::vector<int32_t> row_pix;
+    for (const auto &r : runs)
+      row_pix.insert(row_pix.end(), qm.pix.begin() + r.first, qm.pix.begin() + r.second);
     for (int32_t q = 0; q < Q; q++)
       std::sort(order.begin() + q_ptr[q], order.begin() + q_ptr[q + 1],
                 [&](int32_t a, int32_t b) { return row_pix[a] < row_pix[b]; });
-  up(s.tt_row_grp, row_grp);
-  up(s.tt_grp_ptr, grp_ptr);
-  up(s.tt_order, order);
+  }
+  const bool events = R > 0 && F > 0 && tt_use_events(s);
+  if (req.frame_threading || !events) up(s.tt_order, order);
   if (R > 0 && F > 0) {
-    if (tt_use_events(s))
+    if (events)
       gram_events(s, req, lay, R, G, Q);
     else
       gram_dense(s, req, lay, R, G, Q);

@@ -319,14 +319,15 @@ __global__ void k_tc_final(int32_t F, double inv_npix, const double *__restrict_
   C[i] = (float)v;
 }
 
-// one block per diagonal ff: g2full = its mean; for ff < window, one thread
+// one block per diagonal ff (of q bin q0 + blockIdx.y): g2full = its mean; for ff < window, one thread
 // per window w sums g2partials
 __global__ void __launch_bounds__(256)
-k_tc_diag(int32_t Q, int32_t q, int32_t F, int32_t window, int32_t tp,
-          const double *__restrict__ Cq, float *__restrict__ g2full,
+k_tc_diag(int32_t Q, int32_t q0, int32_t F, int32_t window, int32_t tp,
+          const double *__restrict__ Cd, float *__restrict__ g2full,
           float *__restrict__ g2part) {
   __shared__ double red[256];
-  const int ff = blockIdx.x;
+  const int ff = blockIdx.x, q = q0 + blockIdx.y;
+  const double *Cq = Cd + (size_t)blockIdx.y * F * F;
   double acc = 0.0;
   for (int fx = threadIdx.x; fx < F - ff; fx += blockDim.x) acc += Cq[(size_t)fx * F + fx + ff];
   red[threadIdx.x] = acc;
@@ -365,6 +366,17 @@ EncodeTiledFn encode_fn() {
 }
 
 }  // namespace
+
+void tt_not_counts() {
+  throw Error(XPCS_ERR_INPUT, "EXACT two-time needs integer counts (no flatfield, dense "
+                              "or averaged frames)");
+}
+
+void twotime_exact_diag(Series &s, int32_t window, int32_t Q, int32_t q, int32_t nq) {
+  k_tc_diag<<<dim3(s.F, nq), 256, 0, s.stream>>>(Q, q, s.F, window, s.tt.partials, s.tt_Cq.p,
+                                                 s.tt_full.p, s.tt_part.p);
+  XG_CHECK_LAUNCH();
+}
 
 // Groups and rows as run_twotime builds them; `force_i64` routes every group
 // to the CUDA-core Gram (the check of the tensor-core one).
@@ -425,9 +437,7 @@ void run_twotime_exact(Series &s, const TwoTimeReq &req, const TwoTimeLayout &la
       XG_CUDA(cudaMemcpyAsync(&bound, s.tt_bound.p, sizeof(bound), cudaMemcpyDeviceToHost, st));
       XG_CUDA(cudaMemcpyAsync(&flags, s.tt_flags.p, sizeof(flags), cudaMemcpyDeviceToHost, st));
       XG_CUDA(cudaStreamSynchronize(st));
-      if (flags & 1)
-        throw Error(XPCS_ERR_INPUT, "EXACT two-time needs integer counts (no flatfield, dense "
-                                    "or averaged frames)");
+      if (flags & 1) tt_not_counts();
       double *sgd = sg_host.data() + (size_t)gq * (req.average ? 1 : F);
       double mean = 0.0;
       for (int32_t f = 0; f < F; f++) {
@@ -506,9 +516,7 @@ void run_twotime_exact(Series &s, const TwoTimeReq &req, const TwoTimeLayout &la
           F, inv_npix, s.tt_Cacc.p, s.tt_Cq.p, Cout);
       XG_CHECK_LAUNCH();
     }
-    k_tc_diag<<<F, 256, 0, st>>>(Q, q, F, req.window, o.partials, s.tt_Cq.p, s.tt_full.p,
-                                 s.tt_part.p);
-    XG_CHECK_LAUNCH();
+    twotime_exact_diag(s, req.window, Q, q, 1);
   }
   // sg as float, [G][F] or [G][1]
   std::vector<float> sgf(sg_host.size());

@@ -208,7 +208,6 @@ struct TwoTimeReq {
 };
 // Rows of the processed q bins in mapping order and their grouping.
 struct TwoTimeLayout {
-  std::vector<int32_t> row_pix, row_grp;  // per row: its pixel, its smoothing group
   std::vector<int32_t> grp_ptr{0};        // rows of each smoothing group (contiguous)
   std::vector<int32_t> q_ptr{0};          // rows of each processed q bin (contiguous)
   std::vector<int32_t> q_grp_end;         // static map: end group index of each q bin
@@ -496,6 +495,10 @@ void prepare_framesum_scale(Series &s);  // k_side.cu
 void run_twotime(Series &s, const TwoTimeReq &req, int mode, bool force_i64);
 void run_twotime_exact(Series &s, const TwoTimeReq &req, const TwoTimeLayout &lay,
                        bool force_i64);  // k_twotime_tc.cu
+// g2full and g2partials of the q bins [q, q + nq) of Q from their double
+// matrices in tt_Cq (k_twotime_tc.cu).
+void twotime_exact_diag(Series &s, int32_t window, int32_t Q, int32_t q, int32_t nq);
+[[noreturn]] void tt_not_counts();  // EXACT mode on values that are not counts
 void get_twotime(Series &s, int32_t *qbins, float *sg, float *c2t, float *g2full, float *g2part);
 
 // Dense frames (k_dense.cu)
