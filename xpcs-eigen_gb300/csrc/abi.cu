@@ -1,9 +1,14 @@
 // C ABI of libxpcs_gpu (include/xpcs_gpu.h): series lifecycle, ingest,
 // multi-tau, normalisation, results and the per-stage CUDA-event tracer.
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <algorithm>
 #include <atomic>
 #include <cstring>
 #include <new>
+#include <thread>
+#include <vector>
 
 #include "xpcs_internal.h"
 
@@ -54,6 +59,47 @@ void dev_free(void *p, size_t bytes, cudaStream_t st) {
   if (!p) return;
   cudaFreeAsync(p, st);
   g_dev_used[acct_device()].fetch_sub(bytes);
+}
+
+// Large result buffers are usually fresh: their pages do not exist yet, and a
+// device-to-host copy that makes them one by one on its way ran at 19 GB/s
+// where a copy to existing pages runs at 185 (85 MB of two-time matrices: 4.5
+// ms against 0.46).  Four threads make the pages first: 2.9 ms in all (3.4
+// with two, 3.7 with eight, 4.4 with sixteen, which wait for one another in
+// the kernel).
+// Buffers whose pages exist are left alone (a sample of them is looked at),
+// and where the kernel cannot populate, the copy makes the pages as before.
+void populate_host(void *ptr, size_t bytes) {
+  constexpr size_t MIN_BYTES = (size_t)8 << 20, PART = (size_t)4 << 20;
+  constexpr int POPULATE_WRITE = 23;  // MADV_POPULATE_WRITE (Linux 5.14)
+  if (!ptr || bytes < MIN_BYTES) return;
+  const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+  const uintptr_t a = ((uintptr_t)ptr + page - 1) / page * page;
+  const uintptr_t e = ((uintptr_t)ptr + bytes) / page * page;
+  if (e <= a) return;
+  bool missing = false;
+  for (int k = 0; k < 16 && !missing; k++) {
+    unsigned char in = 1;
+    const uintptr_t at = a + (e - a) / page * k / 16 * page;
+    if (mincore((void *)at, page, &in) == 0) missing = !(in & 1);
+  }
+  if (!missing) return;
+  const size_t parts = (e - a + PART - 1) / PART;
+  const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
+  const size_t n = std::min<size_t>(std::min<size_t>(hw, 4), parts);
+  auto work = [&](size_t t) {
+    for (size_t k = t; k < parts; k += n) {
+      const uintptr_t at = a + k * PART;
+      if (madvise((void *)at, std::min<size_t>(PART, e - at), POPULATE_WRITE) != 0) return;
+    }
+  };
+  std::vector<std::thread> threads;
+  try {
+    for (size_t t = 1; t < n; t++) threads.emplace_back(work, t);
+  } catch (...) {  // fewer threads than wanted: the copy makes the rest
+  }
+  work(0);
+  for (auto &t : threads) t.join();
 }
 }
 
@@ -473,6 +519,7 @@ int xpcs_get_g2ipif(xpcs_series *h, float *G2, float *IP, float *IF) {
     if (!s.have_multitau) throw Error(XPCS_ERR_STATE, "xpcs_multitau has not run");
     DeviceGuard g(s.device);
     const size_t n = (size_t)s.D * s.P;
+    for (float *out : {G2, IP, IF}) populate_host(out, 4 * n);  // while the kernels run
     XG_CUDA(cudaEventRecord(s.ev[9], s.stream));
     if (G2 && n) XG_CUDA(cudaMemcpyAsync(G2, s.G2.p, 4 * n, cudaMemcpyDeviceToHost, s.stream));
     if (IP && n) XG_CUDA(cudaMemcpyAsync(IP, s.IP.p, 4 * n, cudaMemcpyDeviceToHost, s.stream));

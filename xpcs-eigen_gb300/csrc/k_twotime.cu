@@ -877,6 +877,7 @@ void get_twotime(Series &s, int32_t *qbins, float *sg, float *c2t, float *g2full
   if (sg && o.sg_rows)
     XG_CUDA(cudaMemcpyAsync(sg, o.averaged ? s.tt_sga.p : s.tt_sg.p,
                             4 * (size_t)o.sg_rows * o.sg_cols, cudaMemcpyDeviceToHost, st));
+  if (c2t) populate_host(c2t, 4 * Q * F * F);
   if (c2t && Q) XG_CUDA(cudaMemcpyAsync(c2t, s.tt_C.p, 4 * Q * F * F, cudaMemcpyDeviceToHost, st));
   if (g2full && Q) XG_CUDA(cudaMemcpyAsync(g2full, s.tt_full.p, 4 * F * Q, cudaMemcpyDeviceToHost, st));
   if (g2part && Q && o.partials)

@@ -51,6 +51,10 @@ enum : int32_t {
 void *dev_alloc(size_t bytes, cudaStream_t st);
 void dev_free(void *p, size_t bytes, cudaStream_t st);
 
+// Makes the pages of a large, fresh host buffer that a result is about to be
+// copied to (abi.cu).
+void populate_host(void *ptr, size_t bytes);
+
 // A stream-ordered device allocation that grows on demand.
 template <class T>
 struct DBuf {
