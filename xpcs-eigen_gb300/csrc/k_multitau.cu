@@ -517,8 +517,8 @@ __device__ int compact_row(uint32_t *row, int m, int lastframe, int lane) {
 //     the level.  On sorted levels where a fifth of the bins hold an entry,
 //     the prefix-sum array (done with after IP/IF) holds the values by bin
 //     and a source finds each partner by one lookup.  On other sorted levels
-//     of delays <= 64 where the row could reach every delay (m x (thi + 1) >=
-//     lastframe), the same words hold the row's occupancy bitmask: a source
+//     of at most 32 delays, none above 64, where the row could reach every
+//     delay (m x (thi + 1) >= lastframe), the same words hold the row's occupancy bitmask: a source
 //     reads the 64 bins after it, finds its first partner's index by a
 //     population count over the bins below tau_lo and visits only the
 //     occupied bins of the delay window.
@@ -598,7 +598,8 @@ __device__ __forceinline__ void mt_warp_pixel(const McPlan *pl, const McArrays &
           if (tb < lf) acc[k * 32] += vi * S[tb];
         }
       }
-    } else if (sorted && tlo >= 1 && thi <= 64 && lf <= 32 * cap && m * (thi + 1) >= lf) {
+    } else if (sorted && tlo >= 1 && thi <= 64 && L.count <= 32 && lf <= 32 * cap &&
+               m * (thi + 1) >= lf) {
       // about one entry or more per delay window: S (done with after IP/IF)
       // becomes the level's occupancy bitmask.  Bins of the prefix are distinct
       // and increasing, so the entry at bin b is at position popcount(bits
@@ -656,14 +657,17 @@ __device__ __forceinline__ void mt_warp_pixel(const McPlan *pl, const McArrays &
         wj = j < m ? row[j] : 0u;
       }
     }
-    int mine = 0;
-    for (int k = 0; k < L.count; k++) {
-      const int tot = __reduce_add_sync(FULL, acc[k * 32]);
-      if (lane == k) mine = tot;
-    }
-    if (lane < L.count) {
-      const int d = L.first + lane;
-      G2[(size_t)d * P + p] = scaled_quotient(mine, 2 * L.level, ar.denom[d], ar.rcp[d]);
+    for (int k0 = 0; k0 < L.count; k0 += 32) {  // a lane each for 32 delays
+      int mine = 0;
+      const int nk = min(32, L.count - k0);
+      for (int k = 0; k < nk; k++) {
+        const int tot = __reduce_add_sync(FULL, acc[(k0 + k) * 32]);
+        if (lane == k) mine = tot;
+      }
+      if (lane < nk) {
+        const int d = L.first + k0 + lane;
+        G2[(size_t)d * P + p] = scaled_quotient(mine, 2 * L.level, ar.denom[d], ar.rcp[d]);
+      }
     }
     __syncwarp();
   }
