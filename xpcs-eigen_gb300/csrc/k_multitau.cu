@@ -43,6 +43,7 @@
 #include <climits>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 
 #include "mt_replay.cuh"
 #include "xpcs_internal.h"
@@ -54,6 +55,11 @@ constexpr int MT_WARPS = 2;  // warps per block of the thread-per-pixel kernel
 constexpr int WP_WARPS = 8;  // warps per block of the warp-per-pixel kernel
 constexpr int MT_MID_CAP = 1024;  // long rows up to this length: 4 warps per block
 constexpr int MID_WARPS = 4;
+// Bins per entry up to which a level's pairs are taken by byte products
+// (mt_warp_pixel).  The integer rows of 263 x 251 pixels x 16,000 frames, 744
+// events each, take 2.95 / 2.25 / 2.00 / 1.97 / 1.98 ms with 0 (pairs by
+// search and bitmask only) / 4 / 8 / 16 / 40.
+constexpr int MB_RATIO = 16;
 constexpr int LONG_WARPS = 2;  // warps per block for rows of up to MT_LONG_CAP events
 
 // std::lower_bound as libstdc++ implements it (halving the remaining length),
@@ -506,6 +512,34 @@ __device__ int compact_row(uint32_t *row, int m, int lastframe, int lane) {
   return gbase;
 }
 
+// G2 sums of one level from its bins as bytes: S holds the level's values, one
+// byte per bin, zero where no entry is and in the MB_PAD words past the last
+// bin.  Lanes take words of 4 bins: for each delay the bins that far on (byte
+// funnel shifts of the words after) meet the lane's own in a 4-way byte
+// product, so an empty bin costs no test and an occupied one no search.
+// a[k]: this lane's share of delay tlo + k, KM delays from tlo <= 31 on.
+constexpr int MB_PAD = 16;
+template <int KM>
+__device__ __forceinline__ void byte_pairs(const uint32_t *S, int lf, int tlo, int lane,
+                                           unsigned (&a)[KM]) {
+  const uint32_t *T = S + (tlo >> 2);
+  const int sh = (tlo & 3) * 8, nw = (lf + 3) >> 2;
+  for (int w = lane; w < nw; w += 32) {
+    const uint32_t own = S[w];
+    uint32_t x[KM / 4 + 2], z[KM / 4 + 1];
+#pragma unroll
+    for (int j = 0; j < KM / 4 + 2; j++) x[j] = T[w + j];
+#pragma unroll
+    for (int j = 0; j < KM / 4 + 1; j++) z[j] = __funnelshift_r(x[j], x[j + 1], sh);
+#pragma unroll
+    for (int k = 0; k < KM; k++) {
+      const uint32_t p =
+          k % 4 ? __funnelshift_r(z[k / 4], z[k / 4 + 1], 8 * (k % 4)) : z[k / 4];
+      a[k] = __dp4a(own, p, a[k]);
+    }
+  }
+}
+
 // One warp per pixel of `list` (count at *count_p) whose row holds more than
 // min_n and at most `cap` events, packed (frame << 16 | int16 value) in the warp's shared memory, with
 // the row's inclusive prefix sums and per-lane accumulators beside it.
@@ -514,14 +548,18 @@ __device__ int compact_row(uint32_t *row, int m, int lastframe, int lane) {
 //   G2: per level, warp-cooperative compaction, then every lane takes the
 //     sources lane, lane+32, ... in one flat loop over (source, partner)
 //     visits into its own accumulators, summed over the warp at the end of
-//     the level.  On sorted levels where a fifth of the bins hold an entry,
-//     the prefix-sum array (done with after IP/IF) holds the values by bin
-//     and a source finds each partner by one lookup.  On other sorted levels
-//     of at most 32 delays, none above 64, where the row could reach every
-//     delay (m x (thi + 1) >= lastframe), the same words hold the row's occupancy bitmask: a source
-//     reads the 64 bins after it, finds its first partner's index by a
-//     population count over the bins below tau_lo and visits only the
-//     occupied bins of the delay window.
+//     the level.  Where at least one bin in MB_RATIO holds an entry and the
+//     level's bins fit the prefix-sum array (done with after IP/IF) as bytes,
+//     byte products take the place of the visits (byte_pairs); entries that
+//     the reference's search misses (an unsorted buffer) are then taken out
+//     again as partners.  Where only words fit and a fifth of the bins hold an
+//     entry, the array holds the values by bin (counts above 255) and a source
+//     finds each partner by one lookup.  On other sorted levels of at most 32
+//     delays, none above 64, where the row could reach every delay (m x
+//     (thi + 1) >= lastframe), the same words hold the row's occupancy bitmask:
+//     a source reads the 64 bins after it, finds its first partner's index by a
+//     population count over the bins below tau_lo and visits only the occupied
+//     bins of the delay window.
 // One pixel p of a series with a row of n0 events from event b on (min_n < n0
 // <= cap): the body of the warp-per-pixel kernel, shared by its per-series launches and by
 // the batch's work-queue launches.  pl / ar: the plan (shared or global
@@ -581,7 +619,50 @@ __device__ __forceinline__ void mt_warp_pixel(const McPlan *pl, const McArrays &
     const int tlo = L.tau_lo, thi = L.tau_lo + L.count - 1;
     for (int k = 0; k < L.count; k++) acc[k * 32] = 0;
     const int lf = L.lastframe;
-    if (sorted && tlo >= 1 && lf <= cap && 5 * m >= lf) {
+    bool bytes = tlo >= 1 && tlo <= 31 && L.count <= 16 && ((lf + 3) >> 2) + MB_PAD <= cap &&
+                 lf <= MB_RATIO * m;
+    if (bytes) {
+      const int nw = (lf + 3) >> 2;
+      for (int q = lane; q < nw + MB_PAD; q += 32) S[q] = 0;
+      __syncwarp();
+      unsigned most = 0;  // a negative value is past 255 as well
+      for (int k = lane; k < m; k += 32) {
+        const uint32_t e = row[k];
+        most = max(most, (unsigned)pk_v(e));
+        ((uint8_t *)S)[pk_t(e)] = (uint8_t)pk_v(e);
+      }
+      bytes = __reduce_max_sync(FULL, most) <= 255u;
+      __syncwarp();
+    }
+    if (bytes) {
+      const auto level = [&](auto km) {
+        constexpr int KM = decltype(km)::value;
+        unsigned a[KM];
+#pragma unroll
+        for (int k = 0; k < KM; k++) a[k] = 0;
+        byte_pairs<KM>((const uint32_t *)S, lf, tlo, lane, a);
+        if (!sorted) {
+          // partners that lower_bound over the whole buffer does not find: none
+          // up to the tail's first bin when the tail ascends
+          const int tail0 = U && m < n0 ? pk_t(row[m]) : (U ? INT_MAX : -1);
+          for (int i = lane; i < m; i += 32) {
+            const int t = pk_t(row[i]);
+            if (t <= tail0 || lower_bound_row(row, n0, t) == i) continue;
+            const unsigned v = (unsigned)pk_v(row[i]);
+#pragma unroll
+            for (int k = 0; k < KM; k++)
+              if (t - tlo - k >= 0) a[k] -= v * ((const uint8_t *)S)[t - tlo - k];
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < KM; k++)
+          if (k < L.count) acc[k * 32] = (int32_t)a[k];
+      };
+      if (L.count <= 8)
+        level(std::integral_constant<int, 8>{});
+      else
+        level(std::integral_constant<int, 16>{});
+    } else if (sorted && tlo >= 1 && lf <= cap && 5 * m >= lf) {
       // at least a fifth of the level's bins hold an entry: the prefix sums
       // S are done with, and S becomes the row's values by bin, so that each
       // source finds its partner for every delay with one lookup (a missing
