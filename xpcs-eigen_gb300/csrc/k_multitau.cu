@@ -392,8 +392,8 @@ __device__ __forceinline__ void mt_thread_warp(const uint8_t *__restrict__ plan_
   const int P = ((const McPlan *)plan_g)->P, lane = threadIdx.x & 31;
   if (p0 >= P) return;
   const int p = p0 + lane;
-  const int c = p < P ? pclass[p] : PCLASS_FTHREAD;
-  const bool mine = c != PCLASS_FTHREAD;  // those are written by k_mt_fthread
+  const int c = p < P ? pclass[p] : PCLASS_FLOAT;
+  const bool mine = c == PCLASS_THREAD || c == PCLASS_EMPTY;  // the others' kernels write theirs
   if (!__any_sync(0xffffffffu, mine)) return;
   const int n0 = c == PCLASS_THREAD ? row_len[p] : 0;
   if (!__any_sync(0xffffffffu, n0 > 0)) {  // zeros only
@@ -449,6 +449,24 @@ __device__ __forceinline__ void mt_thread_warp(const uint8_t *__restrict__ plan_
   mt_thread_rows<CAP>(plan_g, p, n0, mine, G2, IP, IF, wbase);
 }
 
+// ---------------------------------------------------- overlapping launches
+//
+// The multi-tau kernels of a series write the results of different pixels, so
+// one may begin while the last blocks of the one before still run: each calls
+// overlap_begin first (the next launch_overlapped kernel may start once every
+// block of this one has) and overlap_end last (this kernel is complete only
+// when the one before is, so that what follows in the stream waits for all of
+// them).  What they read was written before the first, which is launched
+// plainly.  The longest rows' launch, a few warps busy for as long as their
+// rows take, comes first and the other launches fill the chip beside it; a
+// counter hands out the rows, since blocks begin at different times (a fixed
+// share for each block: 2.6 ms).  263 x 251 pixels x 16,000 frames, rows of 744
+// events: the integer rows 1.97 ms one launch after the other, 1.62 overlapped.
+__device__ __forceinline__ void overlap_begin() { cudaTriggerProgrammaticLaunchCompletion(); }
+__device__ __forceinline__ void overlap_end() {
+  if (blockIdx.x == 0 && threadIdx.x == 0) cudaGridDependencySynchronize();
+}
+
 template <int CAP>
 __global__ void __launch_bounds__(MT_WARPS * 32, 8)
 k_mt_thread(const uint8_t *__restrict__ plan_g, const int64_t *__restrict__ row_ptr,
@@ -459,8 +477,10 @@ k_mt_thread(const uint8_t *__restrict__ plan_g, const int64_t *__restrict__ row_
   const int scr = ((const McPlan *)plan_g)->scr;
   const int warp = threadIdx.x >> 5;
   uint32_t *wbase = (uint32_t *)smem + (size_t)warp * (CAP + scr) * 32;
+  overlap_begin();
   mt_thread_warp<CAP>(plan_g, row_ptr, row_len, pclass, ev_frame, ev_val, G2, IP, IF,
                       (blockIdx.x * MT_WARPS + warp) * 32, wbase);
+  overlap_end();
 }
 
 // ------------------------------------------------------- warp per pixel
@@ -759,8 +779,12 @@ k_mt_warp(const uint8_t *__restrict__ plan_g, const int32_t *__restrict__ list,
           const int32_t *__restrict__ count_p, int32_t min_n, int32_t cap,
           const int64_t *__restrict__ row_ptr, const int32_t *__restrict__ row_len,
           const int32_t *__restrict__ ev_frame, const float *__restrict__ ev_val,
-          float *__restrict__ G2, float *__restrict__ IP, float *__restrict__ IF) {
+          float *__restrict__ G2, float *__restrict__ IP, float *__restrict__ IF,
+          int32_t *__restrict__ next) {
   extern __shared__ __align__(16) uint8_t smem[];
+  overlap_begin();
+  const int nw = *count_p;
+  if (nw == 0) return overlap_end();
   const int D = ((const McPlan *)plan_g)->D;
   const size_t pb = mc_plan_bytes(D);
   copy_plan(smem, plan_g, pb);
@@ -768,17 +792,22 @@ k_mt_warp(const uint8_t *__restrict__ plan_g, const int32_t *__restrict__ list,
   const McPlan *pl = (const McPlan *)smem;
   const McArrays ar = mc_arrays(smem, D);
   const int ACC = max(pl->acc, pl->nlev);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwb = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t *row = (uint32_t *)(smem + pb) + (size_t)warp * (2 * cap + 32 * ACC);
   int32_t *S = (int32_t *)(row + cap);
   int32_t *acc = S + cap + lane;  // acc[k * 32]: this lane's accumulator k
-  const int nw = *count_p;
-  for (int q = blockIdx.x * nwb + warp; q < nw; q += gridDim.x * nwb) {
+  // rows one by one from a counter: blocks begin as the launch before ends
+  for (;;) {
+    int q = 0;
+    if (lane == 0) q = atomicAdd(next, 1);
+    q = __shfl_sync(0xffffffffu, q, 0);
+    if (q >= nw) break;
     const int p = list[q];
     const int n0 = row_len[p];
     if (n0 <= min_n || n0 > cap) continue;  // another launch's share of the list
     mt_warp_pixel(pl, ar, p, row_ptr[p], n0, ev_frame, ev_val, G2, IP, IF, cap, row, S, acc);
   }
+  overlap_end();
 }
 
 // ------------------------------------------------ batch work-queue launches
@@ -796,6 +825,7 @@ __global__ void __launch_bounds__(MT_WARPS * 32, 8)
 k_mt_thread_queue(const MtQueueMember *__restrict__ tab, int32_t n, int32_t total,
                   int32_t scr_max, int32_t *__restrict__ next) {
   extern __shared__ __align__(16) uint8_t smem[];
+  overlap_begin();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t *wbase = (uint32_t *)smem + (size_t)warp * (CAP + scr_max) * 32;
   for (;;) {
@@ -814,6 +844,7 @@ k_mt_thread_queue(const MtQueueMember *__restrict__ tab, int32_t n, int32_t tota
                         m.IF, (g - m.first) * 32, wbase);
     __syncwarp();
   }
+  overlap_end();
 }
 
 // Warp-per-pixel items: entry q of the members' warp lists (use_long = 0) or
@@ -823,6 +854,7 @@ __global__ void __launch_bounds__(256)
 k_mt_warp_queue(const MtQueueMember *__restrict__ tab, int32_t n, int32_t use_long,
                 int32_t min_n, int32_t cap, int32_t acc_max, int32_t *__restrict__ next) {
   extern __shared__ __align__(16) uint8_t smem[];
+  overlap_begin();
   int32_t *pref = (int32_t *)smem;  // [n + 1]: first entry of each member's list
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) {
@@ -859,6 +891,7 @@ k_mt_warp_queue(const MtQueueMember *__restrict__ tab, int32_t n, int32_t use_lo
     mt_warp_pixel(pl, ar, p, m.row_ptr[p], n0, m.ev_frame, m.ev_val, m.G2, m.IP, m.IF, cap, row,
                   S, acc);
   }
+  overlap_end();
 }
 
 // --------------------------------------------------------- float replay
@@ -1880,6 +1913,31 @@ size_t warp_smem(int D, int acc, int cap, int warps) {
   return mc_plan_bytes(D) + (size_t)warps * (2 * cap + 32 * acc) * sizeof(int32_t);
 }
 
+// A launch whose kernel may start before the one before it in the stream is
+// complete (overlap_begin / overlap_end), also as part of a captured graph.
+template <typename... Params, typename... Args>
+void launch_overlapped(void (*kernel)(Params...), int grid, int block, size_t smem,
+                       cudaStream_t st, Args... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  XG_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...));
+  XG_CHECK_LAUNCH();
+}
+
+// The kernels' row counters, before the first kernel that uses one.
+void reset_counters(Series &s, cudaStream_t st) {
+  constexpr size_t first = offsetof(DevStats, wnext), end = offsetof(DevStats, events);
+  XG_CUDA(cudaMemsetAsync((char *)s.stats.p + first, 0, end - first, st));
+}
+
 // The float rows of a series (flatfield, average, hot pixels, dense data,
 // normalize_by_framesum) on st: the warp-per-row replay when the schedule
 // allows it, else the thread-per-row one.
@@ -1894,7 +1952,6 @@ void launch_float_rows(Series &s, const McPlan &hp, cudaStream_t st, int sms) {
     prepare_framesum_scale(s);
     fscale = s.d_fscale.p;
   }
-  XG_CUDA(cudaMemsetAsync(&s.stats.p->fnext, 0, 2 * sizeof(int32_t), st));  // and ftnext
   if (s.float_cap) {
     const auto kernel = s.desc.delays_per_level <= 4 ? k_mt_fthread<8, 4> : k_mt_fthread<16, 8>;
     int per_sm = 0;
@@ -2023,26 +2080,26 @@ void run_multitau(Series &s, int mode) {
   int sms = 0;
   XG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s.device));
   XG_CUDA(cudaEventRecord(s.ev[4], st));
-  const int per_block = MT_WARPS * 32;
-  ktt<<<(P + per_block - 1) / per_block, per_block, smt, st>>>(
-      s.plan.p, s.row_ptr.p, s.row_len.p, s.pclass.p, s.ev_frame.p, s.ev_val.p, s.G2.p, s.IP.p,
-      s.IF.p);
-  XG_CHECK_LAUNCH();
-  const DevStats *ds = s.stats.p;
-  // rows of 81-256 events; long rows in two launches over one list: up to 1024
-  // events with 4 warps per block, longer ones with 2 warps per block
-  k_mt_warp<<<sms * (int)((227 * 1024) / smw), WP_WARPS * 32, smw, st>>>(
-      s.plan.p, s.wlist.p, &ds->nwarp, 0, MT_WARP_CAP, s.row_ptr.p, s.row_len.p, s.ev_frame.p,
-      s.ev_val.p, s.G2.p, s.IP.p, s.IF.p);
-  XG_CHECK_LAUNCH();
-  k_mt_warp<<<sms * (int)((227 * 1024) / smm), MID_WARPS * 32, smm, st>>>(
-      s.plan.p, s.llist.p, &ds->nlong, MT_WARP_CAP, MT_MID_CAP, s.row_ptr.p, s.row_len.p,
-      s.ev_frame.p, s.ev_val.p, s.G2.p, s.IP.p, s.IF.p);
-  XG_CHECK_LAUNCH();
+  reset_counters(s, st);
+  DevStats *ds = s.stats.p;
+  // long rows in two launches over one list: up to 1024 events with 4 warps per
+  // block, longer ones, first, with 2 warps per block; rows of 81-256 events;
+  // the thread kernel's pixels
   k_mt_warp<<<sms * (int)((227 * 1024) / sml), LONG_WARPS * 32, sml, st>>>(
       s.plan.p, s.llist.p, &ds->nlong, MT_MID_CAP, MT_LONG_CAP, s.row_ptr.p, s.row_len.p,
-      s.ev_frame.p, s.ev_val.p, s.G2.p, s.IP.p, s.IF.p);
+      s.ev_frame.p, s.ev_val.p, s.G2.p, s.IP.p, s.IF.p, &ds->wnext[0]);
   XG_CHECK_LAUNCH();
+  launch_overlapped(k_mt_warp, sms * (int)((227 * 1024) / smm), MID_WARPS * 32, smm, st,
+                    s.plan.p, s.llist.p, &ds->nlong, MT_WARP_CAP, MT_MID_CAP, s.row_ptr.p,
+                    s.row_len.p, s.ev_frame.p, s.ev_val.p, s.G2.p, s.IP.p, s.IF.p,
+                    &ds->wnext[1]);
+  launch_overlapped(k_mt_warp, sms * (int)((227 * 1024) / smw), WP_WARPS * 32, smw, st,
+                    s.plan.p, s.wlist.p, &ds->nwarp, 0, MT_WARP_CAP, s.row_ptr.p, s.row_len.p,
+                    s.ev_frame.p, s.ev_val.p, s.G2.p, s.IP.p, s.IF.p, &ds->wnext[2]);
+  const int per_block = MT_WARPS * 32;
+  launch_overlapped(ktt, (P + per_block - 1) / per_block, per_block, smt, st, s.plan.p,
+                    s.row_ptr.p, s.row_len.p, s.pclass.p, s.ev_frame.p, s.ev_val.p, s.G2.p,
+                    s.IP.p, s.IF.p);
   XG_CUDA(cudaEventRecord(s.ev[5], st));
   launch_float_rows(s, *hp, st, sms);
   XG_CUDA(cudaEventRecord(s.ev[6], st));
@@ -2087,6 +2144,33 @@ void mt_queue_run(const std::vector<Series *> &ss, MtQueue &q, cudaStream_t st) 
   XG_CUDA(cudaGetDevice(&dev));
   XG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   XG_CUDA(cudaMemsetAsync(q.next.p, 0, sizeof(int32_t) * (MT_THREAD_NCAPS + 3), st));
+  // the warp-per-pixel tiers over every member, longest rows first: rows of
+  // 1025-4096, 257-1024 and 81-256 events; then the thread kernels
+  const int tiers[3][4] = {{1, MT_MID_CAP, MT_LONG_CAP, LONG_WARPS},
+                           {1, MT_WARP_CAP, MT_MID_CAP, MID_WARPS},
+                           {0, 0, MT_WARP_CAP, WP_WARPS}};
+  const size_t pref_bytes = mc_align16(sizeof(int32_t) * (size_t)(n + 1));
+  for (int t = 0; t < 3; t++) {
+    const int cap = tiers[t][2], warps = tiers[t][3];
+    const size_t sm = pref_bytes + (size_t)warps * (2 * cap + 32 * q.acc_max) * sizeof(int32_t);
+    if (sm > 227 * 1024)
+      throw Error(XPCS_ERR_INVALID_ARGUMENT, "delay schedule too large for the multi-tau kernels");
+    XG_CUDA(cudaFuncSetAttribute(k_mt_warp_queue, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sm));
+    int per_sm = 0;
+    XG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mt_warp_queue, warps * 32,
+                                                          sm));
+    const int grid = sms * std::max(1, per_sm);
+    int32_t *next = q.next.p + MT_THREAD_NCAPS + t;
+    if (t == 0) {
+      k_mt_warp_queue<<<grid, warps * 32, sm, st>>>(q.tab.p, n, tiers[t][0], tiers[t][1], cap,
+                                                    q.acc_max, next);
+      XG_CHECK_LAUNCH();
+    } else {
+      launch_overlapped(k_mt_warp_queue, grid, warps * 32, sm, st, q.tab.p, n, tiers[t][0],
+                        tiers[t][1], cap, q.acc_max, next);
+    }
+  }
   using QueueKernel = void (*)(const MtQueueMember *, int32_t, int32_t, int32_t, int32_t *);
   const QueueKernel kq[MT_THREAD_NCAPS] = {k_mt_thread_queue<32>, k_mt_thread_queue<48>,
                                            k_mt_thread_queue<64>, k_mt_thread_queue<80>,
@@ -2101,35 +2185,15 @@ void mt_queue_run(const std::vector<Series *> &ss, MtQueue &q, cudaStream_t st) 
     XG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kq[c], MT_WARPS * 32, smt));
     const int blocks = std::min(sms * std::max(1, per_sm), (q.cap_groups[c] + MT_WARPS - 1) /
                                                                MT_WARPS);
-    kq[c]<<<std::max(1, blocks), MT_WARPS * 32, smt, st>>>(q.tab.p + q.cap_first[c],
-                                                           q.cap_count[c], q.cap_groups[c],
-                                                           q.scr_max, q.next.p + c);
-    XG_CHECK_LAUNCH();
-  }
-  // the warp-per-pixel tiers over every member: rows of 81-256, 257-1024 and
-  // 1025-4096 events (the thread kernels above wrote zeros for those pixels)
-  const int tiers[3][4] = {{0, 0, MT_WARP_CAP, WP_WARPS},
-                           {1, MT_WARP_CAP, MT_MID_CAP, MID_WARPS},
-                           {1, MT_MID_CAP, MT_LONG_CAP, LONG_WARPS}};
-  const size_t pref_bytes = mc_align16(sizeof(int32_t) * (size_t)(n + 1));
-  for (int t = 0; t < 3; t++) {
-    const int cap = tiers[t][2], warps = tiers[t][3];
-    const size_t sm = pref_bytes + (size_t)warps * (2 * cap + 32 * q.acc_max) * sizeof(int32_t);
-    if (sm > 227 * 1024)
-      throw Error(XPCS_ERR_INVALID_ARGUMENT, "delay schedule too large for the multi-tau kernels");
-    XG_CUDA(cudaFuncSetAttribute(k_mt_warp_queue, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)sm));
-    int per_sm = 0;
-    XG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mt_warp_queue, warps * 32,
-                                                          sm));
-    k_mt_warp_queue<<<sms * std::max(1, per_sm), warps * 32, sm, st>>>(
-        q.tab.p, n, tiers[t][0], tiers[t][1], cap, q.acc_max, q.next.p + MT_THREAD_NCAPS + t);
-    XG_CHECK_LAUNCH();
+    launch_overlapped(kq[c], std::max(1, blocks), MT_WARPS * 32, smt, st,
+                      q.tab.p + q.cap_first[c], q.cap_count[c], q.cap_groups[c], q.scr_max,
+                      q.next.p + c);
   }
   for (Series *sp : ss) {  // float rows, member by member (none in integer data)
     Series &s = *sp;
     if (s.D == 0 || s.P == 0) continue;
     const McPlan hp = *(const McPlan *)make_plan(s, s.plan_mode).data();
+    reset_counters(s, st);
     launch_float_rows(s, hp, st, sms);
   }
 }

@@ -199,7 +199,10 @@ struct DevStats {
   int32_t nwarp;
   int32_t nlong;
   int32_t nfthread;  // float rows of the thread-per-pixel float kernel
-  int32_t fnext, ftnext;  // ftnext: next 32 pixels of k_mt_fthread; fnext: next float-path pixel to hand out (k_mt_fwarp)
+  // counters from which the multi-tau kernels hand out their rows, zeroed before
+  // each run (wnext up to events): k_mt_warp's three launches (index into its
+  // list), k_mt_fwarp (index into the float list), k_mt_fthread (32 pixels)
+  int32_t wnext[3], fnext, ftnext;
   unsigned long long events;
   unsigned long long dropped;  // K-a items sorted last (unused frames, bad pixel indices)
 };
