@@ -30,10 +30,11 @@
 // k_mt_thread: one thread per pixel, rows packed (frame << 16 | int16 value)
 //   in shared memory with a lane-interleaved layout (conflict-free), outputs
 //   written straight to [D][P] (32 consecutive pixels per warp = coalesced).
-//   Levels of few bins find pairs from an occupancy bitmask of the row in the
-//   thread's scratch words; sparse levels check each source's next two
-//   entries without branching.  Pixels of other classes get zeros here and
-//   are rewritten by the kernels below.
+//   Dense levels take their pairs by byte products over windows of the level's
+//   bins in the thread's scratch words; levels of few bins whose values do not
+//   fit bytes, or with more than 8 delays, find pairs from an occupancy bitmask
+//   there; sparse levels check each source's next two entries without
+//   branching.  Pixels of other classes are left to the kernels below.
 // k_mt_warp:   one warp per pixel, rows packed in shared memory: rows of up
 //   to 256 events (8 warps per block), up to 1024 (4 warps per block) and up
 //   to 4096 (2 warps per block).
@@ -60,6 +61,14 @@ constexpr int MID_WARPS = 4;
 // events each, take 2.95 / 2.25 / 2.00 / 1.97 / 1.98 ms with 0 (pairs by
 // search and bitmask only) / 4 / 8 / 16 / 40.
 constexpr int MB_RATIO = 16;
+// The same for the thread kernel (mt_thread_rows), of the warp's longest row, and
+// the scratch words that its windows have at least.  At 1 Mpx x 10,000 frames,
+// rows of 50 events, the integer rows take 2.53 / 2.29 / 2.27 / 2.26 / 2.25 /
+// 2.41 ms with 0 / 4 / 8 / 12 / 16 / 20 bins per entry; at 512 x 512 x 1,000
+// frames, rows of 10 and 4 delays a level, 161 / 143 / 139 / 141 us with 8 / 10
+// / 12 / 16 words (8 are too few for any level's window).
+constexpr int TB_RATIO = 12;
+constexpr int MT_MIN_SCR = 12;
 constexpr int LONG_WARPS = 2;  // warps per block for rows of up to MT_LONG_CAP events
 
 // std::lower_bound as libstdc++ implements it (halving the remaining length),
@@ -165,6 +174,74 @@ __device__ __forceinline__ void bins_pairs(const uint32_t *row, int m, int lf, i
 #pragma unroll
   for (int k = 0; k < KM; k++)
     if (k < count) acc[k * 32] = a[k];
+}
+
+// Denser levels (at most TB_RATIO bins per entry of the warp's longest row):
+// windows of the level's bins lie in the thread's W scratch words as bytes, one
+// a bin, zero where no entry is.  The partners of 4 bins for delay tlo + k are
+// the 4 bytes tlo + k further on: a funnel shift of two words gives them and a
+// 4-way byte product the sum, so that a word costs 1 + 3 shifts and KM products
+// whatever its bins hold, and no lane waits for another's search.  (Measured
+// beside TB_RATIO; KM = 16 took 107 registers instead of 61 and was slower at
+// every size.)  After a window the words that held only partners move to the
+// front.  False (the same
+// for all lanes): a value of some lane is not within a byte; acc is undefined.
+template <int KM>
+__device__ __forceinline__ bool byte_pairs_thread(const uint32_t *row, int m, int lf, int tlo,
+                                                  int count, int W, int32_t *acc) {
+  constexpr int Q = KM / 4;
+  const int off = tlo >> 2, sh = (tlo & 3) * 8, H = off + Q + 1;  // H: words of partners only
+  int a[KM];
+#pragma unroll
+  for (int k = 0; k < KM; k++) a[k] = 0;
+  for (int q = 0; q < W; q++) acc[q * 32] = 0;
+  unsigned most = 0;  // a negative value is past 255 as well
+  int i = 0;
+  uint32_t e = m > 0 ? row[0] : 0u;
+  for (int b0 = 0;;) {
+    const int bend = b0 + 4 * W;
+    while (i < m && pk_t(e) < bend) {
+      const int r = pk_t(e) - b0;
+      most = max(most, e & 0xffffu);
+      ((uint8_t *)acc)[(r >> 2) * 128 + (r & 3)] = (uint8_t)e;
+      i++;
+      e = row[i * 32];  // one past the row at most: a scratch word, not used
+    }
+    const int nown = min(W - H, (lf - b0 + 3) >> 2);
+    const int32_t *X = acc + off * 32;
+    // s[q][r]: the 4 bytes from 4 (w + q) + tlo + r on
+    uint32_t s[Q][4], x1 = X[32], z = __funnelshift_r(X[0], x1, sh);
+    const auto next = [&](int w, uint32_t (&d)[4]) {  // word w of the shifted stream
+      const uint32_t x2 = X[(w + 2) * 32], z1 = __funnelshift_r(x1, x2, sh);
+      d[0] = z;
+#pragma unroll
+      for (int r = 1; r < 4; r++) d[r] = __funnelshift_r(z, z1, 8 * r);
+      x1 = x2;
+      z = z1;
+    };
+#pragma unroll
+    for (int q = 0; q < Q - 1; q++) next(q, s[q + 1]);
+#pragma unroll 4
+    for (int w = 0; w < nown; w++) {
+#pragma unroll
+      for (int q = 0; q < Q - 1; q++)
+#pragma unroll
+        for (int r = 0; r < 4; r++) s[q][r] = s[q + 1][r];
+      next(w + Q - 1, s[Q - 1]);
+      const uint32_t own = acc[w * 32];
+#pragma unroll
+      for (int k = 0; k < KM; k++) a[k] = (int)__dp4a(own, s[k / 4][k % 4], (unsigned)a[k]);
+    }
+    b0 += 4 * nown;
+    if (b0 >= lf) break;
+    for (int h = 0; h < H; h++) acc[h * 32] = acc[(nown + h) * 32];
+    for (int h = H; h < W; h++) acc[h * 32] = 0;
+  }
+  if (__any_sync(0xffffffffu, most > 255u)) return false;
+#pragma unroll
+  for (int k = 0; k < KM; k++)
+    if (k < count) acc[k * 32] = a[k];
+  return true;
 }
 
 // The 32 consecutive pixels of a warp (this lane's is p; mine: its outputs are
@@ -294,8 +371,34 @@ __device__ __forceinline__ void mt_thread_rows(const uint8_t *__restrict__ plan_
     const bool sorted = mode != XPCS_MODE_REFERENCE || (J && U);
     const int tlo = L.tau_lo, thi = L.tau_lo + L.count - 1;
     // warp-uniform: every lane of the warp sees the same level
+    const int lf = L.lastframe;
+    bool bytes = false;
+    if (tlo >= 1 && L.count <= 8 && (tlo >> 2) + 8 <= scr &&
+        lf <= TB_RATIO * __reduce_max_sync(0xffffffffu, m)) {
+      if (L.count <= 4)
+        bytes = byte_pairs_thread<4>(row, m, lf, tlo, L.count, scr, acc);
+      else
+        bytes = byte_pairs_thread<8>(row, m, lf, tlo, L.count, scr, acc);
+    }
     const bool bins = tlo >= 1 && thi <= 64 && L.count <= 16 && L.lastframe <= 32 * scr;
-    if (bins && sorted) {
+    if (bytes) {
+      if (!sorted) {
+        // taken out again: entries that lower_bound over the whole buffer does
+        // not find (none up to the tail's first bin when the tail ascends)
+        const int tail0 = U && m < n0 ? pk_t(row[m * 32]) : (U ? INT_MAX : -1);
+        for (int j = 1; j < m; j++) {
+          const uint32_t wj = row[j * 32];
+          const int tj = pk_t(wj);
+          if (tj <= tail0 || lower_bound_packed(row, n0, tj) == j) continue;
+          for (int i = j - 1; i >= 0; i--) {
+            const uint32_t wi = row[i * 32];
+            const int d = tj - pk_t(wi);
+            if (d > thi) break;
+            if (d >= tlo) acc[(d - tlo) * 32] -= pk_v(wi) * pk_v(wj);
+          }
+        }
+      }
+    } else if (bins && sorted) {
       // mask words in the scratch: zeroed, then one store per word that holds
       // an entry (the bins increase along the prefix)
       const int nw = (L.lastframe + 31) >> 5;
@@ -468,7 +571,7 @@ __device__ __forceinline__ void overlap_end() {
 }
 
 template <int CAP>
-__global__ void __launch_bounds__(MT_WARPS * 32, 8)
+__global__ void __launch_bounds__(MT_WARPS * 32, 16)
 k_mt_thread(const uint8_t *__restrict__ plan_g, const int64_t *__restrict__ row_ptr,
             const int32_t *__restrict__ row_len, const uint8_t *__restrict__ pclass,
             const int32_t *__restrict__ ev_frame, const float *__restrict__ ev_val,
@@ -821,7 +924,7 @@ k_mt_warp(const uint8_t *__restrict__ plan_g, const int32_t *__restrict__ list,
 // Thread-per-pixel items: group g of the queue is group g - first of the
 // member whose range holds it.  wbase strides by the batch's largest scratch.
 template <int CAP>
-__global__ void __launch_bounds__(MT_WARPS * 32, 8)
+__global__ void __launch_bounds__(MT_WARPS * 32, 16)
 k_mt_thread_queue(const MtQueueMember *__restrict__ tab, int32_t n, int32_t total,
                   int32_t scr_max, int32_t *__restrict__ next) {
   extern __shared__ __align__(16) uint8_t smem[];
@@ -1341,7 +1444,7 @@ __device__ __forceinline__ int na_class(const NaRows &v, int64_t b, int n) {
 // classifying its own; every other pixel gets zeros here, overwritten by the
 // kernels below.
 template <int CAP>
-__global__ void __launch_bounds__(MT_WARPS * 32, 8) k_na_thread(NaRows v) {
+__global__ void __launch_bounds__(MT_WARPS * 32, 16) k_na_thread(NaRows v) {
   extern __shared__ __align__(16) uint8_t smem[];
   const int scr = ((const McPlan *)v.plan)->scr;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1884,7 +1987,7 @@ std::vector<uint8_t> make_plan(const Series &s, int mode) {
   }
   pl->nlev = nlev;
   pl->acc = acc;
-  pl->scr = std::max(acc, nlev) + std::max(0, s.scr_extra);
+  pl->scr = std::max(std::max(acc, nlev), MT_MIN_SCR) + std::max(0, s.scr_extra);
   for (int k = 1; k < D; k++)
     if (t_ip[k] >= t_ip[k - 1] || tau_abs[k] <= tau_abs[k - 1])
       throw Error(XPCS_ERR_INVALID_ARGUMENT, "delay thresholds are not monotone");
