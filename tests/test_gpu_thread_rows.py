@@ -1,10 +1,11 @@
 """Rows of the thread-per-pixel kernel, bit for bit against the oracle in both
 modes: delays per level below, at and above what the byte products of the denser
 levels take, row capacities from the smallest to the largest, series whose
-levels end inside a word of four bins and at its end, rows that are spread out,
-packed into one part of the series or into two (their buffer falls out of order
-at the high levels), empty and full rows, counts that reach 255, 256 and more at
-one level or another in some lanes of a warp, and values below zero."""
+levels end inside a word of four bins and at its end, the last frame that fits
+16 bits, rows that are spread out, packed into one part of the series or into
+two (their buffer falls out of order at the high levels), empty and full rows,
+counts that reach 255, 256 and more at one level or another in some lanes of a
+warp, and values below zero."""
 import numpy as np
 import pytest
 
@@ -25,6 +26,7 @@ CASES = {
     "dpl_9": (1003, 9, 50, 1, 4),
     "dpl_16": (2500, 16, 30, 1, 4),
     "long": (20000, 8, 60, 1, 3),
+    "65536_frames": (65536, 8, 20, 1, 3),
     "short": (61, 4, 15, 1, 3),
     "full": (100, 4, 70, 1, 3),
     "counts_to_255": (402, 4, 9, 60, 256),
