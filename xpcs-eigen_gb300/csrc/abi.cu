@@ -243,6 +243,7 @@ void free_series(Series *s) {
     s->blk_len.release(st);
     s->blk_rp.release(st);
     s->blk_tot.release(st);
+    s->blk_pos.release(st);
     s->stats.release(st);
     cudaStreamSynchronize(st);
     for (auto &e : s->ev)

@@ -1115,9 +1115,18 @@ k_merge_block(int32_t P, int32_t avg, const int64_t *__restrict__ row_ptr,
   const int64_t b = has ? row_ptr[p] : 0;
   const int32_t n = has ? (int32_t)(row_ptr[p + 1] - b) : 0;
   int32_t out = 0;
+  // one coalesced look at the warp's events: no two equal frames in a row, no
+  // repeated frame (equal ones may also be the end of one row and the start of
+  // the next, so the lanes then look for themselves)
+  const int lane = threadIdx.x & 31;
+  const int64_t lo = __shfl_sync(0xffffffffu, b, 0);
+  const int64_t hi = row_ptr[min(p - lane + 32, P)];
+  bool maybe = false;
+  for (int64_t e = lo + 1 + lane; e < hi; e += 32) maybe |= fr[e] == fr[e - 1];
+  maybe = __any_sync(0xffffffffu, maybe);
   if (has && mask[p]) {
     bool dup = false;
-    for (int32_t i = 1; i < n && !dup; i++) dup = fr[b + i] == fr[b + i - 1];
+    for (int32_t i = 1; maybe && i < n && !dup; i++) dup = fr[b + i] == fr[b + i - 1];
     if (dup || avg != 1) {
       const float favg = (float)avg;
       int32_t i = 0;
@@ -1142,35 +1151,76 @@ k_merge_block(int32_t P, int32_t avg, const int64_t *__restrict__ row_ptr,
   }
 }
 
-// Merged row lengths of every block summed per pixel.
+// Merged row lengths of every block summed per pixel; pos: the events that a
+// pixel has before each block.
 __global__ void k_block_totals(int32_t P, int32_t nblk, const int32_t *__restrict__ blk_len,
-                               int32_t *__restrict__ tot) {
+                               int32_t *__restrict__ pos, int32_t *__restrict__ tot) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= P) return;
   int32_t t = 0;
-  for (int32_t k = 0; k < nblk; k++) t += blk_len[(size_t)k * P + p];
+#pragma unroll 4
+  for (int32_t k = 0; k < nblk; k++) {
+    pos[(size_t)k * P + p] = t;
+    t += blk_len[(size_t)k * P + p];
+  }
   tot[p] = t;
 }
 
 // Each pixel's block segments, in block order, copied to its row of the
-// series' event lists.
-__global__ void k_gather_blocks(int32_t P, int32_t nblk, const int64_t *__restrict__ blk_base,
-                                const int32_t *__restrict__ blk_off,
-                                const int32_t *__restrict__ blk_len,
-                                const int32_t *__restrict__ bfr, const float *__restrict__ bval,
-                                const int64_t *__restrict__ row_ptr, int32_t *__restrict__ fr,
-                                float *__restrict__ val) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P) return;
-  int64_t d = row_ptr[p];
-  for (int32_t k = 0; k < nblk; k++) {
-    const int32_t n = blk_len[(size_t)k * P + p];
-    const int64_t src = blk_base[k] + blk_off[(size_t)k * P + p];
-    for (int32_t i = 0; i < n; i++) {
-      fr[d + i] = bfr[src + i];
-      val[d + i] = bval[src + i];
+// series' event lists.  One warp per 32 pixels and block: the segments of
+// consecutive pixels follow each other in a block (with gaps where the merge
+// shortened one), so the lanes take the range's events in order, 4 at a time,
+// find each event's pixel among the 32 starts and place it in that pixel's
+// row.  Warps of one pixel group follow each other, so that the short runs
+// that they write meet in L2.  512 x 512 pixels in 10 blocks, 12.3 M events
+// (bandwidth: 30 us): 228 us with one thread a pixel, 134 with one warp for all
+// blocks of its pixels, 55 so.
+__global__ void __launch_bounds__(256)
+k_gather_blocks(int32_t P, int32_t nblk, const int64_t *__restrict__ blk_base,
+                const int32_t *__restrict__ blk_off, const int32_t *__restrict__ blk_len,
+                const int32_t *__restrict__ pos, const int32_t *__restrict__ bfr,
+                const float *__restrict__ bval, const int64_t *__restrict__ row_ptr,
+                int32_t *__restrict__ fr, float *__restrict__ val) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int64_t w = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int64_t group = w / nblk;
+  if (group * 32 >= P) return;
+  const int k = (int)(w - group * nblk), p0 = (int)group * 32, p = p0 + lane;
+  const int last = min(31, P - 1 - p0);
+  const size_t q = (size_t)k * P + p;
+  const int64_t d0 = row_ptr[p0];
+  // this lane's segment: its place from the first row's start on, its length
+  // and its start in the block
+  const int64_t d = p < P ? row_ptr[p] - d0 + pos[q] : 0;
+  const int32_t n = p < P ? blk_len[q] : 0, off = p < P ? blk_off[q] : INT32_MAX;
+  const int64_t base = blk_base[k];
+  const int32_t lo = __shfl_sync(FULL, off, 0);
+  const int32_t hi = __shfl_sync(FULL, off + n, last);
+  for (int32_t e0 = lo; e0 < hi; e0 += 128) {
+    int32_t f[4];
+    float v[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const int32_t e = e0 + u * 32 + lane;
+      f[u] = e < hi ? bfr[base + e] : 0;
+      v[u] = e < hi ? bval[base + e] : 0.f;
     }
-    d += n;
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const int32_t e = e0 + u * 32 + lane;
+      int own = 0;  // the last lane whose segment starts at or before e
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+        if (__shfl_sync(FULL, off, (own + o) & 31) <= e) own += o;
+      const int32_t i = e - __shfl_sync(FULL, off, own);
+      const int64_t dst = d0 + __shfl_sync(FULL, d, own) + i;
+      const int32_t len = __shfl_sync(FULL, n, own);  // by all lanes
+      if (e < hi && i < len) {
+        fr[dst] = f[u];
+        val[dst] = v[u];
+      }
+    }
   }
 }
 
@@ -1182,12 +1232,15 @@ void gather_blocks(Series &s) {
   const int32_t P = s.P, nblk = (int32_t)s.blk_base.size();
   s.blk_tot.reserve(P, st);
   if (nblk > 0) {
-    k_block_totals<<<(P + 255) / 256, 256, 0, st>>>(P, nblk, s.blk_len.p, s.blk_tot.p);
+    s.blk_pos.reserve((size_t)nblk * P, st);
+    k_block_totals<<<(P + 255) / 256, 256, 0, st>>>(P, nblk, s.blk_len.p, s.blk_pos.p,
+                                                    s.blk_tot.p);
     XG_CHECK_LAUNCH();
     exclusive_scan_i32_i64(s.blk_tot.p, s.row_ptr.p, P, s.scan_tmp.p, st);
-    k_gather_blocks<<<(P + 255) / 256, 256, 0, st>>>(P, nblk, s.d_blk_base.p, s.blk_off.p,
-                                                     s.blk_len.p, s.blk_fr.p, s.blk_val.p,
-                                                     s.row_ptr.p, s.ev_frame.p, s.ev_val.p);
+    const int64_t warps = (int64_t)((P + 31) / 32) * nblk;  // below 2^31 blocks of 8
+    k_gather_blocks<<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(
+        P, nblk, s.d_blk_base.p, s.blk_off.p, s.blk_len.p, s.blk_pos.p, s.blk_fr.p, s.blk_val.p,
+        s.row_ptr.p, s.ev_frame.p, s.ev_val.p);
     XG_CHECK_LAUNCH();
   } else {
     XG_CUDA(cudaMemsetAsync(s.row_ptr.p, 0, sizeof(int64_t) * ((size_t)P + 1), st));

@@ -293,6 +293,7 @@ struct Series {
   DBuf<int32_t> blk_off, blk_len;  // [block][P]: row start in its block, merged length
   DBuf<int64_t> blk_rp;       // row pointers of the block being transposed
   DBuf<int32_t> blk_tot;      // merged events per pixel over every block
+  DBuf<int32_t> blk_pos;      // [block][pixel] events of the pixel before the block
   DBuf<int64_t> row_ptr;    // [P+1]
   DBuf<int32_t> row_len;    // events per pixel after merging duplicates
   DBuf<uint8_t> pclass;
