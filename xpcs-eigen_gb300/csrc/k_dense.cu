@@ -505,6 +505,7 @@ __global__ void k_px_totals(int32_t P, int32_t nblk, const int32_t *__restrict__
 }
 
 constexpr int KB_VT = 128;  // raw values from a pixel's threshold up in its value table
+constexpr int KB_GW = 4;    // warps per block of the gather
 
 struct PxGather {
   int32_t P, F, tcap, fcap, force_float, nblk, has_dark;
@@ -524,93 +525,118 @@ struct PxGather {
   DevStats *stats;
 };
 
-// One block per 32 pixels, each warp taking 4 of them in turn: a pixel's
-// packed entries of every block, in block order, become (frame, value) in its
-// row of the event lists.  For a given pixel the value is a function of the
-// raw value alone: the warp first forms it, as the frame-major write does,
-// for the 128 raw values from the pixel's threshold up (where nearly all kept
-// values lie) and looks those up; others are formed directly.  The row's
-// length, whether every value is an integer and sum |v| are collected on the
-// way, and the block's first warp classifies the 32 pixels as the merge pass
-// does for transposed rows (no row has two events of one frame here).
-__global__ void __launch_bounds__(256)
+// One warp per 32 pixels, one after the other: a pixel's packed entries of
+// every block, in block order, become (frame, value) in its row of the event
+// lists.  For a given pixel the value is a function of the raw value alone: the
+// warp forms it once, as the frame-major write does, for the raw values from
+// the pixel's threshold up, 32 at a time as far as the row's entries need them
+// (up to 128, where nearly all kept values lie) and looks those up; others are
+// formed directly.  The lanes read the 32 pixels' places together, and a pixel's
+// first entries are loaded while the one before is formed.  The row's length,
+// whether every value is an integer and sum |v| are collected on the way, and
+// the warp classifies its 32 pixels as the merge pass does for transposed rows
+// (no row has two events of one frame here).
+// 960 x 960 pixels, rows of 154 entries (bandwidth: 250 us): 1.27 ms with all 128
+// values formed for each pixel and 8 warps waiting for each other, 0.83 ms so.
+__global__ void __launch_bounds__(KB_GW * 32)
 k_dense_gather_px(PxGather g) {
-  __shared__ float s_tab[KB_WARPS][KB_VT];
-  __shared__ int32_t s_n[32], s_nonint[32];
-  __shared__ long long s_tot[32];
+  __shared__ float s_tab[KB_GW][KB_VT];
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int pb = blockIdx.x * 32;
-  for (int q = 0; q < 32 / KB_WARPS; q++) {
-    const int loc = q * KB_WARPS + w, p = pb + loc;
-    if (p >= g.P) break;
-    const int32_t rlo = g.rmin[p];
+  const int p0 = (blockIdx.x * KB_GW + w) * 32, pl = p0 + lane;
+  if (p0 >= g.P) return;
+  const bool has = pl < g.P;
+  float *tab = s_tab[w];
+  // of the lane's pixel: threshold, row, first block's entries
+  const int32_t rl = has ? g.rmin[pl] : KB_NEVER;
+  const bool live = rl < KB_NEVER && g.nblk > 0;
+  const int64_t dl = live ? g.row_ptr[pl] : 0;
+  const int32_t nl = live ? g.blk_len[pl] : 0;
+  const int64_t sl = live ? g.blk_base[0] + g.blk_off[pl] : 0;
+  int32_t c_n = 0;       // the lane's pixel: length, all integers, sum |v|
+  bool c_int = true;
+  int c_tot = 0;
+  uint32_t e[4];
+  const auto load = [&](int64_t src, int32_t i0, int32_t nk, uint32_t (&x)[4]) {
+#pragma unroll
+    for (int h = 0; h < 4; h++) {
+      const int32_t i = i0 + h * 32 + lane;
+      x[h] = i < nk ? __ldcs(g.pk + src + i) : 0u;
+    }
+  };
+  load(__shfl_sync(FULL, sl, 0), 0, __shfl_sync(FULL, nl, 0), e);
+  for (int q = 0; q < 32 && p0 + q < g.P; q++) {
+    const int p = p0 + q;
+    const int32_t rlo = __shfl_sync(FULL, rl, q);
+    int64_t d = __shfl_sync(FULL, dl, q);
+    int64_t src = __shfl_sync(FULL, sl, q);
+    int32_t nk = __shfl_sync(FULL, nl, q);
+    // the next pixel's first entries
+    const int32_t next_n = q < 31 ? __shfl_sync(FULL, nl, q + 1) : 0;
+    uint32_t en[4];
+    load(__shfl_sync(FULL, sl, (q + 1) & 31), 0, next_n, en);
     int32_t n = 0;
     bool nonint = false;
-    long long tot = 0;
+    int tot = 0, built = 0;
     if (rlo < KB_NEVER) {
-      for (int i = lane; i < KB_VT; i += 32)
-        s_tab[w][i] = rlo + i <= 32767
-                          ? dense_event_value(rlo + i, g.has_dark, g.avg, g.flat, g.prep, p)
-                          : 0.f;
-      __syncwarp();
-      int64_t d = g.row_ptr[p];
       for (int32_t k = 0; k < g.nblk; k++) {
-        const int32_t nk = g.blk_len[(size_t)k * g.P + p];
-        const int64_t src = g.blk_base[k] + g.blk_off[(size_t)k * g.P + p];
+        if (k > 0) {
+          nk = g.blk_len[(size_t)k * g.P + p];
+          src = g.blk_base[k] + g.blk_off[(size_t)k * g.P + p];
+          load(src, 0, nk, e);
+        }
         const int32_t r0 = g.blk_r0[k];
-        // four 32-entry chunks' loads in flight before any is used
         for (int32_t i0 = 0; i0 < nk; i0 += 4 * 32) {
-          uint32_t e[4];
+          if (i0 > 0) load(src, i0, nk, e);
+          int top = 0;  // >= 0: kept values pass the threshold
+#pragma unroll
+          for (int h = 0; h < 4; h++)
+            if (i0 + h * 32 + lane < nk) top = max(top, (int32_t)(int16_t)(e[h] & 0xffffu) - rlo);
+          top = min(__reduce_max_sync(FULL, top), KB_VT - 1);
+          for (; built <= top; built += 32)
+            tab[built + lane] = rlo + built + lane <= 32767
+                                    ? dense_event_value(rlo + built + lane, g.has_dark, g.avg,
+                                                        g.flat, g.prep, p)
+                                    : 0.f;
+          __syncwarp();
 #pragma unroll
           for (int h = 0; h < 4; h++) {
             const int32_t i = i0 + h * 32 + lane;
-            e[h] = i < nk ? __ldcs(g.pk + src + i) : 0u;
-          }
-#pragma unroll
-          for (int h = 0; h < 4; h++) {
-            if (i0 + h * 32 >= nk) break;  // the same for every lane
-            const int32_t i = i0 + h * 32 + lane;
-            bool ni = false;
-            unsigned a = 0;
             if (i < nk) {
-              const int32_t raw = (int16_t)(e[h] & 0xffffu);
-              const int32_t t = raw - rlo;  // >= 0: kept values pass the threshold
-              const float v = t < KB_VT ? s_tab[w][t]
+              const int32_t raw = (int16_t)(e[h] & 0xffffu), t = raw - rlo;
+              const float v = t < KB_VT ? tab[t]
                                         : dense_event_value(raw, g.has_dark, g.avg, g.flat,
                                                             g.prep, p);
               g.fr[d + i] = r0 + (int32_t)(e[h] >> 16);
               g.val[d + i] = v;
-              ni = !(v == truncf(v) && fabsf(v) < 16777216.f);
-              a = ni ? 0u : (unsigned)fabsf(v);
+              const bool ni = !(v == truncf(v) && fabsf(v) < 16777216.f);
+              nonint |= ni;
+              // a sum past 2^24 makes a float row whatever it is
+              tot = ni ? tot : min(tot + (int)fabsf(v), 1 << 24);
             }
-            nonint = nonint || __any_sync(FULL, ni);
-            tot += __reduce_add_sync(FULL, a);
           }
         }
         d += nk;
         n += nk;
       }
-      __syncwarp();  // the table is rebuilt for the warp's next pixel
+      __syncwarp();  // the table is rebuilt for the next pixel
     }
-    if (lane == 0) {
-      s_n[loc] = n;
-      s_nonint[loc] = nonint ? 1 : 0;
-      s_tot[loc] = tot;
-      g.row_len[p] = n;
+    nonint = __any_sync(FULL, nonint);
+    tot = __reduce_add_sync(FULL, tot);
+    if (lane == q) {
+      c_n = n;
+      c_int = !nonint;
+      c_tot = tot;
     }
+#pragma unroll
+    for (int h = 0; h < 4; h++) e[h] = en[h];
   }
-  __syncthreads();
-  if (w == 0) {
-    const int p = pb + lane;
-    const bool has = p < g.P;
-    const int32_t n = has ? s_n[lane] : 0;
-    uint8_t c = has && g.mask[p] ? pixel_class(n, s_nonint[lane] == 0, s_tot[lane], g.F, g.tcap)
-                                 : (uint8_t)PCLASS_EMPTY;
-    if (g.force_float && c != PCLASS_EMPTY) c = PCLASS_FLOAT;  // values rescaled later
-    c = float_class(c, n, g.fcap);
-    record_class_warp(has, p, c, n, g.pclass, g.cl, g.stats);
-  }
+  if (has) g.row_len[pl] = c_n;
+  uint8_t c = has && g.mask[pl] ? pixel_class(c_n, c_int, c_tot, g.F, g.tcap)
+                                : (uint8_t)PCLASS_EMPTY;
+  if (g.force_float && c != PCLASS_EMPTY) c = PCLASS_FLOAT;  // values rescaled later
+  c = float_class(c, c_n, g.fcap);
+  record_class_warp(has, pl, c, c_n, g.pclass, g.cl, g.stats);
 }
 
 }  // namespace
@@ -792,7 +818,7 @@ void dense_px_gather(Series &s) {
              s.d_mask.p, s.rmin.p, s.dark_avg.p, s.has_flat ? s.d_flat.p : nullptr,
              (const DensePrep *)s.dn_prep.p, s.ev_frame.p, s.ev_val.p, s.row_len.p, s.pclass.p,
              ClassLists{s.wlist.p, s.llist.p, s.flist.p}, s.stats.p};
-  k_dense_gather_px<<<(P + 31) / 32, KB_WARPS * 32, 0, st>>>(g);
+  k_dense_gather_px<<<(P + 32 * KB_GW - 1) / (32 * KB_GW), KB_GW * 32, 0, st>>>(g);
   XG_CHECK_LAUNCH();
 }
 
