@@ -503,7 +503,7 @@ int xpcs_multitau(xpcs_series *h, int32_t mode) {
     DeviceGuard g(s.device);
     const int64_t l0 = tl_launches;
     XG_CUDA(cudaEventRecord(s.ev[2], s.stream));
-    run_filter_transpose(s);
+    run_filter_transpose(s, true);
     XG_CUDA(cudaEventRecord(s.ev[3], s.stream));
     run_multitau(s, mode);
     s.launches = (int32_t)(tl_launches - l0);
@@ -608,7 +608,7 @@ int xpcs_twotime(xpcs_series *h, const xpcs_twotime_desc *d, int32_t mode,
     req.average = d->average != 0;
     req.window = d->window;
     req.frame_threading = d->frame_threading != 0;
-    run_filter_transpose(s);
+    run_filter_transpose(s, true);
     run_twotime(s, req, mode == XPCS_MODE_REFERENCE ? XPCS_MODE_REFERENCE : XPCS_MODE_EXACT,
                 mode == XPCS_TWOTIME_EXACT_CUDA_CORES);
     sync_and_check(s);

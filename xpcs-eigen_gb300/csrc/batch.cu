@@ -113,7 +113,7 @@ int32_t autotune(Series &s, int mode) {
     float ms = 0.f;
     for (int rep = 0; rep < 2; rep++) {  // the second pass is timed
       XG_CUDA(cudaEventRecord(e0, st));
-      run_filter_transpose(s);
+      run_filter_transpose(s, false);
       run_multitau(s, mode);
       XG_CUDA(cudaEventRecord(e1, st));
       XG_CUDA(cudaEventSynchronize(e1));
@@ -172,7 +172,7 @@ __global__ void k_stamp(unsigned long long *dst) {
 }
 
 void series_pass(Series &s, int mode, uint32_t flags) {
-  run_filter_transpose(s);
+  run_filter_transpose(s, false);
   run_multitau(s, mode);
   run_normalize(s, (flags & XPCS_BATCH_F64) != 0, (flags & XPCS_BATCH_F32) != 0);
 }
@@ -219,7 +219,7 @@ void enqueue(Batch &b, int mode, uint32_t flags, int lanes, bool queue, bool cap
     k_stamp<<<1, 1, 0, s.stream>>>(b.stamps.p + 2 * i);
     XG_CHECK_LAUNCH();
     if (queue) {
-      run_filter_transpose(s);
+      run_filter_transpose(s, false);
     } else {
       series_pass(s, mode, flags);
       k_stamp<<<1, 1, 0, s.stream>>>(b.stamps.p + 2 * i + 1);
@@ -322,7 +322,7 @@ float run_directly(Batch &b, int mode, uint32_t flags) {
   drop_graph(b);
   for (Series *s : b.ss) {
     dense_px_flush(*s);
-    default_knobs(*s);
+    default_knobs(*s, false);
     prepare_multitau(*s, mode);
   }
   try {

@@ -813,7 +813,7 @@ void dense_px_gather(Series &s) {
     XG_CUDA(cudaMemsetAsync(s.blk_tot.p, 0, sizeof(int32_t) * (size_t)P, st));
   }
   exclusive_scan_i32_i64(s.blk_tot.p, s.row_ptr.p, P, s.scan_tmp.p, st);
-  PxGather g{P, s.F, s.thread_cap, s.float_cap, s.desc.normalize_by_framesum, nblk, s.has_dark ? 1 : 0,
+  PxGather g{P, s.F, s.class_cap, s.float_cap, s.desc.normalize_by_framesum, nblk, s.has_dark ? 1 : 0,
              s.d_blk_base.p, s.d_blk_r0.p, s.blk_off.p, s.blk_len.p, s.blk_pk.p, s.row_ptr.p,
              s.d_mask.p, s.rmin.p, s.dark_avg.p, s.has_flat ? s.d_flat.p : nullptr,
              (const DensePrep *)s.dn_prep.p, s.ev_frame.p, s.ev_val.p, s.row_len.p, s.pclass.p,

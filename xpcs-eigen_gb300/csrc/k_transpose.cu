@@ -1073,11 +1073,11 @@ void merge_classify(Series &s, int32_t avg) {
   const double mean = (double)s.raw_events / (double)std::max<int64_t>(s.valid_pixels, 1);
   if (avg == 1 && mean < MS_MEAN_MAX)
     k_merge_short<<<(s.P + MS_WARPS * 32 - 1) / (MS_WARPS * 32), MS_WARPS * 32, 0, s.stream>>>(
-        s.P, s.F, s.thread_cap, s.float_cap, s.desc.normalize_by_framesum, s.row_ptr.p, s.d_mask.p,
+        s.P, s.F, s.class_cap, s.float_cap, s.desc.normalize_by_framesum, s.row_ptr.p, s.d_mask.p,
         s.ev_frame.p, s.ev_val.p, s.row_len.p, s.pclass.p, cl, s.pixels_sum.p, s.stats.p);
   else
     k_merge_rows<<<(s.P + 31) / 32, MC_WARPS * 32, 0, s.stream>>>(
-        s.P, s.F, avg, s.thread_cap, s.float_cap, s.desc.normalize_by_framesum, s.row_ptr.p,
+        s.P, s.F, avg, s.class_cap, s.float_cap, s.desc.normalize_by_framesum, s.row_ptr.p,
         s.d_mask.p, s.ev_frame.p, s.ev_val.p, s.row_len.p, s.pclass.p, cl, s.pixels_sum.p,
         s.stats.p);
   XG_CHECK_LAUNCH();
@@ -1299,7 +1299,16 @@ void reset_blocks(Series &s) {
 // capacity of at least 1.5 mean rows, which the autotuner also picks for mean
 // rows of 25, 52 and 100 events (1 Mi pixels, 5,000-20,000 frames), and the
 // extra scratch words it picks from 16,384 frames on.
-void default_knobs(Series &s) {
+// Series of few pixels (alone: not beside a batch's other members) give every
+// row to a warp: one thread a row leaves most of the chip without work and
+// takes as long as its longest row.  At 1,000 frames the integer rows take, with
+// a thread / a warp a row, at 4,096 pixels and rows of 3, 10, 30 events 35 / 27,
+// 54 / 29 and 83 / 32 us, at 16,384 pixels 36 / 60, 54 / 66 and 127 / 74 us, at
+// 36,864 pixels 39 / 111, 57 / 127 and 129 / 140 us; rows of 80 events (4,000
+// frames) 192 / 103 us at 16,384 and 195 / 201 us at 36,864 pixels.  The line
+// lies where the two meet.  It does not hold for a row capacity that the caller
+// chose.
+void default_knobs(Series &s, bool alone) {
   if (s.valid_pixels < 0) {
     s.valid_pixels = 0;
     for (uint8_t v : s.qmap.valid) s.valid_pixels += v;
@@ -1309,22 +1318,25 @@ void default_knobs(Series &s) {
   // raw events of a row that the filter uses: the stride's skipped sub-frames
   // are among a sparse series' events
   s.float_cap = mt_float_cap(s, mean * s.R_in / (s.desc.dense ? 1 : s.desc.stride_frames));
-  if (s.knobs_set) return;
-  int32_t cap = MT_THREAD_CAPS[MT_THREAD_NCAPS - 1];
-  for (int c : MT_THREAD_CAPS)
-    if (c >= 1.5 * mean) {
-      cap = c;
-      break;
-    }
-  s.thread_cap = cap;
-  s.scr_extra = s.F >= 16384 ? 8 : 0;
+  if (!s.knobs_set) {
+    int32_t cap = MT_THREAD_CAPS[MT_THREAD_NCAPS - 1];
+    for (int c : MT_THREAD_CAPS)
+      if (c >= 1.5 * mean) {
+        cap = c;
+        break;
+      }
+    s.thread_cap = cap;
+    s.scr_extra = s.F >= 16384 ? 8 : 0;
+  }
+  const bool few = s.valid_pixels <= std::min(5000.0 + 800.0 * mean, 32000.0);
+  s.class_cap = few && alone && (s.tuned || !s.knobs_set) ? 0 : s.thread_cap;
 }
 
-void run_filter_transpose(Series &s) {
+void run_filter_transpose(Series &s, bool alone) {
   cudaStream_t st = s.stream;
   const int32_t P = s.P;
   dense_px_flush(s);  // frames still pending become the last block
-  default_knobs(s);
+  default_knobs(s, alone);
   reserve_lists(s);
   const size_t nalloc = s.raw_events > 0 ? (size_t)s.raw_events : 1;
   s.ev_frame.reserve(nalloc, st);
@@ -1414,9 +1426,9 @@ void multitau_rows_upload(Series &s, const int64_t *row_ptr, const int32_t *fram
     XG_CUDA(cudaMemcpyAsync(s.ev_frame.p, frame, sizeof(int32_t) * events, cudaMemcpyHostToDevice, st));
     XG_CUDA(cudaMemcpyAsync(s.ev_val.p, value, sizeof(float) * events, cudaMemcpyHostToDevice, st));
   }
-  default_knobs(s);
+  default_knobs(s, true);
   const int bs = 256;
-  k_classify_rows<<<(P + bs - 1) / bs, bs, 0, st>>>(P, s.F, s.thread_cap, s.row_ptr.p, s.ev_frame.p,
+  k_classify_rows<<<(P + bs - 1) / bs, bs, 0, st>>>(P, s.F, s.class_cap, s.row_ptr.p, s.ev_frame.p,
                                                      s.ev_val.p, s.row_len.p, s.pclass.p,
                                                      ClassLists{s.wlist.p, s.llist.p, s.flist.p},
                                                      s.stats.p);

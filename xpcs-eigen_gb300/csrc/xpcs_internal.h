@@ -321,6 +321,7 @@ struct Series {
   DBuf<uint8_t> plan;       // McPlan + tau_lvl[D] + denom[D]
   int32_t plan_mode = -1;   // mode of the plan in `plan` (-1: none uploaded)
   int32_t thread_cap = MT_THREAD_CAP_DEFAULT;  // rows up to this length: thread per pixel
+  int32_t class_cap = 0;    // the same, or 0: every row to a warp (default_knobs)
   int32_t float_cap = 0;    // float rows up to this length: thread per pixel (default_knobs)
   int32_t scr_extra = 0;    // scratch words beyond max(delays of a level, levels)
   int32_t radix_ipt = 0;    // transpose items per lane (event tile / 256); 0: by series size
@@ -448,9 +449,9 @@ void exclusive_scan_i32_i64(const int32_t *in, int64_t *out, int64_t n, void *ws
                             cudaStream_t st);
 
 // Kernel launchers
-void run_filter_transpose(Series &s);                       // k_transpose.cu
+void run_filter_transpose(Series &s, bool alone);                       // k_transpose.cu
 // Knobs for a series the caller has not tuned, from its mean row length.
-void default_knobs(Series &s);
+void default_knobs(Series &s, bool alone);
 // Incremental transposes: every complete block of ingested frames (k_transpose.cu)
 void transpose_ready_blocks(Series &s);
 void reset_blocks(Series &s);
