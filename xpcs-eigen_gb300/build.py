@@ -56,7 +56,7 @@ def _stale(target: Path, deps) -> bool:
 def build_gpu(force: bool = False, verbose: bool = False) -> Path:
     OBJ.mkdir(parents=True, exist_ok=True)
     headers = [INCLUDE / "xpcs_gpu.h", CSRC / "xpcs_internal.h", CSRC / "f64emu.cuh",
-               CSRC / "mt_replay.cuh",
+               CSRC / "mt_replay.cuh", CSRC / "overlap.cuh",
                CSRC / "classify.cuh"]
     jobs = []
     objs = []

@@ -47,6 +47,7 @@
 #include <type_traits>
 
 #include "mt_replay.cuh"
+#include "overlap.cuh"
 #include "xpcs_internal.h"
 
 namespace xg {
@@ -2039,25 +2040,6 @@ ThreadKernel thread_kernel(int cap) {
 }
 size_t warp_smem(int D, int acc, int cap, int warps) {
   return mc_plan_bytes(D) + (size_t)warps * (2 * cap + 32 * acc) * sizeof(int32_t);
-}
-
-// A launch whose kernel may start before the one before it in the stream is
-// complete (overlap_begin / overlap_end), also as part of a captured graph.
-template <typename... Params, typename... Args>
-void launch_overlapped(void (*kernel)(Params...), int grid, int block, size_t smem,
-                       cudaStream_t st, Args... args) {
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(block);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  XG_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...));
-  XG_CHECK_LAUNCH();
 }
 
 // The kernels' row counters, before the first kernel that uses one.

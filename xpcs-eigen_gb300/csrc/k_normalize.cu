@@ -33,6 +33,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "overlap.cuh"
 #include "xpcs_internal.h"
 
 namespace xg {
@@ -143,6 +144,7 @@ k_norm_part(int D, int P, int NC, const int32_t *__restrict__ ch_k0,
             const int32_t *__restrict__ ch_k1, const int32_t *__restrict__ pix,
             const float *__restrict__ G2, const float *__restrict__ IP,
             const float *__restrict__ IF, double *__restrict__ part) {
+  overlap_after();
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int c = blockIdx.x * NW + (threadIdx.x >> 5), t0 = blockIdx.y * NT;
@@ -297,6 +299,7 @@ __global__ void k_norm_finish(int NQ, int D, const int32_t *__restrict__ qep,
                               const int32_t *__restrict__ ch_k0, const int32_t *__restrict__ ch_k1,
                               const double *__restrict__ part, double *__restrict__ g2,
                               double *__restrict__ se) {
+  overlap_after();
   const int lane = threadIdx.x & 31;
   const int idx = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   if (idx >= NQ * D) return;
@@ -686,16 +689,14 @@ void run_normalize(Series &s, bool want64, bool want32) {
     const int NC = s.n_chunks;
     s.n_part.reserve((size_t)(NC > 0 ? NC : 1) * D * NPART, st);
     if (NC > 0) {
-      k_norm_part<<<dim3((NC + NW - 1) / NW, (D + NT - 1) / NT), NW * 32, 0, st>>>(
-          D, P, NC, s.n_ch_k0.p, s.n_ch_k1.p, s.n_pix.p, s.G2.p, s.IP.p, s.IF.p, s.n_part.p);
-      XG_CHECK_LAUNCH();
+      launch_overlapped(k_norm_part, dim3((NC + NW - 1) / NW, (D + NT - 1) / NT), NW * 32, 0, st,
+                        D, P, NC, s.n_ch_k0.p, s.n_ch_k1.p, s.n_pix.p, s.G2.p, s.IP.p, s.IF.p,
+                        s.n_part.p);
     }
     const int bs = 128;
-    k_norm_finish<<<(unsigned)(((int64_t)NQ * D * 32 + bs - 1) / bs), bs, 0, st>>>(NQ, D, s.n_q_entry_ptr.p, s.n_q_row.p,
-                                                        s.n_e_chunk_ptr.p, s.n_ch_k0.p,
-                                                        s.n_ch_k1.p, s.n_part.p, s.n_g2.p,
-                                                        s.n_se.p);
-    XG_CHECK_LAUNCH();
+    launch_overlapped(k_norm_finish, (unsigned)(((int64_t)NQ * D * 32 + bs - 1) / bs), bs, 0, st,
+                      NQ, D, s.n_q_entry_ptr.p, s.n_q_row.p, s.n_e_chunk_ptr.p, s.n_ch_k0.p,
+                      s.n_ch_k1.p, s.n_part.p, s.n_g2.p, s.n_se.p);
   }
   if (want32) {
     const QMap &qm = s.qmap;

@@ -26,6 +26,7 @@
 
 #include "f64emu.cuh"
 #include "classify.cuh"
+#include "overlap.cuh"
 #include "xpcs_internal.h"
 
 namespace xg {
@@ -89,6 +90,7 @@ struct DigitSums {
 // off[r + 1] - e0.
 __global__ void k_chunk_frames(int32_t nframes, const int64_t *__restrict__ off, int64_t e0,
                                int64_t nchunks, int32_t chunk, int32_t *__restrict__ chunk_frame) {
+  overlap_after();
   const int32_t r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= nframes) return;
   const int64_t c0 = (off[r] - e0 + chunk - 1) / chunk;
@@ -160,6 +162,7 @@ __device__ __forceinline__ int64_t item_index(int tile, int w, int k, int lane) 
 template <int IPT, int DB, bool FIRST>
 __global__ void __launch_bounds__(RS_THREADS)
 k_upsweep(RawCfg rc, PassCfg pc, uint32_t *__restrict__ hist, DigitSums *__restrict__ ds) {
+  overlap_after();
   constexpr int RS_DIGITS = 1 << DB;
   __shared__ uint32_t h[RS_DIGITS];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, tile = blockIdx.x;
@@ -225,6 +228,7 @@ constexpr int DSC_IPT = 8;
 __global__ void __launch_bounds__(DSC_THREADS)
 k_digit_scan(int digits, int ntiles, int hstride, uint32_t *__restrict__ hist,
              DigitSums *__restrict__ ds) {
+  overlap_after();
   __shared__ uint32_t wsum[DSC_THREADS / 32];
   __shared__ bool last;
   const unsigned FULL = 0xffffffffu;
@@ -314,6 +318,7 @@ template <int IPT, int DB, bool FIRST, bool LAST, bool PK>
 __global__ void __launch_bounds__(RS_THREADS)
 k_downsweep(RawCfg rc, PassCfg pc, const uint32_t *__restrict__ offsets,
             const DigitSums *__restrict__ dsum) {
+  overlap_after();
   constexpr int RS_DIGITS = 1 << DB;
   extern __shared__ __align__(16) uint8_t ds_raw[];
   DsSmem<IPT, DB, PK> &sm = *reinterpret_cast<DsSmem<IPT, DB, PK> *>(ds_raw);
@@ -463,6 +468,7 @@ constexpr int RP_U = 4;
 __global__ void __launch_bounds__(256)
 k_row_ptr(const uint32_t *__restrict__ keys, int64_t n, const DevStats *__restrict__ stats,
           int32_t P, int64_t *__restrict__ row_ptr) {
+  overlap_after();
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int64_t nv = n - (int64_t)stats->dropped;
@@ -626,6 +632,7 @@ k_merge_rows(int32_t P, int32_t F, int32_t avg, int32_t tcap, int32_t fcap,
                  int32_t *__restrict__ fr, float *__restrict__ val, int32_t *__restrict__ row_len,
                  uint8_t *__restrict__ pclass, ClassLists cl, float *__restrict__ pixels_sum,
                  DevStats *__restrict__ stats) {
+  overlap_after();
   __shared__ int32_t s_len[32];
   __shared__ uint8_t s_cls[32];
   const unsigned FULL = 0xffffffffu;
@@ -750,6 +757,7 @@ k_merge_short(int32_t P, int32_t F, int32_t tcap, int32_t fcap, int32_t force_fl
               int32_t *__restrict__ fr, float *__restrict__ val, int32_t *__restrict__ row_len,
               uint8_t *__restrict__ pclass, ClassLists cl, float *__restrict__ pixels_sum,
               DevStats *__restrict__ stats) {
+  overlap_after();
   __shared__ float s_val[MS_WARPS][MS_TILE];
   __shared__ uint32_t s_start[MS_WARPS][MS_TILE / 32];
   const unsigned FULL = 0xffffffffu;
@@ -843,8 +851,8 @@ void launch_downsweep(Series &s, int ntiles, const RawCfg &rc, const PassCfg &pc
   const size_t smem = sizeof(DsSmem<IPT, DB, PK>);
   XG_CUDA(cudaFuncSetAttribute(k_downsweep<IPT, DB, FIRST, LAST, PK>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k_downsweep<IPT, DB, FIRST, LAST, PK><<<ntiles, RS_THREADS, smem, s.stream>>>(rc, pc, s.hist.p,
-                                                                               ds);
+  launch_overlapped(k_downsweep<IPT, DB, FIRST, LAST, PK>, ntiles, RS_THREADS, smem, s.stream, rc,
+                    pc, s.hist.p, ds);
 }
 
 // One radix pass: tile histograms, digit-major scan, stable scatter.
@@ -854,13 +862,10 @@ void radix_pass(Series &s, bool first, bool last, const RawCfg &rc, PassCfg pc) 
   const int ntiles = pc.ntiles;
   pc.hstride = (ntiles + 3) & ~3;
   DigitSums *ds = (DigitSums *)(s.hist.p + ((size_t)pc.hstride << DB));
-  if (first)
-    k_upsweep<IPT, DB, true><<<ntiles, RS_THREADS, 0, st>>>(rc, pc, s.hist.p, ds);
-  else
-    k_upsweep<IPT, DB, false><<<ntiles, RS_THREADS, 0, st>>>(rc, pc, s.hist.p, ds);
-  XG_CHECK_LAUNCH();
-  k_digit_scan<<<1 << DB, DSC_THREADS, 0, st>>>(1 << DB, ntiles, pc.hstride, s.hist.p, ds);
-  XG_CHECK_LAUNCH();
+  launch_overlapped(first ? k_upsweep<IPT, DB, true> : k_upsweep<IPT, DB, false>, ntiles,
+                    RS_THREADS, 0, st, rc, pc, s.hist.p, ds);
+  launch_overlapped(k_digit_scan, 1 << DB, DSC_THREADS, 0, st, 1 << DB, ntiles, pc.hstride,
+                    s.hist.p, ds);
   if (first && last)
     launch_downsweep<IPT, DB, true, true, PK>(s, ntiles, rc, pc, ds);
   else if (first)
@@ -1007,9 +1012,8 @@ void transpose_range(Series &s, int32_t r0, int32_t r1, int32_t *ev_fr, float *e
   const int64_t nch = (n + chunk - 1) / chunk;
   const int32_t nfr = r1 - r0;
   s.d_chunk_frame.reserve((size_t)nch, st);
-  k_chunk_frames<<<(nfr + 255) / 256, 256, 0, st>>>(nfr, s.d_frame_off.p + r0, e0, nch, chunk,
-                                                     s.d_chunk_frame.p);
-  XG_CHECK_LAUNCH();
+  launch_overlapped(k_chunk_frames, (nfr + 255) / 256, 256, 0, st, nfr, s.d_frame_off.p + r0, e0,
+                    nch, chunk, s.d_chunk_frame.p);
   RawCfg rc{s.raw_idx.p + e0, dense ? nullptr : s.raw_val.p + e0,
             dense ? s.raw_valf.p + e0 : nullptr, s.d_frame_off.p + r0, s.d_frame_map.p + r0,
             s.d_chunk_frame.p, nfr, e0, n, P, s.F, s.R_in, s.desc.stride_frames,
@@ -1041,8 +1045,8 @@ void transpose_range(Series &s, int32_t r0, int32_t r1, int32_t *ev_fr, float *e
     radix_pass(s, ipt, dg.bits, packed, first, last, rc, pc);
   }
   const uint32_t *keys = (passes % 2 == 0) ? s.keyB.p : s.keyA.p;  // written by the last pass
-  k_row_ptr<<<(unsigned)((n + 1 + RP_U * 1024 - 1) / (RP_U * 1024)), 256, 0, st>>>(keys, n, s.stats.p, P, row_ptr);
-  XG_CHECK_LAUNCH();
+  launch_overlapped(k_row_ptr, (unsigned)((n + 1 + RP_U * 1024 - 1) / (RP_U * 1024)), 256, 0, st,
+                    keys, n, s.stats.p, P, row_ptr);
 }
 
 void reserve_lists(Series &s) {
@@ -1072,15 +1076,15 @@ void merge_classify(Series &s, int32_t avg) {
   const ClassLists cl{s.wlist.p, s.llist.p, s.flist.p};
   const double mean = (double)s.raw_events / (double)std::max<int64_t>(s.valid_pixels, 1);
   if (avg == 1 && mean < MS_MEAN_MAX)
-    k_merge_short<<<(s.P + MS_WARPS * 32 - 1) / (MS_WARPS * 32), MS_WARPS * 32, 0, s.stream>>>(
+    launch_overlapped(
+        k_merge_short, (s.P + MS_WARPS * 32 - 1) / (MS_WARPS * 32), MS_WARPS * 32, 0, s.stream,
         s.P, s.F, s.class_cap, s.float_cap, s.desc.normalize_by_framesum, s.row_ptr.p, s.d_mask.p,
         s.ev_frame.p, s.ev_val.p, s.row_len.p, s.pclass.p, cl, s.pixels_sum.p, s.stats.p);
   else
-    k_merge_rows<<<(s.P + 31) / 32, MC_WARPS * 32, 0, s.stream>>>(
-        s.P, s.F, avg, s.class_cap, s.float_cap, s.desc.normalize_by_framesum, s.row_ptr.p,
+    launch_overlapped(
+        k_merge_rows, (s.P + 31) / 32, MC_WARPS * 32, 0, s.stream, s.P, s.F, avg, s.class_cap, s.float_cap, s.desc.normalize_by_framesum, s.row_ptr.p,
         s.d_mask.p, s.ev_frame.p, s.ev_val.p, s.row_len.p, s.pclass.p, cl, s.pixels_sum.p,
         s.stats.p);
-  XG_CHECK_LAUNCH();
 }
 
 }  // namespace
@@ -1109,6 +1113,7 @@ k_merge_block(int32_t P, int32_t avg, const int64_t *__restrict__ row_ptr,
               const uint8_t *__restrict__ mask, int32_t *__restrict__ fr,
               float *__restrict__ val, int32_t *__restrict__ blk_off,
               int32_t *__restrict__ blk_len) {
+  overlap_after();
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p - (int)(threadIdx.x & 31) >= P) return;  // whole warp past the end
   const bool has = p < P;
@@ -1261,11 +1266,9 @@ void transpose_block(Series &s, int32_t r1) {
   s.blk_len.grow((k + 1) * (size_t)P, k * (size_t)P, st);
   s.blk_rp.reserve((size_t)P + 1, st);
   transpose_range(s, r0, r1, s.blk_fr.p + base, s.blk_val.p + base, s.blk_rp.p);
-  k_merge_block<<<(P + 255) / 256, 256, 0, st>>>(P, s.desc.avg_frames, s.blk_rp.p, s.d_mask.p,
-                                                  s.blk_fr.p + base, s.blk_val.p + base,
-                                                  s.blk_off.p + k * (size_t)P,
-                                                  s.blk_len.p + k * (size_t)P);
-  XG_CHECK_LAUNCH();
+  launch_overlapped(k_merge_block, (P + 255) / 256, 256, 0, st, P, s.desc.avg_frames, s.blk_rp.p,
+                    s.d_mask.p, s.blk_fr.p + base, s.blk_val.p + base,
+                    s.blk_off.p + k * (size_t)P, s.blk_len.p + k * (size_t)P);
   s.blk_base.push_back(base);
   s.blk_events = base + n;
   s.blk_raw_done = r1;
