@@ -62,14 +62,13 @@ constexpr int MID_WARPS = 4;
 // events each, take 2.95 / 2.25 / 2.00 / 1.97 / 1.98 ms with 0 (pairs by
 // search and bitmask only) / 4 / 8 / 16 / 40.
 constexpr int MB_RATIO = 16;
-// The same for the thread kernel (mt_thread_rows), of the warp's longest row, and
-// the scratch words that its windows have at least.  At 1 Mpx x 10,000 frames,
+// The same for the thread kernel (mt_thread_rows), of the warp's longest row; its
+// windows have at least MT_MIN_SCR scratch words.  At 1 Mpx x 10,000 frames,
 // rows of 50 events, the integer rows take 2.53 / 2.29 / 2.27 / 2.26 / 2.25 /
 // 2.41 ms with 0 / 4 / 8 / 12 / 16 / 20 bins per entry; at 512 x 512 x 1,000
 // frames, rows of 10 and 4 delays a level, 161 / 143 / 139 / 141 us with 8 / 10
 // / 12 / 16 words (8 are too few for any level's window).
 constexpr int TB_RATIO = 12;
-constexpr int MT_MIN_SCR = 12;
 constexpr int LONG_WARPS = 2;  // warps per block for rows of up to MT_LONG_CAP events
 
 // std::lower_bound as libstdc++ implements it (halving the remaining length),

@@ -185,7 +185,7 @@ int na_build_plan(int32_t P, int32_t F, int32_t dpl, int32_t mode, uint8_t *buf,
   pl->nlev = nlev;
   pl->acc = 1;
   for (int g = 0; g < nlev; g++) pl->acc = std::max(pl->acc, pl->lv[g].count);
-  pl->scr = std::max(pl->acc, nlev) + (F >= 16384 ? 8 : 0);  // as default_knobs
+  pl->scr = std::max({pl->acc, nlev, MT_MIN_SCR}) + (F >= 16384 ? 8 : 0);  // as default_knobs
   return D;
 }
 

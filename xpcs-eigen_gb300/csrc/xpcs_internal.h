@@ -171,6 +171,7 @@ __host__ __device__ inline McArrays mc_arrays(const void *plan, int D) {
 constexpr int MT_THREAD_CAPS[] = {32, 48, 64, 80, 112};
 constexpr int MT_THREAD_NCAPS = 5;
 constexpr int MT_THREAD_CAP_DEFAULT = 80;
+constexpr int MT_MIN_SCR = 12;  // scratch words a row of the thread kernel has at least
 constexpr int MT_WARP_CAP = 256;
 constexpr int MT_LONG_CAP = 4096;  // an integer row with sum |v| < 4096 has fewer non-zero events
 enum : uint8_t { PCLASS_EMPTY = 0, PCLASS_THREAD = 1, PCLASS_WARP = 2, PCLASS_FLOAT = 3,
