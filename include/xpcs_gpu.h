@@ -374,8 +374,8 @@ int xpcs_get_twotime(xpcs_series *s, int32_t *qbins, float *sg, float *c2t, floa
  * them -- filter/transpose, multi-tau and normalisation -- as one CUDA graph,
  * captured by the second run on the same frames and replayed until a member's
  * frames, the mode or the flags change; a first run enqueues the same schedule
- * directly.  Members are dealt, largest
- * first, onto a number of concurrent chains.  Two forms:
+ * directly.  Members are dealt, largest first, onto a number of concurrent
+ * chains.  Two forms:
  *  - work queue (the default): the chains run every member's transpose, then
  *    the multi-tau of all members runs as persistent launches over a device
  *    work queue -- one per thread-kernel row capacity, pulling 32-pixel groups
