@@ -763,7 +763,6 @@ __device__ __forceinline__ void mt_warp_pixel(const McPlan *pl, const McArrays &
     }
     const bool sorted = mode != XPCS_MODE_REFERENCE || (J && U);
     const int tlo = L.tau_lo, thi = L.tau_lo + L.count - 1;
-    for (int k = 0; k < L.count; k++) acc[k * 32] = 0;
     const int lf = L.lastframe;
     bool bytes = tlo >= 1 && tlo <= 31 && L.count <= 16 && ((lf + 3) >> 2) + MB_PAD <= cap &&
                  lf <= MB_RATIO * m;
@@ -800,15 +799,27 @@ __device__ __forceinline__ void mt_warp_pixel(const McPlan *pl, const McArrays &
               if (t - tlo - k >= 0) a[k] -= v * ((const uint8_t *)S)[t - tlo - k];
           }
         }
+        int mine = 0;
 #pragma unroll
-        for (int k = 0; k < KM; k++)
-          if (k < L.count) acc[k * 32] = (int32_t)a[k];
+        for (int k = 0; k < KM; k++) {
+          if (k >= L.count) break;
+          const int tot = __reduce_add_sync(FULL, (int)a[k]);
+          if (lane == k) mine = tot;
+        }
+        if (lane < L.count) {
+          const int d = L.first + lane;
+          G2[(size_t)d * P + p] = scaled_quotient(mine, 2 * L.level, ar.denom[d], ar.rcp[d]);
+        }
+        __syncwarp();
       };
       if (L.count <= 8)
         level(std::integral_constant<int, 8>{});
       else
         level(std::integral_constant<int, 16>{});
-    } else if (sorted && tlo >= 1 && lf <= cap && 5 * m >= lf) {
+      continue;
+    }
+    for (int k = 0; k < L.count; k++) acc[k * 32] = 0;
+    if (sorted && tlo >= 1 && lf <= cap && 5 * m >= lf) {
       // at least a fifth of the level's bins hold an entry: the prefix sums
       // S are done with, and S becomes the row's values by bin, so that each
       // source finds its partner for every delay with one lookup (a missing

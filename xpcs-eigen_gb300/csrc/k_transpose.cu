@@ -1305,10 +1305,10 @@ void reset_blocks(Series &s) {
 // Series of few pixels (alone: not beside a batch's other members) give every
 // row to a warp: one thread a row leaves most of the chip without work and
 // takes as long as its longest row.  At 1,000 frames the integer rows take, with
-// a thread / a warp a row, at 4,096 pixels and rows of 3, 10, 30 events 35 / 27,
-// 54 / 29 and 83 / 32 us, at 16,384 pixels 36 / 60, 54 / 66 and 127 / 74 us, at
-// 36,864 pixels 39 / 111, 57 / 127 and 129 / 140 us; rows of 80 events (4,000
-// frames) 192 / 103 us at 16,384 and 195 / 201 us at 36,864 pixels.  The line
+// a thread / a warp a row, at 4,096 pixels and rows of 3, 10, 30 events 35 / 26,
+// 54 / 29 and 84 / 30 us, at 16,384 pixels 36 / 57, 54 / 62 and 117 / 65 us, at
+// 36,864 pixels 39 / 102, 58 / 116 and 129 / 125 us; rows of 80 events (4,000
+// frames) 190 / 94 us at 16,384 and 197 / 186 us at 36,864 pixels.  The line
 // lies where the two meet.  It does not hold for a row capacity that the caller
 // chose.
 void default_knobs(Series &s, bool alone) {
