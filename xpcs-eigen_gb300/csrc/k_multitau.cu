@@ -588,10 +588,6 @@ __device__ __forceinline__ void mt_thread_warp(const uint8_t *__restrict__ plan_
 // counter hands out the rows, since blocks begin at different times (a fixed
 // share for each block: 2.6 ms).  263 x 251 pixels x 16,000 frames, rows of 744
 // events: the integer rows 1.97 ms one launch after the other, 1.62 overlapped.
-__device__ __forceinline__ void overlap_begin() { cudaTriggerProgrammaticLaunchCompletion(); }
-__device__ __forceinline__ void overlap_end() {
-  if (blockIdx.x == 0 && threadIdx.x == 0) cudaGridDependencySynchronize();
-}
 
 template <int CAP>
 __global__ void __launch_bounds__(MT_WARPS * 32, 16)

@@ -26,7 +26,7 @@
 //                  of every chunk's own and of n (chunk mean - mean)^2;
 //                  stderr = sqrt(1/n) sqrt(M2/n) (:1043-1087).
 // float32 result (optional, bit-identical to the reference's float output):
-//   k_f32_transpose / k_entry_f32 / k_q_f32 replay the reference's sequential
+//   k_f32_transpose / k_q_f32 / k_entry_f32 / k_q_mean_f32 replay the reference's sequential
 //   float operations in its order, including the running-mean/M2 update of
 //   every pixel.
 #include <algorithm>
@@ -508,6 +508,7 @@ __global__ void k_entry_f32(int NE, int D, int Dp, int FR_CH, const int32_t *__r
                             const float *__restrict__ Tg, const float *__restrict__ Ti,
                             const float *__restrict__ Tf, float *__restrict__ ratio,
                             int32_t *__restrict__ err) {
+  overlap_begin();
   extern __shared__ __align__(16) float fr_buf[];  // [2][3][FR_CH][Dp], then 2 mbarriers
   uint64_t *bar = (uint64_t *)(fr_buf + (size_t)2 * 3 * FR_CH * Dp);
   const int e = blockIdx.x, t = threadIdx.x;
@@ -532,30 +533,39 @@ __global__ void k_entry_f32(int NE, int D, int Dp, int FR_CH, const int32_t *__r
     sf = __fdiv_rn(sf, cnt);
     ratio[(size_t)e * D + t] = __fdiv_rn(sg, __fmul_rn(si, sf));
   }
+  overlap_end();
 }
 
-// One block per q ring, thread tau: g2 = mean of the non-NaN entry ratios
-// (corr.cpp:1018-1040); stderr from the running mean / M2 over the ring's
-// pixels in order, NaN counted as 0 (corr.cpp:1043-1087).
+// g2 of a q bin and tau = mean of the non-NaN entry ratios (corr.cpp:1018-1040).
+__global__ void k_q_mean_f32(int NQ, int D, const int32_t *__restrict__ qep,
+                             const int32_t *__restrict__ qrow, const float *__restrict__ ratio,
+                             float *__restrict__ g2) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= NQ * D) return;
+  const int qi = i / D, t = i - qi * D;
+  float acc = 0.f, cnt = 0.f;
+  for (int e = qep[qi]; e < qep[qi + 1]; e++) {
+    const float r = ratio[(size_t)e * D + t];
+    acc = __fadd_rn(acc, isnan(r) ? 0.f : r);
+    cnt = __fadd_rn(cnt, isnan(r) ? 0.f : 1.f);
+  }
+  g2[(size_t)t * NQ + qrow[qi]] = __fdiv_rn(acc, cnt);
+}
+
+// One block per q ring, thread tau: stderr from the running mean / M2 over the
+// ring's pixels in order, NaN counted as 0 (corr.cpp:1043-1087).  Few blocks,
+// each a long chain: the entries' kernel runs on the other SMs meanwhile (640 x
+// 480 x 2,000 frames with the side statistics: 3.16 ms one after the other, 2.83).
 __global__ void k_q_f32(int NQ, int D, int Dp, int FR_CH, const int32_t *__restrict__ qep,
                         const int32_t *__restrict__ qrow, const int32_t *__restrict__ epp,
-                        const float *__restrict__ ratio, const float *__restrict__ X,
-                        float *__restrict__ g2, float *__restrict__ se,
+                        const float *__restrict__ X, float *__restrict__ se,
                         const int32_t *__restrict__ unsafe, int32_t *__restrict__ err) {
+  overlap_begin();
   extern __shared__ __align__(16) float fr_buf[];  // [2][FR_CH][Dp], then 2 mbarriers
   const bool all_safe = *unsafe == 0;
   uint64_t *bar = (uint64_t *)(fr_buf + (size_t)2 * FR_CH * Dp);
   const int qi = blockIdx.x, t = threadIdx.x;
   const int row = qrow[qi];
-  if (t < D) {
-    float acc = 0.f, cnt = 0.f;
-    for (int e = qep[qi]; e < qep[qi + 1]; e++) {
-      float r = ratio[(size_t)e * D + t];
-      acc = __fadd_rn(acc, isnan(r) ? 0.f : r);
-      cnt = __fadd_rn(cnt, isnan(r) ? 0.f : 1.f);
-    }
-    g2[(size_t)t * NQ + row] = __fdiv_rn(acc, cnt);
-  }
   // The reference's sample count (samples += 1.0f per pixel) is the exact
   // count below 2^24 and stays at 2^24 from there on.  Its correctly rounded
   // reciprocal depends on the count only: the block computes each chunk's
@@ -730,14 +740,15 @@ void run_normalize(Series &s, bool want64, bool want32) {
                                  (int)sm_e));
     XG_CUDA(cudaFuncSetAttribute(k_q_f32, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)sm_q));
-    if (NE > 0) {
-      k_entry_f32<<<NE, bs, sm_e, st>>>(NE, D, Dp, ch_e, s.n_entry_pix_ptr.p, s.n_tg.p,
-                                        s.n_ti.p, s.n_tf.p, s.n_ratio32.p, &s.stats.p->error);
-      XG_CHECK_LAUNCH();
-    }
     k_q_f32<<<NQ, bs, sm_q, st>>>(NQ, D, Dp, ch_q, s.n_q_entry_ptr.p, s.n_q_row.p,
-                                  s.n_entry_pix_ptr.p, s.n_ratio32.p, s.n_tx.p, s.n_g2f.p,
-                                  s.n_sef.p, s.n_unsafe.p, &s.stats.p->error);
+                                  s.n_entry_pix_ptr.p, s.n_tx.p, s.n_sef.p, s.n_unsafe.p,
+                                  &s.stats.p->error);
+    XG_CHECK_LAUNCH();
+    if (NE > 0)
+      launch_overlapped(k_entry_f32, NE, bs, sm_e, st, NE, D, Dp, ch_e, s.n_entry_pix_ptr.p,
+                        s.n_tg.p, s.n_ti.p, s.n_tf.p, s.n_ratio32.p, &s.stats.p->error);
+    k_q_mean_f32<<<(NQ * D + 127) / 128, 128, 0, st>>>(NQ, D, s.n_q_entry_ptr.p, s.n_q_row.p,
+                                                       s.n_ratio32.p, s.n_g2f.p);
     XG_CHECK_LAUNCH();
   }
 }

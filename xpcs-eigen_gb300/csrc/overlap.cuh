@@ -11,7 +11,7 @@ namespace xg {
 
 // A launch whose kernel may start before the one before it in the stream is
 // complete, also as part of a captured graph.  The kernel itself waits for what
-// it needs: overlap_after, or the pairs described in k_multitau.cu.
+// it needs: overlap_after, or overlap_begin / overlap_end.
 template <typename... Params, typename... Args>
 void launch_overlapped(void (*kernel)(Params...), dim3 grid, int block, size_t smem,
                        cudaStream_t st, Args... args) {
@@ -36,6 +36,15 @@ void launch_overlapped(void (*kernel)(Params...), dim3 grid, int block, size_t s
 __device__ __forceinline__ void overlap_after() {
   cudaGridDependencySynchronize();
   cudaTriggerProgrammaticLaunchCompletion();
+}
+
+// Kernels that need nothing from one another, the first launched plainly: each
+// begins with overlap_begin (the next may start once every block of this one has)
+// and ends with overlap_end (this kernel is complete only when the one before is,
+// so that what follows in the stream waits for all of them).
+__device__ __forceinline__ void overlap_begin() { cudaTriggerProgrammaticLaunchCompletion(); }
+__device__ __forceinline__ void overlap_end() {
+  if (blockIdx.x == 0 && threadIdx.x == 0) cudaGridDependencySynchronize();
 }
 
 }  // namespace xg
