@@ -260,3 +260,28 @@ def test_first_run_replay_and_a_change_of_form_give_the_same_bits():
     finally:
         for s in members:
             s.close()
+
+
+@pytest.mark.parametrize("queue", [True, False])
+def test_a_member_run_alone_in_another_mode_leaves_the_batch_its_results(queue):
+    """A member run alone in the other mode holds that mode's plan: the batch
+    puts its own back before its graph is captured and before each replay."""
+    series = [open_member(*synth_member(i, *m)) for i, m in enumerate(MIX[:4])]
+    series.append(open_member(*synth_member(0, *LONG_ROWS[0])))
+    other = {xg.MODE_REFERENCE: xg.MODE_EXACT, xg.MODE_EXACT: xg.MODE_REFERENCE}
+    try:
+        solo = {m: [alone(s, m) for s in series] for m in other}
+        assert any(not same_bits(a["G2"], b["G2"]) for a, b in zip(*solo.values()))
+        with xg.Batch(series) as b:
+            b.set_form(queue)
+            for mode in other:
+                for _ in range(3):  # enqueued directly, captured, replayed
+                    b.run(mode, f64=True, f32=True)
+                    for s, r in zip(series, solo[mode]):
+                        assert_same(results(s), r)
+                    for s in series:
+                        s.multitau(other[mode])
+                        s.synchronize()
+    finally:
+        for s in series:
+            s.close()

@@ -384,6 +384,11 @@ void batch_run(Batch &b, int mode, uint32_t flags) {
       b.last_ms = launch(b);
     }
   } else {
+    // a run of a member alone in another mode has replaced the plan that the
+    // graph's kernels read: put back here, since a capture must not copy from
+    // host memory
+    for (Series *s : b.ss)
+      if (s->plan_mode != mode) prepare_multitau(*s, mode);
     if (!b.exec) {
       mt_queue_build(b.ss, b.mtq, b.origin);
       build_graph(b, mode, flags, b.lanes, b.queue);
