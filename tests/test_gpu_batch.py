@@ -285,3 +285,21 @@ def test_a_member_run_alone_in_another_mode_leaves_the_batch_its_results(queue):
     finally:
         for s in series:
             s.close()
+
+
+def test_a_replay_waits_for_what_a_member_was_asked_alone():
+    """xpcs_multitau returns with its work enqueued on the member's stream: the
+    batch's graph, captured or replayed, starts after it."""
+    series = [open_member(*synth_member(i, *m)) for i, m in enumerate(MIX[1:] + LONG_ROWS)]
+    try:
+        solo = [alone(s, xg.MODE_REFERENCE) for s in series]
+        with xg.Batch(series) as b:
+            for _ in range(6):
+                b.run(xg.MODE_REFERENCE, f64=True, f32=True)
+                for s, r in zip(series, solo):
+                    assert_same(results(s), r)
+                for s in series:
+                    s.multitau(xg.MODE_REFERENCE)
+    finally:
+        for s in series:
+            s.close()

@@ -384,6 +384,9 @@ void batch_run(Batch &b, int mode, uint32_t flags) {
       b.last_ms = launch(b);
     }
   } else {
+    // the graph starts from the origin stream alone: what a member's own calls
+    // enqueued on its stream (xpcs_multitau does not wait) ends first
+    for (Series *s : b.ss) XG_CUDA(cudaStreamSynchronize(s->stream));
     // a run of a member alone in another mode has replaced the plan that the
     // graph's kernels read: put back here, since a capture must not copy from
     // host memory
