@@ -3,6 +3,8 @@ graph.  Each member's G2/IP/IF and g2/stderr (float64 and float32) must be
 bit-identical to the same series run alone, the graph replay must repeat
 them, a member whose frames change must be recaptured, and golden members
 must still match the reference's own outputs."""
+import time
+
 import numpy as np
 import pytest
 
@@ -300,6 +302,34 @@ def test_a_replay_waits_for_what_a_member_was_asked_alone():
                     assert_same(results(s), r)
                 for s in series:
                     s.multitau(xg.MODE_REFERENCE)
+    finally:
+        for s in series:
+            s.close()
+
+
+def test_autotuning_after_a_change_of_form_times_the_chain_counts_again():
+    """A form chosen on frames that the batch has run leaves the chain count to
+    the next autotuned run: that run captures one graph for each of 1, 2, 4 and
+    8 chains and the one it keeps, where a run without autotuning captures one."""
+    series = [open_member(*synth_member(i, *m)) for i, m in enumerate(MIX + LONG_ROWS)]
+    took = {}
+    try:
+        solo = [alone(s, xg.MODE_REFERENCE) for s in series]
+        for tune in (False, True):
+            with xg.Batch(series) as b:
+                b.run(autotune=tune, f32=True)
+                b.run(autotune=tune, f32=True)
+                ms = []
+                for queue in (True, False) * 3:
+                    b.set_form(queue)
+                    t = time.perf_counter()
+                    b.run(autotune=tune, f32=True)
+                    ms.append(time.perf_counter() - t)
+                    assert b.form()[0] == queue
+                    for s, r in zip(series, solo):
+                        assert_same(results(s), r)
+                took[tune] = min(ms)
+        assert took[True] > 2.5 * took[False], took
     finally:
         for s in series:
             s.close()

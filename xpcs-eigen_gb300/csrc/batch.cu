@@ -367,9 +367,9 @@ void tune_form(Batch &b, int mode, uint32_t flags) {
 }  // namespace
 
 void batch_run(Batch &b, int mode, uint32_t flags) {
-  if (stale(b, mode, flags)) {
+  const bool tune = (flags & XPCS_BATCH_AUTOTUNE) != 0, direct = stale(b, mode, flags);
+  if (direct) {
     b.gens.clear();  // stale until this run is through
-    const bool tune = (flags & XPCS_BATCH_AUTOTUNE) != 0;
     if (tune)
       for (Series *s : b.ss)
         if (!s->tuned) autotune(*s, mode);
@@ -378,11 +378,6 @@ void batch_run(Batch &b, int mode, uint32_t flags) {
     b.flags = flags;
     b.gens.resize(b.ss.size());
     for (size_t i = 0; i < b.ss.size(); i++) b.gens[i] = b.ss[i]->generation;
-    if (tune && !b.lanes_tuned) {
-      tune_form(b, mode, flags);
-      build_graph(b, mode, flags, b.lanes, b.queue);
-      b.last_ms = launch(b);
-    }
   } else {
     // the graph starts from the origin stream alone: what a member's own calls
     // enqueued on its stream (xpcs_multitau does not wait) ends first
@@ -392,6 +387,10 @@ void batch_run(Batch &b, int mode, uint32_t flags) {
     // host memory
     for (Series *s : b.ss)
       if (s->plan_mode != mode) prepare_multitau(*s, mode);
+  }
+  const bool chains = tune && !b.lanes_tuned;  // also after a form was chosen (set_form)
+  if (chains) tune_form(b, mode, flags);
+  if (!direct || chains) {
     if (!b.exec) {
       mt_queue_build(b.ss, b.mtq, b.origin);
       build_graph(b, mode, flags, b.lanes, b.queue);
