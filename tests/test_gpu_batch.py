@@ -333,3 +333,31 @@ def test_autotuning_after_a_change_of_form_times_the_chain_counts_again():
     finally:
         for s in series:
             s.close()
+
+
+@pytest.mark.parametrize("queue", [True, False])
+def test_sorts_of_a_members_events_leave_a_captured_batch_its_buffers(queue):
+    """Members transposed in tiles of 16 items per lane; the ordered side
+    statistics and the two-time lists sort their events in tiles of 8, between
+    the capture and the replays of the batch's graph."""
+    flat = golden_member("sparse_flat")[1]
+    plain = [open_member(*synth_member(i, *m)) for i, m in enumerate(MIX[:3])]
+    members = plain + [flat]
+    try:
+        for s in members:
+            s.set_tuning(80, 0, 16)
+        solo = [alone(s, xg.MODE_REFERENCE) for s in members]
+        with xg.Batch(members) as b:
+            b.set_form(queue)
+            for k in range(4):
+                b.run(xg.MODE_REFERENCE, f64=True, f32=True)
+                for s, r in zip(members, solo):
+                    assert_same(results(s), r)
+                if k >= 1:  # the graph exists
+                    for s in members:
+                        s.side_stats(max(s.frames // 10, 1))
+                    plain[0].twotime([1, 2], static_map=True)
+                    plain[2].twotime([1], mode=xg.MODE_EXACT, fetch=False)
+    finally:
+        for s in members:
+            s.close()

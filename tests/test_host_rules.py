@@ -1,0 +1,43 @@
+"""Host rules of the library that decide sizes and kernels, called directly
+(tests/host_rules.cpp, linked against the library; no GPU)."""
+import shutil
+import subprocess
+from pathlib import Path
+
+import pytest
+
+import xpcs_gpu as xg
+
+HERE = Path(__file__).resolve().parent
+ROOT = HERE.parent
+NVCC = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+
+pytestmark = pytest.mark.skipif(not Path(NVCC).exists(), reason="nvcc not found")
+
+
+@pytest.fixture(scope="module")
+def rules(tmp_path_factory):
+    xg.lib()
+    exe = tmp_path_factory.mktemp("rules") / "host_rules"
+    r = subprocess.run([NVCC, "-std=c++17", "-x", "cu", str(HERE / "host_rules.cpp"), "-I",
+                        str(ROOT / "include"), "-I", str(xg.HERE / "csrc"), "-L",
+                        str(xg.LIB.parent), "-lxpcs_gpu", "-Xlinker", f"-rpath={xg.LIB.parent}",
+                        "-o", str(exe)], capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stderr
+
+    def call(*args):
+        out = subprocess.run([str(exe), *map(str, args)], capture_output=True, text=True,
+                             check=True, timeout=60).stdout
+        return [float(x) for x in out.split()]
+    return call
+
+
+def test_no_sort_of_a_series_events_outgrows_its_transposes_histogram(rules):
+    """A captured batch graph holds the histogram's address.  Sorts of at most
+    the transpose's items fit what the transpose reserved, in tiles of 2,048
+    and of 4,096 items, on both sides of where the tile changes."""
+    n = [1, 2047, 2048, 4097, 1 << 20, (1 << 27) - 1, 1 << 27, (1 << 27) + 5, 1 << 31]
+    words = rules("hist", *n)
+    assert words == sorted(words)
+    for k, w in zip(n, words):
+        assert w >= 256 * -(-k // 2048) + 513

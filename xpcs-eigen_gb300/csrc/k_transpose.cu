@@ -905,18 +905,20 @@ void radix_pass(Series &s, int ipt, int bits, bool packed, bool first, bool last
   }
 }
 
-// The histogram of a pass, its rows padded to 16 bytes, and the digits' sums.
-// Sized for 8-bit digits whichever the keys take, so that sorts of one
-// series' events by different keys never move the buffer under a captured
-// batch.
-void reserve_hist(Series &s, int ntiles) {
-  const size_t hstride = ((size_t)ntiles + 3) & ~(size_t)3;
-  s.hist.reserve(hstride * RS_DIGITS_MAX + sizeof(DigitSums) / sizeof(uint32_t), s.stream);
-}
-
 int items_per_lane(int64_t n) { return n >= RS_BIG_N ? 16 : 8; }
 
 }  // namespace
+
+// The histogram of a pass over n items, its rows padded to 16 bytes, and the
+// digits' sums: sized for 8-bit digits and tiles of 8 items per lane whichever
+// a sort takes.  A series' sorts by other keys (side statistics, two-time
+// lists) have their own digits and tiles but never more items than its
+// transpose, so that none of them moves the buffer under a captured batch.
+size_t radix_hist_words(int64_t n) {
+  const int64_t tiles = (n + RS_THREADS * 8 - 1) / (RS_THREADS * 8);
+  return (size_t)((tiles + 3) & ~(int64_t)3) * RS_DIGITS_MAX +
+         sizeof(DigitSums) / sizeof(uint32_t);
+}
 
 // Stable LSD radix sort of (key, a, b) triples by the low `key_bits` bits of
 // key, with the passes above; (key2, a2, b2) is scratch of the same length.
@@ -928,7 +930,7 @@ bool radix_sort_triples(Series &s, uint32_t *key, int32_t *a, float *b, uint32_t
   const int passes = dg.passes;
   const int ipt = items_per_lane(n);
   const int ntiles = (int)((n + RS_THREADS * ipt - 1) / (RS_THREADS * ipt));
-  reserve_hist(s, ntiles);
+  s.hist.reserve(radix_hist_words(n), s.stream);
   RawCfg rc{};
   uint32_t *kb[2] = {key, key2};
   int32_t *ab[2] = {a, a2};
@@ -992,7 +994,7 @@ void transpose_range(Series &s, int32_t r0, int32_t r1, int32_t *ev_fr, float *e
   const int passes = dg.passes;
   const int ipt = s.radix_ipt == 8 || s.radix_ipt == 16 ? s.radix_ipt : items_per_lane(n);
   const int ntiles = (int)((n + RS_THREADS * ipt - 1) / (RS_THREADS * ipt));
-  reserve_hist(s, ntiles);
+  s.hist.reserve(radix_hist_words(n), s.stream);
   // sparse series below 65,536 filter frames carry one packed word per item
   // (frame, raw value) through the passes instead of a frame and a value
   const bool dense = s.desc.dense != 0;

@@ -451,6 +451,7 @@ void exclusive_scan_i32_i64(const int32_t *in, int64_t *out, int64_t n, void *ws
 
 // Kernel launchers
 void run_filter_transpose(Series &s, bool alone);                       // k_transpose.cu
+size_t radix_hist_words(int64_t n);                          // k_transpose.cu
 // Knobs for a series the caller has not tuned, from its mean row length.
 void default_knobs(Series &s, bool alone);
 // Incremental transposes: every complete block of ingested frames (k_transpose.cu)
