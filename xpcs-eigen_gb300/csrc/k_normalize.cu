@@ -288,17 +288,37 @@ __device__ __forceinline__ void warp_sum5(double (&v)[5]) {
   v[4] = __shfl_sync(FULL, c, 20);
 }
 
+// sum (x - mean)^2 over the pixels [k0, k1) in a pass of its own, in FP64, for
+// rings whose chunk sums cancel: nothing is lost however close the ratios lie.
+__device__ double deviations(int k0, int k1, double mean, const int32_t *__restrict__ pix,
+                             const float *__restrict__ g, const float *__restrict__ a,
+                             const float *__restrict__ b) {
+  double M2 = 0.0;
+  for (int k = k0 + (threadIdx.x & 31); k < k1; k += 32) {
+    const int32_t p = pix[k];
+    const double d = to_double(ratio_dw(g[p], a[p], b[p])) - mean;
+    M2 = fma(d, d, M2);
+  }
+  return warp_sum(M2);
+}
+
 // One warp per (q, tau), lanes over the ring's chunks.  Bound by FP64 issue
 // (a division is some 25 instructions at 1/64 of the FP32 rate), so the
 // formulas keep the divisions to one per entry and three per ring.  One
 // thread merging the chunks in turn took 62 us at 18 rings x 88 delays and 40
 // at 9 x 34; 19 and 14 now.
+// A ring whose spread is small beside its shifts' distance from the mean (one
+// pixel, equal ratios, dead pixels first) goes over its pixels again: below a
+// 16th of the terms M2 is the difference of, their rounding would show in it,
+// and could leave it negative.
 __global__ void k_norm_finish(int NQ, int D, const int32_t *__restrict__ qep,
                               const int32_t *__restrict__ qrow,
                               const int32_t *__restrict__ e_chunk_ptr,
                               const int32_t *__restrict__ ch_k0, const int32_t *__restrict__ ch_k1,
-                              const double *__restrict__ part, double *__restrict__ g2,
-                              double *__restrict__ se) {
+                              const double *__restrict__ part, int P,
+                              const int32_t *__restrict__ pix, const float *__restrict__ G2,
+                              const float *__restrict__ IP, const float *__restrict__ IF,
+                              double *__restrict__ g2, double *__restrict__ se) {
   overlap_after();
   const int lane = threadIdx.x & 31;
   const int idx = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
@@ -328,13 +348,20 @@ __global__ void k_norm_finish(int NQ, int D, const int32_t *__restrict__ qep,
   }
   // sum (x - mean)^2 = sum (x - s)^2 + 2 (s - mean) sum (x - s) + n (s - mean)^2
   const double mean = sx / n;
-  double M2 = 0.0;
-  for (int c = e_chunk_ptr[qep[qi]] + lane; c < e_chunk_ptr[qep[qi + 1]]; c += 32) {
+  const int c0 = e_chunk_ptr[qep[qi]], c1 = e_chunk_ptr[qep[qi + 1]];
+  double M2 = 0.0, terms = 0.0;
+  for (int c = c0 + lane; c < c1; c += 32) {
     const double *q = part + ((size_t)c * D + t) * NPART;
     const double nc = (double)(ch_k1[c] - ch_k0[c]), d = q[5] - mean;
     M2 += fma(d, fma(nc, d, 2.0 * q[3]), q[4]);
+    terms += fma(nc * d, d, q[4]);
   }
   M2 = warp_sum(M2);
+  terms = warp_sum(terms);
+  if (M2 < 0.0625 * terms) {  // (not NaN, and not a ring of zeros)
+    const size_t o = (size_t)t * P;
+    M2 = deviations(ch_k0[c0], ch_k1[c1 - 1], mean, pix, G2 + o, IP + o, IF + o);
+  }
   if (lane == 0) {
     const int row = qrow[qi];
     g2[(size_t)t * NQ + row] = gacc / (double)gcnt;
@@ -706,7 +733,8 @@ void run_normalize(Series &s, bool want64, bool want32) {
     const int bs = 128;
     launch_overlapped(k_norm_finish, (unsigned)(((int64_t)NQ * D * 32 + bs - 1) / bs), bs, 0, st,
                       NQ, D, s.n_q_entry_ptr.p, s.n_q_row.p, s.n_e_chunk_ptr.p, s.n_ch_k0.p,
-                      s.n_ch_k1.p, s.n_part.p, s.n_g2.p, s.n_se.p);
+                      s.n_ch_k1.p, s.n_part.p, P, s.n_pix.p, s.G2.p, s.IP.p, s.IF.p, s.n_g2.p,
+                      s.n_se.p);
   }
   if (want32) {
     const QMap &qm = s.qmap;
