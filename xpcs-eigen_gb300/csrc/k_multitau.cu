@@ -2093,8 +2093,7 @@ void launch_float_rows(Series &s, const McPlan &hp, cudaStream_t st, int sms) {
   }
   if (mt_float_rows_warp(hp)) {
     const size_t smf = FW_WARPS * fw_warp_bytes(hp.acc);
-    XG_CUDA(cudaFuncSetAttribute(k_mt_fwarp, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smf));
+    allow_smem(k_mt_fwarp);
     int per_sm = 0;
     XG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mt_fwarp, FW_WARPS * 32,
                                                           smf));
@@ -2201,11 +2200,10 @@ void run_multitau(Series &s, int mode) {
                smw = warp_smem(D, scr, MT_WARP_CAP, WP_WARPS);
   const size_t smm = warp_smem(D, scr, MT_MID_CAP, MID_WARPS);
   const size_t sml = warp_smem(D, scr, MT_LONG_CAP, LONG_WARPS);
-  if (smt > 227 * 1024 || smw > 227 * 1024 || smm > 227 * 1024 || sml > 227 * 1024)
+  if (smt > SMEM_MAX || smw > SMEM_MAX || smm > SMEM_MAX || sml > SMEM_MAX)
     throw Error(XPCS_ERR_INVALID_ARGUMENT, "delay schedule too large for the multi-tau kernels");
-  XG_CUDA(cudaFuncSetAttribute(ktt, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smt));
-  XG_CUDA(cudaFuncSetAttribute(k_mt_warp, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)std::max(std::max(smw, smm), sml)));
+  allow_smem(ktt);
+  allow_smem(k_mt_warp);
   int sms = 0;
   XG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s.device));
   XG_CUDA(cudaEventRecord(s.ev[4], st));
@@ -2214,15 +2212,15 @@ void run_multitau(Series &s, int mode) {
   // long rows in two launches over one list: up to 1024 events with 4 warps per
   // block, longer ones, first, with 2 warps per block; rows of 81-256 events;
   // the thread kernel's pixels
-  k_mt_warp<<<sms * (int)((227 * 1024) / sml), LONG_WARPS * 32, sml, st>>>(
+  k_mt_warp<<<sms * (int)(SMEM_MAX / sml), LONG_WARPS * 32, sml, st>>>(
       s.plan.p, s.llist.p, &ds->nlong, MT_MID_CAP, MT_LONG_CAP, s.row_ptr.p, s.row_len.p,
       s.ev_frame.p, s.ev_val.p, s.G2.p, s.IP.p, s.IF.p, &ds->wnext[0]);
   XG_CHECK_LAUNCH();
-  launch_overlapped(k_mt_warp, sms * (int)((227 * 1024) / smm), MID_WARPS * 32, smm, st,
+  launch_overlapped(k_mt_warp, sms * (int)(SMEM_MAX / smm), MID_WARPS * 32, smm, st,
                     s.plan.p, s.llist.p, &ds->nlong, MT_WARP_CAP, MT_MID_CAP, s.row_ptr.p,
                     s.row_len.p, s.ev_frame.p, s.ev_val.p, s.G2.p, s.IP.p, s.IF.p,
                     &ds->wnext[1]);
-  launch_overlapped(k_mt_warp, sms * (int)((227 * 1024) / smw), WP_WARPS * 32, smw, st,
+  launch_overlapped(k_mt_warp, sms * (int)(SMEM_MAX / smw), WP_WARPS * 32, smw, st,
                     s.plan.p, s.wlist.p, &ds->nwarp, 0, MT_WARP_CAP, s.row_ptr.p, s.row_len.p,
                     s.ev_frame.p, s.ev_val.p, s.G2.p, s.IP.p, s.IF.p, &ds->wnext[2]);
   const int per_block = MT_WARPS * 32;
@@ -2282,10 +2280,9 @@ void mt_queue_run(const std::vector<Series *> &ss, MtQueue &q, cudaStream_t st) 
   for (int t = 0; t < 3; t++) {
     const int cap = tiers[t][2], warps = tiers[t][3];
     const size_t sm = pref_bytes + (size_t)warps * (2 * cap + 32 * q.acc_max) * sizeof(int32_t);
-    if (sm > 227 * 1024)
+    if (sm > SMEM_MAX)
       throw Error(XPCS_ERR_INVALID_ARGUMENT, "delay schedule too large for the multi-tau kernels");
-    XG_CUDA(cudaFuncSetAttribute(k_mt_warp_queue, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)sm));
+    allow_smem(k_mt_warp_queue);
     int per_sm = 0;
     XG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mt_warp_queue, warps * 32,
                                                           sm));
@@ -2307,9 +2304,9 @@ void mt_queue_run(const std::vector<Series *> &ss, MtQueue &q, cudaStream_t st) 
   for (int c = 0; c < MT_THREAD_NCAPS; c++) {
     if (!q.cap_count[c]) continue;
     const size_t smt = thread_smem(q.scr_max, MT_THREAD_CAPS[c]);
-    if (smt > 227 * 1024)
+    if (smt > SMEM_MAX)
       throw Error(XPCS_ERR_INVALID_ARGUMENT, "delay schedule too large for the multi-tau kernels");
-    XG_CUDA(cudaFuncSetAttribute(kq[c], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smt));
+    allow_smem(kq[c]);
     int per_sm = 0;
     XG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kq[c], MT_WARPS * 32, smt));
     const int blocks = std::min(sms * std::max(1, per_sm), (q.cap_groups[c] + MT_WARPS - 1) /
@@ -2337,7 +2334,7 @@ cudaError_t mt_noalloc_setup() {
     cudaError_t e = cudaFuncGetAttributes(&a, f);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               227 * 1024 - (int)a.sharedSizeBytes);
+                               (int)SMEM_MAX - (int)a.sharedSizeBytes);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
@@ -2348,10 +2345,10 @@ cudaError_t mt_noalloc_setup() {
 // thresholds, as make_plan requires.
 bool mt_noalloc_supported(const McPlan &hp, const McArrays &ar) {
   const int scr = std::max(hp.acc, hp.nlev);
-  if (hp.D <= 0 || hp.P > (1 << 30) || hp.acc > 32 || thread_smem(hp.scr, 80) > 227 * 1024 ||
-      warp_smem(0, scr, MT_WARP_CAP, WP_WARPS) > 227 * 1024 ||
-      warp_smem(0, scr, MT_MID_CAP, MID_WARPS) > 227 * 1024 ||
-      warp_smem(0, scr, MT_LONG_CAP, LONG_WARPS) > 227 * 1024)
+  if (hp.D <= 0 || hp.P > (1 << 30) || hp.acc > 32 || thread_smem(hp.scr, 80) > SMEM_MAX ||
+      warp_smem(0, scr, MT_WARP_CAP, WP_WARPS) > SMEM_MAX ||
+      warp_smem(0, scr, MT_MID_CAP, MID_WARPS) > SMEM_MAX ||
+      warp_smem(0, scr, MT_LONG_CAP, LONG_WARPS) > SMEM_MAX)
     return false;
   for (int k = 1; k < hp.D; k++)
     if (ar.t_ip[k] >= ar.t_ip[k - 1] || ar.tau_abs[k] <= ar.tau_abs[k - 1]) return false;
@@ -2388,7 +2385,7 @@ cudaError_t mt_noalloc_rows(const McPlan &hp, const NaRows &v, int sms, cudaStre
                            {MT_MID_CAP, MT_LONG_CAP, LONG_WARPS}};
   for (int t = 0; t < 3; t++) {
     const size_t sm = warp_smem(0, scr, tiers[t][1], tiers[t][2]);
-    k_na_warp<<<sms * std::max(1, (int)((227 * 1024) / sm)), tiers[t][2] * 32, sm, st>>>(
+    k_na_warp<<<sms * std::max(1, (int)(SMEM_MAX / sm)), tiers[t][2] * 32, sm, st>>>(
         v, 1 << t, tiers[t][0], tiers[t][1], v.status + 2 + t);
   }
   if (mt_float_rows_warp(hp))

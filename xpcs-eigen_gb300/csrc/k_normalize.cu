@@ -446,6 +446,7 @@ __device__ __forceinline__ float div_count(float a, float n, int ni, float y) {
 // flight while the threads step through chunk c, so each thread's sequential
 // chain reads shared memory instead of waiting on global loads.
 constexpr int FR_SMEM = 200 * 1024;  // shared memory budget of a replay block
+constexpr int FR_ROWS = 256;         // most rows of a chunk
 constexpr uint32_t FR_WAIT_LIMIT = 1u << 22;  // polls before a wait is given up
 
 __device__ __forceinline__ uint32_t fr_u32(const void *p) {
@@ -598,7 +599,7 @@ __global__ void k_q_f32(int NQ, int D, int Dp, int FR_CH, const int32_t *__restr
   // reciprocal depends on the count only: the block computes each chunk's
   // into a table, off the chain of dependent operations that each tau's
   // running mean is.
-  __shared__ __align__(16) float rtab[256];
+  __shared__ __align__(16) float rtab[FR_ROWS];
   float avg = 0.f, sd = 0.f;
   const int k0 = epp[qep[qi]], n = epp[qep[qi + 1]] - k0;
   const float *src[1] = {X};
@@ -760,14 +761,12 @@ void run_normalize(Series &s, bool want64, bool want32) {
     }
     if (D > 1024) throw Error(XPCS_ERR_INVALID_ARGUMENT, "more than 1024 delays");
     const int bs = (D + 31) / 32 * 32;
-    const int ch_e = std::max(1, std::min(256, (FR_SMEM - 64) / (24 * Dp)));
-    const int ch_q = std::max(1, std::min(256, (FR_SMEM - 64) / (8 * Dp)));
+    const int ch_e = std::max(1, std::min(FR_ROWS, (FR_SMEM - 64) / (24 * Dp)));
+    const int ch_q = std::max(1, std::min(FR_ROWS, (FR_SMEM - 64) / (8 * Dp)));
     const size_t sm_e = sizeof(float) * 2 * 3 * (size_t)ch_e * Dp + 2 * sizeof(uint64_t);
     const size_t sm_q = sizeof(float) * 2 * (size_t)ch_q * Dp + 2 * sizeof(uint64_t);
-    XG_CUDA(cudaFuncSetAttribute(k_entry_f32, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)sm_e));
-    XG_CUDA(cudaFuncSetAttribute(k_q_f32, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)sm_q));
+    allow_smem(k_entry_f32);
+    allow_smem(k_q_f32, sizeof(float) * FR_ROWS);
     k_q_f32<<<NQ, bs, sm_q, st>>>(NQ, D, Dp, ch_q, s.n_q_entry_ptr.p, s.n_q_row.p,
                                   s.n_entry_pix_ptr.p, s.n_tx.p, s.n_sef.p, s.n_unsafe.p,
                                   &s.stats.p->error);

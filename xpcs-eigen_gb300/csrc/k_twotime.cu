@@ -660,8 +660,7 @@ void gram_events(Series &s, const TwoTimeReq &req, const TwoTimeLayout &lay, int
   }
   const int W = tt_columns(F, sizeof(float));
   const size_t smem = sizeof(float) * (size_t)F * W;
-  XG_CUDA(cudaFuncSetAttribute(k_tt_gram_events, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)smem));
+  allow_smem(k_tt_gram_events);
   k_tt_gram_events<<<dim3((F + W - 1) / W, Q), 32 * W, smem, st>>>(
       F, l.q_ptr, s.tt_cols.p, ab.first, ab.second, s.tt_row_pix.p, s.row_ptr.p, s.ev_frame.p,
       s.tt_V.p, s.tt_C.p);
@@ -722,8 +721,7 @@ bool gram_counts(Series &s, const TwoTimeReq &req, const TwoTimeLayout &lay, int
     XG_CHECK_LAUNCH();
   }
   const size_t smem = col * (size_t)F * W;
-  XG_CUDA(cudaFuncSetAttribute(k_tt_gram_counts, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)smem));
+  allow_smem(k_tt_gram_counts);
   // q bins at a time: their double matrices within 2 GB
   const size_t F2 = (size_t)F * F;
   const int32_t step = (int32_t)std::max<size_t>(1, std::min<size_t>(Q, (2ull << 30) / (8 * F2)));

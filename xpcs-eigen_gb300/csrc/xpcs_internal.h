@@ -28,6 +28,17 @@ struct Error : std::runtime_error {
                         std::string(#call) + ": " + cudaGetErrorString(e_));          \
   } while (0)
 
+// Lifts a kernel's limit of dynamic shared memory to all that a block may have
+// beside its static arrays.  The limit belongs to the kernel on its device and
+// not to a launch: were it set to each call's own size, a call on another
+// thread could lower it between the two.
+constexpr size_t SMEM_MAX = 227 * 1024;
+template <class... P>
+void allow_smem(void (*kernel)(P...), size_t static_bytes = 0) {
+  XG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)(SMEM_MAX - static_bytes)));
+}
+
 // Kernels launched by this thread (the stage tracer reports per-call deltas).
 extern thread_local int64_t tl_launches;
 #define XG_CHECK_LAUNCH()          \
