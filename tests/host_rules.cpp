@@ -1,6 +1,9 @@
 // Prints what the library's host rules (csrc/xpcs_internal.h) give, one value
 // per line, for tests/test_host_rules.py.  No device is touched.
 //   host_rules hist N ...      words of the radix sorts' histogram for N items
+//   host_rules rows P E F      rows the caller holds, P pixels, E events, F frames:
+//                              thread kernel's row capacity, and the longest row that
+//                              a series takes by thread (0: every row to a warp)
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -11,5 +14,13 @@ int main(int argc, char **argv) {
   if (argc > 1 && !std::strcmp(argv[1], "hist"))
     for (int k = 2; k < argc; k++)
       std::printf("%zu\n", xg::radix_hist_words(std::atoll(argv[k])));
+  if (argc == 5 && !std::strcmp(argv[1], "rows")) {
+    xg::Series s;
+    s.P = std::atoi(argv[2]);
+    s.raw_events = std::atoll(argv[3]);
+    s.F = std::atoi(argv[4]);
+    xg::default_knobs(s, true);
+    std::printf("%d\n%d\n", s.thread_cap, s.class_cap);
+  }
   return 0;
 }

@@ -41,3 +41,14 @@ def test_no_sort_of_a_series_events_outgrows_its_transposes_histogram(rules):
     assert words == sorted(words)
     for k, w in zip(n, words):
         assert w >= 256 * -(-k // 2048) + 513
+
+
+@pytest.mark.parametrize("pixels,mean,cap,by_thread", [
+    (1 << 20, 3, 32, True), (1 << 20, 50, 80, True), (36864, 10, 32, True), (16384, 3, 32, True),
+    (4096, 10, 32, False), (16384, 80, 112, False),
+])
+def test_caller_held_rows_choose_their_kernel_by_pixels_and_row_length(rules, pixels, mean, cap,
+                                                                       by_thread):
+    """Rows without a partition map: every pixel counts, so rows of many pixels
+    keep a thread each and the mean row length picks the capacity."""
+    assert rules("rows", pixels, pixels * mean, 4000) == [cap, cap if by_thread else 0]

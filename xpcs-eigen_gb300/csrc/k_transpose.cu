@@ -1317,6 +1317,7 @@ void default_knobs(Series &s, bool alone) {
   if (s.valid_pixels < 0) {
     s.valid_pixels = 0;
     for (uint8_t v : s.qmap.valid) s.valid_pixels += v;
+    if (s.qmap.valid.empty()) s.valid_pixels = s.P;  // caller-held rows have no map
   }
   const double mean =
       (double)s.raw_events / ((double)std::max<int64_t>(s.valid_pixels, 1) * s.R_in);
