@@ -361,3 +361,31 @@ def test_sorts_of_a_members_events_leave_a_captured_batch_its_buffers(queue):
     finally:
         for s in members:
             s.close()
+
+
+def test_a_capacity_set_after_autotuning_holds_for_few_pixels():
+    """48 x 48 pixels, 4,000 frames, rows of up to 100 events: a warp a row by
+    default, a thread a row once the caller chose a capacity, before or after
+    an autotune.  One thread a row takes several times as long here."""
+    acq, dq, sq, frames = synth_member(2, 48, 4000, 0.02, 8, (10, 900))
+
+    def int_ms(s):
+        ms = []
+        for _ in range(8):
+            s.multitau()
+            s.synchronize()
+            ms.append(s.stage_times()["multitau_int_ms"])
+        return min(ms)
+
+    s = open_member(acq, dq, sq, frames)
+    try:
+        warp = int_ms(s)
+        s.set_tuning(112, 0, 0)
+        thread = int_ms(s)
+        assert thread > 1.5 * warp  # or the rest says nothing
+        s.autotune()
+        assert int_ms(s) < 1.3 * warp  # the faster of both forms
+        s.set_tuning(112, 0, 0)
+        assert int_ms(s) > 1.3 * warp
+    finally:
+        s.close()

@@ -52,3 +52,12 @@ def test_caller_held_rows_choose_their_kernel_by_pixels_and_row_length(rules, pi
     """Rows without a partition map: every pixel counts, so rows of many pixels
     keep a thread each and the mean row length picks the capacity."""
     assert rules("rows", pixels, pixels * mean, 4000) == [cap, cap if by_thread else 0]
+
+
+@pytest.mark.parametrize("pixels,by_thread,alone", [(4096, 1, 48), (4096, 0, 0),
+                                                    (1 << 20, 1, 48), (1 << 20, 0, 48)])
+def test_a_tuned_series_of_few_pixels_keeps_a_capacity_that_was_chosen(rules, pixels, by_thread,
+                                                                       alone):
+    """The caller's row capacity, also one set after an autotune, and the thread
+    form where the autotuner found it faster, hold for few pixels too."""
+    assert rules("tuned", pixels, pixels * 20, 1000, by_thread) == [alone, 48]

@@ -97,7 +97,9 @@ Batch *batch_create(Series *const *ss, int32_t n) {
 //      which decide up to which level (32 x words bins) the pair search runs
 //      on the occupancy bitmask instead of the sparse two-candidate checks;
 //   3. the event tile of the transpose: 8 or 16 items per lane (tiles of
-//      2,048 or 4,096 events).
+//      2,048 or 4,096 events);
+//   4. for a series of few pixels (default_knobs), whether alone it gives every
+//      row to a warp or keeps the thread kernel up to the capacity found.
 // A change of any knob changes the work (pixel classes, kernel launch), so it
 // counts as a change of the series for captured batch graphs.  Results do not
 // depend on the knobs.
@@ -107,13 +109,13 @@ int32_t autotune(Series &s, int mode) {
   XG_CUDA(cudaEventCreate(&e0));
   XG_CUDA(cudaEventCreate(&e1));
   const int32_t cap0 = s.thread_cap, scr0 = s.scr_extra, ipt0 = s.radix_ipt;
-  const bool set0 = s.knobs_set;
+  const bool set0 = s.knobs_set, thread0 = s.by_thread;
   s.knobs_set = true;  // the candidates below are not replaced by the defaults
-  auto time_pass = [&]() {
+  auto time_pass = [&](bool alone) {
     float ms = 0.f;
     for (int rep = 0; rep < 2; rep++) {  // the second pass is timed
       XG_CUDA(cudaEventRecord(e0, st));
-      run_filter_transpose(s, false);
+      run_filter_transpose(s, alone);
       run_multitau(s, mode);
       XG_CUDA(cudaEventRecord(e1, st));
       XG_CUDA(cudaEventSynchronize(e1));
@@ -128,7 +130,7 @@ int32_t autotune(Series &s, int mode) {
     bool first = true;
     for (int32_t v : values) {
       knob = v;
-      const float ms = time_pass();
+      const float ms = time_pass(false);
       if (first || ms < best_ms) {
         best_ms = ms;
         best = v;
@@ -143,11 +145,15 @@ int32_t autotune(Series &s, int mode) {
     search(s.thread_cap, {32, 48, 64, 80, 112});
     search(s.scr_extra, {0, 8});
     search(s.radix_ipt, {8, 16});
+    s.by_thread = false;
+    default_knobs(s, true);
+    if (s.class_cap == 0) s.by_thread = time_pass(false) < time_pass(true);
   } catch (...) {
     s.thread_cap = cap0;
     s.scr_extra = scr0;
     s.radix_ipt = ipt0;
     s.knobs_set = set0;
+    s.by_thread = thread0;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     throw;

@@ -1312,7 +1312,7 @@ void reset_blocks(Series &s) {
 // 36,864 pixels 39 / 102, 58 / 116 and 129 / 125 us; rows of 80 events (4,000
 // frames) 190 / 94 us at 16,384 and 197 / 186 us at 36,864 pixels.  The line
 // lies where the two meet.  It does not hold for a row capacity that the caller
-// chose.
+// chose, and the autotuner times both forms of such a series.
 void default_knobs(Series &s, bool alone) {
   if (s.valid_pixels < 0) {
     s.valid_pixels = 0;
@@ -1335,7 +1335,7 @@ void default_knobs(Series &s, bool alone) {
     s.scr_extra = s.F >= 16384 ? 8 : 0;
   }
   const bool few = s.valid_pixels <= std::min(5000.0 + 800.0 * mean, 32000.0);
-  s.class_cap = few && alone && (s.tuned || !s.knobs_set) ? 0 : s.thread_cap;
+  s.class_cap = few && alone && !s.by_thread ? 0 : s.thread_cap;
 }
 
 void run_filter_transpose(Series &s, bool alone) {

@@ -340,6 +340,8 @@ struct Series {
   int32_t plan_scr = -1;    // scratch words of the uploaded plan
   bool tuned = false;       // thread_cap, scr_extra, radix_ipt chosen by xpcs_autotune
   bool knobs_set = false;   // chosen by the caller or the autotuner (else: default_knobs)
+  bool by_thread = false;   // few pixels: rows keep the thread kernel alone as well, by the
+                            // caller's capacity or the autotuner's times
   int64_t valid_pixels = -1;  // pixels of the q-map mask (counted once)
   DBuf<float> G2, IP, IF;
   bool have_multitau = false;
