@@ -80,3 +80,63 @@ def test_device_properties_and_bad_ordinal():
     with pytest.raises(xg.XpcsError) as e:
         xg.device_sm_count(1 << 20)
     assert e.value.code == 1
+
+
+def _flat_series(F=300):
+    W, H = 310, 300
+    rng = np.random.default_rng(5)
+    n = rng.poisson(0.04, (F, W * H))
+    hit = n > 0
+    nnz, idx, val = hit.sum(1).astype(np.uint32), np.nonzero(hit)[1], n[hit]
+    dq = np.ones((H, W), np.int32)
+    s = xg.Series(W, H, F, 8, dq, dq, flatfield=rng.uniform(0.8, 1.2, W * H))
+    s.ingest_sparse(nnz, idx.astype(np.int32), val.astype(np.int16))
+    s.synchronize()
+    return s, idx.size
+
+
+def test_float_rows_within_what_a_limit_left_them_before():
+    """The scratch of the thread-per-pixel float kernel (as large as G2, IP and
+    IF, and its rows' slots) is no condition of a call: a limit that leaves room
+    for the event lists (54 B per event), the per-pixel tables and the results
+    is enough, alone and in a batch; what a call did take of it is given back."""
+    try:
+        s, events = _flat_series()
+        with s:
+            s.multitau(xg.MODE_REFERENCE)
+            want = s.g2ipif()
+            assert s.info().float_path_pixels > s.P // 2
+            room = s.P * (12 * s.D + 64) + 54 * events + (4 << 20)
+        for limited_room in (room, 1 << 34):
+            s, _ = _flat_series()
+            with s:
+                xg.set_device_memory_limit(0, xg.device_memory(0)[0] + limited_room)
+                for _ in range(2):
+                    s.multitau(xg.MODE_REFERENCE)
+                    for g, w in zip(s.g2ipif(), want):
+                        assert same_bits(g, w)
+                    assert s.info().float_path_pixels > s.P // 2
+                    s.normalize(f32=False)
+                with xg.Batch([s]) as b:
+                    for queue in (True, False):
+                        b.set_form(queue)
+                        for k in range(3):
+                            b.run(f64=False)
+                            for g, w in zip(s.g2ipif(), want):
+                                assert same_bits(g, w)
+                            if k == 1:
+                                s.multitau(xg.MODE_REFERENCE)
+                assert xg.device_memory(0)[0] < xg.device_memory(0)[1] - limited_room + room
+                xg.set_device_memory_limit(0, 0)
+                b = xg.Batch([s])
+                b.run(f64=False)
+                b.run(f64=False)  # captured with the scratch, which the next call gives back
+                xg.set_device_memory_limit(0, xg.device_memory(0)[0] + limited_room)
+                s.multitau(xg.MODE_REFERENCE)
+                b.run(f64=False)
+                for g, w in zip(s.g2ipif(), want):
+                    assert same_bits(g, w)
+                b.close()
+                xg.set_device_memory_limit(0, 0)
+    finally:
+        xg.set_device_memory_limit(0, 0)

@@ -55,6 +55,8 @@ void *dev_alloc(size_t bytes, cudaStream_t st) {
   return q;
 }
 
+bool dev_limited() { return g_dev_limit[acct_device()].load() != 0; }
+
 void dev_free(void *p, size_t bytes, cudaStream_t st) {
   if (!p) return;
   cudaFreeAsync(p, st);

@@ -2054,6 +2054,51 @@ void reset_counters(Series &s, cudaStream_t st) {
   XG_CUDA(cudaMemsetAsync((char *)s.stats.p + first, 0, end - first, st));
 }
 
+// Given back: a captured batch graph that holds the addresses is stale with it.
+void release_float_thread(Series &s, cudaStream_t st) {
+  if (s.ft_slots.p || s.ft_list.p || s.ft_out.p) s.generation++;
+  s.ft_slots.release(st);
+  s.ft_list.release(st);
+  s.ft_out.release(st);
+}
+
+// The scratch of k_mt_fthread, up to 3 GB of slots and as much as G2, IP and IF
+// together; false where it is not to be had (the rows then go to the warp-per-row
+// kernel, which needs none).  A captured graph allocates nothing.
+bool reserve_float_thread(Series &s, cudaStream_t st, size_t slots, size_t list, size_t out) {
+  if (slots <= s.ft_slots.cap && list <= s.ft_list.cap && out <= s.ft_out.cap) return true;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  XG_CUDA(cudaStreamIsCapturing(st, &cap));
+  if (cap != cudaStreamCaptureStatusNone) return false;
+  try {
+    s.ft_slots.reserve(slots, st);
+    s.ft_list.reserve(list, st);
+    s.ft_out.reserve(out, st);
+    return true;
+  } catch (const Error &e) {
+    if (e.code != XPCS_ERR_OUT_OF_MEMORY) throw;
+    release_float_thread(s, st);
+    return false;
+  }
+}
+
+// The rows of the thread-per-pixel float kernel moved to the list of the
+// warp-per-row one.
+__global__ void k_ft_to_warps(int32_t P, const uint8_t *__restrict__ pclass,
+                              int32_t *__restrict__ flist, DevStats *__restrict__ stats) {
+  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool mine = p < P && pclass[p] == PCLASS_FTHREAD;
+  const unsigned m = __ballot_sync(0xffffffffu, mine);
+  const int lane = threadIdx.x & 31;
+  int base = 0;
+  if (lane == 0 && m) {
+    base = atomicAdd(&stats->nfloat, __popc(m));
+    atomicSub(&stats->nfthread, __popc(m));
+  }
+  base = __shfl_sync(0xffffffffu, base, 0);
+  if (mine) flist[base + __popc(m & ((1u << lane) - 1u))] = (int32_t)p;
+}
+
 // The float rows of a series (flatfield, average, hot pixels, dense data,
 // normalize_by_framesum) on st: the thread-per-pixel kernel's rows, and for the
 // others the warp-per-row replay when the schedule allows it (beside the last
@@ -2070,7 +2115,7 @@ void launch_float_rows(Series &s, const McPlan &hp, cudaStream_t st, int sms) {
     prepare_framesum_scale(s);
     fscale = s.d_fscale.p;
   }
-  const bool thread_rows = s.float_cap > 0;
+  bool thread_rows = s.float_cap > 0;
   const int Dp = (s.D + 3) & ~3;  // padded delays of k_mt_fthread's staged results
   if (thread_rows) {
     const auto kernel = s.desc.delays_per_level <= 4 ? k_mt_fthread<8, 4> : k_mt_fthread<16, 8>;
@@ -2081,14 +2126,17 @@ void launch_float_rows(Series &s, const McPlan &hp, cudaStream_t st, int sms) {
     per_sm = std::min(per_sm, (int)(FT_SLOT_BYTES / (block_bytes * (size_t)sms)));
     const int windows = (P + FT_WIN_PIX - 1) / FT_WIN_PIX;
     const int blocks = std::min(sms * std::max(1, per_sm), windows * (FT_WIN_PIX / 32 / FT_WARPS));
-    s.ft_slots.reserve(blocks * block_bytes, st);
-    s.ft_list.reserve((size_t)windows * FT_WIN_PIX, st);
-    s.ft_out.reserve((size_t)P * 3 * Dp, st);
-    k_ft_sort<<<windows, 256, 0, st>>>(P, s.row_len.p, s.pclass.p, s.ft_list.p);
-    XG_CHECK_LAUNCH();
-    kernel<<<blocks, FT_WARPS * 32, 0, st>>>(
-        s.plan.p, s.float_cap, (uint2 *)s.ft_slots.p, s.ft_list.p, s.row_ptr.p, s.row_len.p,
-        s.ev_frame.p, s.ev_val.p, fscale, s.stats.p, Dp, s.ft_out.p);
+    thread_rows = reserve_float_thread(s, st, blocks * block_bytes,
+                                       (size_t)windows * FT_WIN_PIX, (size_t)P * 3 * Dp);
+    if (thread_rows) {
+      k_ft_sort<<<windows, 256, 0, st>>>(P, s.row_len.p, s.pclass.p, s.ft_list.p);
+      XG_CHECK_LAUNCH();
+      kernel<<<blocks, FT_WARPS * 32, 0, st>>>(
+          s.plan.p, s.float_cap, (uint2 *)s.ft_slots.p, s.ft_list.p, s.row_ptr.p, s.row_len.p,
+          s.ev_frame.p, s.ev_val.p, fscale, s.stats.p, Dp, s.ft_out.p);
+    } else {
+      k_ft_to_warps<<<(P + 255) / 256, 256, 0, st>>>(P, s.pclass.p, s.flist.p, s.stats.p);
+    }
     XG_CHECK_LAUNCH();
   }
   if (mt_float_rows_warp(hp)) {
@@ -2118,6 +2166,11 @@ void launch_float_rows(Series &s, const McPlan &hp, cudaStream_t st, int sms) {
     k_ft_out<<<(P + 31) / 32, 256, 0, st>>>(P, s.D, Dp, s.pclass.p, s.ft_out.p, s.G2.p, s.IP.p,
                                             s.IF.p);
     XG_CHECK_LAUNCH();
+    // under a memory limit the scratch is the call's alone: what follows, and
+    // other handles, have what they had without this kernel
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    XG_CUDA(cudaStreamIsCapturing(st, &cap));
+    if (cap == cudaStreamCaptureStatusNone && dev_limited()) release_float_thread(s, st);
   }
 }
 

@@ -61,6 +61,8 @@ enum : int32_t {
 // XPCS_ERR_OUT_OF_MEMORY before CUDA is asked (abi.cu).
 void *dev_alloc(size_t bytes, cudaStream_t st);
 void dev_free(void *p, size_t bytes, cudaStream_t st);
+// Whether the current device has a memory limit (xpcs_set_device_memory_limit).
+bool dev_limited();
 
 // Makes the pages of a large, fresh host buffer that a result is about to be
 // copied to (abi.cu).
