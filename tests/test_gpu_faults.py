@@ -82,6 +82,40 @@ def test_device_properties_and_bad_ordinal():
     assert e.value.code == 1
 
 
+@pytest.mark.parametrize("mode,side,F,density,need", [
+    # REFERENCE: the dense rows [P][F]; EXACT: X^T of a group and F x F matrices
+    (xg.MODE_REFERENCE, 200, 100, 0.39, lambda P, F: 4 * P * F),
+    (xg.MODE_EXACT, 20, 900, 0.04, lambda P, F: 20 * F * F + (8 << 20)),
+    (xg.MODE_EXACT, 300, 100, 0.05, lambda P, F: 2 * 128 * P // 6 + 20 * F * F + (1 << 19)),
+])
+def test_two_time_within_what_a_limit_left_it_before(mode, side, F, density, need):
+    """Event lists are no condition of a two-time call: a limit that leaves room
+    for the dense forms and the results is enough."""
+    rng = np.random.default_rng(F)
+    P = side * side
+    sq = (np.arange(P) * 6 // P + 1).astype(np.int32).reshape(side, side)
+    hit = rng.random((F, P)) < density
+    nnz, idx = hit.sum(1).astype(np.uint32), np.nonzero(hit)[1].astype(np.int32)
+    try:
+        out = []
+        for limit in (False, True):
+            with xg.Series(side, side, F, 2, sq, sq) as s:
+                s.ingest_sparse(nnz, idx, np.ones(idx.size, np.int16))
+                s.multitau()
+                s.synchronize()
+                if limit:
+                    xg.set_device_memory_limit(0, xg.device_memory(0)[0] + 16 * P + 4 * 7 * F * F
+                                               + need(P, F) + (1 << 20))
+                out.append(s.twotime(range(1, 7), window=2, mode=mode))
+        a, b = out
+        for q in range(1, 7):
+            assert same_bits(a["c2t"][q], b["c2t"][q])
+        for k in ("sg", "g2full", "g2partials"):
+            assert same_bits(a[k], b[k]), k
+    finally:
+        xg.set_device_memory_limit(0, 0)
+
+
 def _flat_series(F=300):
     W, H = 310, 300
     rng = np.random.default_rng(5)

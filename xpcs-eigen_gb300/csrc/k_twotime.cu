@@ -552,6 +552,16 @@ __global__ void k_tt_diag(int32_t Q, int32_t F, int32_t window, int32_t tp,
   }
 }
 
+// Device memory that the event lists and their tables would still have to
+// allocate.
+size_t lists_bytes(const Series &s, int32_t R, int32_t G, int32_t Q) {
+  const size_t n = (size_t)std::max<int64_t>(s.raw_events, 1);
+  return s.keyA.more(n) + s.keyB.more(n) + s.frA.more(n) + s.frB.more(n) + s.vA.more(n) +
+         s.vB.more(n) + s.hist.more(radix_hist_words(n)) + s.tt_len.more(R) +
+         s.tt_cpos.more((size_t)R + 1) + s.tt_cols.more((size_t)Q * s.F + 1) +
+         s.tt_qptr.more(2 * (size_t)Q + G + 2) + s.scan_tmp.more(scan_workspace_bytes(R));
+}
+
 // Whether the rows are sparse enough for the event Gram, from the mean number
 // of events per pixel and frame, d.  Its work grows as d^2, the tiled Gram's
 // not at all, and short columns are cheap at any density.  Whole calls in ms,
@@ -562,8 +572,13 @@ __global__ void k_tt_diag(int32_t Q, int32_t F, int32_t window, int32_t tp,
 //   128^2    2,000  1.10/6.61   2.50/6.74   7.95/7.02   28.5/7.5
 //   256^2      700  1.20/12.5   3.03/12.6   10.1/12.8   36.8/13.2
 //   64^2     4,096  1.58/5.60   3.10/5.75   9.03/6.09   32.0/7.0
-bool tt_use_events(Series &s) {
+// Under a memory limit the form that takes less more of it is chosen, so that
+// no call is refused for the lists.
+bool tt_use_events(Series &s, int32_t R, int32_t G, int32_t Q) {
   if (tt_columns(s.F, sizeof(float)) == 0) return false;
+  if (dev_limited() && lists_bytes(s, R, G, Q) + s.tt_V.more(s.raw_events) >
+                           s.tt_V.more((size_t)R * s.F))
+    return false;
   const double most = std::min(0.4, std::max(0.15, 40.0 / s.F));
   return (double)s.raw_events <= most * (double)s.qmap.pix.size() * s.R_in * s.F;
 }
@@ -689,6 +704,16 @@ bool gram_counts(Series &s, const TwoTimeReq &req, const TwoTimeLayout &lay, int
   const size_t col = sizeof(int32_t) + (multi ? sizeof(double) : 0);
   const int W = tt_columns(F, col);
   if (W == 0) return false;
+  const size_t F2 = (size_t)F * F;
+  // q bins at a time: their double matrices within 2 GB
+  int32_t step = (int32_t)std::max<size_t>(1, std::min<size_t>(Q, (2ull << 30) / (8 * F2)));
+  if (dev_limited()) {  // as in tt_use_events
+    step = 1;
+    if (lists_bytes(s, R, G, Q) + s.tt_Cq.more(F2) + s.tt_sgd.more(2 * (size_t)G * F) +
+            s.tt_bound.more(G) >
+        twotime_exact_bytes(s, lay))
+      return false;
+  }
   int64_t n = 0;
   int32_t flags = 0;
   std::vector<unsigned long long> bound(G);
@@ -722,9 +747,6 @@ bool gram_counts(Series &s, const TwoTimeReq &req, const TwoTimeLayout &lay, int
   }
   const size_t smem = col * (size_t)F * W;
   allow_smem(k_tt_gram_counts);
-  // q bins at a time: their double matrices within 2 GB
-  const size_t F2 = (size_t)F * F;
-  const int32_t step = (int32_t)std::max<size_t>(1, std::min<size_t>(Q, (2ull << 30) / (8 * F2)));
   s.tt_Cq.reserve(F2 * step, st);
   for (int32_t q = 0; q < Q; q += step) {
     const int32_t nq = std::min(step, Q - q);
@@ -852,7 +874,7 @@ void run_twotime(Series &s, const TwoTimeReq &req, int mode, bool force_i64) {
       std::sort(order.begin() + q_ptr[q], order.begin() + q_ptr[q + 1],
                 [&](int32_t a, int32_t b) { return row_pix[a] < row_pix[b]; });
   }
-  const bool events = R > 0 && F > 0 && tt_use_events(s);
+  const bool events = R > 0 && F > 0 && tt_use_events(s, R, G, Q);
   if (req.frame_threading || !events) up(s.tt_order, order);
   if (R > 0 && F > 0) {
     if (events)

@@ -378,6 +378,16 @@ void twotime_exact_diag(Series &s, int32_t window, int32_t Q, int32_t q, int32_t
   XG_CHECK_LAUNCH();
 }
 
+size_t twotime_exact_bytes(const Series &s, const TwoTimeLayout &lay) {
+  const size_t F2 = (size_t)s.F * s.F, G = lay.grp_ptr.size() - 1;
+  const size_t Fp = ((size_t)s.F + TC_BN - 1) / TC_BN * TC_BN;
+  size_t Kp = TC_BK;
+  for (size_t g = 0; g < G; g++)
+    Kp = std::max(Kp, ((size_t)(lay.grp_ptr[g + 1] - lay.grp_ptr[g]) + TC_BK - 1) / TC_BK * TC_BK);
+  return s.tt_XT.more(Fp * Kp) + s.tt_Gf.more(Fp * Fp) + s.tt_Cacc.more(F2 + 1) +
+         s.tt_Cq.more(F2 + 1) + s.tt_sgd.more(G * ((size_t)s.F + 1)) + s.tt_S.more(s.F + 1);
+}
+
 // Groups and rows as run_twotime builds them; `force_i64` routes every group
 // to the CUDA-core Gram (the check of the tensor-core one).
 void run_twotime_exact(Series &s, const TwoTimeReq &req, const TwoTimeLayout &lay,

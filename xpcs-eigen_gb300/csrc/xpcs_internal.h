@@ -80,6 +80,8 @@ struct DBuf {
     p = q;
     cap = n;
   }
+  // bytes that reserve(n) would allocate
+  size_t more(size_t n) const { return n > cap ? sizeof(T) * n : 0; }
   // grow keeping the first `keep` elements
   void grow(size_t n, size_t keep, cudaStream_t st) {
     if (n <= cap) return;
@@ -521,6 +523,8 @@ void prepare_framesum_scale(Series &s);  // k_side.cu
 void run_twotime(Series &s, const TwoTimeReq &req, int mode, bool force_i64);
 void run_twotime_exact(Series &s, const TwoTimeReq &req, const TwoTimeLayout &lay,
                        bool force_i64);  // k_twotime_tc.cu
+// Device memory that it would still have to allocate.
+size_t twotime_exact_bytes(const Series &s, const TwoTimeLayout &lay);
 // g2full and g2partials of the q bins [q, q + nq) of Q from their double
 // matrices in tt_Cq (k_twotime_tc.cu).
 void twotime_exact_diag(Series &s, int32_t window, int32_t Q, int32_t q, int32_t nq);
