@@ -174,3 +174,34 @@ def test_float_rows_within_what_a_limit_left_them_before():
                 xg.set_device_memory_limit(0, 0)
     finally:
         xg.set_device_memory_limit(0, 0)
+
+
+def test_blocks_joined_within_what_a_limit_left_them_before():
+    """The places of the blocks' rows (4 B per pixel and block) are no condition
+    of the join: 260 blocks of one frame under a limit that leaves room for the
+    event lists and the results."""
+    W, H, F = 300, 290, 260
+    rng = np.random.default_rng(8)
+    n = rng.poisson(0.01, (F, W * H))
+    hit = n > 0
+    nnz, idx, val = hit.sum(1).astype(np.uint32), np.nonzero(hit)[1], n[hit]
+    dq = np.ones((H, W), np.int32)
+    try:
+        out = []
+        for block in (0, 1):
+            with xg.Series(W, H, F, 4, dq, dq) as s:
+                s.set_block_frames(block)
+                s.ingest_sparse(nnz, idx.astype(np.int32), val.astype(np.int16))
+                s.synchronize()
+                used = xg.device_memory(0)[0]
+                if block:
+                    xg.set_device_memory_limit(0, used + s.P * (12 * s.D + 64) + 54 * idx.size
+                                               + (4 << 20))
+                for _ in range(2):
+                    s.multitau(xg.MODE_REFERENCE)
+                    out.append(s.g2ipif())
+        for r in out[1:]:
+            for g, w in zip(r, out[0]):
+                assert same_bits(g, w)
+    finally:
+        xg.set_device_memory_limit(0, 0)

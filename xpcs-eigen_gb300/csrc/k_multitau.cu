@@ -2070,16 +2070,11 @@ bool reserve_float_thread(Series &s, cudaStream_t st, size_t slots, size_t list,
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   XG_CUDA(cudaStreamIsCapturing(st, &cap));
   if (cap != cudaStreamCaptureStatusNone) return false;
-  try {
-    s.ft_slots.reserve(slots, st);
-    s.ft_list.reserve(list, st);
-    s.ft_out.reserve(out, st);
+  if (s.ft_slots.try_reserve(slots, st) && s.ft_list.try_reserve(list, st) &&
+      s.ft_out.try_reserve(out, st))
     return true;
-  } catch (const Error &e) {
-    if (e.code != XPCS_ERR_OUT_OF_MEMORY) throw;
-    release_float_thread(s, st);
-    return false;
-  }
+  release_float_thread(s, st);
+  return false;
 }
 
 // The rows of the thread-per-pixel float kernel moved to the list of the

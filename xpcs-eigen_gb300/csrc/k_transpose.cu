@@ -1159,7 +1159,7 @@ k_merge_block(int32_t P, int32_t avg, const int64_t *__restrict__ row_ptr,
 }
 
 // Merged row lengths of every block summed per pixel; pos: the events that a
-// pixel has before each block.
+// pixel has before each block (null: not wanted).
 __global__ void k_block_totals(int32_t P, int32_t nblk, const int32_t *__restrict__ blk_len,
                                int32_t *__restrict__ pos, int32_t *__restrict__ tot) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1167,7 +1167,7 @@ __global__ void k_block_totals(int32_t P, int32_t nblk, const int32_t *__restric
   int32_t t = 0;
 #pragma unroll 4
   for (int32_t k = 0; k < nblk; k++) {
-    pos[(size_t)k * P + p] = t;
+    if (pos) pos[(size_t)k * P + p] = t;
     t += blk_len[(size_t)k * P + p];
   }
   tot[p] = t;
@@ -1181,7 +1181,8 @@ __global__ void k_block_totals(int32_t P, int32_t nblk, const int32_t *__restric
 // row.  Warps of one pixel group follow each other, so that the short runs
 // that they write meet in L2.  512 x 512 pixels in 10 blocks, 12.3 M events
 // (bandwidth: 30 us): 228 us with one thread a pixel, 134 with one warp for all
-// blocks of its pixels, 55 so.
+// blocks of its pixels, 55 so.  Without pos (4 bytes a pixel and block that a
+// memory limit refuses) each warp adds up the lengths before its block.
 __global__ void __launch_bounds__(256)
 k_gather_blocks(int32_t P, int32_t nblk, const int64_t *__restrict__ blk_base,
                 const int32_t *__restrict__ blk_off, const int32_t *__restrict__ blk_len,
@@ -1199,7 +1200,10 @@ k_gather_blocks(int32_t P, int32_t nblk, const int64_t *__restrict__ blk_base,
   const int64_t d0 = row_ptr[p0];
   // this lane's segment: its place from the first row's start on, its length
   // and its start in the block
-  const int64_t d = p < P ? row_ptr[p] - d0 + pos[q] : 0;
+  int32_t before = 0;
+  if (p < P && pos) before = pos[q];
+  for (int j = 0; p < P && !pos && j < k; j++) before += blk_len[(size_t)j * P + p];
+  const int64_t d = p < P ? row_ptr[p] - d0 + before : 0;
   const int32_t n = p < P ? blk_len[q] : 0, off = p < P ? blk_off[q] : INT32_MAX;
   const int64_t base = blk_base[k];
   const int32_t lo = __shfl_sync(FULL, off, 0);
@@ -1239,16 +1243,17 @@ void gather_blocks(Series &s) {
   const int32_t P = s.P, nblk = (int32_t)s.blk_base.size();
   s.blk_tot.reserve(P, st);
   if (nblk > 0) {
-    s.blk_pos.reserve((size_t)nblk * P, st);
-    k_block_totals<<<(P + 255) / 256, 256, 0, st>>>(P, nblk, s.blk_len.p, s.blk_pos.p,
-                                                    s.blk_tot.p);
+    const bool pos = s.blk_pos.try_reserve((size_t)nblk * P, st);
+    k_block_totals<<<(P + 255) / 256, 256, 0, st>>>(P, nblk, s.blk_len.p,
+                                                    pos ? s.blk_pos.p : nullptr, s.blk_tot.p);
     XG_CHECK_LAUNCH();
     exclusive_scan_i32_i64(s.blk_tot.p, s.row_ptr.p, P, s.scan_tmp.p, st);
     const int64_t warps = (int64_t)((P + 31) / 32) * nblk;  // below 2^31 blocks of 8
     k_gather_blocks<<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(
-        P, nblk, s.d_blk_base.p, s.blk_off.p, s.blk_len.p, s.blk_pos.p, s.blk_fr.p, s.blk_val.p,
-        s.row_ptr.p, s.ev_frame.p, s.ev_val.p);
+        P, nblk, s.d_blk_base.p, s.blk_off.p, s.blk_len.p, pos ? s.blk_pos.p : nullptr, s.blk_fr.p,
+        s.blk_val.p, s.row_ptr.p, s.ev_frame.p, s.ev_val.p);
     XG_CHECK_LAUNCH();
+    if (dev_limited()) s.blk_pos.release(st);  // the call's alone
   } else {
     XG_CUDA(cudaMemsetAsync(s.row_ptr.p, 0, sizeof(int64_t) * ((size_t)P + 1), st));
   }

@@ -82,6 +82,16 @@ struct DBuf {
   }
   // bytes that reserve(n) would allocate
   size_t more(size_t n) const { return n > cap ? sizeof(T) * n : 0; }
+  // false where the memory is not to be had
+  bool try_reserve(size_t n, cudaStream_t st) {
+    try {
+      reserve(n, st);
+      return true;
+    } catch (const Error &e) {
+      if (e.code != XPCS_ERR_OUT_OF_MEMORY) throw;
+      return false;
+    }
+  }
   // grow keeping the first `keep` elements
   void grow(size_t n, size_t keep, cudaStream_t st) {
     if (n <= cap) return;
