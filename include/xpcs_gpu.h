@@ -419,7 +419,9 @@ void xpcs_batch_destroy(xpcs_batch *b);
  * An acquisition is submitted with its series description and expected event
  * count; it is admitted -- its series created on the GPU -- as soon as its
  * estimated device footprint (raw events, resident rows and work buffers,
- * ~54 B per event, plus 12 B per pixel and delay for G2/IP/IF) fits
+ * ~54 B per event, 12 B per pixel and delay for G2/IP/IF, 12 B per pixel and
+ * block of 512 frames, and the float rows' scratch of flatfield and averaged
+ * acquisitions) fits
  * `memory_budget`, in submission order (an acquisition larger than the budget
  * is admitted when nothing else is active).  Frames pushed before admission
  * wait in host memory.  push copies frames into the acquisition's resident

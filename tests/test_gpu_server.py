@@ -186,3 +186,30 @@ def test_close_after_finish_without_result():
         srv2.push(i, *fr)
         srv2.finish(i)
         check(srv2.result(i, g2ipif=True), alone(acq, dq, sq, fr))
+
+
+@pytest.mark.parametrize("flat,stride,average,F", [(True, 1, 1, 300), (False, 1, 2, 300),
+                                                  (False, 1, 1, 2600)])
+def test_an_acquisitions_footprint_covers_what_it_takes(flat, stride, average, F):
+    """The device memory that a streamed acquisition holds at its end, the float
+    rows' scratch (flatfield, averaging) and the blocks' tables included, is
+    within what the server counts for it when it admits it."""
+    W, H = 760, 700
+    rng = np.random.default_rng(F)
+    frames = [np.flatnonzero(rng.random(W * H) < 0.002).astype(np.int32)
+              for _ in range(F * stride * average)]
+    events = sum(f.size for f in frames)
+    dq = np.ones((H, W), np.int32)
+    before = xg.device_memory(0)[0]
+    with xg.Server(memory_budget=64 << 30) as srv:
+        i = srv.submit(W, H, F, 8, dq, dq, expected_events=events,
+                       flatfield=rng.uniform(0.9, 1.1, W * H) if flat else None, stride=stride,
+                       average=average)
+        counted = srv.stats()["used_bytes"]
+        for f in frames:
+            srv.push(i, np.array([f.size], np.uint32), f, np.ones(f.size, np.int16))
+        srv.finish(i)
+        srv.result(i)
+        held = xg.device_memory(0)[0] - before
+        assert held <= counted, (held, counted)
+        srv.release(i)

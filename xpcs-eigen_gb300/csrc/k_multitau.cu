@@ -2054,6 +2054,20 @@ void reset_counters(Series &s, cudaStream_t st) {
   XG_CUDA(cudaMemsetAsync((char *)s.stats.p + first, 0, end - first, st));
 }
 
+// Blocks of k_mt_fthread, the slots within FT_SLOT_BYTES, and its scratch.
+struct FtScratch {
+  int blocks;
+  size_t slots, list, out;  // bytes, pixels, floats
+};
+FtScratch ft_scratch(const Series &s, int32_t cap, int sms, int per_sm) {
+  const size_t block_bytes = (size_t)FT_WARPS * 32 * cap * sizeof(uint2);
+  per_sm = std::min(per_sm, (int)(FT_SLOT_BYTES / (block_bytes * (size_t)sms)));
+  const int windows = (s.P + FT_WIN_PIX - 1) / FT_WIN_PIX;
+  const int blocks = std::min(sms * std::max(1, per_sm), windows * (FT_WIN_PIX / 32 / FT_WARPS));
+  return {blocks, blocks * block_bytes, (size_t)windows * FT_WIN_PIX,
+          (size_t)s.P * 3 * ((s.D + 3) & ~3)};
+}
+
 // Given back: a captured batch graph that holds the addresses is stale with it.
 void release_float_thread(Series &s, cudaStream_t st) {
   if (s.ft_slots.p || s.ft_list.p || s.ft_out.p) s.generation++;
@@ -2065,13 +2079,13 @@ void release_float_thread(Series &s, cudaStream_t st) {
 // The scratch of k_mt_fthread, up to 3 GB of slots and as much as G2, IP and IF
 // together; false where it is not to be had (the rows then go to the warp-per-row
 // kernel, which needs none).  A captured graph allocates nothing.
-bool reserve_float_thread(Series &s, cudaStream_t st, size_t slots, size_t list, size_t out) {
-  if (slots <= s.ft_slots.cap && list <= s.ft_list.cap && out <= s.ft_out.cap) return true;
+bool reserve_float_thread(Series &s, cudaStream_t st, const FtScratch &f) {
+  if (f.slots <= s.ft_slots.cap && f.list <= s.ft_list.cap && f.out <= s.ft_out.cap) return true;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   XG_CUDA(cudaStreamIsCapturing(st, &cap));
   if (cap != cudaStreamCaptureStatusNone) return false;
-  if (s.ft_slots.try_reserve(slots, st) && s.ft_list.try_reserve(list, st) &&
-      s.ft_out.try_reserve(out, st))
+  if (s.ft_slots.try_reserve(f.slots, st) && s.ft_list.try_reserve(f.list, st) &&
+      s.ft_out.try_reserve(f.out, st))
     return true;
   release_float_thread(s, st);
   return false;
@@ -2116,17 +2130,13 @@ void launch_float_rows(Series &s, const McPlan &hp, cudaStream_t st, int sms) {
     const auto kernel = s.desc.delays_per_level <= 4 ? k_mt_fthread<8, 4> : k_mt_fthread<16, 8>;
     int per_sm = 0;
     XG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, FT_WARPS * 32, 0));
-    // the slots of the grid within FT_SLOT_BYTES
-    const size_t block_bytes = (size_t)FT_WARPS * 32 * s.float_cap * sizeof(uint2);
-    per_sm = std::min(per_sm, (int)(FT_SLOT_BYTES / (block_bytes * (size_t)sms)));
-    const int windows = (P + FT_WIN_PIX - 1) / FT_WIN_PIX;
-    const int blocks = std::min(sms * std::max(1, per_sm), windows * (FT_WIN_PIX / 32 / FT_WARPS));
-    thread_rows = reserve_float_thread(s, st, blocks * block_bytes,
-                                       (size_t)windows * FT_WIN_PIX, (size_t)P * 3 * Dp);
+    const FtScratch f = ft_scratch(s, s.float_cap, sms, per_sm);
+    thread_rows = reserve_float_thread(s, st, f);
     if (thread_rows) {
-      k_ft_sort<<<windows, 256, 0, st>>>(P, s.row_len.p, s.pclass.p, s.ft_list.p);
+      k_ft_sort<<<(unsigned)(f.list / FT_WIN_PIX), 256, 0, st>>>(P, s.row_len.p, s.pclass.p,
+                                                                s.ft_list.p);
       XG_CHECK_LAUNCH();
-      kernel<<<blocks, FT_WARPS * 32, 0, st>>>(
+      kernel<<<f.blocks, FT_WARPS * 32, 0, st>>>(
           s.plan.p, s.float_cap, (uint2 *)s.ft_slots.p, s.ft_list.p, s.row_ptr.p, s.row_len.p,
           s.ev_frame.p, s.ev_val.p, fscale, s.stats.p, Dp, s.ft_out.p);
     } else {
@@ -2214,6 +2224,14 @@ int32_t mt_float_cap(const Series &s, double mean) {
   static_assert(FT_MAXC == FT_MAXD, "a level's largest delay is at most 2 dpl bins");
   const double factor = std::min(s.desc.dense ? 6.0 : 3.0, FT_PIX_FACTOR * s.P);
   return factor < 1.25 ? 0 : (int32_t)std::min<double>(s.F, factor * mean + 64.0);
+}
+
+size_t mt_float_bytes(const Series &s, int32_t float_cap, int sms) {
+  if (float_cap <= 0) return 0;
+  // as many blocks on an SM as their shared memory lets there be
+  const FtScratch f =
+      ft_scratch(s, float_cap, sms, (int)(SMEM_MAX / (sizeof(float) * FT_WARPS * FT_WORDS)));
+  return f.slots + sizeof(int32_t) * f.list + sizeof(float) * f.out;
 }
 
 std::vector<uint8_t> prepare_multitau(Series &s, int mode) {

@@ -122,13 +122,25 @@ constexpr int32_t SERVER_BLOCK_FRAMES = 512;
 
 // Device footprint of an acquisition: raw events, the resident block rows and
 // the transpose/list buffers (~54 B per event), per-pixel tables and G2/IP/IF
-// (12 B per delay), and every block's row offsets and lengths (8 B per pixel).
-uint64_t estimate_footprint(const xpcs_series_desc &d, int64_t events) {
+// (12 B per delay), every block's row offsets, lengths and places (12 B per
+// pixel), and with flatfield or averaging the float rows' scratch.
+uint64_t estimate_footprint(const xpcs_series_desc &d, int64_t events, int sms) {
   const uint64_t P = (uint64_t)d.width * d.height;
   const DelaySchedule ds = delay_schedule(d.frames, d.delays_per_level);
   const uint64_t blocks = (uint64_t)std::max(d.frames, 0) / SERVER_BLOCK_FRAMES + 1;
-  return P * (12ull * ds.level.size() + 64 + 8 * blocks) +
-         (uint64_t)std::max<int64_t>(events, 0) * 54 + (64ull << 20);
+  events = std::max<int64_t>(events, 0);
+  Series s;
+  s.desc = d;
+  s.P = (int32_t)P;
+  s.F = d.frames;
+  s.D = (int32_t)ds.level.size();
+  s.has_flat = d.flatfield != nullptr;
+  int64_t valid = 0;
+  for (uint64_t p = 0; p < P; p++) valid += d.dqmap[p] > 0 && d.sqmap[p] > 0;
+  const double mean =
+      (double)events / ((double)std::max<int64_t>(valid, 1) * std::max(d.stride_frames, 1));
+  return P * (12ull * ds.level.size() + 64 + 12 * blocks) + (uint64_t)events * 54 +
+         mt_float_bytes(s, mt_float_cap(s, mean), sms) + (64ull << 20);
 }
 
 void check_rc(int rc) {
@@ -283,7 +295,9 @@ int64_t server_submit(void *h, const xpcs_series_desc &desc, int64_t expected_ev
   sl->dq.assign(desc.dqmap, desc.dqmap + P);
   sl->sq.assign(desc.sqmap, desc.sqmap + P);
   if (desc.flatfield) sl->flat.assign(desc.flatfield, desc.flatfield + P);
-  sl->footprint = estimate_footprint(desc, expected_events);
+  int sms = 0;
+  XG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, srv.device));
+  sl->footprint = estimate_footprint(desc, expected_events, sms);
   std::vector<std::shared_ptr<Slot>> go;
   {
     std::lock_guard<std::mutex> g(srv.mu);

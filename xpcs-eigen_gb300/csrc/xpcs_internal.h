@@ -493,6 +493,8 @@ bool mt_float_rows_warp(const McPlan &hp);                    // k_multitau.cu
 // Longest row of the thread-per-pixel float kernel for a series whose rows
 // hold `mean` events on average, 0 for no row at all.
 int32_t mt_float_cap(const Series &s, double mean);           // k_multitau.cu
+// The most device memory that kernel's scratch takes (k_multitau.cu).
+size_t mt_float_bytes(const Series &s, int32_t float_cap, int sms);
 // The rows of xpcs_multitau2_noalloc (k_multitau.cu): the caller's arrays and
 // the fixed scratch.  No allocation, no exception.
 enum : int32_t { NA_INT = 0, NA_FLOAT = 8, NA_IRREGULAR = 16 };  // kinds of rows in status[1]
