@@ -74,3 +74,30 @@ def test_exact_twotime_from_event_lists_equals_the_int64_gram(W, H, F, density, 
         assert same_bits_nan(e["c2t"][q], i["c2t"][q])
     for k in ("sg", "g2full", "g2partials"):
         assert same_bits_nan(e[k], i[k]), k
+
+
+@pytest.mark.parametrize("average", [False, True])
+def test_exact_twotime_of_more_smoothing_groups_than_a_grid_has_rows(average):
+    """68,644 static bins of one pixel each: with counts of 1, 2 and 4 every
+    pixel's smoothed pair of events is 1 to the bit (or, averaged over the
+    frames, its counts over their mean), and C is their number over the pixels."""
+    W = H = 262
+    P, F = W * H, 6
+    rng = np.random.default_rng(3)
+    sq = np.arange(1, P + 1, dtype=np.int32).reshape(H, W)
+    v = np.where(rng.random((F, P)) < 0.04, 2 ** rng.integers(0, 3, (F, P)), 0)
+    hit = v > 0
+    nnz, idx = hit.sum(1).astype(np.uint32), np.nonzero(hit)[1].astype(np.int32)
+    with xg.Series(W, H, F, 4, np.ones((H, W), np.int32), sq) as s:
+        s.ingest_sparse(nnz, idx, v[hit].astype(np.int16))
+        r = s.twotime([1], static_map=True, average=average, mode=xg.MODE_EXACT)
+    want = np.zeros((F, F))
+    sg = v.mean(0) if average else None
+    for a in range(F):
+        for b in range(a, F):
+            both = hit[a] & hit[b]
+            w = (v[a] * v[b])[both] / sg[both] ** 2 if average else np.ones(np.count_nonzero(both))
+            want[a, b] = w.sum() / P
+    assert np.allclose(r["c2t"][1], want, rtol=2.0 ** -23, atol=0)
+    assert np.array_equal(r["sg"], v.mean(0).astype(np.float32)[:, None] if average
+                          else v.T.astype(np.float32))

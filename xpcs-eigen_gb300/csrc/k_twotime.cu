@@ -420,7 +420,8 @@ __global__ void k_tt_sg_counts(int32_t F, const int32_t *__restrict__ grp_ptr,
                                const float *__restrict__ ev_val, double *__restrict__ sgd,
                                double *__restrict__ isg, float *__restrict__ sg) {
   const int lane = threadIdx.x & 31;
-  const int f = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5), g = blockIdx.y;
+  const int nb = (F + 7) / 8;  // blocks of 8 frames; any number of groups in one dimension
+  const int f = (int)(blockIdx.x % nb) * 8 + (threadIdx.x >> 5), g = (int)(blockIdx.x / nb);
   if (f >= F) return;
   const int r0 = grp_ptr[g], r1 = grp_ptr[g + 1];
   const int64_t c = (int64_t)grp_q[g] * F + f;
@@ -698,15 +699,17 @@ bool gram_counts(Series &s, const TwoTimeReq &req, const TwoTimeLayout &lay, int
   cudaStream_t st = s.stream;
   const int32_t F = s.F;
   const double most = std::min(0.06, 65.0 / F);
-  if (F > 65535 || (double)s.raw_events > most * (double)s.qmap.pix.size() * s.R_in * F)
+  if (F > 65535 || (int64_t)(F + 7) / 8 * G > INT32_MAX ||
+      (double)s.raw_events > most * (double)s.qmap.pix.size() * s.R_in * F)
     return false;
   const bool multi = G > Q;
   const size_t col = sizeof(int32_t) + (multi ? sizeof(double) : 0);
   const int W = tt_columns(F, col);
   if (W == 0) return false;
   const size_t F2 = (size_t)F * F;
-  // q bins at a time: their double matrices within 2 GB
-  int32_t step = (int32_t)std::max<size_t>(1, std::min<size_t>(Q, (2ull << 30) / (8 * F2)));
+  // q bins at a time: their double matrices within 2 GB, and a grid's rows
+  int32_t step = (int32_t)std::max<size_t>(
+      1, std::min<size_t>(std::min(Q, 65535), (2ull << 30) / (8 * F2)));
   if (dev_limited()) {  // as in tt_use_events
     step = 1;
     if (lists_bytes(s, R, G, Q) + s.tt_Cq.more(F2) + s.tt_sgd.more(2 * (size_t)G * F) +
@@ -736,10 +739,9 @@ bool gram_counts(Series &s, const TwoTimeReq &req, const TwoTimeLayout &lay, int
   const auto ab = lists_build(s, l, R, Q, nullptr);
   s.tt_sgd.reserve(2 * (size_t)G * F, st);
   double *sgd = s.tt_sgd.p, *isg = sgd + (size_t)G * F;
-  k_tt_sg_counts<<<dim3(tt_warps(F), G), 256, 0, st>>>(F, s.tt_grp_ptr.p, l.grp_q, s.tt_cols.p,
-                                                       ab.first, ab.second, s.tt_row_pix.p,
-                                                       s.row_ptr.p, s.ev_val.p, sgd, isg,
-                                                       s.tt_sg.p);
+  k_tt_sg_counts<<<(unsigned)((F + 7) / 8) * (unsigned)G, 256, 0, st>>>(
+      F, s.tt_grp_ptr.p, l.grp_q, s.tt_cols.p, ab.first, ab.second, s.tt_row_pix.p, s.row_ptr.p,
+      s.ev_val.p, sgd, isg, s.tt_sg.p);
   XG_CHECK_LAUNCH();
   if (req.average) {
     k_tt_sg_counts_avg<<<(G + 31) / 32, 32, 0, st>>>(G, F, sgd, isg, s.tt_sga.p);
