@@ -464,17 +464,47 @@ k_downsweep(RawCfg rc, PassCfg pc, const uint32_t *__restrict__ offsets,
 // without events) together.  Bound by HBM: 4 B per event read.  One binary
 // search per pixel took 64 us at 49.6 M events in 1 Mi pixels and 12 at 2.5 M
 // in 512^2, this pass 64 and 9.
+// One warp fills 7,600 rows of a gap in a microsecond, too few where most of a
+// large detector is one gap (events in one corner, or none kept): the filter of
+// 20,000 events on 4,096 x 4,096 pixels took 2.84 ms so, 0.65 with the events
+// all over the detector, and as long as that now.  So the grid's first gap_blocks take the rows in
+// aligned spans of RP_SPAN, a warp each, and fill those that lie in one gap
+// (two binary searches tell); the warp that finds the gap leaves them out.
 constexpr int RP_U = 4;
+constexpr int RP_SPAN = 4096;
+__device__ __forceinline__ int64_t first_key(const uint32_t *__restrict__ keys, int64_t n,
+                                             int32_t p) {  // the first that is >= p
+  int64_t first = 0;
+  while (n > 0) {
+    const int64_t h = n >> 1;
+    if ((int32_t)keys[first + h] < p) {
+      first += h + 1;
+      n -= h + 1;
+    } else {
+      n = h;
+    }
+  }
+  return first;
+}
 __global__ void __launch_bounds__(256)
 k_row_ptr(const uint32_t *__restrict__ keys, int64_t n, const DevStats *__restrict__ stats,
-          int32_t P, int64_t *__restrict__ row_ptr) {
+          int32_t P, int32_t gap_blocks, int64_t *__restrict__ row_ptr) {
   overlap_after();
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int64_t nv = n - (int64_t)stats->dropped;
+  if ((int)blockIdx.x < gap_blocks) {
+    const int64_t p0 = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * RP_SPAN;
+    if (p0 + RP_SPAN - 1 > P) return;  // rows 0 .. P
+    const int64_t at = first_key(keys, nv, (int32_t)p0 + (lane & 1) * (RP_SPAN - 1));
+    const int64_t pos = __shfl_sync(FULL, at, 0);
+    if (pos != __shfl_sync(FULL, at, 1)) return;
+    for (int k = lane; k < RP_SPAN; k += 32) row_ptr[p0 + k] = pos;
+    return;
+  }
   // the warp's first key; position nv is the end of the last rows
   const int64_t w0 =
-      (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (RP_U * 128);
+      (((int64_t)(blockIdx.x - gap_blocks) * blockDim.x + threadIdx.x) >> 5) * (RP_U * 128);
   if (w0 > nv) return;
   int32_t key[RP_U][5];  // keys i0 - 1 .. i0 + 3 of a group: -1 before the first, P past the end
 #pragma unroll
@@ -516,7 +546,14 @@ k_row_ptr(const uint32_t *__restrict__ keys, int64_t n, const DevStats *__restri
         const int32_t a = __shfl_sync(FULL, key[u][k - 1], l);
         const int32_t e = __shfl_sync(FULL, key[u][k], l);
         const int64_t pos = __shfl_sync(FULL, i0 - 1 + k, l);
-        for (int32_t p = a + 1 + lane; p <= e; p += 32) row_ptr[p] = pos;
+        // whole spans [s0, s1) of the gap's rows a + 1 .. e are the gap blocks'
+        int32_t s0 = e + 1, s1 = e + 1;
+        if (gap_blocks) {
+          s0 = min((a + RP_SPAN) / RP_SPAN * RP_SPAN, e + 1);
+          s1 = max((e + 1) / RP_SPAN * RP_SPAN, s0);
+        }
+        for (int32_t p = a + 1 + lane; p < s0; p += 32) row_ptr[p] = pos;
+        for (int32_t p = s1 + lane; p <= e; p += 32) row_ptr[p] = pos;
       }
     }
   }
@@ -1047,8 +1084,10 @@ void transpose_range(Series &s, int32_t r0, int32_t r1, int32_t *ev_fr, float *e
     radix_pass(s, ipt, dg.bits, packed, first, last, rc, pc);
   }
   const uint32_t *keys = (passes % 2 == 0) ? s.keyB.p : s.keyA.p;  // written by the last pass
-  launch_overlapped(k_row_ptr, (unsigned)((n + 1 + RP_U * 1024 - 1) / (RP_U * 1024)), 256, 0, st,
-                    keys, n, s.stats.p, P, row_ptr);
+  // smaller detectors' gaps take a warp at most 17 us, no longer than the searches
+  const int gaps = P >= 1 << 17 ? (int)(((int64_t)P + 1 + 8 * RP_SPAN - 1) / (8 * RP_SPAN)) : 0;
+  launch_overlapped(k_row_ptr, (unsigned)(gaps + (n + 1 + RP_U * 1024 - 1) / (RP_U * 1024)), 256, 0,
+                    st, keys, n, s.stats.p, P, gaps, row_ptr);
 }
 
 void reserve_lists(Series &s) {
