@@ -137,3 +137,34 @@ def test_twotime_frame_counts_around_the_tiles(frames, static_map):
     assert same_bits_nan(r["g2full"], o["g2full"])
     assert same_bits_nan(r["g2partials"], o["g2partials"])
     assert same_bits_nan(t["g2full"], c["g2full"])
+
+
+@pytest.mark.parametrize("side,frames,groups,density", [
+    (96, 700, 1, 0.1), (96, 700, 4, 0.12), (64, 1100, 2, 0.08), (131, 257, 1, 0.3), (40, 130, 8, 0.9),
+])
+@pytest.mark.parametrize("static_map,average", [(True, False), (False, True)])
+def test_tensor_core_gram_of_many_k_tiles_and_column_tiles(side, frames, groups, density,
+                                                           static_map, average):
+    """Counts too dense for the event lists, so that the tensor-core Gram runs
+    (it reports its time): groups of up to 268 k tiles over the four-stage ring,
+    last tiles partly filled, up to five column tiles; equal to the int64
+    CUDA-core Gram in every output."""
+    rng = np.random.default_rng(side + frames)
+    P = side * side
+    sq = (np.arange(P) * groups // P + 1).astype(np.int32).reshape(side, side)
+    dq = (sq + 1) // 2
+    hit = rng.random((frames, P)) < density
+    nnz, idx = hit.sum(1).astype(np.uint32), np.nonzero(hit)[1].astype(np.int32)
+    val = rng.integers(1, 10, idx.size).astype(np.int16)
+    out = []
+    for mode in (xg.MODE_EXACT, xg.TWOTIME_EXACT_CUDA_CORES):
+        with xg.Series(side, side, frames, 4, dq, sq) as s:
+            s.ingest_sparse(nnz, idx, val)
+            out.append(s.twotime(range(1, int(dq.max()) + 1), static_map=static_map,
+                                 average=average, window=5, mode=mode))
+    t, c = out
+    assert t["gram_ms"] > 0 and c["gram_ms"] == 0
+    for q in t["c2t"]:
+        assert np.count_nonzero(t["c2t"][q]) > 0 and same_bits_nan(t["c2t"][q], c["c2t"][q]), q
+    for k in ("sg", "g2full", "g2partials"):
+        assert same_bits_nan(t[k], c[k]), k
