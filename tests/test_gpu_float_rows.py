@@ -59,3 +59,30 @@ def test_float_rows_vs_oracle(name, mode):
     want = oracle.multitau2(rows, F, dpl, mode)
     for g, w, which in zip(got, want, ("G2", "IP", "IF")):
         assert same_bits(g, w), (which, int(np.count_nonzero(g != w)))
+
+
+@pytest.mark.parametrize("mode", [xg.MODE_REFERENCE, xg.MODE_EXACT])
+@pytest.mark.parametrize("flat,dpl,average", [(False, 8, 1), (True, 4, 1), (False, 8, 2)])
+def test_framesum_normalised_float_rows_vs_oracle(flat, dpl, average, mode):
+    """normalize_by_framesum through the thread-per-pixel float kernel, with and
+    without a flatfield and averaging, and rows past its capacity."""
+    W, H, F = 310, 300, 150
+    rng = np.random.default_rng(dpl + average)
+    P, R = W * H, F * average
+    hit = rng.random((R, P)) < rng.uniform(0.05, 0.15, (R, 1)) / average
+    hit[:, :40] |= rng.random((R, 40)) < np.linspace(0.1, 1.0, 40)
+    nnz, idx = hit.sum(1).astype(np.uint32), np.nonzero(hit)[1].astype(np.int32)
+    val = rng.integers(1, 6, idx.size).astype(np.int16)
+    gain = rng.uniform(0.8, 1.2, P) if flat else None
+    dq = np.ones((H, W), np.int32)
+    with xg.Series(W, H, F, dpl, dq, dq, flatfield=gain, average=average,
+                   normalize_by_framesum=True) as s:
+        s.ingest_sparse(nnz, idx, val)
+        s.multitau(mode)
+        got = s.g2ipif()
+        assert s.info().float_path_pixels == P
+    rows, side = oracle.sparse_filter(oracle.QMap(dq, dq), nnz, idx, val, F, average=average,
+                                      flat=gain)
+    want = oracle.multitau2(oracle.framesum_normalize(rows, side["frames_sum"], F), F, dpl, mode)
+    for g, w, which in zip(got, want, ("G2", "IP", "IF")):
+        assert same_bits(g, w), (which, int(np.count_nonzero(g != w)))
