@@ -308,9 +308,9 @@ __device__ double deviations(int k0, int k1, double mean, const int32_t *__restr
 // thread merging the chunks in turn took 62 us at 18 rings x 88 delays and 40
 // at 9 x 34; 19 and 14 now.
 // A ring whose spread is small beside its shifts' distance from the mean (one
-// pixel, equal ratios, dead pixels first) goes over its pixels again: below a
-// 16th of the terms M2 is the difference of, their rounding would show in it,
-// and could leave it negative.
+// pixel, equal ratios, dead pixels first) goes over its pixels again: where M2 is
+// less than a 16th of sum (x - s)^2, their rounding would show in it, and could
+// leave it negative.
 __global__ void k_norm_finish(int NQ, int D, const int32_t *__restrict__ qep,
                               const int32_t *__restrict__ qrow,
                               const int32_t *__restrict__ e_chunk_ptr,
@@ -349,16 +349,23 @@ __global__ void k_norm_finish(int NQ, int D, const int32_t *__restrict__ qep,
   // sum (x - mean)^2 = sum (x - s)^2 + 2 (s - mean) sum (x - s) + n (s - mean)^2
   const double mean = sx / n;
   const int c0 = e_chunk_ptr[qep[qi]], c1 = e_chunk_ptr[qep[qi + 1]];
-  double M2 = 0.0, terms = 0.0;
+  double about = 0.0, shift = 0.0;  // sum (x - s)^2, and the rest
   for (int c = c0 + lane; c < c1; c += 32) {
     const double *q = part + ((size_t)c * D + t) * NPART;
     const double nc = (double)(ch_k1[c] - ch_k0[c]), d = q[5] - mean;
-    M2 += fma(d, fma(nc, d, 2.0 * q[3]), q[4]);
-    terms += fma(nc * d, d, q[4]);
+    about += q[4];
+    shift = fma(d, fma(nc, d, 2.0 * q[3]), shift);
   }
-  M2 = warp_sum(M2);
-  terms = warp_sum(terms);
-  if (M2 < 0.0625 * terms) {  // (not NaN, and not a ring of zeros)
+  {  // both over the warp, a half-warp each, in as many FP64 additions as one takes
+    const bool up = lane & 16;
+    double v = (up ? shift : about) + __shfl_xor_sync(0xffffffffu, up ? about : shift, 16);
+#pragma unroll
+    for (int w = 8; w > 0; w >>= 1) v += __shfl_xor_sync(0xffffffffu, v, w);
+    about = __shfl_sync(0xffffffffu, v, 0);
+    shift = __shfl_sync(0xffffffffu, v, 16);
+  }
+  double M2 = about + shift;
+  if (M2 < 0.0625 * about) {  // (not NaN, and not a ring of zeros)
     const size_t o = (size_t)t * P;
     M2 = deviations(ch_k0[c0], ch_k1[c1 - 1], mean, pix, G2 + o, IP + o, IF + o);
   }
