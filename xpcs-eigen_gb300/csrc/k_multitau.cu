@@ -537,39 +537,37 @@ __device__ __forceinline__ void mt_thread_warp(const uint8_t *__restrict__ plan_
   // 32 events in flight per lane.  Positions are relative to the warp's first
   // event: when a lane owns a packed row every frame is below 65536, so the
   // 32 rows span fewer than 2^21 events.
-  if (__any_sync(0xffffffffu, n0 > 0)) {
-    const unsigned FULL = 0xffffffffu;
-    const int plast = min(p0 + 32, P);
-    const int64_t e0 = row_ptr[p0];
-    const int nw = (int)(row_ptr[plast] - e0);
-    const int my_b = p < P ? (int)(row_ptr[p] - e0) : nw;
-    const int lo = __reduce_min_sync(FULL, n0 > 0 ? my_b : INT_MAX);
-    const int hi = __reduce_max_sync(FULL, n0 > 0 ? my_b + n0 : 0);
-    for (int base = lo; base < hi; base += 128) {
-      int dst[4], fr[4];
-      float vl[4];
+  const unsigned FULL = 0xffffffffu;
+  const int plast = min(p0 + 32, P);
+  const int64_t e0 = row_ptr[p0];
+  const int nw = (int)(row_ptr[plast] - e0);
+  const int my_b = p < P ? (int)(row_ptr[p] - e0) : nw;
+  const int lo = __reduce_min_sync(FULL, n0 > 0 ? my_b : INT_MAX);
+  const int hi = __reduce_max_sync(FULL, n0 > 0 ? my_b + n0 : 0);
+  for (int base = lo; base < hi; base += 128) {
+    int dst[4], fr[4];
+    float vl[4];
 #pragma unroll
-      for (int u = 0; u < 4; u++) {
-        const int e = base + u * 32 + lane;
-        int owner = 0;  // last lane whose row starts at or before e
+    for (int u = 0; u < 4; u++) {
+      const int e = base + u * 32 + lane;
+      int owner = 0;  // last lane whose row starts at or before e
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          const int cand = owner + o;
-          const int cb = __shfl_sync(FULL, my_b, cand & 31);
-          if (cand < 32 && cb <= e) owner = cand;
-        }
-        const int slot = e - __shfl_sync(FULL, my_b, owner);
-        const int olen = __shfl_sync(FULL, n0, owner);
-        dst[u] = (e < hi && slot < olen) ? slot * 32 + owner : -1;
-        if (dst[u] >= 0) {
-          fr[u] = ev_frame[e0 + e];
-          vl[u] = ev_val[e0 + e];
-        }
+      for (int o = 16; o > 0; o >>= 1) {
+        const int cand = owner + o;
+        const int cb = __shfl_sync(FULL, my_b, cand & 31);
+        if (cand < 32 && cb <= e) owner = cand;
       }
-#pragma unroll
-      for (int u = 0; u < 4; u++)
-        if (dst[u] >= 0) wbase[dst[u]] = pk(fr[u], __float2int_rn(vl[u]));
+      const int slot = e - __shfl_sync(FULL, my_b, owner);
+      const int olen = __shfl_sync(FULL, n0, owner);
+      dst[u] = (e < hi && slot < olen) ? slot * 32 + owner : -1;
+      if (dst[u] >= 0) {
+        fr[u] = ev_frame[e0 + e];
+        vl[u] = ev_val[e0 + e];
+      }
     }
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      if (dst[u] >= 0) wbase[dst[u]] = pk(fr[u], __float2int_rn(vl[u]));
   }
   __syncwarp();
   mt_thread_rows<CAP>(plan_g, p, n0, mine, G2, IP, IF, wbase);

@@ -1019,7 +1019,6 @@ void transpose_range(Series &s, int32_t r0, int32_t r1, int32_t *ev_fr, float *e
   cudaStream_t st = s.stream;
   const int32_t P = s.P;
   const int64_t e0 = s.frame_off[r0], n = s.frame_off[r1] - e0;
-  s.scan_tmp.reserve(scan_workspace_bytes(P), st);
   if (n <= 0) {
     XG_CUDA(cudaMemsetAsync(row_ptr, 0, sizeof(int64_t) * ((size_t)P + 1), st));
     return;

@@ -865,8 +865,9 @@ void run_twotime(Series &s, const TwoTimeReq &req, int mode, bool force_i64) {
     o.ready = true;
     return;
   }
-  // Gram order of every q bin's rows
-  std::vector<int32_t> order(R);
+  const bool events = R > 0 && F > 0 && tt_use_events(s, R, G, Q);
+  // Gram order of every q bin's rows (event lists take the mapping order as it is)
+  std::vector<int32_t> order(req.frame_threading || !events ? R : 0);
   std::iota(order.begin(), order.end(), 0);
   if (req.frame_threading) {
     std::vector<int32_t> row_pix;
@@ -876,8 +877,7 @@ void run_twotime(Series &s, const TwoTimeReq &req, int mode, bool force_i64) {
       std::sort(order.begin() + q_ptr[q], order.begin() + q_ptr[q + 1],
                 [&](int32_t a, int32_t b) { return row_pix[a] < row_pix[b]; });
   }
-  const bool events = R > 0 && F > 0 && tt_use_events(s, R, G, Q);
-  if (req.frame_threading || !events) up(s.tt_order, order);
+  if (!order.empty()) up(s.tt_order, order);
   if (R > 0 && F > 0) {
     if (events)
       gram_events(s, req, lay, R, G, Q);
