@@ -226,7 +226,10 @@ int xpcs_get_normalized(xpcs_series *s, double *g2, double *stderr_, float *g2_f
  * Until xpcs_series_set_tuning or xpcs_autotune sets them, each multi-tau
  * derives the first two from the series: thread_cap the smallest capacity of
  * at least 1.5 mean rows (events per mapped pixel), scratch_extra 8 from
- * 16,384 frames on (before the first multi-tau: 80 and 0). */
+ * 16,384 frames on (before the first multi-tau: 80 and 0).  A series of few
+ * pixels (up to 5,000, and 800 more per event of the mean row, at most 32,000)
+ * gives every row to a warp when it runs alone, until the caller sets a
+ * capacity. */
 typedef struct {
   int32_t thread_cap;
   int32_t scratch_extra;
@@ -238,8 +241,9 @@ int xpcs_series_set_tuning(xpcs_series *s, const xpcs_tuning *t);
 /* Autotuner (no reference counterpart).  Times the filter and multi-tau
  * passes of the ingested frames over the knobs above, one knob at a time
  * (thread_cap, then scratch_extra, then radix_items_per_lane), keeping the
- * fastest value of each, and sets them on the series.  *thread_cap (may be
- * NULL) receives the chosen row capacity; xpcs_series_get_tuning gives all
+ * fastest value of each, and sets them on the series; then, for a series of
+ * few pixels, whether alone it keeps the capacity found or gives every row to
+ * a warp, whichever was faster.  *thread_cap (may be NULL) receives the chosen row capacity; xpcs_series_get_tuning gives all
  * three. */
 int xpcs_autotune(xpcs_series *s, int32_t mode, int32_t *thread_cap);
 
@@ -254,7 +258,9 @@ int xpcs_get_stage_times(xpcs_series *s, xpcs_stage_times *t);
  * library's total on that device past `bytes` fails with
  * XPCS_ERR_OUT_OF_MEMORY (message naming the limit) before CUDA is asked, and
  * the handle stays usable: destroy or reset it, or raise the limit and call
- * again.  0 = no limit (the default).  xpcs_get_device_memory reports the
+ * again.  Work buffers that only save time (the thread-per-pixel float kernel's
+ * scratch, the places of a streamed series' rows, two-time event lists) give
+ * way to slower forms instead.  0 = no limit (the default).  xpcs_get_device_memory reports the
  * bytes the library holds on the device and the limit. */
 int xpcs_set_device_memory_limit(int32_t device, uint64_t bytes);
 /* Streaming multiprocessors and compute capability of a device (no reference
@@ -333,11 +339,13 @@ int xpcs_multitau2_noalloc(const int64_t *row_ptr, const int32_t *frame, const f
  * (twotimeQBinThreading) or ascending pixel index with frame_threading
  * (twotimeFrameThreading).
  * mode EXACT: needs integer counts; the Gram products of the raw counts of
- * every smoothing group are exact integers, computed on the tensor cores
- * (fp16 operands, fp32 accumulation: exact while the counts are <= 2048 and
- * sum over pixels of (max count)^2 < 2^24; other groups use an int64 CUDA-core
- * Gram), and the smoothing and reductions are applied in float64 (rounded to
- * float32 on output).  XPCS_TWOTIME_EXACT_CUDA_CORES computes the same with
+ * every smoothing group are exact integers: for sparse counts (fewer events
+ * per pixel and frame than min(0.06, 65 / frames)) int32 sums over event lists
+ * (exact while sum over a group's pixels of (max count)^2 < 2^31), else on the
+ * tensor cores (fp16 operands, fp32 accumulation: exact while the counts are
+ * <= 2048 and that sum is < 2^24; other groups use an int64 CUDA-core Gram).
+ * The smoothing and reductions are applied in float64 (rounded to float32 on
+ * output); the forms give the same bits.  XPCS_TWOTIME_EXACT_CUDA_CORES computes the same with
  * the int64 CUDA-core Gram for every group.
  * Runs the filter/transpose itself. */
 #define XPCS_TWOTIME_EXACT_CUDA_CORES 2
@@ -355,9 +363,11 @@ typedef struct {
   int32_t window;
   int32_t partials;         /* (F - window) / window */
   int32_t sg_rows, sg_cols;
-  float gram_ms;            /* EXACT mode: device time of the tensor-core Gram kernels */
-  double gram_flop;         /* EXACT mode: their multiply-add work, 2 x M x N x K per tile */
-  double gram_flop_algorithmic; /* EXACT mode: the upper triangle's own work,
+  /* of the tensor-core Gram kernels (EXACT mode); all three 0 where none ran:
+   * event lists, the int64 Gram, REFERENCE mode */
+  float gram_ms;            /* device time */
+  double gram_flop;         /* multiply-add work, 2 x M x N x K per tile */
+  double gram_flop_algorithmic; /* the upper triangle's own work,
                                    2 x rows x F (F + 1) / 2 per smoothing group */
 } xpcs_twotime_info;
 int xpcs_twotime(xpcs_series *s, const xpcs_twotime_desc *d, int32_t mode,

@@ -1427,8 +1427,9 @@ k_mt_fwarp(const uint8_t *__restrict__ plan_g, const int32_t *__restrict__ flist
 // rows take the kernels of a series, the others the replay (noalloc.cu).
 // status[1] collects the kinds of rows seen, so that a kernel without rows
 // returns at once; status[2 ..] are the kernels' pixel counters.
-// Measured (256 x 250 pixels, 3,000 frames, 2.8 M events): the call 4,700 us
-// with one thread replaying each row from global memory, 574 us now.
+// Measured (256 x 250 pixels, 3,000 frames, 2.8 M events): the call 4,530 us
+// with one thread replaying each row from global memory, 300 us now, 202 of them
+// in k_na_thread: 2,000 warps, less than one wave, 33 % issue.
 constexpr int NA_GRAB = 4;  // pixels a warp takes at a time
 
 // Row p: its first event and length; false (and the status bit) when it lies
@@ -1604,8 +1605,9 @@ __global__ void __launch_bounds__(FW_WARPS * 32, 7) k_na_fwarp(NaRows v, int32_t
 // earlier entry, which is also the order of the later one).  The IF sums
 // start at their first entry; the IP sums are one running sum, read off where
 // it passes each delay's threshold.
-// Bound by instruction issue (about 94 k warp instructions for 32 rows of 154
-// events, 60 % issue) and, where the slots outgrow the L2, by their traffic.
+// Bound by instruction issue (95 k warp instructions for 32 rows of 154 events,
+// 56 % issue) and, where the slots outgrow the L2, by their traffic (27 % of DRAM
+// throughput there).
 // Measured against the warp-per-row kernel, which spends about 430 warp
 // instructions on 32 entries of one row (float rows as a whole, ms):
 //   dense  960^2 x 2,000 frames, 154 events a row   11.15 -> 4.53

@@ -250,7 +250,7 @@ struct TwoTimeOut {
   std::vector<int32_t> qbins;  // processed q bins present in the mapping, in mapping order
   int32_t frames = 0, window = 1, partials = 0, sg_rows = 0, sg_cols = 0;
   bool averaged = false;    // sg is the frames' mean (sg_cols 1; a one-frame series has 1 as well)
-  float gram_ms = 0.f;      // EXACT: tensor-core Gram kernel time
+  float gram_ms = 0.f;      // EXACT: tensor-core Gram kernel time (0 from event lists)
   double gram_flop = 0.0;      // multiply-adds of the tiles computed (2 x M x N x K each)
   double gram_flop_alg = 0.0;  // of the upper triangle alone (2 x rows x F(F+1)/2)
 };
