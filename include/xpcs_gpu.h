@@ -340,7 +340,8 @@ int xpcs_multitau2_noalloc(const int64_t *row_ptr, const int32_t *frame, const f
  * (twotimeFrameThreading).
  * mode EXACT: needs integer counts; the Gram products of the raw counts of
  * every smoothing group are exact integers: for sparse counts (fewer events
- * per pixel and frame than min(0.06, 65 / frames)) int32 sums over event lists
+ * per pixel and frame than min(0.06, 65 / frames), on the detector and in the
+ * processed q bins) int32 sums over event lists
  * (exact while sum over a group's pixels of (max count)^2 < 2^31), else on the
  * tensor cores (fp16 operands, fp32 accumulation: exact while the counts are
  * <= 2048 and that sum is < 2^24; other groups use an int64 CUDA-core Gram).

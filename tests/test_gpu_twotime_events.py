@@ -2,6 +2,8 @@
 against the oracle: one frame, frame counts around the warp, the tile and the
 columns per block, rows and columns of more than 32 events, and densities on
 both sides of the rule that chooses between the two."""
+import time
+
 import numpy as np
 import pytest
 
@@ -101,3 +103,64 @@ def test_exact_twotime_of_more_smoothing_groups_than_a_grid_has_rows(average):
     assert np.allclose(r["c2t"][1], want, rtol=2.0 ** -23, atol=0)
     assert np.array_equal(r["sg"], v.mean(0).astype(np.float32)[:, None] if average
                           else v.T.astype(np.float32))
+
+
+def _bright_ring(W, H, F, ring, density, seed=0):
+    """A q bin of `ring` pixels hit in `density` of the frames on a detector that
+    is dark elsewhere."""
+    rng = np.random.default_rng(seed)
+    P = W * H
+    dq = np.full(P, 2, np.int32)
+    dq[rng.choice(P - 2, ring, replace=False) + 1] = 1
+    hit = rng.random((F, P)) < np.where(dq == 1, density, 0.002)
+    nnz, idx = hit.sum(1).astype(np.uint32), np.nonzero(hit)[1].astype(np.int32)
+    return dq.reshape(H, W), nnz, idx, rng.integers(1, 5, idx.size).astype(np.int16)
+
+
+def test_a_bright_ring_alone_takes_the_dense_forms():
+    """The lists' work is in pairs of events of the processed rows, whatever the
+    rest of the detector holds: EXACT mode runs the tensor-core Gram (it reports
+    its time), with the int64 Gram's bits, and REFERENCE mode the tiled Gram: it
+    takes about as long as with the same rows dense enough by themselves."""
+    W, H, F, ring = 200, 180, 700, 1500
+    dq, nnz, idx, val = _bright_ring(W, H, F, ring, 0.9)
+    keep = dq.ravel()[idx] == 1
+    alone = (np.bincount(np.repeat(np.arange(F), nnz)[keep], minlength=F).astype(np.uint32),
+             idx[keep], val[keep])
+    only = np.where(dq == 1, 1, 0).astype(np.int32)
+    out = {}
+    for name, m, frames in (("all", dq, (nnz, idx, val)), ("only", only, alone)):
+        with xg.Series(W, H, F, 4, m, m) as s:
+            s.ingest_sparse(*frames)
+            for mode in (xg.MODE_REFERENCE, xg.MODE_EXACT, xg.TWOTIME_EXACT_CUDA_CORES):
+                ms = []
+                for _ in range(4):
+                    t = time.perf_counter()
+                    r = s.twotime([1], window=3, mode=mode)
+                    ms.append(time.perf_counter() - t)
+                out[name, mode] = r, min(ms)
+    for mode in (xg.MODE_REFERENCE, xg.MODE_EXACT, xg.TWOTIME_EXACT_CUDA_CORES):
+        a, o = out["all", mode], out["only", mode]
+        assert same_bits_nan(a[0]["c2t"][1], o[0]["c2t"][1])
+        if mode == xg.MODE_REFERENCE:
+            assert a[1] < 2 * o[1] + 1e-3, (a[1], o[1])
+    assert out["all", xg.MODE_EXACT][0]["gram_ms"] > 0
+    assert same_bits_nan(out["all", xg.MODE_EXACT][0]["c2t"][1],
+                         out["all", xg.TWOTIME_EXACT_CUDA_CORES][0]["c2t"][1])
+
+
+@pytest.mark.parametrize("threading", [False, True])
+def test_a_bright_ring_in_the_reference_order_vs_oracle(threading):
+    W, H, F = 40, 36, 90
+    dq, nnz, idx, val = _bright_ring(W, H, F, 60, 0.95, seed=2)
+    with xg.Series(W, H, F, 4, dq, dq) as s:
+        s.ingest_sparse(nnz, idx, val)
+        for qs in ([1], [2], [1, 2]):
+            r = s.twotime(qs, static_map=True, window=3, frame_threading=threading)
+            qm = oracle.QMap(dq, dq)
+            rows, _ = oracle.sparse_filter(qm, nnz, idx, val, F)
+            o = oracle.twotime(qm, rows, F, qs, True, False, 3, sort_pixels=threading)
+            for q in qs:
+                assert same_bits_nan(r["c2t"][q], o["c2t"][q])
+            for k in ("sg", "g2full", "g2partials"):
+                assert same_bits_nan(r[k], o[k]), k

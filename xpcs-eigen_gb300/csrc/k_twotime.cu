@@ -22,6 +22,7 @@
 //   - g2full[ff] = the float mean of diagonal ff in order; g2partials[ff][w]
 //     the float sum of window w (`window` entries) of diagonal ff / window.
 #include <algorithm>
+#include <cmath>
 #include <numeric>
 #include <utility>
 
@@ -155,12 +156,25 @@ __global__ void k_tt_groups(int32_t R, int32_t G, const int32_t *__restrict__ gr
 // sorted by (q, frame), stably from row order, which gives every column's
 // rows in the order its sums take them.
 
-// Events of row order[j] (order null: row j) in build order.
-__global__ void k_tt_lens(int32_t R, const int32_t *__restrict__ order,
-                          const int32_t *__restrict__ row_pix,
-                          const int32_t *__restrict__ row_len, int32_t *__restrict__ len) {
+// Events of row order[j] (order null: row j) in build order, and the rows' ordered
+// pairs of events, sum n (n - 1).
+__global__ void __launch_bounds__(256)
+k_tt_lens(int32_t R, const int32_t *__restrict__ order, const int32_t *__restrict__ row_pix,
+          const int32_t *__restrict__ row_len, int32_t *__restrict__ len,
+          unsigned long long *__restrict__ pairs) {
+  __shared__ unsigned long long s_pairs[8];
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j < R) len[j] = row_len[row_pix[order ? order[j] : j]];
+  const int n = j < R ? row_len[row_pix[order ? order[j] : j]] : 0;
+  if (j < R) len[j] = n;
+  unsigned long long x = (unsigned long long)n * (unsigned)max(n - 1, 0);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  if ((threadIdx.x & 31) == 0) s_pairs[threadIdx.x >> 5] = x;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; w++) x += s_pairs[w];
+    if (x) atomicAdd(pairs, x);
+  }
 }
 
 // One warp per row in build order: (key = q F + frame, a = row, b = the
@@ -559,12 +573,20 @@ size_t lists_bytes(const Series &s, int32_t R, int32_t G, int32_t Q) {
   const size_t n = (size_t)std::max<int64_t>(s.raw_events, 1);
   return s.keyA.more(n) + s.keyB.more(n) + s.frA.more(n) + s.frB.more(n) + s.vA.more(n) +
          s.vB.more(n) + s.hist.more(radix_hist_words(n)) + s.tt_len.more(R) +
-         s.tt_cpos.more((size_t)R + 1) + s.tt_cols.more((size_t)Q * s.F + 1) +
+         s.tt_cpos.more((size_t)R + 2) + s.tt_cols.more((size_t)Q * s.F + 1) +
          s.tt_qptr.more(2 * (size_t)Q + G + 2) + s.scan_tmp.more(scan_workspace_bytes(R));
 }
 
-// Whether the rows are sparse enough for the event Gram, from the mean number
-// of events per pixel and frame, d.  Its work grows as d^2, the tiled Gram's
+// The density of rows with the given ordered pairs of events, as if every frame of
+// every row had it: what the lists' work, which is in pairs, goes by where some
+// of the processed rows are far brighter than the detector.
+double pair_density(int64_t pairs, int32_t R, int32_t F) {
+  return std::sqrt((double)pairs / R) / F;
+}
+
+// The density up to which the event Gram is taken, of the mapped pixels before its
+// lists are made and of the processed rows' pairs then (events per pixel and frame,
+// d).  Its work grows as d^2, the tiled Gram's
 // not at all, and short columns are cheap at any density.  Whole calls in ms,
 // event lists / tiled (random events, 3 q bins):
 //   pixels  frames   d = 0.05      0.1         0.2         0.4
@@ -575,13 +597,14 @@ size_t lists_bytes(const Series &s, int32_t R, int32_t G, int32_t Q) {
 //   64^2     4,096  1.58/5.60   3.10/5.75   9.03/6.09   32.0/7.0
 // Under a memory limit the form that takes less more of it is chosen, so that
 // no call is refused for the lists.
+double tt_events_most(int32_t F) { return std::min(0.4, std::max(0.15, 40.0 / F)); }
 bool tt_use_events(Series &s, int32_t R, int32_t G, int32_t Q) {
   if (tt_columns(s.F, sizeof(float)) == 0) return false;
   if (dev_limited() && lists_bytes(s, R, G, Q) + s.tt_V.more(s.raw_events) >
                            s.tt_V.more((size_t)R * s.F))
     return false;
-  const double most = std::min(0.4, std::max(0.15, 40.0 / s.F));
-  return (double)s.raw_events <= most * (double)s.qmap.pix.size() * s.R_in * s.F;
+  return (double)s.raw_events <=
+         tt_events_most(s.F) * (double)s.qmap.pix.size() * s.R_in * s.F;
 }
 
 // Warps of 256-thread blocks for k units of one warp.
@@ -593,7 +616,8 @@ struct EventLists {
 };
 
 // Row counts for the lists, and the tables of q bins and groups; enqueues the
-// copy of the event count to *n (valid after a synchronisation).
+// copy of the rows' events and ordered pairs of events to n[0] and n[1] (valid
+// after a synchronisation).
 EventLists lists_prepare(Series &s, const TwoTimeLayout &lay, int32_t R, int32_t G, int32_t Q,
                          const int32_t *order, int64_t *n) {
   cudaStream_t st = s.stream;
@@ -607,13 +631,15 @@ EventLists lists_prepare(Series &s, const TwoTimeLayout &lay, int32_t R, int32_t
   s.tt_qptr.reserve(tab.size(), st);
   XG_CUDA(cudaMemcpyAsync(s.tt_qptr.p, tab.data(), 4 * tab.size(), cudaMemcpyHostToDevice, st));
   s.tt_len.reserve(R, st);
-  s.tt_cpos.reserve((size_t)R + 1, st);
+  s.tt_cpos.reserve((size_t)R + 2, st);
   s.tt_cols.reserve((size_t)Q * s.F + 1, st);
   s.scan_tmp.reserve(scan_workspace_bytes(R), st);
-  k_tt_lens<<<(R + 255) / 256, 256, 0, st>>>(R, order, s.tt_row_pix.p, s.row_len.p, s.tt_len.p);
+  XG_CUDA(cudaMemsetAsync(s.tt_cpos.p + R + 1, 0, sizeof(int64_t), st));
+  k_tt_lens<<<(R + 255) / 256, 256, 0, st>>>(R, order, s.tt_row_pix.p, s.row_len.p, s.tt_len.p,
+                                             (unsigned long long *)s.tt_cpos.p + R + 1);
   XG_CHECK_LAUNCH();
   exclusive_scan_i32_i64(s.tt_len.p, s.tt_cpos.p, R, s.scan_tmp.p, st);
-  if (n) XG_CUDA(cudaMemcpyAsync(n, s.tt_cpos.p + R, sizeof(*n), cudaMemcpyDeviceToHost, st));
+  if (n) XG_CUDA(cudaMemcpyAsync(n, s.tt_cpos.p + R, 2 * sizeof(*n), cudaMemcpyDeviceToHost, st));
   const int32_t *q_ptr = s.tt_qptr.p;
   return {q_ptr, q_ptr + Q + 1, q_ptr + Q + 1 + G, 0};
 }
@@ -646,15 +672,16 @@ std::pair<const int32_t *, const float *> lists_build(Series &s, const EventList
   return {in_b ? s.frB.p : s.frA.p, in_b ? s.vB.p : s.vA.p};
 }
 
-// C, sg and sga from event lists.
-void gram_events(Series &s, const TwoTimeReq &req, const TwoTimeLayout &lay, int32_t R, int32_t G,
+// C, sg and sga from event lists; false when the processed rows are too dense.
+bool gram_events(Series &s, const TwoTimeReq &req, const TwoTimeLayout &lay, int32_t R, int32_t G,
                  int32_t Q) {
   cudaStream_t st = s.stream;
   const int32_t F = s.F;
-  int64_t n = 0;
-  EventLists l = lists_prepare(s, lay, R, G, Q, nullptr, &n);
+  int64_t n[2] = {0, 0};
+  EventLists l = lists_prepare(s, lay, R, G, Q, nullptr, n);
   XG_CUDA(cudaStreamSynchronize(st));
-  l.n = n;
+  if (pair_density(n[1], R, F) > tt_events_most(F)) return false;
+  l.n = n[0];
   auto ab = lists_build(s, l, R, Q, nullptr);  // mapping order
   k_tt_sg_events<<<dim3(tt_warps(F), G), 256, 0, st>>>(F, s.tt_grp_ptr.p, l.grp_q, s.tt_cols.p,
                                                        ab.first, ab.second, s.tt_row_pix.p,
@@ -681,11 +708,12 @@ void gram_events(Series &s, const TwoTimeReq &req, const TwoTimeLayout &lay, int
       F, l.q_ptr, s.tt_cols.p, ab.first, ab.second, s.tt_row_pix.p, s.row_ptr.p, s.ev_frame.p,
       s.tt_V.p, s.tt_C.p);
   XG_CHECK_LAUNCH();
+  return true;
 }
 
 // EXACT mode from the counts' event lists; false when the series takes the
-// other forms: rows too dense for the lists, or counts too large for int32
-// sums.  The lists' work grows with the square of the events per pixel and
+// other forms: pixels, or the processed rows by their pairs of events, too dense
+// for the lists, or counts too large for int32 sums.  The lists' work grows with the square of the events per pixel and
 // frame, d, and the tensor-core Gram's hardly at all; longer columns leave the
 // lists fewer warps per SM.  Whole calls in ms, lists / tensor cores:
 //   pixels  frames  q bins   d = 0.01       0.02        0.03        0.05
@@ -717,7 +745,7 @@ bool gram_counts(Series &s, const TwoTimeReq &req, const TwoTimeLayout &lay, int
         twotime_exact_bytes(s, lay))
       return false;
   }
-  int64_t n = 0;
+  int64_t n[2] = {0, 0};
   int32_t flags = 0;
   std::vector<unsigned long long> bound(G);
   s.tt_bound.reserve(std::max(G, 2), st);
@@ -727,13 +755,14 @@ bool gram_counts(Series &s, const TwoTimeReq &req, const TwoTimeLayout &lay, int
   k_tt_check<<<tt_warps(R), 256, 0, st>>>(R, s.tt_row_pix.p, s.tt_row_grp.p, s.row_ptr.p,
                                           s.row_len.p, s.ev_val.p, s.tt_bound.p, s.tt_flags.p);
   XG_CHECK_LAUNCH();
-  EventLists l = lists_prepare(s, lay, R, G, Q, nullptr, &n);
+  EventLists l = lists_prepare(s, lay, R, G, Q, nullptr, n);
   XG_CUDA(cudaMemcpyAsync(bound.data(), s.tt_bound.p, sizeof(unsigned long long) * G,
                           cudaMemcpyDeviceToHost, st));
   XG_CUDA(cudaMemcpyAsync(&flags, s.tt_flags.p, sizeof(flags), cudaMemcpyDeviceToHost, st));
   XG_CUDA(cudaStreamSynchronize(st));
-  l.n = n;
+  l.n = n[0];
   if (flags & 1) tt_not_counts();
+  if (pair_density(n[1], R, F) > most) return false;
   for (unsigned long long b : bound)
     if (b >= (1ull << 31)) return false;
   const auto ab = lists_build(s, l, R, Q, nullptr);
@@ -865,24 +894,26 @@ void run_twotime(Series &s, const TwoTimeReq &req, int mode, bool force_i64) {
     o.ready = true;
     return;
   }
-  const bool events = R > 0 && F > 0 && tt_use_events(s, R, G, Q);
-  // Gram order of every q bin's rows (event lists take the mapping order as it is)
-  std::vector<int32_t> order(req.frame_threading || !events ? R : 0);
-  std::iota(order.begin(), order.end(), 0);
-  if (req.frame_threading) {
-    std::vector<int32_t> row_pix;
-    for (const auto &r : runs)
-      row_pix.insert(row_pix.end(), qm.pix.begin() + r.first, qm.pix.begin() + r.second);
-    for (int32_t q = 0; q < Q; q++)
-      std::sort(order.begin() + q_ptr[q], order.begin() + q_ptr[q + 1],
-                [&](int32_t a, int32_t b) { return row_pix[a] < row_pix[b]; });
-  }
-  if (!order.empty()) up(s.tt_order, order);
+  // Gram order of every q bin's rows
+  const auto upload_order = [&] {
+    std::vector<int32_t> order(R);
+    std::iota(order.begin(), order.end(), 0);
+    if (req.frame_threading) {
+      std::vector<int32_t> row_pix;
+      for (const auto &r : runs)
+        row_pix.insert(row_pix.end(), qm.pix.begin() + r.first, qm.pix.begin() + r.second);
+      for (int32_t q = 0; q < Q; q++)
+        std::sort(order.begin() + q_ptr[q], order.begin() + q_ptr[q + 1],
+                  [&](int32_t a, int32_t b) { return row_pix[a] < row_pix[b]; });
+    }
+    up(s.tt_order, order);
+  };
   if (R > 0 && F > 0) {
-    if (events)
-      gram_events(s, req, lay, R, G, Q);
-    else
+    if (req.frame_threading) upload_order();  // event lists take the mapping order as it is
+    if (!tt_use_events(s, R, G, Q) || !gram_events(s, req, lay, R, G, Q)) {
+      if (!req.frame_threading) upload_order();
       gram_dense(s, req, lay, R, G, Q);
+    }
     k_tt_diag<<<dim3((F + 127) / 128, Q), 128, 0, st>>>(Q, F, req.window, o.partials, s.tt_C.p,
                                                        s.tt_full.p, s.tt_part.p);
     XG_CHECK_LAUNCH();
