@@ -205,3 +205,31 @@ def test_blocks_joined_within_what_a_limit_left_them_before():
                 assert same_bits(g, w)
     finally:
         xg.set_device_memory_limit(0, 0)
+
+
+def test_counts_too_large_for_the_lists_within_what_the_int64_gram_takes():
+    """EXACT two-time that first looks at the counts' lists and then takes the
+    int64 Gram needs no more than asking for that Gram does."""
+    side, F = 300, 100
+    rng = np.random.default_rng(4)
+    P = side * side
+    sq = (np.arange(P) * 2 // P + 1).astype(np.int32).reshape(side, side)
+    hit = rng.random((F, P)) < 0.02
+    nnz, idx = hit.sum(1).astype(np.uint32), np.nonzero(hit)[1].astype(np.int32)
+    val = rng.integers(1, 30000, idx.size).astype(np.int16)
+    try:
+        out, need = [], 0
+        for mode in (xg.TWOTIME_EXACT_CUDA_CORES, xg.MODE_EXACT):
+            with xg.Series(side, side, F, 2, sq, sq) as s:
+                s.ingest_sparse(nnz, idx, val)
+                s.multitau()
+                s.synchronize()
+                used = xg.device_memory(0)[0]
+                xg.set_device_memory_limit(0, used + (need + 4096 if need else 1 << 34))
+                out.append(s.twotime([1, 2], window=2, mode=mode))
+                need = xg.device_memory(0)[0] - used
+                xg.set_device_memory_limit(0, 0)
+        for q in (1, 2):
+            assert same_bits(out[0]["c2t"][q], out[1]["c2t"][q])
+    finally:
+        xg.set_device_memory_limit(0, 0)

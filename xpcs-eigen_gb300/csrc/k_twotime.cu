@@ -644,6 +644,17 @@ EventLists lists_prepare(Series &s, const TwoTimeLayout &lay, int32_t R, int32_t
   return {q_ptr, q_ptr + Q + 1, q_ptr + Q + 1 + G, 0};
 }
 
+// The lists are not taken after all: under a memory limit their tables give way to
+// the other form's buffers.
+bool lists_refused(Series &s) {
+  if (dev_limited()) {
+    s.tt_len.release(s.stream);
+    s.tt_cpos.release(s.stream);
+    s.tt_cols.release(s.stream);
+  }
+  return false;
+}
+
 // Sorts the rows' events by (q, frame) from the given row order (null: mapping
 // order); the sorted (row, position) pairs, and the columns' first events in
 // tt_cols.
@@ -680,7 +691,7 @@ bool gram_events(Series &s, const TwoTimeReq &req, const TwoTimeLayout &lay, int
   int64_t n[2] = {0, 0};
   EventLists l = lists_prepare(s, lay, R, G, Q, nullptr, n);
   XG_CUDA(cudaStreamSynchronize(st));
-  if (pair_density(n[1], R, F) > tt_events_most(F)) return false;
+  if (pair_density(n[1], R, F) > tt_events_most(F)) return lists_refused(s);
   l.n = n[0];
   auto ab = lists_build(s, l, R, Q, nullptr);  // mapping order
   k_tt_sg_events<<<dim3(tt_warps(F), G), 256, 0, st>>>(F, s.tt_grp_ptr.p, l.grp_q, s.tt_cols.p,
@@ -762,9 +773,9 @@ bool gram_counts(Series &s, const TwoTimeReq &req, const TwoTimeLayout &lay, int
   XG_CUDA(cudaStreamSynchronize(st));
   l.n = n[0];
   if (flags & 1) tt_not_counts();
-  if (pair_density(n[1], R, F) > most) return false;
+  if (pair_density(n[1], R, F) > most) return lists_refused(s);
   for (unsigned long long b : bound)
-    if (b >= (1ull << 31)) return false;
+    if (b >= (1ull << 31)) return lists_refused(s);
   const auto ab = lists_build(s, l, R, Q, nullptr);
   s.tt_sgd.reserve(2 * (size_t)G * F, st);
   double *sgd = s.tt_sgd.p, *isg = sgd + (size_t)G * F;
